@@ -2,81 +2,255 @@
 // fused multiply-adds, float32 out.  No tensor cores and no reduced-precision mode.
 //
 // Every output element is accumulated over k = 0 .. K-1 in that order by one thread, so its
-// value does not depend on M, on the tile it falls in, or on what else is in the batch.
+// value does not depend on M, on the kernel or the tile it falls in, or on what else is in the batch.
 // The reference has no 32-bit path (rapid_llm/models/config.py:134-146 downgrades float32
 // checkpoints); its products go through a library call (rapid_llm/kernels/ops/gemm/linear.py:17-40).
+#include <atomic>
+
 #include "common.cuh"
 
 namespace rl {
 
-constexpr int kTileM = 64, kTileN = 64, kTileK = 16;
+__device__ __forceinline__ void f32_copy16(float* shared, const float* global, bool ok) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(shared))),
+               "l"(global), "r"(ok ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void f32_copy4(float* shared, const float* global, bool ok) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(shared))),
+               "l"(global), "r"(ok ? 4 : 0) : "memory");
+}
 
-template <bool kAligned>
-__global__ void __launch_bounds__(256)
+// ------------------------------------------------------------------ tiles
+// What bounds them: shared memory hands a multiprocessor 128 bytes a cycle, broadcasts included, and a thread's kTm x kTn
+// outputs take (kTm + kTn) * 4 bytes a column for kTm * kTn multiply-adds, so tiles of few outputs a thread starve the FMA
+// pipe and tiles of many leave multiprocessors without a tile.  203 rows (us, before / now; K = 4,096): N = 6,144
+// 477 / 353, N = 4,096 347 / 256, N = 24,576 1,627 / 1,087 (37 TFLOP/s); N = 4,096 with K = 12,288 1,021 / 749.  Before:
+// 64 x 64 tiles, 4 x 4 outputs a thread, one buffer.  Tried and slower there: 8 x 8 and 8 x 16 outputs a thread
+// on 128 x 128 tiles (393 at N = 4,096; ahead only from 512 rows on, 1,410 against 1,611 us at 2,048), operands
+// transposed on their way into shared memory, and packed pairs of multiply-adds (the packing costs what they save).
+constexpr int kF32TileK = 32, kF32Stages = 3;
+constexpr int kF32Stride = kF32TileK + 4;      // floats between two rows in shared memory: eight neighbouring rows meet in no bank
+
+template <int kTx, int kTy, int kTm, int kTn>
+constexpr int f32_stage_floats() { return (kTy * kTm + kTx * kTn) * kF32Stride; }
+
+// kTx x kTy threads with kTm x kTn outputs each.  Both operands lie in shared memory as they lie in memory, rows of 32
+// columns, brought by asynchronous copies two steps ahead; a thread takes four columns of a row in one 16-byte fetch.
+template <int kTx, int kTy, int kTm, int kTn, bool kAligned>
+__global__ void __launch_bounds__(kTx * kTy)
 gemm_f32_kernel(const float* __restrict__ a, const float* __restrict__ w,
                 const float* __restrict__ bias, float* __restrict__ c, int m, int n, int k,
                 int lda, int ldc) {
-  __shared__ float a_tile[kTileK][kTileM + 4];
-  __shared__ float w_tile[kTileK][kTileN + 4];
+  constexpr int kThreads = kTx * kTy, kTileM = kTy * kTm, kTileN = kTx * kTn;
+  extern __shared__ __align__(16) float f32_ring[];
   const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;          // 16 x 16 threads, 4 x 4 outputs each
+  const int tx = tid % kTx, ty = tid / kTx;
   const int m0 = blockIdx.y * kTileM, n0 = blockIdx.x * kTileN;
-  const int load_row = tid >> 2, load_k = (tid & 3) * 4;
+  const int steps = (k + kF32TileK - 1) / kF32TileK;
 
-  float acc[4][4];
+  auto fill = [&](int step) {
+    float* sa = f32_ring + (step % kF32Stages) * f32_stage_floats<kTx, kTy, kTm, kTn>();
+    const int k0 = step * kF32TileK;
+    constexpr int kPiece = kAligned ? 4 : 1, kPieces = kF32TileK / kPiece;
+    static_assert((kTileM + kTileN) * kPieces % kThreads == 0, "every thread copies as many pieces");
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
-
-  for (int k0 = 0; k0 < k; k0 += kTileK) {
-    float av[4] = {0.f, 0.f, 0.f, 0.f}, wv[4] = {0.f, 0.f, 0.f, 0.f};
-    const int am = m0 + load_row, wn = n0 + load_row, kk = k0 + load_k;
-    if (kAligned) {
-      if (am < m && kk < k) {
-        const float4 v = *reinterpret_cast<const float4*>(a + static_cast<size_t>(am) * lda + kk);
-        av[0] = v.x; av[1] = v.y; av[2] = v.z; av[3] = v.w;
-      }
-      if (wn < n && kk < k) {
-        const float4 v = *reinterpret_cast<const float4*>(w + static_cast<size_t>(wn) * k + kk);
-        wv[0] = v.x; wv[1] = v.y; wv[2] = v.z; wv[3] = v.w;
-      }
-    } else {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        if (am < m && kk + e < k) av[e] = a[static_cast<size_t>(am) * lda + kk + e];
-        if (wn < n && kk + e < k) wv[e] = w[static_cast<size_t>(wn) * k + kk + e];
-      }
+    for (int at = 0; at < (kTileM + kTileN) * kPieces; at += kThreads) {
+      const int idx = at + tid, r = idx / kPieces, col = (idx % kPieces) * kPiece;
+      const bool is_a = r < kTileM;
+      const int row = is_a ? m0 + r : n0 + r - kTileM;
+      const bool ok = row < (is_a ? m : n) && k0 + col < k;
+      const float* from = is_a ? a + static_cast<size_t>(row) * lda : w + static_cast<size_t>(row) * k;
+      from = ok ? from + k0 + col : w;
+      if constexpr (kAligned) f32_copy16(sa + r * kF32Stride + col, from, ok);
+      else f32_copy4(sa + r * kF32Stride + col, from, ok);
     }
+  };
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      a_tile[load_k + e][load_row] = av[e];
-      w_tile[load_k + e][load_row] = wv[e];
+  for (int s = 0; s < kF32Stages - 1; ++s) {
+    if (s < steps) fill(s);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  float acc[kTm][kTn];
+#pragma unroll
+  for (int i = 0; i < kTm; ++i)
+#pragma unroll
+    for (int j = 0; j < kTn; ++j) acc[i][j] = 0.0f;
+  for (int step = 0; step < steps; ++step) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kF32Stages - 2) : "memory");
+    __syncthreads();      // the step has landed for every thread, and the stage refilled below has been read
+    if (step + kF32Stages - 1 < steps) fill(step + kF32Stages - 1);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const float* sa = f32_ring + (step % kF32Stages) * f32_stage_floats<kTx, kTy, kTm, kTn>() + ty * kF32Stride;
+    const float* sw = f32_ring + (step % kF32Stages) * f32_stage_floats<kTx, kTy, kTm, kTn>() + (kTileM + tx) * kF32Stride;
+#pragma unroll 1      // unrolled further it runs out of registers and slows down
+    for (int kk = 0; kk < kF32TileK; kk += 4) {
+      float4 ar[kTm], wr[kTn];
+#pragma unroll
+      for (int i = 0; i < kTm; ++i) ar[i] = *reinterpret_cast<const float4*>(sa + i * kTy * kF32Stride + kk);
+#pragma unroll
+      for (int j = 0; j < kTn; ++j) wr[j] = *reinterpret_cast<const float4*>(sw + j * kTx * kF32Stride + kk);
+#pragma unroll
+      for (int i = 0; i < kTm; ++i)
+#pragma unroll
+        for (int j = 0; j < kTn; ++j) acc[i][j] = fmaf(ar[i].x, wr[j].x, acc[i][j]);
+#pragma unroll
+      for (int i = 0; i < kTm; ++i)
+#pragma unroll
+        for (int j = 0; j < kTn; ++j) acc[i][j] = fmaf(ar[i].y, wr[j].y, acc[i][j]);
+#pragma unroll
+      for (int i = 0; i < kTm; ++i)
+#pragma unroll
+        for (int j = 0; j < kTn; ++j) acc[i][j] = fmaf(ar[i].z, wr[j].z, acc[i][j]);
+#pragma unroll
+      for (int i = 0; i < kTm; ++i)
+#pragma unroll
+        for (int j = 0; j < kTn; ++j) acc[i][j] = fmaf(ar[i].w, wr[j].w, acc[i][j]);
     }
-    __syncthreads();
-#pragma unroll
-    for (int kk2 = 0; kk2 < kTileK; ++kk2) {
-      const float4 a4 = *reinterpret_cast<const float4*>(&a_tile[kk2][ty * 4]);
-      const float4 w4 = *reinterpret_cast<const float4*>(&w_tile[kk2][tx * 4]);
-      const float ar[4] = {a4.x, a4.y, a4.z, a4.w};
-      const float wr[4] = {w4.x, w4.y, w4.z, w4.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(ar[i], wr[j], acc[i][j]);
-    }
-    __syncthreads();
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int row = m0 + ty * 4 + i;
+  for (int i = 0; i < kTm; ++i) {
+    const int row = m0 + ty + kTy * i;
     if (row >= m) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int col = n0 + tx * 4 + j;
+    for (int j = 0; j < kTn; ++j) {
+      const int col = n0 + tx + kTx * j;
       if (col < n) c[static_cast<size_t>(row) * ldc + col] = acc[i][j] + (bias ? bias[col] : 0.0f);
     }
   }
+}
+
+// ------------------------------------------------------------------ few rows
+// Up to kG * kPer rows of A (decoding, the head behind a step's prompts): bound by the weights' stream.  A block brings a
+// band of W's rows kBk columns at a time through a ring in shared memory; a lane owns kR weight rows, a warp kPer rows
+// of A, so an output's sum still runs down k in one thread.  kG of the four warps share the rows of A, the others take
+// bands of their own.  Fetches of A are broadcasts but cost shared memory as much as any other, so with many weight rows
+// (where blocks are plenty) a lane owns two of them.  Measured (us, 64 x 64 tiles before / now, K = 4,096): 1 row
+// 292 / 26 at N = 4,096, 501 / 80 at N = 24,576 (5.0 TB/s); 5 rows of the head, N = 151,936, 2,321 / 484 (5.1 TB/s);
+// 16 rows 292 / 60 and 505 / 176; 32 rows 293 / 78 and 505 / 212.
+constexpr int kFewThreads = 128;
+
+template <int kPer, int kG, int kR, int kBk, int kStages>
+struct Few {
+  static constexpr int kRows = 32 * kR * (4 / kG);
+  static constexpr int kStride = kBk + 4;
+  static constexpr int kStageFloats = kRows * kStride + kG * kPer * kBk;
+  static constexpr int kSmem = kStages * kStageFloats * 4;
+};
+
+template <int kPer, int kG, int kR, int kBk, int kStages>
+__global__ void __launch_bounds__(kFewThreads)
+gemm_f32_few_kernel(const float* __restrict__ a, const float* __restrict__ w, const float* __restrict__ bias,
+                    float* __restrict__ c, int m, int n, int k, int lda, int ldc) {
+  using F = Few<kPer, kG, kR, kBk, kStages>;
+  extern __shared__ __align__(16) float few_ring[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int group = warp % kG, band = warp / kG;
+  const int n0 = blockIdx.x * F::kRows;
+  const int steps = (k + kBk - 1) / kBk;
+  auto fill = [&](int step) {
+    float* sw = few_ring + (step % kStages) * F::kStageFloats;
+    float* sa = sw + F::kRows * F::kStride;
+    const int k0 = step * kBk;
+    constexpr int kPieces = kBk / 4;
+#pragma unroll
+    for (int i = 0; i < F::kRows * kPieces / kFewThreads; ++i) {
+      const int idx = tid + i * kFewThreads, r = idx / kPieces, col = (idx % kPieces) * 4;
+      const bool ok = n0 + r < n && k0 + col < k;
+      f32_copy16(sw + r * F::kStride + col, ok ? w + static_cast<size_t>(n0 + r) * k + k0 + col : w, ok);
+    }
+    for (int idx = tid; idx < kG * kPer * kPieces; idx += kFewThreads) {
+      const int r = idx / kPieces, col = (idx % kPieces) * 4;
+      const bool ok = r < m && k0 + col < k;
+      f32_copy16(sa + r * kBk + col, ok ? a + static_cast<size_t>(r) * lda + k0 + col : a, ok);
+    }
+  };
+#pragma unroll
+  for (int s = 0; s < kStages - 1; ++s) {
+    if (s < steps) fill(s);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  float acc[kR][kPer];
+#pragma unroll
+  for (int r = 0; r < kR; ++r)
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) acc[r][i] = 0.0f;
+  const bool works = group * kPer < m;      // a warp without rows of A only copies
+  for (int step = 0; step < steps; ++step) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+    __syncthreads();      // the step has landed for every thread, and the stage refilled below has been read
+    if (step + kStages - 1 < steps) fill(step + kStages - 1);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    if (!works) continue;
+    const float* sw = few_ring + (step % kStages) * F::kStageFloats;
+    const float* mine = sw + (band * 32 * kR + lane) * F::kStride;
+    const float* sa = sw + F::kRows * F::kStride + group * kPer * kBk;
+#pragma unroll
+    for (int kk = 0; kk < kBk; kk += 4) {
+      float4 w4[kR];
+#pragma unroll
+      for (int r = 0; r < kR; ++r) w4[r] = *reinterpret_cast<const float4*>(mine + r * 32 * F::kStride + kk);
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) {
+        const float4 a4 = *reinterpret_cast<const float4*>(sa + i * kBk + kk);
+#pragma unroll
+        for (int r = 0; r < kR; ++r) {
+          acc[r][i] = fmaf(a4.x, w4[r].x, acc[r][i]);
+          acc[r][i] = fmaf(a4.y, w4[r].y, acc[r][i]);
+          acc[r][i] = fmaf(a4.z, w4[r].z, acc[r][i]);
+          acc[r][i] = fmaf(a4.w, w4[r].w, acc[r][i]);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < kR; ++r) {
+    const int col = n0 + (band * kR + r) * 32 + lane;
+    if (col >= n) continue;
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      const int row = group * kPer + i;
+      if (row < m) c[static_cast<size_t>(row) * ldc + col] = acc[r][i] + (bias ? bias[col] : 0.0f);
+    }
+  }
+}
+
+// More than 48 KB of shared memory has to be allowed once per kernel and device (a bit each in `done`).
+template <typename Kernel>
+static cudaError_t f32_allow_shared(Kernel kernel, int bytes, std::atomic<unsigned long long>& done) {
+  int device = 0;
+  const cudaError_t found = cudaGetDevice(&device);
+  if (found != cudaSuccess) return found;
+  const unsigned long long bit = 1ull << (device & 63);
+  if (device < 64 && (done.load(std::memory_order_acquire) & bit)) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess && device < 64) done.fetch_or(bit, std::memory_order_release);
+  return e;
+}
+
+template <int kTx, int kTy, int kTm, int kTn>
+static int launch_f32_tiles(bool aligned, const float* a, const float* w, const float* bias, float* c, int m, int n, int k,
+                            int lda, int ldc, cudaStream_t stream) {
+  const dim3 grid((n + kTx * kTn - 1) / (kTx * kTn), (m + kTy * kTm - 1) / (kTy * kTm));
+  if (grid.y > 65535) return static_cast<int>(cudaErrorInvalidValue);
+  constexpr int smem = kF32Stages * f32_stage_floats<kTx, kTy, kTm, kTn>() * static_cast<int>(sizeof(float));
+  auto kernel = aligned ? gemm_f32_kernel<kTx, kTy, kTm, kTn, true> : gemm_f32_kernel<kTx, kTy, kTm, kTn, false>;
+  static std::atomic<unsigned long long> configured[2];
+  const cudaError_t e = f32_allow_shared(kernel, smem, configured[aligned]);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  kernel<<<grid, kTx * kTy, smem, stream>>>(a, w, bias, c, m, n, k, lda, ldc);
+  return launch_status();
+}
+
+template <int kPer, int kG, int kR, int kBk, int kStages>
+static int launch_f32_few(const float* a, const float* w, const float* bias, float* c, int m, int n, int k, int lda, int ldc,
+                          cudaStream_t stream) {
+  using F = Few<kPer, kG, kR, kBk, kStages>;
+  auto kernel = gemm_f32_few_kernel<kPer, kG, kR, kBk, kStages>;
+  static std::atomic<unsigned long long> configured;
+  const cudaError_t e = f32_allow_shared(kernel, F::kSmem, configured);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  kernel<<<(n + F::kRows - 1) / F::kRows, kFewThreads, F::kSmem, stream>>>(a, w, bias, c, m, n, k, lda, ldc);
+  return launch_status();
 }
 
 }  // namespace rl
@@ -86,13 +260,26 @@ extern "C" int rl_gemm_f32(const float* a, const float* w, const float* bias, fl
                            int n, int k, int lda, int ldc, cudaStream_t stream) {
   if (m == 0 || n == 0) return 0;
   if (k <= 0 || lda < k || ldc < n) return static_cast<int>(cudaErrorInvalidValue);
-  const dim3 grid((n + rl::kTileN - 1) / rl::kTileN, (m + rl::kTileM - 1) / rl::kTileM);
   const bool aligned = (k % 4 == 0) && (lda % 4 == 0) &&
                        (reinterpret_cast<uintptr_t>(a) % 16 == 0) &&
                        (reinterpret_cast<uintptr_t>(w) % 16 == 0);
-  if (aligned)
-    rl::gemm_f32_kernel<true><<<grid, 256, 0, stream>>>(a, w, bias, c, m, n, k, lda, ldc);
-  else
-    rl::gemm_f32_kernel<false><<<grid, 256, 0, stream>>>(a, w, bias, c, m, n, k, lda, ldc);
-  return rl::launch_status();
+  if (aligned && m <= 32) {
+    // a lane with two weight rows halves the blocks: from 16,384 rows on there are enough of them.  One weight row against
+    // two, us at N = 4,096 and 24,576: 8 rows of A 35 and 150 against 125 and 132, 16 rows 60 and 215 against 107 and
+    // 176, 32 rows 78 and 340 against 96 and 212; up to 4 rows one is ahead at both (26 and 80 against 80 and 99)
+    const bool many = n >= 16384;
+    if (m <= 4) return rl::launch_f32_few<1, 4, 1, 64, 6>(a, w, bias, c, m, n, k, lda, ldc, stream);
+    if (m <= 8) return many ? rl::launch_f32_few<8, 1, 2, 32, 3>(a, w, bias, c, m, n, k, lda, ldc, stream)
+                            : rl::launch_f32_few<2, 4, 1, 64, 6>(a, w, bias, c, m, n, k, lda, ldc, stream);
+    if (m <= 16) return many ? rl::launch_f32_few<8, 2, 2, 32, 4>(a, w, bias, c, m, n, k, lda, ldc, stream)
+                             : rl::launch_f32_few<4, 4, 1, 64, 6>(a, w, bias, c, m, n, k, lda, ldc, stream);
+    return many ? rl::launch_f32_few<8, 4, 2, 64, 3>(a, w, bias, c, m, n, k, lda, ldc, stream)
+                : rl::launch_f32_few<8, 4, 1, 64, 6>(a, w, bias, c, m, n, k, lda, ldc, stream);
+  }
+  // 64 x 64 tiles (4 x 8 outputs a thread) or 112 x 64 (7 x 8): a round of tiles on all multiprocessors takes about 115 and
+  // 180 us at K = 4,096 (measured over 40 to 2,048 rows), so the rule compares the rounds
+  const long long wide = (n + 63) / 64, sms = 148;
+  const long long low = (((m + 63) / 64) * wide + sms - 1) / sms, high = (((m + 111) / 112) * wide + sms - 1) / sms;
+  if (180 * high < 115 * low) return rl::launch_f32_tiles<8, 16, 7, 8>(aligned, a, w, bias, c, m, n, k, lda, ldc, stream);
+  return rl::launch_f32_tiles<8, 16, 4, 8>(aligned, a, w, bias, c, m, n, k, lda, ldc, stream);
 }

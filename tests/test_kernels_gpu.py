@@ -100,6 +100,25 @@ def test_gemm_f32(m, n, k_):
     torch.testing.assert_close(out, want, rtol=1e-5, atol=1e-5 * math.sqrt(k_))
 
 
+@pytest.mark.parametrize("n,k_", [(70, 100), (300, 36), (16400, 68), (129, 35)])
+def test_gemm_f32_rows_are_the_same_in_every_kernel(n, k_):
+    """Every edge of the dispatch: 1 to 4, 8, 16, 32 rows, both tiles and their remainders, weights on both sides of 16,384
+    rows, columns that are no multiple of a step or of four; an output is one sum in the order of k wherever it is formed."""
+    torch.manual_seed(3)
+    rows = [1, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65, 112, 113, 240]
+    a, w, bias = torch.randn(max(rows), k_, device=DEV), torch.randn(n, k_, device=DEV), torch.randn(n, device=DEV)
+    want = (a.double() @ w.double().t() + bias.double()).cpu()
+    first = None
+    for m in rows:
+        wide = torch.full((m, n + 4), 7.0, device=DEV)
+        k().gemm_f32(a[:m], w, wide[:, :n], bias)
+        assert bool((wide[:, n:] == 7.0).all())
+        # k sums, each rounded to 2^-24 of a partial sum that stays below 2 k
+        assert float((wide[:, :n].double().cpu() - want[:m]).abs().max()) < 2.0 * k_ * k_ * 2.0 ** -24
+        first = wide[:1, :n].clone() if first is None else first
+        assert torch.equal(wide[:1, :n], first)
+
+
 def test_gemm_f32_rows_do_not_depend_on_the_batch():
     a = rand((70, 300), torch.float32, seed=6).to(DEV)
     w = rand((90, 300), torch.float32, seed=7).to(DEV)
