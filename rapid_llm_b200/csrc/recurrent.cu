@@ -539,12 +539,25 @@ __global__ void rotate_heads_kernel(const T* in, int in_stride, int q_col0, int 
 //   out = (S + diag(bonus) k v^T)^T q;   S <- decay * S + k v^T
 // Query/key head of head h is h / (heads / kv_heads).
 //
-// A block owns (entry, head, a tile of columns of S) and walks the entry's tokens in order.  A column
-// is shared by `partners` lanes of one warp, each holding kRows consecutive rows of it in registers;
-// sums over rows end in a fixed tree of shuffles, so a token's result depends on nothing but the
-// tokens before it.  q, k, row decays, v and the per-token numbers of a run of tokens are brought into
-// shared memory by asynchronous copies while the run before is walked.  In the slot's row a head's
-// state lies column by column (S^T, [vdim][dim]), so that a lane's rows are consecutive floats.
+// A block owns (entry, head, a tile of columns of S) and walks the entry's tokens in order.
+//
+// A column of S is shared by kPartners lanes of one warp, a lane holds kRows of its rows in registers (pieces of four,
+// kPartners pieces apart) for kCols neighbouring columns; sums over rows run down a lane's rows and then over lanes in a
+// fixed tree of exchanges (offsets from kPartners / 2 down), so a token's result depends on nothing but the tokens before
+// it: not on the step it came in, the group of tokens it was walked in, or kCols.  In the slot's row a head's state lies
+// column by column (S^T, [vdim][dim]).
+//
+// What bounds the walk: a token's k, q and row decays are wanted by every column, and shared memory hands a multiprocessor
+// 128 bytes a cycle, broadcasts included: with one column a lane the fetches took four times as long as the multiply-adds.
+// Then the instructions a token takes (about 90 a warp) with one warp a scheduler to issue them (0.3 a cycle): a walk from
+// end to end cannot use the rest of the GPU, so in 16-bit engines long prompts are walked in pieces (below).
+// A correction (beta) makes a token wait for the sum over the whole column of the token before it: there a column has
+// few lanes with many rows each, since an exchange between lanes waits as long as eight multiply-adds.
+// 2,048 tokens, us, before / from end to end / in pieces: 16 heads of 128, fixed decay 432 / 288 / 183; 32 heads of 64, row
+// decays 380 / 249 / 136; with a bonus 333 / 270 / 148; 32 heads of 128, fixed, 3 prompts 551 / 420 / 331; with a
+// correction, 16 heads of 128, 632 / 567 / 433.  64 single tokens: 64 heads of 64, row decays 54 / 31 (4.3 TB/s), 16 heads of
+// 128, fixed 53 / 31 (see the kernel).  Against 64 bits the error is what it was (1.1e-7; fixed decays 2.6e-7; with a correction
+// 1.4e-7 from end to end and 1.41e-7 in pieces of 256, 1.54e-7 in pieces of 128).
 struct ScanArgs {
   const float* q; int q_stride;
   const float* k; int k_stride;
@@ -558,12 +571,99 @@ struct ScanArgs {
   float* state; long long state_stride; int state_off;
   const int* cu_seqlens; const int* entry_slot; const int* entry_start;
   int heads, kv_heads, dim, vdim, slots;
-  int partners, run;
+  int run;
   int wide_in;      // q, k, v (and row decays) can be fetched 16 bytes at a time
   int* fault;
+  int entries;
+  int segment;            // 0: a block walks its entry from end to end; else at most so many tokens, from a state of its own
+  float* seg_states;      // [pieces, heads, vdim, dim]: what a piece alone leaves, then what it starts from
+  float* seg_decays;      // [pieces, heads, dim]: the product of a piece's decays
+  float* seg_mats;        // [pieces, heads, dim, dim]: with beta, what a piece makes of each unit column
 };
 
-constexpr int kScanThreads = 256;
+// The piece that block `index` owns: of which entry, which one of the entry's, its tokens, its place in the arrays of
+// pieces (entries of one piece have none: they start from the slot's state and leave it there); false behind the last.
+struct ScanPiece { int entry, number, first, length, of, place; };
+__device__ __forceinline__ bool scan_piece(const ScanArgs& a, int index, ScanPiece& s) {
+  if (a.segment == 0) {
+    s = {index, 0, a.cu_seqlens[index], a.cu_seqlens[index + 1] - a.cu_seqlens[index], 1, 0};
+    return true;
+  }
+  int at = 0, place = 0;
+  for (int e = 0; e < a.entries; ++e) {
+    const int first = a.cu_seqlens[e], length = a.cu_seqlens[e + 1] - first;
+    const int count = (length + a.segment - 1) / a.segment;
+    if (index < at + count) {
+      const int number = index - at, skipped = number * a.segment;
+      s = {e, number, first + skipped, min(a.segment, length - skipped), count, count > 1 ? place + number : 0};
+      return true;
+    }
+    at += count;
+    if (count > 1) place += count;
+  }
+  return false;
+}
+// The pieces of entry `e` and the place of its first.
+__device__ __forceinline__ int scan_pieces_of(const ScanArgs& a, int e, int& place) {
+  place = 0;
+  int count = 0;
+  for (int i = 0; i <= e; ++i) {
+    if (count > 1) place += count;
+    count = (a.cu_seqlens[i + 1] - a.cu_seqlens[i] + a.segment - 1) / a.segment;
+  }
+  return count;
+}
+
+constexpr int kScanThreads = 128, kScanWarps = kScanThreads / 32;
+constexpr int kScanPlain = 0, kScanDelta = 1, kScanBonus = 2;
+
+// Two neighbouring rows and their arithmetic, each half rounded by itself: packed into one instruction for the walks, plain
+// where what counts is the loads in flight (packed, the register pairs cost the single tokens' kernel 5 to 20 us of 35).
+struct PackedPair {
+  unsigned long long both;
+};
+struct PlainPair {
+  float x, y;
+};
+template <typename P>
+__device__ __forceinline__ P pair_of(float x, float y) {
+  if constexpr (std::is_same_v<P, PlainPair>) {
+    return {x, y};
+  } else {
+    PackedPair out;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(out.both) : "f"(x), "f"(y));
+    return out;
+  }
+}
+__device__ __forceinline__ float2 pair_halves(PlainPair a) { return make_float2(a.x, a.y); }
+__device__ __forceinline__ float2 pair_halves(PackedPair a) {
+  float2 out;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(out.x), "=f"(out.y) : "l"(a.both));
+  return out;
+}
+__device__ __forceinline__ PlainPair pair_fma(PlainPair a, PlainPair b, PlainPair c) { return {fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y)}; }
+__device__ __forceinline__ PlainPair pair_mul(PlainPair a, PlainPair b) { return {__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y)}; }
+__device__ __forceinline__ PlainPair pair_add(PlainPair a, PlainPair b) { return {__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y)}; }
+__device__ __forceinline__ PackedPair pair_fma(PackedPair a, PackedPair b, PackedPair c) {
+  PackedPair out;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(out.both) : "l"(a.both), "l"(b.both), "l"(c.both));
+  return out;
+}
+__device__ __forceinline__ PackedPair pair_mul(PackedPair a, PackedPair b) {
+  PackedPair out;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(out.both) : "l"(a.both), "l"(b.both));
+  return out;
+}
+__device__ __forceinline__ PackedPair pair_add(PackedPair a, PackedPair b) {
+  PackedPair out;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(out.both) : "l"(a.both), "l"(b.both));
+  return out;
+}
+template <typename P>
+__device__ __forceinline__ float pair_sum(P a) {
+  const float2 both = pair_halves(a);
+  return __fadd_rn(both.x, both.y);
+}
 
 __device__ __forceinline__ void copy_async4(float* shared, const float* global) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(shared))),
@@ -577,38 +677,215 @@ __device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.com
 template <int kPending>
 __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory"); }
 
-template <int kRows, int kPartners>
+// The numbers of one token that a lane works with.
+template <int kRows, int kCols, bool kRowDecay, typename P>
+struct ScanToken {
+  P k[kRows / 2], q[kRows / 2], g[kRowDecay ? kRows / 2 : 1];
+  float v[kCols];
+  float strength;
+};
+
+// A lane's share of S and what it does to it, one token at a time.
+template <int kRows, int kPartners, int kCols, int kKind, bool kRowDecay, bool kRead, typename P>
+struct ScanColumns {
+  P S[kCols][kRows / 2];
+  P bonus[kKind == kScanBonus ? kRows / 2 : 1];
+
+  __device__ __forceinline__ void take(const ScanToken<kRows, kCols, kRowDecay, P>& t, float decay, bool scaled, float (&o)[kCols]) {
+    const P d2 = pair_of<P>(decay, decay);
+    if constexpr (kKind == kScanDelta) {
+      float seen[kCols];
+#pragma unroll
+      for (int c = 0; c < kCols; ++c) {
+        P sum[2] = {pair_of<P>(0.0f, 0.0f), pair_of<P>(0.0f, 0.0f)};
+#pragma unroll
+        for (int r = 0; r < kRows / 2; ++r) {
+          S[c][r] = pair_mul(S[c][r], kRowDecay ? t.g[r] : d2);
+          sum[r & 1] = pair_fma(S[c][r], t.k[r], sum[r & 1]);
+        }
+        seen[c] = pair_sum(pair_add(sum[0], sum[1]));
+      }
+#pragma unroll
+      for (int off = kPartners / 2; off >= 1; off >>= 1) {
+#pragma unroll
+        for (int c = 0; c < kCols; ++c) seen[c] += __shfl_xor_sync(0xffffffffu, seen[c], off);
+      }
+#pragma unroll
+      for (int c = 0; c < kCols; ++c) {
+        const float u = t.strength * (t.v[c] - seen[c]);
+        const P u2 = pair_of<P>(u, u);
+        P sum[2] = {pair_of<P>(0.0f, 0.0f), pair_of<P>(0.0f, 0.0f)};
+#pragma unroll
+        for (int r = 0; r < kRows / 2; ++r) {
+          S[c][r] = pair_fma(t.k[r], u2, S[c][r]);
+          if constexpr (kRead) sum[r & 1] = pair_fma(S[c][r], t.q[r], sum[r & 1]);
+        }
+        if constexpr (kRead) o[c] = pair_sum(pair_add(sum[0], sum[1]));
+      }
+    } else {
+#pragma unroll
+      for (int c = 0; c < kCols; ++c) {
+        const float u = scaled ? t.strength * t.v[c] : t.v[c];
+        const P u2 = pair_of<P>(u, u);
+        P sum[2] = {pair_of<P>(0.0f, 0.0f), pair_of<P>(0.0f, 0.0f)};
+#pragma unroll
+        for (int r = 0; r < kRows / 2; ++r) {
+          const P kv = pair_mul(t.k[r], u2);
+          if constexpr (kKind == kScanBonus) {
+            // read the state as the tokens before left it, the token's own pair weighed by the bonus; then decay and add
+            sum[r & 1] = pair_fma(pair_fma(bonus[r], kv, S[c][r]), t.q[r], sum[r & 1]);
+            S[c][r] = pair_fma(S[c][r], kRowDecay ? t.g[r] : d2, kv);
+          } else {
+            S[c][r] = pair_fma(S[c][r], kRowDecay ? t.g[r] : d2, kv);
+            if constexpr (kRead) sum[r & 1] = pair_fma(S[c][r], t.q[r], sum[r & 1]);
+          }
+        }
+        if constexpr (kRead) o[c] = pair_sum(pair_add(sum[0], sum[1]));
+      }
+    }
+  }
+
+  // Column c of the lane's columns at `home`; `left` columns exist.
+  __device__ __forceinline__ void load(const float* home, int dim, int part, int left, bool wide) {
+#pragma unroll
+    for (int c = 0; c < kCols; ++c) {
+#pragma unroll
+      for (int j = 0; j < kRows / 4; ++j) {
+        const int row = (j * kPartners + part) * 4;
+        float x[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if (c < left) {
+          const float* p = home + static_cast<size_t>(c) * dim + row;
+          if (wide) {
+            if (row < dim) {
+              const float4 four = *reinterpret_cast<const float4*>(p);
+              x[0] = four.x; x[1] = four.y; x[2] = four.z; x[3] = four.w;
+            }
+          } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (row + e < dim) x[e] = p[e];
+          }
+        }
+        S[c][2 * j] = pair_of<P>(x[0], x[1]);
+        S[c][2 * j + 1] = pair_of<P>(x[2], x[3]);
+      }
+    }
+  }
+  // Column c becomes the unit vector of row `row0 + c`; columns before row 0 stay as they are.
+  __device__ __forceinline__ void units(int row0, int part) {
+#pragma unroll
+    for (int c = 0; c < kCols; ++c) {
+#pragma unroll
+      for (int r = 0; r < kRows / 2; ++r) {
+        const int row = ((r / 2) * kPartners + part) * 4 + (r & 1) * 2;
+        if (row0 + c >= 0) S[c][r] = pair_of<P>(row == row0 + c ? 1.0f : 0.0f, row + 1 == row0 + c ? 1.0f : 0.0f);
+      }
+    }
+  }
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int c = 0; c < kCols; ++c)
+#pragma unroll
+      for (int r = 0; r < kRows / 2; ++r) S[c][r] = pair_of<P>(0.0f, 0.0f);
+  }
+  __device__ __forceinline__ void store(float* home, int dim, int part, int left, bool wide) const {
+#pragma unroll
+    for (int c = 0; c < kCols; ++c) {
+      if (c >= left) break;
+#pragma unroll
+      for (int j = 0; j < kRows / 4; ++j) {
+        const int row = (j * kPartners + part) * 4;
+        float* p = home + static_cast<size_t>(c) * dim + row;
+        const float2 lower = pair_halves(S[c][2 * j]), upper = pair_halves(S[c][2 * j + 1]);
+        const float x[4] = {lower.x, lower.y, upper.x, upper.y};
+        if (wide) {
+          if (row < dim) *reinterpret_cast<float4*>(p) = make_float4(x[0], x[1], x[2], x[3]);
+        } else {
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (row + e < dim) p[e] = x[e];
+        }
+      }
+    }
+  }
+};
+
+// Sums kCount values over the kPartners lanes of a column, value i of every lane with value i of the others.  Where there
+// are more values than one, each exchange also halves the values a lane keeps: the result is values[0 .. kept - 1], which
+// are the sums of values `first` (returned) and up.  The tree is the same for any kCount.
+template <int kPartners, int kCount>
+__device__ __forceinline__ int scan_sums(float (&values)[kCount], int part) {
+  int first = 0;
+#pragma unroll
+  for (int off = kPartners / 2, count = kCount; off >= 1; off >>= 1) {
+    const bool upper = part & off;
+    if (count > 1) {
+      count >>= 1;
+#pragma unroll
+      for (int i = 0; i < kCount / 2; ++i) {
+        if (i < count) {
+          const float keep = upper ? values[i + count] : values[i], send = upper ? values[i] : values[i + count];
+          values[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+        }
+      }
+      first += upper ? count : 0;
+    } else {
+      values[0] += __shfl_xor_sync(0xffffffffu, values[0], off);
+    }
+  }
+  return first;
+}
+
+// Floats of shared memory a token takes.
+template <int kRows, int kPartners, int kCols, bool kRowDecay, bool kRead>
+__host__ __device__ constexpr int scan_token_floats() {
+  return ((kRowDecay ? 2 : 1) + (kRead ? 1 : 0)) * kPartners * kRows + kScanWarps * (32 / kPartners) * kCols + 2;
+}
+
+// Walks an entry's tokens; q, k, row decays, v and the per-token numbers of a run of tokens are brought into shared memory
+// by asynchronous copies while the run before is walked, and a token's numbers into registers while the one before is taken.
+// With `segment` a prompt's tokens are walked in pieces side by side: every piece from zeros without its read-outs
+// (kRead false; scan_join_kernel then makes each piece's true start out of them), and again from its true start.
+template <int kRows, int kPartners, int kCols, int kKind, bool kRowDecay, bool kRead>
 __global__ void __launch_bounds__(kScanThreads) linear_scan_kernel(const ScanArgs a) {
   extern __shared__ __align__(16) float staged[];
   // Its successor is let in only when the walk is over (below): a kernel that waits at its start still holds
   // warp slots, and the walk is bound by its own latencies, which more resident warps do not shorten.
-  const int e = blockIdx.x, head = blockIdx.y;
-  constexpr int partners = kPartners, cols_per_warp = 32 / kPartners;
+  const int head = blockIdx.y;
+  ScanPiece seg;
+  // the last piece of an entry is walked once: nothing starts from what it leaves
+  if (!scan_piece(a, blockIdx.x, seg) || (!kRead && seg.number == seg.of - 1)) {
+    pdl_wait();
+    return;
+  }
+  const int e = seg.entry;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int part = lane / cols_per_warp, col_in_warp = lane - part * cols_per_warp;
-  constexpr int tile_cols = (kScanThreads / 32) * cols_per_warp;
-  const int col_in_tile = warp * cols_per_warp + col_in_warp;
-  const int col = blockIdx.z * tile_cols + col_in_tile;
-  const bool col_ok = col < a.vdim;
-  const int row0 = part * kRows;
-  constexpr int dim_padded = partners * kRows;
+  const int part = lane % kPartners;
+  constexpr int kSpread = 32 / kPartners;      // groups of kCols columns a warp has
+  constexpr int kTile = kScanWarps * kSpread * kCols;
+  constexpr int kPadded = kPartners * kRows;
+  const int col_in_tile = (warp * kSpread + lane / kPartners) * kCols;
+  const int col = blockIdx.z * kTile + col_in_tile;
+  // columns of this lane that exist; with a correction a piece also takes the unit columns, which lie behind the values'
+  const int left = a.vdim + (!kRead && kKind == kScanDelta ? a.dim : 0) - col;
   const int kv_head = head / (a.heads / a.kv_heads);
 
-  const int first = a.cu_seqlens[e], length = a.cu_seqlens[e + 1] - first, start = a.entry_start[e];
+  const int first = seg.first, length = seg.length, start = a.entry_start[e];
   int slot = a.entry_slot[e];
   const bool slot_ok = slot >= 0 && slot < a.slots;
   if (!slot_ok) {
     if (threadIdx.x == 0) atomicOr(a.fault, kFaultSlot);
     slot = 0;
   }
-  float* home = a.state + slot * a.state_stride + a.state_off + static_cast<size_t>(head) * a.dim * a.vdim +
-                static_cast<size_t>(col_ok ? col : 0) * a.dim + row0;
-  const bool wide = (a.dim & 3) == 0 && (reinterpret_cast<uintptr_t>(home) & 15) == 0;   // kRows is a multiple of 4
+  const size_t in_head = static_cast<size_t>(left > 0 ? col : 0) * a.dim;
+  float* home = a.state + slot * a.state_stride + a.state_off + static_cast<size_t>(head) * a.dim * a.vdim + in_head;
+  const bool wide = (a.dim & 3) == 0 && (reinterpret_cast<uintptr_t>(home) & 15) == 0;
+  const size_t own = (static_cast<size_t>(seg.place) * a.heads + head) * a.dim;      // of this piece in the three arrays
 
-  // two buffers, each: k, q (and row decays) [run][dim_padded]; v [run][tile_cols]; write strength, decay [run]
+  // two buffers, each: k, q (and row decays) [run][kPadded]; v [run][kTile]; write strength, decay [run]
   const int run = a.run;
-  const int per_token = (a.decay_mode == 2 ? 3 : 2) * dim_padded + tile_cols + 2;
-  const int buffer_floats = (run * per_token + 3) & ~3;      // both buffers start on 16 bytes
+  constexpr int kPerToken = scan_token_floats<kRows, kPartners, kCols, kRowDecay, kRead>();
+  const int buffer_floats = (run * kPerToken + 3) & ~3;      // both buffers start on 16 bytes
   const float fixed_decay = a.decay_mode == 0 ? a.decay[head] : 1.0f;
   const float skip = a.skip ? a.skip[head] : 0.0f;
   const float* strength = a.beta ? a.beta : a.v_scale;
@@ -616,51 +893,64 @@ __global__ void __launch_bounds__(kScanThreads) linear_scan_kernel(const ScanArg
   auto stage = [&](int base, float* buffer) {
     const int count = min(run, length - base);
     float* sk = buffer;
-    float* sq = sk + run * dim_padded;
-    float* sg = sq + run * dim_padded;
-    float* sv = sg + (a.decay_mode == 2 ? run * dim_padded : 0);
-    float* sbeta = sv + run * tile_cols;
+    float* sq = sk + run * kPadded;
+    float* sg = sq + (kRead ? run * kPadded : 0);
+    float* sv = sg + (kRowDecay ? run * kPadded : 0);
+    float* sbeta = sv + run * kTile;
     float* sdecay = sbeta + run;
+    // a row decay that is not one per row is spread over the rows here
+    auto spread = [&](size_t t) { return a.decay_mode == 1 ? a.decay[t * a.heads + head] : fixed_decay; };
     if (a.wide_in) {
-      const int quads = dim_padded >> 2, tile_quads = tile_cols >> 2;
+      constexpr int quads = kPadded / 4, tile_quads = kTile / 4;
       for (int idx = threadIdx.x; idx < count * quads; idx += kScanThreads) {
         const int tt = idx / quads, i = (idx - tt * quads) << 2;
         const size_t t = static_cast<size_t>(first + base + tt);
-        const int at = tt * dim_padded + i;
+        const int at = tt * kPadded + i;
         if (i < a.dim) {
           copy_async16(sk + at, a.k + t * a.k_stride + kv_head * a.dim + i);
-          copy_async16(sq + at, a.q + t * a.q_stride + kv_head * a.dim + i);
-          if (a.decay_mode == 2) copy_async16(sg + at, a.decay + (t * a.heads + head) * a.dim + i);
+          if constexpr (kRead) copy_async16(sq + at, a.q + t * a.q_stride + kv_head * a.dim + i);
         } else {
           *reinterpret_cast<float4*>(sk + at) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          *reinterpret_cast<float4*>(sq + at) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          if (a.decay_mode == 2) *reinterpret_cast<float4*>(sg + at) = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+          if constexpr (kRead) *reinterpret_cast<float4*>(sq + at) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+        if constexpr (kRowDecay) {
+          if (a.decay_mode != 2) {
+            const float d = spread(t);
+            *reinterpret_cast<float4*>(sg + at) = make_float4(d, d, d, d);
+          } else if (i < a.dim) {
+            copy_async16(sg + at, a.decay + (t * a.heads + head) * a.dim + i);
+          } else {
+            *reinterpret_cast<float4*>(sg + at) = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+          }
         }
       }
       for (int idx = threadIdx.x; idx < count * tile_quads; idx += kScanThreads) {
         const int tt = idx / tile_quads, j = (idx - tt * tile_quads) << 2;
-        const int c = blockIdx.z * tile_cols + j;
-        float* to = sv + tt * tile_cols + j;
+        const int c = blockIdx.z * kTile + j;
+        float* to = sv + tt * kTile + j;
         if (c < a.vdim) copy_async16(to, a.v + static_cast<size_t>(first + base + tt) * a.v_stride + head * a.vdim + c);
         else *reinterpret_cast<float4*>(to) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       }
     } else {
-      for (int idx = threadIdx.x; idx < count * dim_padded; idx += kScanThreads) {
-        const int tt = idx / dim_padded, i = idx - tt * dim_padded;
+      for (int idx = threadIdx.x; idx < count * kPadded; idx += kScanThreads) {
+        const int tt = idx / kPadded, i = idx - tt * kPadded;
         const size_t t = static_cast<size_t>(first + base + tt);
         if (i < a.dim) {
           copy_async4(sk + idx, a.k + t * a.k_stride + kv_head * a.dim + i);
-          copy_async4(sq + idx, a.q + t * a.q_stride + kv_head * a.dim + i);
-          if (a.decay_mode == 2) copy_async4(sg + idx, a.decay + (t * a.heads + head) * a.dim + i);
+          if constexpr (kRead) copy_async4(sq + idx, a.q + t * a.q_stride + kv_head * a.dim + i);
         } else {
           sk[idx] = 0.0f;
-          sq[idx] = 0.0f;
-          if (a.decay_mode == 2) sg[idx] = 1.0f;
+          if constexpr (kRead) sq[idx] = 0.0f;
+        }
+        if constexpr (kRowDecay) {
+          if (a.decay_mode != 2) sg[idx] = spread(t);
+          else if (i < a.dim) copy_async4(sg + idx, a.decay + (t * a.heads + head) * a.dim + i);
+          else sg[idx] = 1.0f;
         }
       }
-      for (int idx = threadIdx.x; idx < count * tile_cols; idx += kScanThreads) {
-        const int tt = idx / tile_cols, j = idx - tt * tile_cols;
-        const int c = blockIdx.z * tile_cols + j;
+      for (int idx = threadIdx.x; idx < count * kTile; idx += kScanThreads) {
+        const int tt = idx / kTile, j = idx - tt * kTile;
+        const int c = blockIdx.z * kTile + j;
         if (c < a.vdim) copy_async4(sv + idx, a.v + static_cast<size_t>(first + base + tt) * a.v_stride + head * a.vdim + c);
         else sv[idx] = 0.0f;
       }
@@ -675,29 +965,30 @@ __global__ void __launch_bounds__(kScanThreads) linear_scan_kernel(const ScanArg
 
   pdl_wait();
   if (length > 0) stage(0, staged);
-  float S[kRows];
+  using P = PackedPair;
+  ScanColumns<kRows, kPartners, kCols, kKind, kRowDecay, kRead, P> mine;
+  if constexpr (!kRead) {
+    mine.clear();
+    if constexpr (kKind == kScanDelta) mine.units(col - a.vdim, part);
+  } else if (seg.of == 1) {
+    if (start > 0) mine.load(home, a.dim, part, left, wide); else mine.clear();
+  } else if (start > 0 || seg.number > 0) {
+    mine.load(a.seg_states + own * a.vdim + in_head, a.dim, part, left, true);
+  } else {
+    mine.clear();
+  }
+  P product[kRowDecay ? kRows / 2 : 1];      // of the piece's decays
 #pragma unroll
-  for (int r = 0; r < kRows; ++r) S[r] = 0.0f;
-  if (start > 0 && col_ok) {
-    if (wide) {
+  for (int r = 0; r < (kRowDecay ? kRows / 2 : 1); ++r) product[r] = pair_of<P>(1.0f, 1.0f);
+  if constexpr (kKind == kScanBonus) {
 #pragma unroll
-      for (int r = 0; r < kRows; r += 4) {
-        if (row0 + r < a.dim) {
-          const float4 four = *reinterpret_cast<const float4*>(home + r);
-          S[r] = four.x; S[r + 1] = four.y; S[r + 2] = four.z; S[r + 3] = four.w;
-        }
-      }
-    } else {
-#pragma unroll
-      for (int r = 0; r < kRows; ++r)
-        if (row0 + r < a.dim) S[r] = home[r];
+    for (int r = 0; r < kRows / 2; ++r) {
+      const int row = ((r / 2) * kPartners + part) * 4 + (r & 1) * 2;
+      const float* p = a.bonus + static_cast<size_t>(head) * a.dim + row;
+      mine.bonus[r] = pair_of<P>(row < a.dim ? p[0] : 0.0f, row + 1 < a.dim ? p[1] : 0.0f);
     }
   }
-
-  float bonus[kRows];
-#pragma unroll
-  for (int r = 0; r < kRows; ++r)
-    bonus[r] = (a.bonus && row0 + r < a.dim) ? a.bonus[static_cast<size_t>(head) * a.dim + row0 + r] : 0.0f;
+  const bool scaled = strength != nullptr;
 
   int flip = 0;
   for (int base = 0; base < length; base += run, flip ^= 1) {
@@ -711,153 +1002,313 @@ __global__ void __launch_bounds__(kScanThreads) linear_scan_kernel(const ScanArg
     }
     __syncthreads();
     const float* sk = buffer;
-    const float* sq = sk + run * dim_padded;
-    const float* sg = sq + run * dim_padded;
-    const float* sv = sg + (a.decay_mode == 2 ? run * dim_padded : 0);
-    const float* sbeta = sv + run * tile_cols;
+    const float* sq = sk + run * kPadded;
+    const float* sg = sq + (kRead ? run * kPadded : 0);
+    const float* sv = sg + (kRowDecay ? run * kPadded : 0);
+    const float* sbeta = sv + run * kTile;
     const float* sdecay = sbeta + run;
-    // a lane's rows are 16-byte aligned runs of shared memory: fetched four at a time, no two lanes of a
-    // quarter-warp meet in a bank; every pointer of the walk moves by a constant per token
-    const float* kp = sk + row0;
-    const float* qp = sq + row0;
-    const float* gp = sg + row0;
-    const float* vp = sv + col_in_tile;
-    float* op = a.out + static_cast<size_t>(first + base) * a.out_stride + head * a.vdim + (col_ok ? col : 0);
-    const bool writes = part == 0 && col_ok;
-    // Tokens are walked in groups of four: the state passes from one to the next, but their read-outs' sums over
-    // lanes are independent and run side by side after the group, one shuffle's wait for four.  A token's own
-    // arithmetic is the same whatever group it falls into.
-    auto walk = [&](auto group_size, int tt) {
-      constexpr int kGroup = decltype(group_size)::value;
-      float o[kGroup], vv[kGroup];
+    auto fetch = [&](ScanToken<kRows, kCols, kRowDecay, P>& t, int tt) {
+      const int at = tt * kPadded + part * 4;
+      auto two = [&](const float* from, P& lower, P& upper) {
+        const ulonglong2 four = *reinterpret_cast<const ulonglong2*>(from);
+        lower.both = four.x;
+        upper.both = four.y;
+      };
+#pragma unroll
+      for (int j = 0; j < kRows / 4; ++j) {
+        two(sk + at + j * kPartners * 4, t.k[2 * j], t.k[2 * j + 1]);
+        if constexpr (kRead) two(sq + at + j * kPartners * 4, t.q[2 * j], t.q[2 * j + 1]);
+        if constexpr (kRowDecay) two(sg + at + j * kPartners * 4, t.g[2 * j], t.g[2 * j + 1]);
+      }
+      const float* pv = sv + tt * kTile + col_in_tile;
+      if constexpr (kCols == 4) {
+        const float4 v4 = *reinterpret_cast<const float4*>(pv);
+        t.v[0] = v4.x; t.v[1] = v4.y; t.v[2] = v4.z; t.v[3] = v4.w;
+      } else if constexpr (kCols == 2) {
+        const float2 v2 = *reinterpret_cast<const float2*>(pv);
+        t.v[0] = v2.x; t.v[1] = v2.y;
+      } else {
+        t.v[0] = pv[0];
+      }
+      t.strength = scaled ? sbeta[tt] : 1.0f;
+    };
+    // Read-outs of kGroup tokens are summed over lanes together after the group: their exchanges run side by side and
+    // a lane ends up with its share of the sums.
+    auto finish = [&](auto group, float (&o)[decltype(group)::value * kCols], int tt) {
+      constexpr int kCount = decltype(group)::value * kCols;
+      const int at0 = scan_sums<kPartners, kCount>(o, part);
+      constexpr int kKept = kCount > kPartners ? kCount / kPartners : 1;
+      // lanes that hold the same sum: the last exchanges' offsets tell them apart
+      constexpr int kSame = kPartners > kCount ? kPartners / kCount : 1;
+      if (part % kSame != 0) return;
+#pragma unroll
+      for (int i = 0; i < kKept; ++i) {
+        const int g = (at0 + i) / kCols, c = (at0 + i) % kCols;
+        if (c < left) {
+          float sum = o[i];
+          if (a.skip) sum += skip * sv[(tt + g) * kTile + col_in_tile + c];
+          a.out[static_cast<size_t>(first + base + tt + g) * a.out_stride + head * a.vdim + col + c] = sum;
+        }
+      }
+    };
+    auto multiply = [&](const ScanToken<kRows, kCols, kRowDecay, P>& t, float decay) {
+#pragma unroll
+      for (int r = 0; r < (kRowDecay ? kRows / 2 : 1); ++r)
+        product[r] = pair_mul(product[r], kRowDecay ? t.g[r] : pair_of<P>(decay, decay));
+    };
+    constexpr int kGroup = 4;
+    const int whole = count / kGroup * kGroup;
+    ScanToken<kRows, kCols, kRowDecay, P> next;
+    if (whole) fetch(next, 0);
+    for (int tt = 0; tt < whole; tt += kGroup) {
+      float o[kGroup * kCols];
 #pragma unroll
       for (int g = 0; g < kGroup; ++g) {
-        float kk[kRows], qq[kRows];
+        const ScanToken<kRows, kCols, kRowDecay, P> now = next;
+        fetch(next, min(tt + g + 1, count - 1));      // the next token's numbers are on their way during this one's sums
+        float one[kCols];
+        const float decay = kRowDecay ? 1.0f : sdecay[tt + g];
+        mine.take(now, decay, scaled, one);
+        if constexpr (kRead) {
 #pragma unroll
-        for (int r = 0; r < kRows; r += 4) {
-          const float4 k4 = *reinterpret_cast<const float4*>(kp + g * dim_padded + r);
-          const float4 q4 = *reinterpret_cast<const float4*>(qp + g * dim_padded + r);
-          kk[r] = k4.x; kk[r + 1] = k4.y; kk[r + 2] = k4.z; kk[r + 3] = k4.w;
-          qq[r] = q4.x; qq[r + 1] = q4.y; qq[r + 2] = q4.z; qq[r + 3] = q4.w;
+          for (int c = 0; c < kCols; ++c) o[g * kCols + c] = one[c];
+        } else if constexpr (kKind != kScanDelta) {
+          multiply(now, decay);
         }
-        const float vj = vp[g * tile_cols];
-        if (a.bonus) {
-          // read the state as the tokens before left it, the token's own pair weighed by the bonus; then decay and add
-          float gg[kRows];
-          if (a.decay_mode == 2) {
-#pragma unroll
-            for (int r = 0; r < kRows; r += 4) {
-              const float4 g4 = *reinterpret_cast<const float4*>(gp + g * dim_padded + r);
-              gg[r] = g4.x; gg[r + 1] = g4.y; gg[r + 2] = g4.z; gg[r + 3] = g4.w;
-            }
-          } else {
-            const float d = sdecay[tt + g];
-#pragma unroll
-            for (int r = 0; r < kRows; ++r) gg[r] = d;
-          }
-          const float uj = sbeta[tt + g] * vj;
-          float even = 0.0f, odd = 0.0f;
-#pragma unroll
-          for (int r = 0; r < kRows; r += 2) {
-            const float kv0 = kk[r] * uj, kv1 = kk[r + 1] * uj;
-            even += (S[r] + bonus[r] * kv0) * qq[r];
-            odd += (S[r + 1] + bonus[r + 1] * kv1) * qq[r + 1];
-            S[r] = S[r] * gg[r] + kv0;
-            S[r + 1] = S[r + 1] * gg[r + 1] + kv1;
-          }
-          o[g] = even + odd;
-          vv[g] = vj;
-          continue;
-        }
-        if (a.beta == nullptr) {
-          // nothing of the state enters what is added to it: decay and sum are one multiply-add, the only step that a
-          // token has to wait for the one before it
-          const float uj = sbeta[tt + g] * vj;
-          float even = 0.0f, odd = 0.0f;
-          if (a.decay_mode == 2) {
-#pragma unroll
-            for (int r = 0; r < kRows; r += 4) {
-              const float4 g4 = *reinterpret_cast<const float4*>(gp + g * dim_padded + r);
-              S[r] = fmaf(S[r], g4.x, kk[r] * uj);
-              S[r + 1] = fmaf(S[r + 1], g4.y, kk[r + 1] * uj);
-              S[r + 2] = fmaf(S[r + 2], g4.z, kk[r + 2] * uj);
-              S[r + 3] = fmaf(S[r + 3], g4.w, kk[r + 3] * uj);
-            }
-          } else {
-            const float d = sdecay[tt + g];
-#pragma unroll
-            for (int r = 0; r < kRows; ++r) S[r] = fmaf(S[r], d, kk[r] * uj);
-          }
-#pragma unroll
-          for (int r = 0; r < kRows; r += 2) {
-            even += S[r] * qq[r];
-            odd += S[r + 1] * qq[r + 1];
-          }
-          o[g] = even + odd;
-          vv[g] = vj;
-          continue;
-        }
-        if (a.decay_mode == 2) {
-#pragma unroll
-          for (int r = 0; r < kRows; r += 4) {
-            const float4 g4 = *reinterpret_cast<const float4*>(gp + g * dim_padded + r);
-            S[r] *= g4.x; S[r + 1] *= g4.y; S[r + 2] *= g4.z; S[r + 3] *= g4.w;
-          }
-        } else {
-          const float d = sdecay[tt + g];
-#pragma unroll
-          for (int r = 0; r < kRows; ++r) S[r] *= d;
-        }
-        float seen = 0.0f, seen_odd = 0.0f;
-#pragma unroll
-        for (int r = 0; r < kRows; r += 2) {
-          seen += S[r] * kk[r];
-          seen_odd += S[r + 1] * kk[r + 1];
-        }
-        seen += seen_odd;
-#pragma unroll
-        for (int offset = cols_per_warp; offset < 32; offset <<= 1) seen += __shfl_xor_sync(0xffffffffu, seen, offset);
-        const float u = sbeta[tt + g] * (vj - seen);
-        float even = 0.0f, odd = 0.0f;
-#pragma unroll
-        for (int r = 0; r < kRows; r += 2) {
-          S[r] += kk[r] * u;
-          S[r + 1] += kk[r + 1] * u;
-          even += S[r] * qq[r];
-          odd += S[r + 1] * qq[r + 1];
-        }
-        o[g] = even + odd;
-        vv[g] = vj;
       }
-#pragma unroll
-      for (int offset = cols_per_warp; offset < 32; offset <<= 1) {
-#pragma unroll
-        for (int g = 0; g < kGroup; ++g) o[g] += __shfl_xor_sync(0xffffffffu, o[g], offset);
-      }
-      if (writes) {
-#pragma unroll
-        for (int g = 0; g < kGroup; ++g) op[static_cast<size_t>(g) * a.out_stride] = o[g] + skip * vv[g];
-      }
-      kp += kGroup * dim_padded; qp += kGroup * dim_padded; gp += kGroup * dim_padded; vp += kGroup * tile_cols;
-      op += static_cast<size_t>(kGroup) * a.out_stride;
-    };
-    int tt = 0;
-    for (; tt + 4 <= count; tt += 4) walk(std::integral_constant<int, 4>{}, tt);
-    for (; tt < count; ++tt) walk(std::integral_constant<int, 1>{}, tt);
+      if constexpr (kRead) finish(std::integral_constant<int, kGroup>{}, o, tt);
+    }
+    for (int tt = whole; tt < count; ++tt) {
+      ScanToken<kRows, kCols, kRowDecay, P> now;
+      fetch(now, tt);
+      float o[kCols];
+      const float decay = kRowDecay ? 1.0f : sdecay[tt];
+      mine.take(now, decay, scaled, o);
+      if constexpr (kRead) finish(std::integral_constant<int, 1>{}, o, tt);
+      else if constexpr (kKind != kScanDelta) multiply(now, decay);
+    }
     __syncthreads();     // the buffer is free for the run after the next
   }
   pdl_trigger();
-  if (slot_ok && col_ok) {
-    if (wide) {
+  if (left <= 0) return;
+  if constexpr (!kRead) {
+    const int values = a.vdim - col;      // columns of this lane in front of the unit columns
+    // (a lane's columns are all values' or all units': vdim is a multiple of kCols here)
+    if (values > 0) mine.store(a.seg_states + own * a.vdim + in_head, a.dim, part, min(left, values), true);
+    if constexpr (kKind == kScanDelta) {
+      if (values <= 0) mine.store(a.seg_mats + own * a.dim + static_cast<size_t>(-values) * a.dim, a.dim, part, left, true);
+    } else if (blockIdx.z == 0 && threadIdx.x < kPartners) {
 #pragma unroll
-      for (int r = 0; r < kRows; r += 4)
-        if (row0 + r < a.dim) *reinterpret_cast<float4*>(home + r) = make_float4(S[r], S[r + 1], S[r + 2], S[r + 3]);
-    } else {
+      for (int r = 0; r < kRows / 2; ++r) {
+        const int row = ((r / 2) * kPartners + part) * 4 + (r & 1) * 2;
+        const float2 both = pair_halves(product[kRowDecay ? r : 0]);
+        if (row < a.dim) a.seg_decays[own + row] = both.x;
+        if (row + 1 < a.dim) a.seg_decays[own + row + 1] = both.y;
+      }
+    }
+  } else if (slot_ok && seg.number == seg.of - 1) {
+    mine.store(home, a.dim, part, left, wide);
+  }
+}
+
+// What each piece starts from, in place of what it left: start' = decays * start + left, from the slot's state on.
+// A thread owns four rows of a column and goes through the entry's pieces in order; their loads do not wait for one another.
+__global__ void __launch_bounds__(256) scan_join_kernel(const ScanArgs a) {
+  const int e = blockIdx.x, head = blockIdx.y;
+  const int quads = a.dim >> 2, at = blockIdx.z * blockDim.x + threadIdx.x;
+  const int col = at / quads, row = (at - col * quads) * 4;
+  int place;
+  const int pieces = scan_pieces_of(a, e, place);
+  int slot = a.entry_slot[e];
+  if (slot < 0 || slot >= a.slots) slot = 0;      // the walk says so in the fault word
+  pdl_wait();
+  if (col >= a.vdim || pieces <= 1) return;
+  float4 S = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  if (a.entry_start[e] > 0) {
+    const float* home = a.state + slot * a.state_stride + a.state_off + static_cast<size_t>(head) * a.dim * a.vdim +
+                        static_cast<size_t>(col) * a.dim + row;
+    S = make_float4(home[0], home[1], home[2], home[3]);
+  }
+  const size_t step = static_cast<size_t>(a.heads) * a.dim;
+  size_t own = (static_cast<size_t>(place) * a.heads + head) * a.dim;
+#pragma unroll 4
+  for (int p = 0; p < pieces; ++p, own += step) {
+    float4* state = reinterpret_cast<float4*>(a.seg_states + own * a.vdim + static_cast<size_t>(col) * a.dim + row);
+    if (p == pieces - 1) {
+      *state = S;
+      break;
+    }
+    const float4 left = *state, d = *reinterpret_cast<const float4*>(a.seg_decays + own + row);
+    *state = S;
+    S.x = fmaf(S.x, d.x, left.x); S.y = fmaf(S.y, d.y, left.y); S.z = fmaf(S.z, d.z, left.z); S.w = fmaf(S.w, d.w, left.w);
+  }
+}
+
+// The same with a correction: start' = M start + left, M the piece's matrix (its unit columns).  A block owns eight columns
+// of S, which lie in shared memory; a thread forms two rows of them, the matrix read once per block from L2, sixteen of its
+// columns on their way while sixteen are multiplied (without that a piece took 14 us, with it 7).
+constexpr int kJoinCols = 8, kJoinThreads = 64;
+__global__ void __launch_bounds__(kJoinThreads) scan_join_delta_kernel(const ScanArgs a) {
+  __shared__ __align__(16) float start[2 * kJoinThreads][kJoinCols];
+  const int e = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * kJoinCols;
+  int place;
+  const int pieces = scan_pieces_of(a, e, place);
+  int slot = a.entry_slot[e];
+  if (slot < 0 || slot >= a.slots) slot = 0;      // the walk says so in the fault word
+  pdl_wait();
+  if (pieces <= 1) return;
+  const bool carried = a.entry_start[e] > 0;
+  const float* home = a.state + slot * a.state_stride + a.state_off + static_cast<size_t>(head) * a.dim * a.vdim;
+  const int count = min(kJoinCols, a.vdim - col0);
+  const int rows[2] = {min(static_cast<int>(threadIdx.x), a.dim - 1), min(static_cast<int>(threadIdx.x) + kJoinThreads, a.dim - 1)};
+  float S[2][kJoinCols];
 #pragma unroll
-      for (int r = 0; r < kRows; ++r)
-        if (row0 + r < a.dim) home[r] = S[r];
+  for (int h = 0; h < 2; ++h) {
+    const int row = threadIdx.x + h * kJoinThreads;
+#pragma unroll
+    for (int c = 0; c < kJoinCols; ++c)
+      S[h][c] = carried && row < a.dim && c < count ? home[static_cast<size_t>(col0 + c) * a.dim + row] : 0.0f;
+  }
+  for (int p = 0; p < pieces; ++p) {
+    const size_t own = (static_cast<size_t>(place + p) * a.heads + head) * a.dim;
+    float* states = a.seg_states + own * a.vdim + static_cast<size_t>(col0) * a.dim;
+    const float* mat = a.seg_mats + own * a.dim;
+    const bool last = p == pieces - 1;
+    constexpr int kAhead = 16;
+    float m[2][kAhead][2];
+    auto fetch = [&](int buffer, int j0) {
+#pragma unroll
+      for (int j = 0; j < kAhead; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) m[buffer][j][h] = mat[static_cast<size_t>(min(j0 + j, a.dim - 1)) * a.dim + rows[h]];
+    };
+    if (!last) fetch(0, 0);
+    float next[2][kJoinCols];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const bool mine = static_cast<int>(threadIdx.x) + h * kJoinThreads < a.dim;
+#pragma unroll
+      for (int c = 0; c < kJoinCols; ++c) next[h][c] = mine && c < count && !last ? states[static_cast<size_t>(c) * a.dim + rows[h]] : 0.0f;
+#pragma unroll
+      for (int c = 0; c < kJoinCols; ++c)
+        if (mine && c < count) states[static_cast<size_t>(c) * a.dim + rows[h]] = S[h][c];
+    }
+    if (last) break;
+    __syncthreads();      // the piece before has been read
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int c = 0; c < kJoinCols; ++c) start[threadIdx.x + h * kJoinThreads][c] = S[h][c];
+    __syncthreads();
+    auto multiply = [&](int buffer, int j0) {
+#pragma unroll
+      for (int j = 0; j < kAhead; ++j) {
+        if (j0 + j >= a.dim) break;
+        float s[kJoinCols];
+#pragma unroll
+        for (int c = 0; c < kJoinCols; c += 4) {
+          const float4 four = *reinterpret_cast<const float4*>(&start[j0 + j][c]);
+          s[c] = four.x; s[c + 1] = four.y; s[c + 2] = four.z; s[c + 3] = four.w;
+        }
+#pragma unroll
+        for (int c = 0; c < kJoinCols; ++c) {
+          next[0][c] = fmaf(m[buffer][j][0], s[c], next[0][c]);
+          next[1][c] = fmaf(m[buffer][j][1], s[c], next[1][c]);
+        }
+      }
+    };
+    for (int j0 = 0; j0 < a.dim; j0 += 2 * kAhead) {
+      fetch(1, j0 + kAhead);
+      multiply(0, j0);
+      fetch(0, j0 + 2 * kAhead);
+      multiply(1, j0 + kAhead);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int c = 0; c < kJoinCols; ++c) S[h][c] = next[h][c];
+  }
+}
+
+// A step of single tokens: bound by the states' way through memory, so nothing is staged.  A lane's numbers of the token
+// come straight from the rows; with four columns a lane it has four 16-byte pieces of the state on their way.
+template <int kRows, int kPartners, int kCols, int kKind, bool kRowDecay>
+__global__ void __launch_bounds__(kScanThreads) linear_scan_single_kernel(const ScanArgs a) {
+  pdl_trigger();
+  const int e = blockIdx.x, head = blockIdx.y;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, part = lane % kPartners;
+  constexpr int kSpread = 32 / kPartners, kTile = kScanWarps * kSpread * kCols;
+  const int col = blockIdx.z * kTile + (warp * kSpread + lane / kPartners) * kCols;
+  const int left = a.vdim - col;
+  const int kv_head = head / (a.heads / a.kv_heads);
+  const int first = a.cu_seqlens[e], length = a.cu_seqlens[e + 1] - first, start = a.entry_start[e];
+  int slot = a.entry_slot[e];
+  const bool slot_ok = slot >= 0 && slot < a.slots;
+  if (!slot_ok) {
+    if (threadIdx.x == 0) atomicOr(a.fault, kFaultSlot);
+    slot = 0;
+  }
+  float* home = a.state + slot * a.state_stride + a.state_off + static_cast<size_t>(head) * a.dim * a.vdim +
+                static_cast<size_t>(left > 0 ? col : 0) * a.dim;
+  const bool wide = (reinterpret_cast<uintptr_t>(home) & 15) == 0;
+  const float* strength = a.beta ? a.beta : a.v_scale;
+  const bool scaled = strength != nullptr;
+  const float skip = a.skip ? a.skip[head] : 0.0f;
+  const float fixed_decay = a.decay_mode == 0 ? a.decay[head] : 1.0f;
+  using P = PlainPair;
+  ScanColumns<kRows, kPartners, kCols, kKind, kRowDecay, true, P> mine;
+  if constexpr (kKind == kScanBonus) {
+#pragma unroll
+    for (int j = 0; j < kRows / 4; ++j) {
+      const int row = (j * kPartners + part) * 4;
+      const float* p = a.bonus + static_cast<size_t>(head) * a.dim + row;
+      mine.bonus[2 * j] = row < a.dim ? pair_of<P>(p[0], p[1]) : pair_of<P>(0.0f, 0.0f);
+      mine.bonus[2 * j + 1] = row < a.dim ? pair_of<P>(p[2], p[3]) : pair_of<P>(0.0f, 0.0f);
     }
   }
+  pdl_wait();
+  if (start > 0) mine.load(home, a.dim, part, left, wide); else mine.clear();
+  for (int i = 0; i < length; ++i) {
+    const size_t t = static_cast<size_t>(first) + i;
+    ScanToken<kRows, kCols, kRowDecay, P> now;
+    const float decay = a.decay_mode == 1 ? a.decay[t * a.heads + head] : fixed_decay;
+    auto rows = [&](const float* p, int j, float otherwise, P& lower, P& upper) {
+      const int row = (j * kPartners + part) * 4;
+      float4 four = make_float4(otherwise, otherwise, otherwise, otherwise);
+      if (row < a.dim) four = *reinterpret_cast<const float4*>(p + row);
+      lower = pair_of<P>(four.x, four.y);
+      upper = pair_of<P>(four.z, four.w);
+    };
+#pragma unroll
+    for (int j = 0; j < kRows / 4; ++j) {
+      rows(a.k + t * a.k_stride + kv_head * a.dim, j, 0.0f, now.k[2 * j], now.k[2 * j + 1]);
+      rows(a.q + t * a.q_stride + kv_head * a.dim, j, 0.0f, now.q[2 * j], now.q[2 * j + 1]);
+      if constexpr (kRowDecay) {
+        if (a.decay_mode == 2) rows(a.decay + (t * a.heads + head) * a.dim, j, 1.0f, now.g[2 * j], now.g[2 * j + 1]);
+        else now.g[2 * j] = now.g[2 * j + 1] = pair_of<P>(decay, decay);
+      }
+    }
+    const float* v = a.v + t * a.v_stride + head * a.vdim + col;
+#pragma unroll
+    for (int c = 0; c < kCols; ++c) now.v[c] = c < left ? v[c] : 0.0f;
+    now.strength = scaled ? strength[t * a.heads + head] : 1.0f;
+    float o[kCols];
+    mine.take(now, decay, scaled, o);
+    const int at0 = scan_sums<kPartners, kCols>(o, part);
+    constexpr int kSame = kPartners > kCols ? kPartners / kCols : 1, kKept = kCols > kPartners ? kCols / kPartners : 1;
+    if (part % kSame == 0) {
+#pragma unroll
+      for (int c = 0; c < kKept; ++c) {
+        const int at = at0 + c;
+        if (at < left) {
+          float sum = o[c];
+          if (a.skip) sum += skip * v[at];
+          a.out[t * a.out_stride + head * a.vdim + col + at] = sum;
+        }
+      }
+    }
+  }
+  if (slot_ok && left > 0) mine.store(home, a.dim, part, left, wide);
 }
 
 // ------------------------------------------------------------ norm and gate after a mixer
@@ -1041,6 +1492,71 @@ inline unsigned flat_blocks(long long total, int threads) {
 
 }  // namespace rl
 
+namespace rl {
+
+template <int kRows, int kPartners, int kCols, int kKind, bool kRowDecay, bool kRead = true>
+static int launch_scan(ScanArgs a, int blocks, int pdl, cudaStream_t stream) {
+  constexpr int kTile = kScanWarps * (32 / kPartners) * kCols;
+  constexpr int kPerToken = scan_token_floats<kRows, kPartners, kCols, kRowDecay, kRead>();
+  constexpr int kRun = 20 * 1024 / 4 / kPerToken;      // two buffers of a run each within 40 KB
+  a.run = kRun > 16 ? 16 : (kRun < 1 ? 1 : kRun);
+  const size_t smem = 2 * static_cast<size_t>((a.run * kPerToken + 3) & ~3) * sizeof(float);
+  const int columns = a.vdim + (!kRead && kKind == kScanDelta ? a.dim : 0);
+  const dim3 grid(blocks, a.heads, (columns + kTile - 1) / kTile);
+  return launch_kernel(linear_scan_kernel<kRows, kPartners, kCols, kKind, kRowDecay, kRead>, grid, dim3(kScanThreads), smem,
+                       stream, pdl != 0, a);
+}
+
+// Rows a lane and lanes a column are a matter of the head's size alone, since they fix the order of a column's sums.
+template <int kKind, bool kRowDecay>
+static int launch_plain_scan(const ScanArgs& a, int blocks, int pdl, cudaStream_t stream) {
+  const int dim = a.dim;
+  if (dim <= 4) return launch_scan<4, 1, 2, kKind, kRowDecay>(a, blocks, pdl, stream);
+  if (dim <= 8) return launch_scan<4, 2, 2, kKind, kRowDecay>(a, blocks, pdl, stream);
+  if (dim <= 16) return launch_scan<4, 4, 2, kKind, kRowDecay>(a, blocks, pdl, stream);
+  if (dim <= 32) return launch_scan<4, 8, 2, kKind, kRowDecay>(a, blocks, pdl, stream);
+  if (dim <= 64) return launch_scan<4, 16, 2, kKind, kRowDecay>(a, blocks, pdl, stream);
+  if (dim <= 128) return launch_scan<4, 32, 2, kKind, kRowDecay>(a, blocks, pdl, stream);
+  if (dim <= 256) return launch_scan<8, 32, 2, kKind, kRowDecay>(a, blocks, pdl, stream);
+  if (dim <= 512) return launch_scan<16, 32, 1, kKind, kRowDecay>(a, blocks, pdl, stream);
+  return launch_scan<32, 32, 1, kKind, kRowDecay>(a, blocks, pdl, stream);
+}
+
+static int launch_delta_scan(const ScanArgs& a, int blocks, int pdl, cudaStream_t stream) {
+  const int dim = a.dim;
+  if (dim <= 4) return launch_scan<4, 1, 2, kScanDelta, true>(a, blocks, pdl, stream);
+  if (dim <= 8) return launch_scan<4, 2, 2, kScanDelta, true>(a, blocks, pdl, stream);
+  if (dim <= 16) return launch_scan<4, 4, 2, kScanDelta, true>(a, blocks, pdl, stream);
+  if (dim <= 32) return launch_scan<8, 4, 2, kScanDelta, true>(a, blocks, pdl, stream);
+  if (dim <= 64) return launch_scan<16, 4, 2, kScanDelta, true>(a, blocks, pdl, stream);
+  if (dim <= 128) return launch_scan<16, 8, 2, kScanDelta, true>(a, blocks, pdl, stream);
+  if (dim <= 256) return launch_scan<16, 16, 2, kScanDelta, true>(a, blocks, pdl, stream);
+  if (dim <= 512) return launch_scan<16, 32, 1, kScanDelta, true>(a, blocks, pdl, stream);
+  return launch_scan<32, 32, 1, kScanDelta, true>(a, blocks, pdl, stream);
+}
+
+// In pieces there are blocks enough: more rows a lane and four columns, fewer exchanges and fetches a column.
+template <int kKind, bool kRowDecay, bool kRead>
+static int launch_pieces(const ScanArgs& a, int blocks, int pdl, cudaStream_t stream) {
+  if constexpr (kKind == kScanDelta) {
+    // four columns a lane where a column has eight lanes and its read-outs are summed: 194 -> 163 us at 16 heads of 128
+    if (a.dim <= 64) return launch_scan<16, 4, 2, kKind, true, kRead>(a, blocks, pdl, stream);
+    return launch_scan<16, 8, kRead ? 4 : 2, kKind, true, kRead>(a, blocks, pdl, stream);
+  } else {
+    return a.dim <= 64 ? launch_scan<8, 8, 4, kKind, kRowDecay, kRead>(a, blocks, pdl, stream)
+                       : launch_scan<8, 16, 4, kKind, kRowDecay, kRead>(a, blocks, pdl, stream);
+  }
+}
+
+template <int kRows, int kPartners, int kCols, int kKind, bool kRowDecay>
+static int launch_single_scan(const ScanArgs& a, int pdl, cudaStream_t stream) {
+  constexpr int kTile = kScanWarps * (32 / kPartners) * kCols;
+  return launch_kernel(linear_scan_single_kernel<kRows, kPartners, kCols, kKind, kRowDecay>,
+                       dim3(a.entries, a.heads, (a.vdim + kTile - 1) / kTile), dim3(kScanThreads), 0, stream, pdl != 0, a);
+}
+
+}  // namespace rl
+
 extern "C" {
 
 // out = silu(conv(x)) for every row of the step, then the slots' tails are brought up to date.
@@ -1185,40 +1701,68 @@ int rl_rotate_heads(int dtype, const void* in, int in_stride, int q_col0, int k_
 int rl_linear_scan(const float* q, int q_stride, const float* k, int k_stride, const float* v, int v_stride,
                    const float* decay, int decay_mode, const float* beta, const float* v_scale, const float* skip,
                    const float* bonus, float* out, int out_stride, float* state, long long state_stride, int state_off,
-                   const int* cu_seqlens, const int* entry_slot, const int* entry_start, int entries, int heads,
-                   int kv_heads, int dim, int vdim, int slots, int* fault, int pdl, cudaStream_t stream) {
+                   const int* cu_seqlens, const int* entry_slot, const int* entry_start, int entries, int tokens, int heads,
+                   int kv_heads, int dim, int vdim, int slots, int* fault, int segment, int segments, float* seg_states,
+                   float* seg_decays, float* seg_mats, int pdl, cudaStream_t stream) {
   if (entries == 0) return 0;
   if (heads < 1 || kv_heads < 1 || heads % kv_heads || dim < 1 || dim > 1024 || vdim < 1 || decay_mode < 0 ||
       decay_mode > 2 || decay == nullptr || (bonus != nullptr && beta != nullptr))
     return static_cast<int>(cudaErrorInvalidValue);
-  // rows a lane holds: few, so that a column's work spreads over many lanes; as many lanes a column as it takes
-  const int rows = dim <= 32 ? 4 : (dim <= 256 ? 8 : (dim <= 512 ? 16 : 32));
-  int partners = 1;
-  while (partners * rows < dim) partners *= 2;
   rl::ScanArgs a;
   a.q = q; a.q_stride = q_stride; a.k = k; a.k_stride = k_stride; a.v = v; a.v_stride = v_stride;
   a.decay = decay; a.decay_mode = decay_mode; a.beta = beta; a.v_scale = v_scale; a.skip = skip; a.bonus = bonus;
   a.out = out; a.out_stride = out_stride; a.state = state; a.state_stride = state_stride; a.state_off = state_off;
   a.cu_seqlens = cu_seqlens; a.entry_slot = entry_slot; a.entry_start = entry_start;
-  a.heads = heads; a.kv_heads = kv_heads; a.dim = dim; a.vdim = vdim; a.slots = slots; a.partners = partners;
+  a.heads = heads; a.kv_heads = kv_heads; a.dim = dim; a.vdim = vdim; a.slots = slots;
   a.fault = fault;
   auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   a.wide_in = dim % 4 == 0 && vdim % 4 == 0 && q_stride % 4 == 0 && k_stride % 4 == 0 && v_stride % 4 == 0 &&
               aligned(q) && aligned(k) && aligned(v) && (decay_mode != 2 || aligned(decay));
-  const int tile_cols = (rl::kScanThreads / 32) * (32 / partners);
-  const int dim_padded = partners * rows;
-  const int per_token = (decay_mode == 2 ? 3 : 2) * dim_padded + tile_cols + 2;
-  int run = (20 * 1024 / 4) / per_token;      // two buffers of a run each within 40 KB
-  a.run = run > 16 ? 16 : (run < 1 ? 1 : run);
-  const size_t smem = 2 * static_cast<size_t>((a.run * per_token + 3) & ~3) * sizeof(float);
-  const dim3 grid(entries, heads, (vdim + tile_cols - 1) / tile_cols), block(rl::kScanThreads);
-#define RL_SCAN(R, P) \
-  if (rows == R && partners == P) return rl::launch_kernel(rl::linear_scan_kernel<R, P>, grid, block, smem, stream, pdl != 0, a)
-  RL_SCAN(4, 1); RL_SCAN(4, 2); RL_SCAN(4, 4); RL_SCAN(4, 8);
-  RL_SCAN(8, 8); RL_SCAN(8, 16); RL_SCAN(8, 32);
-  RL_SCAN(16, 32); RL_SCAN(32, 32);
-#undef RL_SCAN
-  return static_cast<int>(cudaErrorInvalidValue);
+  a.entries = entries;
+  a.segment = segment;
+  a.seg_states = seg_states; a.seg_decays = seg_decays; a.seg_mats = seg_mats;
+  using namespace rl;
+  // single tokens of the common head sizes: the same rows a lane and lanes a column as the walk, so the same sums
+  if (segment == 0 && tokens == entries && a.wide_in && dim > 32 && dim <= 128) {
+    if (beta)
+      return dim <= 64 ? launch_single_scan<16, 4, 2, kScanDelta, true>(a, pdl, stream)
+                       : launch_single_scan<16, 8, 2, kScanDelta, true>(a, pdl, stream);
+    if (bonus)
+      return dim <= 64 ? launch_single_scan<4, 16, 4, kScanBonus, true>(a, pdl, stream)
+                       : launch_single_scan<4, 32, 4, kScanBonus, true>(a, pdl, stream);
+    if (decay_mode == 2)
+      return dim <= 64 ? launch_single_scan<4, 16, 4, kScanPlain, true>(a, pdl, stream)
+                       : launch_single_scan<4, 32, 4, kScanPlain, true>(a, pdl, stream);
+    return dim <= 64 ? launch_single_scan<4, 16, 4, kScanPlain, false>(a, pdl, stream)
+                     : launch_single_scan<4, 32, 4, kScanPlain, false>(a, pdl, stream);
+  }
+  if (segment == 0) {
+    if (beta) return launch_delta_scan(a, entries, pdl, stream);
+    if (bonus) return launch_plain_scan<kScanBonus, true>(a, entries, pdl, stream);
+    if (decay_mode == 2) return launch_plain_scan<kScanPlain, true>(a, entries, pdl, stream);
+    return launch_plain_scan<kScanPlain, false>(a, entries, pdl, stream);
+  }
+  // in pieces side by side: sizes and pieces the kernels are made for
+  if (segment < 0 || dim <= 32 || dim > 128 || dim % 4 || vdim % 4 || segments < 1 || seg_states == nullptr ||
+      (beta ? seg_mats == nullptr : seg_decays == nullptr) || !aligned(seg_states) || !aligned(seg_decays) || !aligned(seg_mats))
+    return static_cast<int>(cudaErrorInvalidValue);
+  int e;
+  if (beta) {
+    e = launch_pieces<kScanDelta, true, false>(a, segments, pdl, stream);
+    if (e == 0)
+      e = launch_kernel(scan_join_delta_kernel, dim3(entries, heads, (vdim + kJoinCols - 1) / kJoinCols), dim3(kJoinThreads), 0,
+                        stream, pdl != 0, a);
+    return e ? e : launch_pieces<kScanDelta, true, true>(a, segments, pdl, stream);
+  }
+  // with a bonus the state moves as without one
+  e = bonus || decay_mode == 2 ? launch_pieces<kScanPlain, true, false>(a, segments, pdl, stream)
+                               : launch_pieces<kScanPlain, false, false>(a, segments, pdl, stream);
+  if (e == 0)
+    e = launch_kernel(scan_join_kernel, dim3(entries, heads, (vdim * (dim / 4) + 255) / 256), dim3(256), 0, stream, pdl != 0, a);
+  if (e) return e;
+  if (bonus) return launch_pieces<kScanBonus, true, true>(a, segments, pdl, stream);
+  if (decay_mode == 2) return launch_pieces<kScanPlain, true, true>(a, segments, pdl, stream);
+  return launch_pieces<kScanPlain, false, true>(a, segments, pdl, stream);
 }
 
 // y_f32: y is float32 whatever the engine's dtype (the result of a recurrence); else y has the engine's dtype.

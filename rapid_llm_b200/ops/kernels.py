@@ -1101,7 +1101,7 @@ def recurrent() -> ctypes.CDLL:
         lib.rl_linear_scan.argtypes = [
             c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
             c_void_p, c_int, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-            c_int, c_int, c_void_p, c_int, c_void_p,
+            c_int, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
         ]
         lib.rl_exp_decay.argtypes = [c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]
         lib.rl_low_rank_decay.argtypes = [c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_float, c_void_p,
@@ -1230,10 +1230,31 @@ def rotate_heads(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.T
     return out
 
 
+def scan_piece(heads: int, vdim: int, corrected: bool) -> int:
+    """Tokens of a piece of a prompt that is walked in pieces side by side: as many pieces as it takes to fill the GPU, and no
+    more, since what joins them costs by the piece (a matrix product each with a correction, else one more pass over the
+    pieces' states).  2,048 tokens in pieces of 64, 128, 256, us: 16 heads of 128, fixed decays 206, 187, 202; 32 heads 556,
+    374, 332; with a correction, 16 heads, 663, 508, 469."""
+    return 256 if corrected or heads * vdim >= 4096 else 128
+
+
+def scan_pieces_from(heads: int, vdim: int, corrected: bool) -> int:
+    """The shortest prompt that is walked in pieces: every piece but the last is walked twice, and what joins them comes on
+    top.  From end to end and in pieces, us: 8 heads of 128, 300 tokens 43 and 56; 32 heads of 128, 1,015 tokens beside
+    shorter ones 420 and 331; with a correction, 32 heads of 64, the same prompts 252 and 275, 2,048 tokens of 16 heads 567
+    and 433."""
+    return scan_piece(heads, vdim, corrected) * (4 if corrected else 3)
+
+
+def scan_takes_pieces(dim: int, vdim: int) -> bool:
+    """Whether the recurrence's kernels walk prompts of this head size in pieces."""
+    return 32 < dim <= 128 and dim % 4 == 0 and vdim % 4 == 0
+
+
 def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, out: torch.Tensor,
                 state: torch.Tensor, batch, *, heads: int, kv_heads: int, dim: int, vdim: int,
                 beta: torch.Tensor | None = None, v_scale: torch.Tensor | None = None,
-                skip: torch.Tensor | None = None, bonus: torch.Tensor | None = None) -> torch.Tensor:
+                skip: torch.Tensor | None = None, bonus: torch.Tensor | None = None, pieces=None) -> torch.Tensor:
     """The recurrence ``S <- decay * S; u = beta * (v - S^T k)`` (or ``v_scale * v`` without ``beta``);
     ``S <- S + k u^T; out = S^T q + skip * v`` per head over every entry's tokens, from and into
     ``state [slots, heads * dim * vdim]`` (float32; a request at position 0 starts from zeros).  With ``bonus``
@@ -1243,6 +1264,9 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.
     All operands float32: ``q``, ``k`` ``[T, kv_heads * dim]`` and ``v`` ``[T, heads * vdim]`` (views of columns
     are fine), ``decay`` ``[heads]`` (fixed), ``[T, heads]`` or ``[T, heads * dim]`` (one per row of ``S``),
     ``beta``/``v_scale`` ``[T, heads]``, ``skip`` ``[heads]``, ``out`` ``[T, heads * vdim]``.
+
+    With ``pieces`` (a workspace) a step with a long enough prompt (:func:`scan_pieces_from`) is walked in pieces side by side: the
+    same sums in another order, which depends on where the step cuts the request.
     """
     _need_cuda(q, k, v, decay, out, state, beta, v_scale, skip, bonus)
     for name, tensor in (("q", q), ("k", k), ("v", v), ("decay", decay), ("out", out), ("beta", beta),
@@ -1269,12 +1293,23 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.
     # before it still fills most multiprocessors, several of its few blocks on the same ones (measured: 1.1 ms instead
     # of 0.6 ms for 2,048 tokens).  Steps of single tokens have many short blocks and keep the early start.
     early = PDL and tokens < 8 * batch.num_entries
+    piece = blocks = 0
+    states = decays = mats = None
+    if pieces is not None and scan_takes_pieces(dim, vdim) and batch.max_query_len >= scan_pieces_from(heads, vdim, beta is not None):
+        piece = scan_piece(heads, vdim, beta is not None)
+        blocks = tokens // piece + batch.num_entries
+        kept = tokens // piece + min(batch.num_entries, tokens // (piece + 1))      # of entries longer than a piece
+        states = pieces.get("scan_states", kept, heads * dim * vdim, torch.float32, min_rows=kept)
+        if beta is None:
+            decays = pieces.get("scan_decays", kept, heads * dim, torch.float32, min_rows=kept)
+        else:
+            mats = pieces.get("scan_mats", kept, heads * dim * dim, torch.float32, min_rows=kept)
     _check(
         recurrent().rl_linear_scan(
             _ptr(q), _row_stride("q", q), _ptr(k), _row_stride("k", k), _ptr(v), _row_stride("v", v), _ptr(decay), mode,
             _ptr(beta), _ptr(v_scale), _ptr(skip), _ptr(bonus), _ptr(out), _row_stride("out", out), _ptr(state), stride, 0,
-            _ptr(batch.cu_seqlens), _ptr(batch.entry_slot), _ptr(batch.entry_start), batch.num_entries, heads, kv_heads,
-            dim, vdim, slots, _ptr(batch.fault), int(early), _stream()),
+            _ptr(batch.cu_seqlens), _ptr(batch.entry_slot), _ptr(batch.entry_start), batch.num_entries, tokens, heads, kv_heads,
+            dim, vdim, slots, _ptr(batch.fault), piece, blocks, _ptr(states), _ptr(decays), _ptr(mats), int(early), _stream()),
         f"linear_scan(dim={dim}, vdim={vdim})",
     )
     return out

@@ -53,6 +53,18 @@ class _Recurrent(Mixer):
     def state_need(self) -> StateNeed:
         return StateNeed((self.state_size + self.tail_size,), torch.float32)
 
+    def _pieces(self, batch):
+        """Where a long prompt is walked in pieces side by side: in bfloat16.  The 32-bit path walks a request's tokens one
+        after the other, so that its rows are the same bit for bit however they are cut into steps."""
+        return batch.workspace if self.dtype == torch.bfloat16 else None
+
+    def _pieces_elements(self, heads: int, dim: int, vdim: int, corrected: bool = False) -> int:
+        """Elements of the engine's dtype a token's share of the pieces' states takes at most."""
+        if self.dtype != torch.bfloat16 or not kernels.scan_takes_pieces(dim, vdim):
+            return 0
+        floats = heads * dim * (vdim + (dim if corrected else 1))
+        return 2 * 2 * -(-floats // kernels.scan_piece(heads, vdim, corrected))
+
     def _state_views(self, cache) -> tuple[torch.Tensor, torch.Tensor]:
         state = cache.state
         if state is None or state.shape[1] != self.state_size + self.tail_size or state.dtype != torch.float32:
@@ -160,7 +172,8 @@ class ChannelDeltaRule(_Recurrent):
             raise KeyError(name)
 
     def workspace_elements_per_token(self) -> int:
-        return 3 * (self.w_in.shape[0] + self.w_high.shape[0]) + self.ra + self.rg + self.hidden
+        return (3 * (self.w_in.shape[0] + self.w_high.shape[0]) + self.ra + self.rg + self.hidden
+                + self._pieces_elements(self.h, self.dim, self.vdim, corrected=True))
 
     def forward(self, x, batch, cache):
         rows, space, f32 = x.shape[0], batch.workspace, torch.float32
@@ -177,7 +190,7 @@ class ChannelDeltaRule(_Recurrent):
         kernels.decay_gate(high[:, : self.h * self.dim], self.rate, self.dt_bias, self.dim, decay)
         read = space.get("delta_read", rows, self.cv, f32)
         kernels.linear_scan(conv[:, : self.cq], conv[:, self.cq : 2 * self.cq], conv[:, 2 * self.cq :], decay, read, S,
-                            batch, heads=self.h, kv_heads=self.hk, dim=self.dim, vdim=self.vdim, beta=beta)
+                            batch, heads=self.h, kv_heads=self.hk, dim=self.dim, vdim=self.vdim, beta=beta, pieces=self._pieces(batch))
         normed = space.get("delta_normed", rows, self.cv, x.dtype)
         kernels.gated_norm(read, normed, group=self.vdim, gate=high[:, self.h * self.dim :], act=kernels.GATE_SIGMOID,
                            weight=self.norm, eps=self.eps)
@@ -238,7 +251,7 @@ class Retention(_Recurrent):
             raise KeyError(name)
 
     def workspace_elements_per_token(self) -> int:
-        return 4 * self.w_in.shape[0] + self.hidden
+        return 4 * self.w_in.shape[0] + self.hidden + self._pieces_elements(self.h, self.dim, self.vdim)
 
     def forward(self, x, batch, cache):
         rows, space, f32 = x.shape[0], batch.workspace, torch.float32
@@ -250,7 +263,8 @@ class Retention(_Recurrent):
                              self.inv_freq, heads=self.h, dim=self.dim, vdim=self.vdim, k_scale=self.dim ** -0.5)
         read = space.get("ret_read", rows, cv, f32)
         kernels.linear_scan(qkv[:, :cq], qkv[:, cq : 2 * cq], qkv[:, 2 * cq :], self.decay, read, S, batch,
-                            heads=self.h, kv_heads=self.h, dim=self.dim, vdim=self.vdim)
+                            heads=self.h, kv_heads=self.h, dim=self.dim, vdim=self.vdim,
+                            pieces=self._pieces(batch))
         normed = space.get("ret_normed", rows, cv, x.dtype)
         kernels.gated_norm(read, normed, group=self.vdim, gate=proj[:, 2 * cq + cv :], act=kernels.GATE_SILU, eps=self.eps)
         return gemm.linear(normed, self.o, space.get("ret_out", rows, self.hidden, x.dtype), batch.fault)
@@ -307,7 +321,7 @@ class Lightning(_Recurrent):
             raise KeyError(name)
 
     def workspace_elements_per_token(self) -> int:
-        return 4 * self.w_in.shape[0] + self.hidden
+        return 4 * self.w_in.shape[0] + self.hidden + self._pieces_elements(self.h, self.dim, self.vdim)
 
     def forward(self, x, batch, cache):
         rows, space, f32 = x.shape[0], batch.workspace, torch.float32
@@ -317,7 +331,8 @@ class Lightning(_Recurrent):
         qkv = kernels.activate_rows(proj[:, : 2 * cq + cv], space.get("lightning_qkv", rows, 2 * cq + cv, f32), act=True)
         read = space.get("lightning_read", rows, cv, f32)
         kernels.linear_scan(qkv[:, :cq], qkv[:, cq : 2 * cq], qkv[:, 2 * cq :], self.decay, read, S, batch,
-                            heads=self.h, kv_heads=self.h, dim=self.dim, vdim=self.vdim)
+                            heads=self.h, kv_heads=self.h, dim=self.dim, vdim=self.vdim,
+                            pieces=self._pieces(batch))
         normed = space.get("lightning_normed", rows, cv, x.dtype)
         kernels.gated_norm(read, normed, group=cv, gate=proj[:, 2 * cq + cv :], act=kernels.GATE_SIGMOID,
                            weight=self.norm, eps=self.eps)
@@ -392,7 +407,7 @@ class StateSpaceDual(_Recurrent):
             raise KeyError(name)
 
     def workspace_elements_per_token(self) -> int:
-        return 4 * self.w_in.shape[0] + self.hidden
+        return 4 * self.w_in.shape[0] + self.hidden + self._pieces_elements(self.h, self.n, self.vdim)
 
     def forward(self, x, batch, cache):
         rows, space, f32 = x.shape[0], batch.workspace, torch.float32
@@ -405,7 +420,8 @@ class StateSpaceDual(_Recurrent):
         kernels.decay_gate(proj[:, inner + mixed :], self.rate, self.dt_bias, 1, decay, step)
         read = space.get("ssd_read", rows, inner, f32)
         kernels.linear_scan(conv[:, inner + gn :], conv[:, inner : inner + gn], conv[:, :inner], decay, read, S, batch,
-                            heads=self.h, kv_heads=self.groups, dim=self.n, vdim=self.vdim, v_scale=step, skip=self.skip)
+                            heads=self.h, kv_heads=self.groups, dim=self.n, vdim=self.vdim, v_scale=step, skip=self.skip,
+                            pieces=self._pieces(batch))
         normed = space.get("ssd_normed", rows, inner, x.dtype)
         kernels.gated_norm(read, normed, group=inner // self.norm_groups, gate=proj[:, :inner], act=kernels.GATE_SILU,
                            gate_first=True, weight=self.norm, eps=self.eps)
@@ -483,7 +499,8 @@ class ShiftedDecay(_Recurrent):
             raise KeyError(name)
 
     def workspace_elements_per_token(self) -> int:
-        return 5 * self.hidden + 4 * self.c + 2 * (4 * self.c) + 2 * self.rank + self.hidden
+        return (5 * self.hidden + 4 * self.c + 2 * (4 * self.c) + 2 * self.rank + self.hidden
+                + self._pieces_elements(self.h, self.dim, self.dim))
 
     def forward(self, x, batch, cache):
         rows, space, f32, c = x.shape[0], batch.workspace, torch.float32, self.c
@@ -502,7 +519,8 @@ class ShiftedDecay(_Recurrent):
         rkv = kernels.activate_rows(proj[: 3 * rows], space.get("wkv_rkv", 3 * rows, c, f32), act=False)
         read = space.get("wkv_read", rows, c, f32)
         kernels.linear_scan(rkv[:rows], rkv[rows : 2 * rows], rkv[2 * rows :], decay, read, S, batch, heads=self.h,
-                            kv_heads=self.h, dim=self.dim, vdim=self.dim, bonus=self.bonus)
+                            kv_heads=self.h, dim=self.dim, vdim=self.dim, bonus=self.bonus,
+                            pieces=self._pieces(batch))
         normed = space.get("wkv_normed", rows, c, x.dtype)
         kernels.gated_norm(read, normed, group=self.dim, gate=proj[3 * rows :], act=kernels.GATE_SILU, weight=self.norm,
                            eps=self.eps)
@@ -576,7 +594,8 @@ class GatedLinear(_Recurrent):
 
     def workspace_elements_per_token(self) -> int:
         # the product, the float32 q, k, v, decays and read-out, the normed heads and the result
-        return self.w_in.shape[0] + 2 * (3 * self.cq + 2 * self.cv) + self.cv + self.hidden
+        return (self.w_in.shape[0] + 2 * (3 * self.cq + 2 * self.cv) + self.cv + self.hidden
+                + self._pieces_elements(self.h, self.dim, self.vdim))
 
     def forward(self, x, batch, cache):
         rows, space, f32 = x.shape[0], batch.workspace, torch.float32
@@ -589,7 +608,8 @@ class GatedLinear(_Recurrent):
                                self.tau, qkv, decay)
         read = space.get("gla_read", rows, cv, f32)
         kernels.linear_scan(qkv[:, :cq], qkv[:, cq : 2 * cq], qkv[:, 2 * cq :], decay, read, S, batch,
-                            heads=self.h, kv_heads=self.h, dim=self.dim, vdim=self.vdim)
+                            heads=self.h, kv_heads=self.h, dim=self.dim, vdim=self.vdim,
+                            pieces=self._pieces(batch))
         normed = space.get("gla_normed", rows, cv, x.dtype)
         kernels.gated_norm(read, normed, group=self.vdim, gate=proj[:, self.g_col0 : self.g_col0 + cv], act=kernels.GATE_SILU,
                            weight=self.norm, eps=self.eps * self.dim)

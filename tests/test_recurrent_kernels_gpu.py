@@ -132,6 +132,67 @@ def test_the_recurrence_over_steps_and_slots(kind, dim, vdim, heads, kv_heads):
         torch.testing.assert_close(torch.cat(got[i]).double(), want[i], rtol=2e-4, atol=2e-4)
 
 
+@pytest.mark.parametrize("kind", ["fixed", "per_token", "per_row", "bonus", "delta"])
+@pytest.mark.parametrize("dim,vdim", [(36, 44), (64, 64), (128, 128), (100, 132)])
+def test_prompts_walked_in_pieces(kind, dim, vdim):
+    """Entries of one piece, of exactly two, of five with a remainder and of a single token, from zeros and from a carried
+    state, in pieces against the walk from end to end (the same sums in another order) and its final states; and single tokens
+    of the same heads, alone and behind another entry, bit for bit as the walk takes them."""
+    from rapid_llm_b200.engine.batch import Workspace
+    from rapid_llm_b200.ops import kernels
+
+    heads, kv_heads = 4, 2
+    piece = kernels.scan_piece(heads, vdim, kind == "delta")
+    lengths, starts, slots = [4 * piece + 37, 1, piece, 2 * piece], [0, 9, 5, 700], [3, 1, 0, 2]
+    tokens = sum(lengths)
+    torch.manual_seed(dim)
+    q, k = torch.randn(tokens, kv_heads * dim, device=DEV) / dim ** 0.5, torch.randn(tokens, kv_heads * dim, device=DEV)
+    k = (k.view(tokens, kv_heads, dim) / k.view(tokens, kv_heads, dim).norm(dim=-1, keepdim=True)).reshape(tokens, -1).contiguous()
+    v, options = torch.randn(tokens, heads * vdim, device=DEV), {}
+    if kind == "fixed":
+        decay = torch.rand(heads, device=DEV) * 0.1 + 0.9
+    elif kind == "per_token":
+        decay = torch.rand(tokens, heads, device=DEV) * 0.1 + 0.9
+        options = {"v_scale": torch.rand(tokens, heads, device=DEV), "skip": torch.rand(heads, device=DEV)}
+    else:
+        decay = torch.rand(tokens, heads * dim, device=DEV) * 0.1 + 0.9
+        if kind == "bonus":
+            options = {"bonus": torch.randn(heads, dim, device=DEV)}
+        elif kind == "delta":
+            options = {"beta": torch.rand(tokens, heads, device=DEV)}
+    given = torch.randn(4, heads * dim * vdim, device=DEV) * 0.3
+    results = []
+    for pieces in (None, Workspace(64, torch.device(DEV))):
+        batch = _batch(lengths, slots, starts)
+        batch.max_query_len = max(lengths)
+        out, state = torch.empty(tokens, heads * vdim, device=DEV), given.clone()
+        kernels.linear_scan(q, k, v, decay, out, state, batch, heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, pieces=pieces, **options)
+        assert int(batch.fault.item()) == 0
+        results.append((out, state))
+    (walked, walked_state), (out, state) = results
+    # two float32 sums of over a thousand terms each, decayed to about 20 that count: 20 * 2^-24 of a value's size, ten-fold
+    size = float(walked.abs().max())
+    assert float((out - walked).abs().max()) <= 200 * 2.0 ** -24 * max(size, 1.0)
+    assert float((state - walked_state).abs().max()) <= 200 * 2.0 ** -24 * max(float(walked_state.abs().max()), 1.0)
+    if dim % 4 == 0 and vdim % 4 == 0:
+        per_token = {name: t for name, t in options.items() if t.shape[0] == tokens}
+        fixed = {name: t for name, t in options.items() if t.shape[0] != tokens}
+        rows = torch.tensor([3, 4 * piece + 37, 5], device=DEV)      # any three tokens, as single tokens and in an entry of two
+
+        def taken(index):
+            return (q[index].contiguous(), k[index].contiguous(), v[index].contiguous(), decay if kind == "fixed" else decay[index].contiguous(),
+                    {**fixed, **{name: t[index].contiguous() for name, t in per_token.items()}})
+
+        singles, mixed = [], []
+        for index, cut, into in ((rows, [1, 1, 1], singles), (torch.cat([rows, rows[:1]]), [1, 1, 2], mixed)):
+            a, b, c, d, more = taken(index)
+            batch = _batch(cut, [1, 2, 0], [4, 0, 8])
+            out, state = torch.empty(len(index), heads * vdim, device=DEV), given.clone()
+            kernels.linear_scan(a, b, c, d, out, state, batch, heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, **more)
+            into.extend([out[:3], state[1:3]])
+        assert all(torch.equal(one, other) for one, other in zip(singles, mixed))
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_norm_and_gate_in_their_three_orders(dtype):
     from rapid_llm_b200.ops import kernels
