@@ -42,6 +42,25 @@ __device__ __forceinline__ float2 load_pair<__nv_bfloat16>(const __nv_bfloat16* 
   return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
 }
 
+// Four neighbouring elements as floats, 8 or 16 bytes at once.
+__device__ __forceinline__ void load_four(const float* p, float (&v)[4]) {
+  const float4 four = *reinterpret_cast<const float4*>(p);
+  v[0] = four.x; v[1] = four.y; v[2] = four.z; v[3] = four.w;
+}
+__device__ __forceinline__ void load_four(const __nv_bfloat16* p, float (&v)[4]) {
+  const uint2 raw = *reinterpret_cast<const uint2*>(p);
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+  const float2 lo = __bfloat1622float2(h[0]), hi = __bfloat1622float2(h[1]);
+  v[0] = lo.x; v[1] = lo.y; v[2] = hi.x; v[3] = hi.y;
+}
+__device__ __forceinline__ void store_four(float* p, const float (&v)[4]) {
+  *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
+__device__ __forceinline__ void store_four(__nv_bfloat16* p, const float (&v)[4]) {
+  __nv_bfloat162 h[2] = {__floats2bfloat162_rn(v[0], v[1]), __floats2bfloat162_rn(v[2], v[3])};
+  *reinterpret_cast<uint2*>(p) = *reinterpret_cast<const uint2*>(h);
+}
+
 // A thread owns kLanes (1 or 2) neighbouring channels over kConvRows consecutive packed rows and slides the taps'
 // window down them, so a row of x is fetched once, not once per tap.  kLanes == 2 wants even C, col0 and x_stride.
 // kTaps > 0: the taps' number is known when compiling and the window lives in registers; 0: any number up to kMaxTaps.
@@ -196,6 +215,31 @@ __global__ void activate_rows_kernel(const T* x, int x_stride, int col0, float* 
     const int c = static_cast<int>(idx - t * C);
     const float v = to_float(x[static_cast<size_t>(t) * x_stride + col0 + c]);
     out[idx] = act ? silu_f(v) : v;
+  }
+}
+
+// The same for rows that can be fetched four columns at a time: four rows a thread, their loads in flight together.  Bound by
+// its bytes: 2,048 rows of 12,288, 16 bits in, 32 out, 81 -> 27 us (5.6 TB/s).
+constexpr int kActivateRows = 4;
+template <typename T>
+__global__ void __launch_bounds__(256) activate_rows_wide_kernel(const T* x, int x_stride, int col0, float* out, int tokens, int C,
+                                                                 int act) {
+  pdl_trigger();
+  const int c = (blockIdx.x * 256 + threadIdx.x) * 4, t0 = blockIdx.y * kActivateRows;
+  pdl_wait();
+  if (c >= C) return;
+  float v[kActivateRows][4];
+#pragma unroll
+  for (int i = 0; i < kActivateRows; ++i)
+    if (t0 + i < tokens) load_four(x + static_cast<size_t>(t0 + i) * x_stride + col0 + c, v[i]);
+#pragma unroll
+  for (int i = 0; i < kActivateRows; ++i) {
+    if (t0 + i >= tokens) break;
+    if (act) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[i][j] = silu_f(v[i][j]);
+    }
+    store_four(out + static_cast<size_t>(t0 + i) * C + c, v[i]);
   }
 }
 
@@ -439,6 +483,42 @@ __global__ void unit_heads_kernel(float* __restrict__ rows, int stride, int col0
   for (int i = threadIdx.x; i < gates; i += blockDim.x)
     gate_out[static_cast<size_t>(t) * gates + i] =
         sigmoid_f(to_float(gate_in[static_cast<size_t>(t) * gate_stride + gate_col0 + i]));
+}
+
+// The same with kLanes lanes of a warp per head, four entries a lane, read and written once; blocks behind the heads' form
+// the gates.  2,048 tokens, 32 heads of 128: 22.5 -> 17 us.
+template <typename T, int kLanes>
+__global__ void __launch_bounds__(256) unit_heads_wide_kernel(float* rows, int stride, int col0, int heads, int dim, float eps,
+                                                              int split, float scale_low, float scale_high, const T* gate_in,
+                                                              int gate_stride, int gate_col0, int gates, float* gate_out,
+                                                              int tokens, int head_blocks) {
+  pdl_trigger();
+  if (static_cast<int>(blockIdx.x) >= head_blocks) {
+    const long long idx = (static_cast<long long>(blockIdx.x) - head_blocks) * 256 + threadIdx.x;
+    pdl_wait();
+    if (idx >= static_cast<long long>(tokens) * gates) return;
+    const long long t = idx / gates;
+    const int i = static_cast<int>(idx - t * gates);
+    gate_out[idx] = sigmoid_f(to_float(gate_in[static_cast<size_t>(t) * gate_stride + gate_col0 + i]));
+    return;
+  }
+  const int lane = threadIdx.x % kLanes;
+  const long long index = blockIdx.x * static_cast<long long>(256 / kLanes) + threadIdx.x / kLanes;
+  const bool mine = index < static_cast<long long>(tokens) * heads;
+  const long long t = mine ? index / heads : 0;
+  const int head = mine ? static_cast<int>(index - t * heads) : 0;
+  float* p = rows + static_cast<size_t>(t) * stride + col0 + static_cast<size_t>(head) * dim + lane * 4;
+  const bool reads = mine && lane * 4 < dim;
+  pdl_wait();
+  float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  if (reads) load_four(p, v);
+  float sum_sq = v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + v[3] * v[3];
+#pragma unroll
+  for (int off = kLanes / 2; off >= 1; off >>= 1) sum_sq += __shfl_xor_sync(0xffffffffu, sum_sq, off);
+  const float factor = (head < split ? scale_low : scale_high) / sqrtf(sum_sq + eps);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) v[j] *= factor;
+  if (reads) store_four(p, v);
 }
 
 // ------------------------------------------------------------ rotation for heads without a cache
@@ -1354,85 +1434,118 @@ __global__ void gated_norm_kernel(const TY* y, int y_stride, const T* g, int g_s
   }
 }
 
-// The same with one warp per (token, group), for groups that are a multiple of 4 columns: four columns a lane and
-// step, no shared memory, no barrier; the second pass finds its rows in L1.
-template <typename TY, typename T>
-__global__ void gated_norm_warp_kernel(const TY* y, int y_stride, const T* g, int g_stride,
-                                       int g_col0, int act, int gate_first, int norm, const float* __restrict__ weight,
-                                       int weight_period, float eps, T* __restrict__ out, int group, int groups,
-                                       long long total, int wide) {
-  pdl_trigger();
-  pdl_wait();
-  const long long index = blockIdx.x * static_cast<long long>(blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (index >= total) return;
-  const int lane = threadIdx.x & 31;
-  const long long t = index / groups;
-  const int part = static_cast<int>(index - t * groups);
-  const TY* yr = y + static_cast<size_t>(t) * y_stride + static_cast<size_t>(part) * group;
-  const T* gr = (g && act != 0) ? g + static_cast<size_t>(t) * g_stride + g_col0 + static_cast<size_t>(part) * group : nullptr;
-  T* o = out + (static_cast<size_t>(t) * groups + part) * group;
-  auto load4 = [&](const auto* p, float (&v)[4]) {      // `wide`: every run of four starts on a vector's boundary
-    using E = std::remove_cv_t<std::remove_reference_t<decltype(*p)>>;
-    if (wide) {
-      if constexpr (sizeof(E) == 4) {
-        const float4 f = *reinterpret_cast<const float4*>(p);
-        v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
-      } else {
-        const uint2 raw = *reinterpret_cast<const uint2*>(p);
-        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
-        const float2 lo = __bfloat1622float2(h[0]), hi = __bfloat1622float2(h[1]);
-        v[0] = lo.x; v[1] = lo.y; v[2] = hi.x; v[3] = hi.y;
+// What the two kernels below share: a thread's columns (runs of four, `apart` columns from one to the next) and their gates,
+// read once, from the loads to the sum of squares and from the norm to the store.  `wide`: every run of four starts on a
+// vector's boundary.
+template <typename TY, typename T, int kPer>
+struct GatedColumns {
+  float z[kPer][4], gate[kPer][4];
+
+  __device__ __forceinline__ float take(const TY* yr, const T* gr, int first, int apart, int group, int act, int gate_first, int wide) {
+#pragma unroll
+    for (int p = 0; p < kPer; ++p) {
+      const int i = first + p * apart;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        z[p][j] = 0.0f;
+        gate[p][j] = 1.0f;
       }
-    } else {
+      if (i >= group) continue;
+      if (wide) {
+        load_four(yr + i, z[p]);
+        if (gr) load_four(gr + i, gate[p]);
+      } else {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) v[j] = to_float(p[j]);
+        for (int j = 0; j < 4; ++j) {
+          z[p][j] = to_float(yr[i + j]);
+          if (gr) gate[p][j] = to_float(gr[i + j]);
+        }
+      }
     }
-  };
-  auto four = [&](int i, float (&z)[4], float (&gate)[4]) {
-    load4(yr + i, z);
-    float raw[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    if (gr) load4(gr + i, raw);
+    float sum_sq = 0.0f;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      gate[j] = gr ? (act == 1 ? sigmoid_f(raw[j]) : silu_f(raw[j])) : 1.0f;
-      if (gate_first) z[j] *= gate[j];
+    for (int p = 0; p < kPer; ++p) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (gr) gate[p][j] = act == 1 ? sigmoid_f(gate[p][j]) : silu_f(gate[p][j]);
+        if (gate_first) z[p][j] *= gate[p][j];
+        sum_sq += z[p][j] * z[p][j];
+      }
     }
-  };
+    return sum_sq;
+  }
+  __device__ __forceinline__ void give(T* o, float inv, const float* weight, int weight_at, int weight_period, int first, int apart,
+                                       int group, int gate_first, int wide) {
+#pragma unroll
+    for (int p = 0; p < kPer; ++p) {
+      const int i = first + p * apart;
+      if (i >= group) break;
+      int at = weight ? (weight_at + i) % weight_period : 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        z[p][j] *= inv;
+        if (weight) {
+          z[p][j] *= weight[at];
+          at = at + 1 == weight_period ? 0 : at + 1;
+        }
+        if (!gate_first) z[p][j] *= gate[p][j];
+      }
+      if (wide) {
+        store_four(o + i, z[p]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o[i + j] = from_float<T>(z[p][j]);
+      }
+    }
+  }
+};
+
+// The same with kLanes lanes of a warp per (token, group), for groups of at most kLanes * 4 * kPer columns, a multiple of 4.
+// 2,048 tokens, us: 32 heads of 64 33 -> 15 (half a warp idled), 16 heads of 128 18 -> 15.
+template <typename TY, typename T, int kLanes, int kPer>
+__global__ void __launch_bounds__(256) gated_norm_warp_kernel(
+    const TY* y, int y_stride, const T* g, int g_stride, int g_col0, int act, int gate_first, int norm,
+    const float* __restrict__ weight, int weight_period, float eps, T* out, int group, int groups, long long total, int wide) {
+  pdl_trigger();
+  const int lane = threadIdx.x % kLanes;
+  const long long index = blockIdx.x * static_cast<long long>(256 / kLanes) + threadIdx.x / kLanes;
+  const bool mine = index < total;
+  const long long t = mine ? index / groups : 0;
+  const int part = mine ? static_cast<int>(index - t * groups) : 0;
+  const int columns = mine ? group : 0;
+  const T* gr = (g && act != 0) ? g + static_cast<size_t>(t) * g_stride + g_col0 + static_cast<size_t>(part) * group : nullptr;
+  GatedColumns<TY, T, kPer> own;
+  pdl_wait();
+  float sum_sq = own.take(y + static_cast<size_t>(t) * y_stride + static_cast<size_t>(part) * group, gr, lane * 4, kLanes * 4, columns,
+                          act, gate_first, wide);
   float inv = 1.0f;
   if (norm) {
-    float sum_sq = 0.0f;
-    for (int i = lane * 4; i < group; i += 128) {
-      float z[4], gate[4];
-      four(i, z, gate);
-      sum_sq += z[0] * z[0] + z[1] * z[1] + z[2] * z[2] + z[3] * z[3];
-    }
-    sum_sq = warp_sum(sum_sq);
+#pragma unroll
+    for (int off = kLanes / 2; off >= 1; off >>= 1) sum_sq += __shfl_xor_sync(0xffffffffu, sum_sq, off);
     inv = 1.0f / sqrtf(sum_sq / static_cast<float>(group) + eps);
   }
-  for (int i = lane * 4; i < group; i += 128) {
-    float z[4], gate[4];
-    four(i, z, gate);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      z[j] *= inv;
-      if (norm && weight) z[j] *= weight[(part * group + i + j) % weight_period];
-      if (!gate_first) z[j] *= gate[j];
-    }
-    if (wide) {
-      if constexpr (sizeof(T) == 4) {
-        *reinterpret_cast<float4*>(o + i) = make_float4(z[0], z[1], z[2], z[3]);
-      } else {
-        uint2 packed;
-        __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&packed);
-        h[0] = __floats2bfloat162_rn(z[0], z[1]);
-        h[1] = __floats2bfloat162_rn(z[2], z[3]);
-        *reinterpret_cast<uint2*>(o + i) = packed;
-      }
-    } else {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) o[i + j] = from_float<T>(z[j]);
-    }
-  }
+  const int weight_at = weight ? static_cast<int>(static_cast<long long>(part) * group % weight_period) : 0;
+  own.give(out + (static_cast<size_t>(t) * groups + part) * group, inv, norm ? weight : nullptr, weight_at, weight_period, lane * 4,
+           kLanes * 4, columns, gate_first, wide);
+}
+
+// One block per (token, group) for groups of thousands of columns, up to 256 * 4 * kPer.  2,048 rows of 4,096: 48 -> 21 us.
+template <typename TY, typename T, int kPer>
+__global__ void __launch_bounds__(256) gated_norm_row_kernel(
+    const TY* y, int y_stride, const T* g, int g_stride, int g_col0, int act, int gate_first, int norm,
+    const float* __restrict__ weight, int weight_period, float eps, T* out, int group, int groups) {
+  __shared__ float scratch[32];
+  pdl_trigger();
+  const int t = blockIdx.x, part = blockIdx.y, first = threadIdx.x * 4;
+  const T* gr = (g && act != 0) ? g + static_cast<size_t>(t) * g_stride + g_col0 + static_cast<size_t>(part) * group : nullptr;
+  GatedColumns<TY, T, kPer> own;
+  pdl_wait();
+  const float sum_sq = own.take(y + static_cast<size_t>(t) * y_stride + static_cast<size_t>(part) * group, gr, first, 1024, group, act,
+                                gate_first, 1);
+  const float inv = norm ? 1.0f / sqrtf(block_sum(sum_sq, scratch) / static_cast<float>(group) + eps) : 1.0f;
+  const int weight_at = weight ? static_cast<int>(static_cast<long long>(part) * group % weight_period) : 0;
+  own.give(out + (static_cast<size_t>(t) * groups + part) * group, inv, norm ? weight : nullptr, weight_at, weight_period, first, 1024,
+           group, gate_first, 1);
 }
 
 // ------------------------------------------------------------ xIELU
@@ -1493,6 +1606,42 @@ inline unsigned flat_blocks(long long total, int threads) {
 }  // namespace rl
 
 namespace rl {
+
+// A group of up to 512 columns takes the lanes of a warp that hold four columns each (a warp's part, so that no lane idles at
+// heads of 64 and 32), one of thousands a block; odd sizes go element by element.
+template <typename TY, typename T>
+static int launch_gated_norm(const TY* y, int y_stride, const T* g, int g_stride, int g_col0, int act, int gate_first, int norm,
+                             const float* weight, int weight_period, float eps, T* out, int tokens, int group, int groups,
+                             int pdl, cudaStream_t stream) {
+  const bool wide = ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(out)) & 15) == 0 &&
+                    y_stride % 4 == 0 && g_stride % 4 == 0 && g_col0 % 4 == 0;
+  const long long total = static_cast<long long>(tokens) * groups;
+  auto warps = [&](auto kernel, int lanes) {
+    const long long per = 256 / lanes;
+    return launch_kernel(kernel, dim3(static_cast<unsigned>((total + per - 1) / per)), dim3(256), 0, stream, pdl != 0, y, y_stride,
+                         g, g_stride, g_col0, act, gate_first, norm, weight, weight_period, eps, out, group, groups, total,
+                         static_cast<int>(wide));
+  };
+  if (group % 4 == 0 && group <= 512) {
+    if (group <= 32) return warps(gated_norm_warp_kernel<TY, T, 8, 1>, 8);
+    if (group <= 64) return warps(gated_norm_warp_kernel<TY, T, 16, 1>, 16);
+    if (group <= 128) return warps(gated_norm_warp_kernel<TY, T, 32, 1>, 32);
+    if (group <= 256) return warps(gated_norm_warp_kernel<TY, T, 32, 2>, 32);
+    return warps(gated_norm_warp_kernel<TY, T, 32, 4>, 32);
+  }
+  auto rows = [&](auto kernel, int threads) {
+    return launch_kernel(kernel, dim3(tokens, groups), dim3(threads), 0, stream, pdl != 0, y, y_stride, g, g_stride, g_col0, act,
+                         gate_first, norm, weight, weight_period, eps, out, group, groups);
+  };
+  if (group % 4 == 0 && wide && group <= 8192) {
+    if (group <= 2048) return rows(gated_norm_row_kernel<TY, T, 2>, 256);
+    if (group <= 4096) return rows(gated_norm_row_kernel<TY, T, 4>, 256);
+    return rows(gated_norm_row_kernel<TY, T, 8>, 256);
+  }
+  int threads = 32;
+  while (threads < 256 && threads * 2 <= group) threads *= 2;
+  return rows(gated_norm_kernel<TY, T>, threads);
+}
 
 template <int kRows, int kPartners, int kCols, int kKind, bool kRowDecay, bool kRead = true>
 static int launch_scan(ScanArgs a, int blocks, int pdl, cudaStream_t stream) {
@@ -1592,7 +1741,13 @@ int rl_activate_rows(int dtype, const void* x, int x_stride, int col0, float* ou
                      int pdl, cudaStream_t stream) {
   if (tokens == 0 || channels == 0) return 0;
   if (act < 0 || act > 1) return static_cast<int>(cudaErrorInvalidValue);
+  const int row_blocks = (tokens + rl::kActivateRows - 1) / rl::kActivateRows;
+  const bool wide = channels % 4 == 0 && col0 % 4 == 0 && x_stride % 4 == 0 && row_blocks <= 65535 &&
+                    ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
   RL_DISPATCH_DTYPE(dtype, {
+    if (wide)
+      return rl::launch_kernel(rl::activate_rows_wide_kernel<scalar_t>, dim3((channels + 1023) / 1024, row_blocks), dim3(256), 0,
+                               stream, pdl != 0, static_cast<const scalar_t*>(x), x_stride, col0, out, tokens, channels, act);
     return rl::launch_kernel(rl::activate_rows_kernel<scalar_t>,
                              dim3(rl::flat_blocks(static_cast<long long>(tokens) * channels, 256)), dim3(256), 0, stream,
                              pdl != 0, static_cast<const scalar_t*>(x), x_stride, col0, out, tokens, channels, act);
@@ -1674,7 +1829,19 @@ int rl_unit_heads(int dtype, float* rows, int stride, int col0, int heads, int d
                   float scale_low, float scale_high, const void* gate_in, int gate_stride, int gate_col0, int gates,
                   float* gate_out, int tokens, int pdl, cudaStream_t stream) {
   if (tokens == 0) return 0;
+  const bool wide = dim % 4 == 0 && dim <= 128 && heads > 0 && stride % 4 == 0 && col0 % 4 == 0 && (reinterpret_cast<uintptr_t>(rows) & 15) == 0;
   RL_DISPATCH_DTYPE(dtype, {
+    if (wide) {
+      const int lanes = dim <= 32 ? 8 : dim <= 64 ? 16 : 32, per = 256 / lanes;
+      const long long head_blocks = (static_cast<long long>(tokens) * heads + per - 1) / per;
+      const long long gate_blocks = (static_cast<long long>(tokens) * gates + 255) / 256;
+      auto kernel = lanes == 8 ? rl::unit_heads_wide_kernel<scalar_t, 8>
+                               : lanes == 16 ? rl::unit_heads_wide_kernel<scalar_t, 16> : rl::unit_heads_wide_kernel<scalar_t, 32>;
+      return rl::launch_kernel(kernel, dim3(static_cast<unsigned>(head_blocks + gate_blocks)), dim3(256), 0, stream, pdl != 0,
+                               rows, stride, col0, heads, dim, eps, split, scale_low, scale_high,
+                               static_cast<const scalar_t*>(gate_in), gate_stride, gate_col0, gates, gate_out, tokens,
+                               static_cast<int>(head_blocks));
+    }
     return rl::launch_kernel(rl::unit_heads_kernel<scalar_t>, dim3(tokens), dim3(128), 0, stream, pdl != 0, rows,
                              stride, col0, heads, dim, eps, split, scale_low, scale_high,
                              static_cast<const scalar_t*>(gate_in), gate_stride, gate_col0, gates, gate_out, tokens);
@@ -1772,38 +1939,14 @@ int rl_gated_norm(int dtype, int y_f32, const void* y, int y_stride, const void*
   if (tokens == 0 || groups == 0) return 0;
   if (group < 1 || act < 0 || act > 2 || (weight != nullptr && weight_period < 1))
     return static_cast<int>(cudaErrorInvalidValue);
-  int threads = 32;
-  while (threads < 256 && threads * 2 <= group) threads *= 2;
-  const dim3 grid(tokens, groups), block(threads);
-  // a warp per (token, group) while a group is a warp's work; a group of thousands of columns (one norm over all
-  // heads) takes a block, or the few warps of a small step would each walk it alone
-  if (group % 4 == 0 && group <= 512) {
-    const long long total = static_cast<long long>(tokens) * groups;
-    const dim3 warp_grid(static_cast<unsigned>((total + 7) / 8)), warp_block(256);
-    const bool wide = ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(out)) & 15) == 0 &&
-                      y_stride % 4 == 0 && g_stride % 4 == 0 && g_col0 % 4 == 0;
-    RL_DISPATCH_DTYPE(dtype, {
-      if (y_f32)
-        return rl::launch_kernel(rl::gated_norm_warp_kernel<float, scalar_t>, warp_grid, warp_block, 0, stream, pdl != 0,
-                                 static_cast<const float*>(y), y_stride, static_cast<const scalar_t*>(g), g_stride,
-                                 g_col0, act, gate_first, norm, weight, weight_period, eps,
-                                 static_cast<scalar_t*>(out), group, groups, total, static_cast<int>(wide));
-      return rl::launch_kernel(rl::gated_norm_warp_kernel<scalar_t, scalar_t>, warp_grid, warp_block, 0, stream, pdl != 0,
-                               static_cast<const scalar_t*>(y), y_stride, static_cast<const scalar_t*>(g), g_stride,
-                               g_col0, act, gate_first, norm, weight, weight_period, eps,
-                               static_cast<scalar_t*>(out), group, groups, total, static_cast<int>(wide));
-    });
-  }
   RL_DISPATCH_DTYPE(dtype, {
     if (y_f32)
-      return rl::launch_kernel(rl::gated_norm_kernel<float, scalar_t>, grid, block, 0, stream, pdl != 0,
-                               static_cast<const float*>(y), y_stride, static_cast<const scalar_t*>(g), g_stride,
-                               g_col0, act, gate_first, norm, weight, weight_period, eps, static_cast<scalar_t*>(out),
-                               group, groups);
-    return rl::launch_kernel(rl::gated_norm_kernel<scalar_t, scalar_t>, grid, block, 0, stream, pdl != 0,
-                             static_cast<const scalar_t*>(y), y_stride, static_cast<const scalar_t*>(g), g_stride,
-                             g_col0, act, gate_first, norm, weight, weight_period, eps, static_cast<scalar_t*>(out),
-                             group, groups);
+      return rl::launch_gated_norm<float, scalar_t>(static_cast<const float*>(y), y_stride, static_cast<const scalar_t*>(g),
+                                                    g_stride, g_col0, act, gate_first, norm, weight, weight_period, eps,
+                                                    static_cast<scalar_t*>(out), tokens, group, groups, pdl, stream);
+    return rl::launch_gated_norm<scalar_t, scalar_t>(static_cast<const scalar_t*>(y), y_stride, static_cast<const scalar_t*>(g),
+                                                     g_stride, g_col0, act, gate_first, norm, weight, weight_period, eps,
+                                                     static_cast<scalar_t*>(out), tokens, group, groups, pdl, stream);
   });
   return 0;
 }

@@ -223,6 +223,38 @@ def test_norm_and_gate_in_their_three_orders(dtype):
     torch.testing.assert_close(out.double().cpu(), rows.double() * torch.sigmoid(g), rtol=1e-2 if dtype == torch.bfloat16 else 1e-6, atol=1e-6)
 
 
+@pytest.mark.parametrize("group,groups", [(4, 3), (32, 5), (36, 2), (64, 7), (128, 2), (132, 3), (512, 2), (516, 1), (2048, 2), (4100, 1), (8192, 1), (8196, 1)])
+def test_norms_and_unit_vectors_at_the_edges_of_their_groups(group, groups):
+    """Each number of lanes, columns a lane and block size of the gated norm, the sizes behind them, on rows that start on a
+    vector's boundary and on rows that do not; unit vectors and plain activations of the same sizes."""
+    from rapid_llm_b200.ops import kernels
+
+    torch.manual_seed(group)
+    tokens, width = 9, group * groups
+    for shift in (0, 1):
+        wide_y = torch.randn(tokens, width + 4, device=DEV)
+        wide_g = torch.randn(tokens, width + 4, device=DEV).to(torch.bfloat16)
+        y, gate = wide_y[:, shift : shift + width], wide_g[:, shift : shift + width]
+        weight = torch.randn(width, device=DEV)
+        out = torch.empty(tokens, width, dtype=torch.bfloat16, device=DEV)
+        kernels.gated_norm(y, out, group=group, gate=gate, act=kernels.GATE_SILU, weight=weight, eps=1e-5)
+        want = (unit_rms(y.double().cpu().reshape(tokens, groups, group), 1e-5).reshape(tokens, width) * weight.double().cpu()
+                * silu(gate.double().cpu()))
+        torch.testing.assert_close(out.double().cpu(), want, rtol=2.0 ** -8, atol=1e-5)      # half a step of bfloat16, twice
+        plain = kernels.activate_rows(gate, torch.empty(tokens, width, device=DEV), act=True)
+        torch.testing.assert_close(plain.double().cpu(), silu(gate.double().cpu()), rtol=1e-5, atol=1e-6)
+        if group <= 512:
+            rows = wide_y.clone()
+            raw, beta = torch.randn(tokens, 3, device=DEV).to(torch.bfloat16), torch.empty(tokens, 3, device=DEV)
+            kernels.unit_heads(rows[:, shift : shift + width], heads=groups, dim=group, eps=1e-6, split=1, scale_low=0.5, scale_high=2.0,
+                               gate_in=raw, gate_out=beta)
+            v = y.double().cpu().reshape(tokens, groups, group)
+            v = v / torch.sqrt((v * v).sum(-1, keepdim=True) + 1e-6) * torch.tensor([0.5] + [2.0] * (groups - 1)).view(1, -1, 1)
+            torch.testing.assert_close(rows[:, shift : shift + width].double().cpu(), v.reshape(tokens, width), rtol=1e-5, atol=1e-6)
+            torch.testing.assert_close(beta.double().cpu(), torch.sigmoid(raw.double().cpu()), rtol=1e-5, atol=1e-6)
+            assert torch.equal(rows[:, shift + width :], wide_y[:, shift + width :])
+
+
 def test_activation_decays_unit_heads_and_rotation():
     from rapid_llm_b200.ops import kernels
 
