@@ -24,9 +24,10 @@
 // A row's result does not depend on its tile's other rows or on the order in which the pairs of an
 // expert were laid out: the inner sums run over k in a fixed order per row.
 //
-// Three product kernels: float32 FMA tiles (the 32-bit engine; any sizes), mma.sync m16n8k16 tiles for
-// bfloat16 (float32 accumulators; any sizes), and the same instruction behind a cp.async ring with
-// ldmatrix fragments on tiles of 64 pairs for bfloat16 operands whose rows are multiples of 16 bytes.
+// Five product kernels: float32 FMA tiles (the 32-bit engine; any sizes), mma.sync m16n8k16 tiles for
+// bfloat16 (float32 accumulators; any sizes), and for bfloat16 operands whose rows are multiples of 16 bytes: the same
+// instruction with the weights straight from memory on tiles of 16 pairs (few pairs: bound by the weights' stream),
+// behind a cp.async ring with ldmatrix fragments on tiles of 64 pairs, and tcgen05 on tiles of 128 (moe_tc.cu).
 // The plan is made for the tile the product kernels will use (`tile_m`).
 #include "common.cuh"
 
@@ -39,6 +40,13 @@ constexpr int kMoeThreads = 256;
 constexpr int kMoeWideM = 64;     // pairs per tile of the pipelined bfloat16 kernel
 constexpr int kMoeWideK = 64;
 constexpr int kMoeStages = 3;
+constexpr int kMoeFewM = 16;      // pairs per tile of the kernel for few pairs
+constexpr int kMoeTensorM = 128;  // pairs per tile of the tensor cores' kernel
+
+// moe_tc.cu
+int grouped_linear_tc(const void* a, int a_stride, const void* w, int experts, const int* sorted, const int* meta,
+                      const float* pair_weight, int top, int by_token, int n, int k, int gated, void* out_act, float* out_y,
+                      int most_tiles, float glu_limit, float glu_alpha, int* fault, int pdl, cudaStream_t stream);
 
 __device__ __forceinline__ float moe_sigmoid(float x) { return 1.0f / (1.0f + expf(-x)); }
 
@@ -274,36 +282,58 @@ __global__ void moe_plan_kernel(const int* __restrict__ ids, int pairs, int expe
   for (int e = threadIdx.x; e < experts; e += blockDim.x) counts[e] = 0;
   pdl_wait();
   __syncthreads();
-  for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
-    const int e = ids[i];
-    if (e >= 0 && e < experts) atomicAdd(&counts[e], 1);
+  // a warp's pairs of one expert count at once: one addition to shared memory for all of them
+  const int lane = threadIdx.x & 31;
+  auto claim = [&](int* table, int e) {
+    const unsigned same = __match_any_sync(0xffffffffu, e);
+    const int leader = __ffs(same) - 1;
+    int at = 0;
+    if (lane == leader && e >= 0) at = atomicAdd(&table[e], __popc(same));
+    return __shfl_sync(0xffffffffu, at, leader) + __popc(same & ((1u << lane) - 1u));
+  };
+  const int rounded = (pairs + blockDim.x - 1) / blockDim.x * blockDim.x;      // whole warps take part
+  for (int i = threadIdx.x; i < rounded; i += blockDim.x) {
+    const int id = i < pairs ? ids[i] : -1;
+    claim(counts, id >= 0 && id < experts ? id : -1);
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {
+    // 32 experts at a time: where each one's pairs and tiles start, by sums over the lanes
     int at = 0, tiles = 0;
-    for (int e = 0; e < experts; ++e) {
-      cursor[e] = at;
-      for (int row = 0; row < counts[e]; row += tile_m) {
-        if (tiles < max_tiles) {
-          meta[1 + 3 * tiles] = e;
-          meta[2 + 3 * tiles] = at + row;
-          meta[3 + 3 * tiles] = min(tile_m, counts[e] - row);
+    for (int e0 = 0; e0 < experts; e0 += 32) {
+      const int e = e0 + lane, count = e < experts ? counts[e] : 0, own = (count + tile_m - 1) / tile_m;
+      int place = count, tile = own;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int p = __shfl_up_sync(0xffffffffu, place, off), t = __shfl_up_sync(0xffffffffu, tile, off);
+        if (lane >= off) {
+          place += p;
+          tile += t;
         }
-        ++tiles;
       }
-      at += counts[e];
+      const int first = at + place - count, first_tile = tiles + tile - own;
+      if (e < experts) cursor[e] = first;
+      for (int i = 0; i < own && first_tile + i < max_tiles; ++i) {
+        meta[1 + 3 * (first_tile + i)] = e;
+        meta[2 + 3 * (first_tile + i)] = first + i * tile_m;
+        meta[3 + 3 * (first_tile + i)] = min(tile_m, count - i * tile_m);
+      }
+      at += __shfl_sync(0xffffffffu, place, 31);
+      tiles += __shfl_sync(0xffffffffu, tile, 31);
     }
-    if (tiles > max_tiles) {
-      atomicOr(fault, kFaultSlot);
-      tiles = max_tiles;
+    if (lane == 0) {
+      if (tiles > max_tiles) {
+        atomicOr(fault, kFaultSlot);
+        tiles = max_tiles;
+      }
+      meta[0] = tiles;
     }
-    meta[0] = tiles;
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
-    const int e = ids[i];
-    if (e < 0 || e >= experts) continue;
-    const int p = atomicAdd(&cursor[e], 1);
+  for (int i = threadIdx.x; i < rounded; i += blockDim.x) {
+    const int id = i < pairs ? ids[i] : -1, e = id >= 0 && id < experts ? id : -1;
+    const int p = claim(cursor, e);
+    if (e < 0) continue;
     sorted[p] = i;
     place_of[i] = p;
   }
@@ -682,7 +712,185 @@ grouped_linear_wide_kernel(const __nv_bfloat16* a, int a_stride, const __nv_bflo
   }
 }
 
+// ------------------------------------------------------------------ few pairs
+// Tiles of up to 16 pairs: bound by the weights' stream, and before that by how much of it is on its way.  A block owns 32
+// weight rows (gated: 16 gate rows and the 16 up rows beside them), its eight warps share the inner range, and a lane
+// fetches eight neighbouring columns of its rows 16 bytes at a time straight into the product's fragments: with the
+// columns of 32 renamed (lane q of four holds columns 8 q .. 8 q + 7, which serve as columns 2 q, 2 q + 1, 2 q + 8, 2 q + 9
+// of two instructions) both operands are read as they lie.  The pairs' rows wait in shared memory.  The warps' partial sums
+// are added in the order of the inner range, so an output does not depend on its tile.
+constexpr int kMoeFewWarps = 8;
+constexpr int kMoeFewAhead = 4;      // steps of 32 columns on their way per warp
+
+template <bool kGated, int kNt>
+__global__ void __launch_bounds__(kMoeFewWarps * 32)
+grouped_linear_few_kernel(const __nv_bfloat16* a, int a_stride, const __nv_bfloat16* __restrict__ w, const int* sorted,
+                          const int* meta, const float* pair_weight, int top, int by_token, int n, int k,
+                          __nv_bfloat16* out_act, float* out_y, float glu_limit, float glu_alpha) {
+  extern __shared__ __align__(16) unsigned char moe_few_smem[];
+  constexpr int kPairs = 8 * kNt;
+  __shared__ int s_pair[kPairs];
+  __shared__ float partial[kMoeFewWarps][2][16][kPairs + 1];
+  const int steps = (k + 31) / 32, stride = steps * 32 + 32;      // 64 bytes between rows' ends: neighbouring rows meet in no bank
+  __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(moe_few_smem);
+  pdl_trigger();
+  pdl_wait();
+  const int tile = blockIdx.y;
+  if (tile >= meta[0]) return;
+  const int expert = meta[1 + 3 * tile], place0 = meta[2 + 3 * tile], rows = meta[3 + 3 * tile];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int n0 = blockIdx.x * (kGated ? 16 : 32);
+  if (tid < kPairs) s_pair[tid] = tid < rows ? sorted[place0 + tid] : -1;
+  __syncthreads();
+  for (int idx = tid; idx < kPairs * steps * 4; idx += kMoeFewWarps * 32) {
+    const int r = idx / (steps * 4), c = (idx - r * (steps * 4)) * 8;
+    const int pair = s_pair[r];
+    const bool ok = pair >= 0 && c < k;
+    const size_t row = ok ? (by_token ? static_cast<size_t>(pair / top) : static_cast<size_t>(place0 + r)) : 0;
+    moe_cp_async16(xs + r * stride + c, ok ? a + row * a_stride + c : a, ok);
+  }
+  asm volatile("cp.async.commit_group;\n" ::);
+  // rows g and g + 8 of both groups of sixteen; q: which eight columns of a step
+  const int g = lane >> 2, q = lane & 3;
+  const size_t w_rows = kGated ? 2 * static_cast<size_t>(n) : static_cast<size_t>(n);
+  const __nv_bfloat16* we = w + static_cast<size_t>(expert) * w_rows * k;
+  const __nv_bfloat16* from[2][2];
+  bool live[2][2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int col = n0 + g + 8 * i + (kGated ? 0 : 16 * h);
+      live[h][i] = col < n;
+      from[h][i] = we + (static_cast<size_t>(live[h][i] ? col : 0) + (kGated && h ? n : 0)) * k + q * 8;
+    }
+  }
+  const int per = (steps + kMoeFewWarps - 1) / kMoeFewWarps, begin = warp * per, end = min(steps, begin + per);
+  float acc[2][kNt][4];
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int nt = 0; nt < kNt; ++nt)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[h][nt][c] = 0.0f;
+  uint4 ahead[kMoeFewAhead][2][2];
+  auto fetch = [&](uint4 (&to)[2][2], int step) {
+    const bool inside = step < end && step * 32 + q * 8 < k;
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        to[h][i] = inside && live[h][i] ? __ldg(reinterpret_cast<const uint4*>(from[h][i] + step * 32)) : make_uint4(0u, 0u, 0u, 0u);
+  };
+#pragma unroll
+  for (int s = 0; s < kMoeFewAhead; ++s) fetch(ahead[s], begin + s);
+  asm volatile("cp.async.wait_group 0;\n" ::);
+  __syncthreads();
+  for (int step0 = begin; step0 < end; step0 += kMoeFewAhead) {
+#pragma unroll
+    for (int s = 0; s < kMoeFewAhead; ++s) {
+      const int step = step0 + s;
+      if (step < end) {
+        uint4 x4[kNt];
+#pragma unroll
+        for (int nt = 0; nt < kNt; ++nt)
+          x4[nt] = *reinterpret_cast<const uint4*>(xs + (nt * 8 + g) * stride + step * 32 + q * 8);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const uint4 lo = ahead[s][h][0], hi = ahead[s][h][1];
+          const uint32_t first[4] = {lo.x, hi.x, lo.y, hi.y}, second[4] = {lo.z, hi.z, lo.w, hi.w};
+#pragma unroll
+          for (int nt = 0; nt < kNt; ++nt) {
+            moe_mma_bf16(acc[h][nt], first, x4[nt].x, x4[nt].y);
+            moe_mma_bf16(acc[h][nt], second, x4[nt].z, x4[nt].w);
+          }
+        }
+        fetch(ahead[s], step + kMoeFewAhead);
+      }
+    }
+  }
+  // accumulator: rows g, g + 8 of the weights; pairs 2 q, 2 q + 1 of a group of eight
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int nt = 0; nt < kNt; ++nt)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) partial[warp][h][g + 8 * (c >> 1)][nt * 8 + 2 * q + (c & 1)] = acc[h][nt][c];
+  __syncthreads();
+  for (int idx = tid; idx < 16 * kPairs; idx += kMoeFewWarps * 32) {
+    const int r = idx & 15, p = idx >> 4, pair = s_pair[p];
+    if (pair < 0) continue;
+    float sum[2] = {0.0f, 0.0f};
+#pragma unroll
+    for (int s = 0; s < kMoeFewWarps; ++s) {
+      sum[0] += partial[s][0][r][p];
+      sum[1] += partial[s][1][r][p];
+    }
+    const int col = n0 + r;
+    if constexpr (kGated) {
+      const float scale = pair_weight ? pair_weight[pair] : 1.0f;
+      if (col < n)
+        out_act[static_cast<size_t>(place0 + p) * n + col] = __float2bfloat16_rn(moe_unit(sum[0] * scale, sum[1] * scale, glu_limit, glu_alpha));
+    } else {
+      if (col < n) out_y[static_cast<size_t>(pair) * n + col] = sum[0];
+      if (col + 16 < n) out_y[static_cast<size_t>(pair) * n + col + 16] = sum[1];
+    }
+  }
+}
+
 // ------------------------------------------------------------------ combine
+// Four columns a thread and access where the row length and the addresses allow it: bound by its bytes.
+template <typename T>
+__global__ void __launch_bounds__(256) moe_combine_wide_kernel(const float* y, int top, const T* shared, const float* gate,
+                                                               int gate_stride, T* out, int tokens, int hidden, const float* weights,
+                                                               const int* ids, int experts, const T* x, int x_stride) {
+  pdl_trigger();
+  const int c = (blockIdx.x * 256 + threadIdx.x) * 4, t = blockIdx.y;
+  pdl_wait();
+  if (c >= hidden) return;
+  float own[4] = {0.0f, 0.0f, 0.0f, 0.0f}, sum[4] = {0.0f, 0.0f, 0.0f, 0.0f}, also[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  auto four = [](const T* p, float (&v)[4]) {
+    if constexpr (sizeof(T) == 2) {
+      const uint2 raw = *reinterpret_cast<const uint2*>(p);
+      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+      const float2 lo = __bfloat1622float2(h[0]), hi = __bfloat1622float2(h[1]);
+      v[0] = lo.x; v[1] = lo.y; v[2] = hi.x; v[3] = hi.y;
+    } else {
+      const float4 f = *reinterpret_cast<const float4*>(p);
+      v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+    }
+  };
+  // a choice at or behind `experts` is an identity expert: its result is the token's own row, and no tile wrote y
+  if (ids) four(x + static_cast<size_t>(t) * x_stride + c, own);
+  if (shared) four(shared + static_cast<size_t>(t) * hidden + c, also);
+  for (int j = 0; j < top; ++j) {
+    const size_t pair = static_cast<size_t>(t) * top + j;
+    float v[4];
+    if (ids && ids[pair] >= experts) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[i] = own[i];
+    } else {
+      const float4 f = *reinterpret_cast<const float4*>(y + pair * hidden + c);
+      v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+    }
+    const float weight = weights ? weights[pair] : 1.0f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sum[i] = weights ? fmaf(weight, v[i], sum[i]) : sum[i] + v[i];
+  }
+  if (shared) {
+    const float by = gate ? gate[static_cast<size_t>(t) * gate_stride] : 1.0f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sum[i] += by * also[i];
+  }
+  T* o = out + static_cast<size_t>(t) * hidden + c;
+  if constexpr (sizeof(T) == 2) {
+    const __nv_bfloat162 h[2] = {__floats2bfloat162_rn(sum[0], sum[1]), __floats2bfloat162_rn(sum[2], sum[3])};
+    *reinterpret_cast<uint2*>(o) = *reinterpret_cast<const uint2*>(h);
+  } else {
+    *reinterpret_cast<float4*>(o) = make_float4(sum[0], sum[1], sum[2], sum[3]);
+  }
+}
+
 template <typename T>
 __global__ void moe_combine_kernel(const float* __restrict__ y, int top, const T* shared, const float* __restrict__ gate,
                                    int gate_stride, T* __restrict__ out, int tokens, int hidden, const float* weights,
@@ -758,7 +966,10 @@ __global__ void moe_combine_layernorm_kernel(const float* __restrict__ y, int to
 
 extern "C" {
 
-int rl_moe_tile_rows(int wide) { return wide ? rl::kMoeWideM : rl::kMoeTileM; }
+// kind 0: the plain tiles, 1: the pipelined bfloat16 ones, 2: few pairs, 3: the tensor cores'
+int rl_moe_tile_rows(int kind) {
+  return kind == 3 ? rl::kMoeTensorM : kind == 2 ? rl::kMoeFewM : kind == 1 ? rl::kMoeWideM : rl::kMoeTileM;
+}
 
 int rl_router_topk(int dtype, const void* x, int x_stride, const float* w, int hidden, int experts, int gates, int top,
                    int* ids, float* weights, float* gate_out, float* scores_out, int tokens, const float* bias,
@@ -797,7 +1008,7 @@ int rl_moe_plan(const int* ids, int pairs, int experts, int* sorted, int* place_
                 int tile_m, int* fault, int pdl, cudaStream_t stream) {
   if (pairs == 0) return 0;
   const size_t smem = 2 * static_cast<size_t>(experts) * sizeof(int);
-  if (experts < 1 || smem > 48 * 1024 || max_tiles < 1 || (tile_m != rl::kMoeTileM && tile_m != rl::kMoeWideM))
+  if (experts < 1 || smem > 48 * 1024 || max_tiles < 1 || (tile_m != rl::kMoeTileM && tile_m != rl::kMoeWideM && tile_m != rl::kMoeFewM && tile_m != rl::kMoeTensorM))
     return static_cast<int>(cudaErrorInvalidValue);
   return rl::launch_kernel(rl::moe_plan_kernel, dim3(1), dim3(1024), smem, stream, pdl != 0, ids, pairs, experts,
                            sorted, place_of, meta, max_tiles, tile_m, fault);
@@ -829,7 +1040,7 @@ extern "C" {
 // tile_m: the rows of a tile the plan was made with; kMoeWideM selects the pipelined bfloat16 kernel.
 int rl_grouped_linear(int dtype, const void* a, int a_stride, const void* w, const int* sorted, const int* meta,
                       const float* pair_weight, int top, int by_token, int n, int k, int gated, void* out_act,
-                      float* out_y, int max_tiles, int tile_m, float glu_limit, float glu_alpha, int pdl,
+                      float* out_y, int max_tiles, int tile_m, float glu_limit, float glu_alpha, int experts, int* fault, int pdl,
                       cudaStream_t stream) {
   if (max_tiles == 0) return 0;
   if (tile_m == rl::kMoeWideM) {
@@ -845,6 +1056,26 @@ int rl_grouped_linear(int dtype, const void* a, int a_stride, const void* w, con
     return launch_grouped_wide<false>(wide_grid, stream, pdl != 0, static_cast<const bf*>(a), a_stride,
                                       static_cast<const bf*>(w), sorted, meta, pair_weight, top, by_token, n, k,
                                       static_cast<bf*>(out_act), out_y, glu_limit, glu_alpha);
+  }
+  if (tile_m == rl::kMoeFewM || tile_m == rl::kMoeTensorM) {
+    using bf = __nv_bfloat16;
+    if (dtype != rl::kBF16 || (gated ? out_act == nullptr : out_y == nullptr)) return static_cast<int>(cudaErrorInvalidValue);
+    if (tile_m == rl::kMoeTensorM)
+      return rl::grouped_linear_tc(a, a_stride, w, experts, sorted, meta, pair_weight, top, by_token, n, k, gated, out_act, out_y,
+                                   max_tiles, glu_limit, glu_alpha, fault, pdl, stream);
+    const size_t smem = static_cast<size_t>(rl::kMoeFewM) * ((k + 31) / 32 * 32 + 32) * sizeof(bf);
+    if (k % 8 != 0 || a_stride % 8 != 0 || n < 1 || k < 1 || top < 1 || max_tiles > 65535 || smem > 200 * 1024 ||
+        ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) & 15) != 0)
+      return static_cast<int>(cudaErrorInvalidValue);
+    auto kernel = gated ? rl::grouped_linear_few_kernel<true, 2> : rl::grouped_linear_few_kernel<false, 2>;
+    if (smem > 30 * 1024) {      // with its own 17 KB beyond what a kernel has without asking
+      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+      if (e != cudaSuccess) return static_cast<int>(e);
+    }
+    const int columns = gated ? 16 : 32;
+    return rl::launch_kernel(kernel, dim3((n + columns - 1) / columns, max_tiles), dim3(rl::kMoeFewWarps * 32), smem, stream, pdl != 0,
+                             static_cast<const bf*>(a), a_stride, static_cast<const bf*>(w), sorted, meta, pair_weight, top, by_token,
+                             n, k, static_cast<bf*>(out_act), out_y, glu_limit, glu_alpha);
   }
   if (tile_m != rl::kMoeTileM) return static_cast<int>(cudaErrorInvalidValue);
   if (n < 1 || k < 1 || top < 1 || (gated && out_act == nullptr) || (!gated && out_y == nullptr) || max_tiles > 65535)
@@ -880,7 +1111,14 @@ int rl_moe_combine(int dtype, const float* y, int top, const void* shared, const
   const long long total = static_cast<long long>(tokens) * hidden;
   long long blocks = (total + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
+  const bool wide = hidden % 4 == 0 && tokens <= 65535 && (ids == nullptr || x_stride % 4 == 0) &&
+                    ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(shared) | reinterpret_cast<uintptr_t>(out) |
+                      reinterpret_cast<uintptr_t>(x)) & 15) == 0;
   RL_DISPATCH_DTYPE(dtype, {
+    if (wide)
+      return rl::launch_kernel(rl::moe_combine_wide_kernel<scalar_t>, dim3((hidden + 1023) / 1024, tokens), dim3(256), 0, stream,
+                               pdl != 0, y, top, static_cast<const scalar_t*>(shared), gate, gate_stride, static_cast<scalar_t*>(out),
+                               tokens, hidden, weights, ids, experts, static_cast<const scalar_t*>(x), x_stride);
     return rl::launch_kernel(rl::moe_combine_kernel<scalar_t>, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, stream,
                              pdl != 0, y, top, static_cast<const scalar_t*>(shared), gate, gate_stride,
                              static_cast<scalar_t*>(out), tokens, hidden, weights, ids, experts,

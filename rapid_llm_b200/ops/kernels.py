@@ -1556,7 +1556,7 @@ def moe_lib() -> ctypes.CDLL:
         lib.rl_moe_tile_rows.argtypes = [c_int]
         lib.rl_grouped_linear.argtypes = [c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
                                           c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_float, c_float, c_int,
-                                          c_void_p]
+                                          c_void_p, c_int, c_void_p]
         lib.rl_moe_combine.argtypes = [c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p,
                                        c_void_p, c_int, c_void_p, c_int, c_int, c_void_p]
         lib.rl_moe_combine_layernorm.argtypes = [c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p,
@@ -1568,17 +1568,33 @@ def moe_lib() -> ctypes.CDLL:
     return _MOE_LIB
 
 
-def moe_tile_rows(wide: bool) -> int:
-    """Pairs per tile: of the plain tiles, or of the pipelined bfloat16 kernel's (``wide``)."""
-    return int(moe_lib().rl_moe_tile_rows(int(bool(wide))))
+MOE_KINDS = {False: 0, True: 1, "few": 2, "tensor": 3}
+
+
+def moe_tile_rows(wide) -> int:
+    """Pairs per tile of a product kernel: ``False`` the plain tiles, ``True`` the pipelined bfloat16 ones, ``"few"`` the one
+    for few pairs, ``"tensor"`` the tensor cores' (tcgen05)."""
+    return int(moe_lib().rl_moe_tile_rows(MOE_KINDS[wide]))
 
 
 def moe_wide_takes(dtype: torch.dtype, *inner_sizes: int) -> bool:
-    """Whether the pipelined bfloat16 kernel takes products with these inner sizes (16-byte rows)."""
+    """Whether the bfloat16 kernels for rows of whole 16-byte pieces take products with these inner sizes."""
     return dtype == torch.bfloat16 and all(size % 8 == 0 for size in inner_sizes)
 
 
-def moe_max_tiles(pairs: int, experts: int, wide: bool = False) -> int:
+MOE_FEW_PAIRS, MOE_TENSOR_PAIRS = 8, 32      # pairs per expert up to and from which a kernel is the fastest
+
+
+def moe_kind(dtype: torch.dtype, pairs: int, experts: int, hidden: int, inter: int):
+    """Which product kernels a step's pairs run on (see :func:`moe_tile_rows`)."""
+    if not moe_wide_takes(dtype, hidden, inter):
+        return False
+    if pairs <= MOE_FEW_PAIRS * experts and max(hidden, inter) <= 6144:
+        return "few"
+    return "tensor" if pairs >= MOE_TENSOR_PAIRS * experts else True
+
+
+def moe_max_tiles(pairs: int, experts: int, wide=False) -> int:
     """Most tiles the (token, expert) pairs of a step can fall into."""
     return -(-int(pairs) // moe_tile_rows(wide)) + int(experts)
 
@@ -1623,7 +1639,7 @@ def router_topk(x: torch.Tensor, weight: torch.Tensor, *, experts: int, top: int
 
 
 def moe_plan(ids: torch.Tensor, experts: int, sorted_pairs: torch.Tensor, place_of: torch.Tensor, meta: torch.Tensor,
-             fault: torch.Tensor, wide: bool = False) -> int:
+             fault: torch.Tensor, wide=False) -> int:
     """Groups the pairs ``ids [T, top]`` by expert on the device, in tiles of :func:`moe_tile_rows` pairs; returns the
     most tiles there can be.  The products over the plan must be asked for with the same ``wide``."""
     _need_cuda(ids, sorted_pairs, place_of, meta, fault)
@@ -1640,8 +1656,8 @@ def moe_plan(ids: torch.Tensor, experts: int, sorted_pairs: torch.Tensor, place_
 
 def grouped_linear(a: torch.Tensor, weight: torch.Tensor, sorted_pairs: torch.Tensor, meta: torch.Tensor, *, top: int,
                    by_token: bool, max_tiles: int, pair_weight: torch.Tensor | None = None,
-                   out_act: torch.Tensor | None = None, out_y: torch.Tensor | None = None, wide: bool = False,
-                   clamp: tuple[float, float] | None = None) -> None:
+                   out_act: torch.Tensor | None = None, out_y: torch.Tensor | None = None, wide=False,
+                   fault: torch.Tensor | None = None, clamp: tuple[float, float] | None = None) -> None:
     """Products over the pairs grouped by expert: ``weight [E, N or 2 N, K]``.  With ``out_act`` (engine dtype,
     by place) the weight is gate rows then up rows and ``out_act = silu(w g) * (w u)`` with the pair's weight ``w``,
     or with ``clamp = (limit, alpha)`` the clamped unit ``g' sigmoid(alpha g') (u' + 1)``, ``g' = min(g, limit)``,
@@ -1659,10 +1675,12 @@ def grouped_linear(a: torch.Tensor, weight: torch.Tensor, sorted_pairs: torch.Te
     n = (out_act if gated else out_y).shape[1]
     if weight.shape[1] != (2 * n if gated else n) or (gated and out_act.dtype != a.dtype):
         raise KernelError("grouped_linear: the result's width does not fit the weight")
+    if wide == "tensor" and fault is None:
+        raise KernelError("grouped_linear: the tensor cores' tiles need the fault word")
     _check(moe_lib().rl_grouped_linear(dtype_tag(a.dtype), _ptr(a), _row_stride("a", a), _ptr(weight), _ptr(sorted_pairs),
                                        _ptr(meta), _ptr(pair_weight), int(top), int(by_token), n, a.shape[1], int(gated),
                                        _ptr(out_act), _ptr(out_y), int(max_tiles), moe_tile_rows(wide), limit, alpha,
-                                       int(PDL), _stream()),
+                                       weight.shape[0], _ptr(fault), int(PDL), _stream()),
            "grouped_linear")
 
 

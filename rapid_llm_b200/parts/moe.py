@@ -169,16 +169,17 @@ class RoutedExperts(FeedForward):
                             correction=self.correction, groups=self.groups, keep=self.keep)
         order = space.get("moe_sorted", tokens, top, i32).view(-1)
         place = space.get("moe_place", tokens, top, i32).view(-1)
-        wide = kernels.moe_wide_takes(x.dtype, self.hidden, self.inter)      # the pipelined bfloat16 tiles
-        most = kernels.moe_max_tiles(max(space.max_tokens, tokens) * top, experts)
+        wide = kernels.moe_kind(x.dtype, pairs, experts, self.hidden, self.inter)      # which product kernels
+        most = kernels.moe_max_tiles(max(space.max_tokens, tokens) * top, experts, "few")      # the smallest tiles
         meta = space.get("moe_meta", 1, 1 + 3 * most, i32, min_rows=1).view(-1)
         max_tiles = kernels.moe_plan(ids, experts, order, place, meta, batch.fault, wide=wide)
         act = space.get("moe_act", tokens, top * self.inter, x.dtype).view(pairs, self.inter)
         kernels.grouped_linear(x, self.gate_up, order, meta, top=top, by_token=True, max_tiles=max_tiles,
                                pair_weight=weights.view(-1) if self.scale_input else None, out_act=act, wide=wide,
-                               clamp=self.clamp)
+                               clamp=self.clamp, fault=batch.fault)
         each = space.get("moe_each", tokens, top * self.hidden, f32).view(pairs, self.hidden)
-        kernels.grouped_linear(act, self.down, order, meta, top=top, by_token=False, max_tiles=max_tiles, out_y=each, wide=wide)
+        kernels.grouped_linear(act, self.down, order, meta, top=top, by_token=False, max_tiles=max_tiles, out_y=each, wide=wide,
+                               fault=batch.fault)
         shared = None if self.shared is None else self.shared.forward(x, batch)
         if closing is not None and shared is None and hasattr(closing.norm, "bias") and closing.norm.gain == 1.0:
             out = space.get("stream_rows", tokens, self.hidden, x.dtype)

@@ -67,6 +67,65 @@ def test_products_over_pairs_grouped_by_expert(tokens, experts, top, hidden, int
     torch.testing.assert_close(out.float(), want, **bound)
 
 
+@pytest.mark.parametrize("kind", ["few", "tensor"])
+@pytest.mark.parametrize("tokens,experts,top,hidden,inter", [(1, 3, 2, 64, 32), (8, 16, 2, 2048, 512), (17, 1, 1, 40, 24), (130, 2, 2, 200, 136),
+                                                             (400, 3, 1, 64, 264), (2048, 16, 2, 256, 64), (300, 40, 3, 72, 8)])
+def test_products_over_few_and_over_many_pairs(tokens, experts, top, hidden, inter, kind):
+    """The kernels for few pairs a tile and on the tensor cores, at edges of their tiles (16 and 128 pairs, 16 and 128 gated
+    columns, 32 and 256 plain ones, 32 and 64 inner columns) with unit, clamp and pair weights, against each expert's rows in
+    float32; identity experts' pairs are in no tile, and nothing is written past the pairs."""
+    from rapid_llm_b200.ops import kernels
+
+    torch.manual_seed(tokens)
+    bf = torch.bfloat16
+    x = torch.randn(tokens, hidden + 8, device=DEVICE).to(bf)[:, :hidden]
+    gate_up = (torch.randn(experts, 2 * inter, hidden, device=DEVICE) / hidden ** 0.5).to(bf)
+    down = (torch.randn(experts, hidden, inter, device=DEVICE) / inter ** 0.5).to(bf)
+    ids = torch.rand(tokens, experts + 1, device=DEVICE).argsort(-1)[:, :top].to(torch.int32).contiguous()      # id `experts`: an identity expert
+    weights = torch.rand(tokens, top, device=DEVICE)
+    pairs = tokens * top
+    fault = torch.zeros(1, dtype=torch.int32, device=DEVICE)
+    order, place = torch.zeros(pairs, dtype=torch.int32, device=DEVICE), torch.zeros(pairs, dtype=torch.int32, device=DEVICE)
+    meta = torch.zeros(1 + 3 * kernels.moe_max_tiles(pairs, experts, kind), dtype=torch.int32, device=DEVICE)
+    tiles = kernels.moe_plan(ids, experts, order, place, meta, fault, wide=kind)
+    chosen = ids.view(-1).long()
+    mine = chosen < experts
+    for clamp in (None, (0.5, 1.702)):
+        act = torch.full((pairs + 1, inter), 7.0, dtype=bf, device=DEVICE)
+        kernels.grouped_linear(x, gate_up, order, meta, top=top, by_token=True, max_tiles=tiles, pair_weight=weights.view(-1),
+                               out_act=act[:pairs], wide=kind, clamp=clamp, fault=fault)
+        each = torch.full((pairs + 1, hidden), 7.0, device=DEVICE)
+        kernels.grouped_linear(act[:pairs], down, order, meta, top=top, by_token=False, max_tiles=tiles, out_y=each[:pairs], wide=kind, fault=fault)
+        assert int(fault.item()) == 0
+        assert bool((act[pairs] == 7.0).all()) and bool((each[pairs] == 7.0).all()) and bool((each[:pairs][~mine] == 7.0).all())
+        rows = x.float().repeat_interleave(top, dim=0)
+        for e in range(experts):
+            at = (chosen == e).nonzero(as_tuple=True)[0]
+            if not at.numel():
+                continue
+            both = (rows[at] @ gate_up[e].float().t()) * weights.view(-1)[at][:, None]
+            g, u = both[:, :inter], both[:, inter:]
+            if clamp is None:
+                unit = g * torch.sigmoid(g) * u
+            else:
+                g, u = g.clamp(max=clamp[0]), u.clamp(-clamp[0], clamp[0])
+                unit = g * torch.sigmoid(clamp[1] * g) * (u + 1.0)
+            got = act[place.long()[at]].float()
+            torch.testing.assert_close(got, unit, rtol=2.0 ** -7, atol=1e-3)            # one rounding to bfloat16
+            torch.testing.assert_close(each[at], got @ down[e].float().t(), rtol=1e-4, atol=1e-4)      # float32 sums
+    # a row does not depend on what else is in its tile
+    alone_ids = ids[:1].contiguous()
+    order1, place1 = torch.zeros(top, dtype=torch.int32, device=DEVICE), torch.zeros(top, dtype=torch.int32, device=DEVICE)
+    meta1 = torch.zeros(1 + 3 * kernels.moe_max_tiles(top, experts, kind), dtype=torch.int32, device=DEVICE)
+    tiles1 = kernels.moe_plan(alone_ids, experts, order1, place1, meta1, fault, wide=kind)
+    act1 = torch.empty(top, inter, dtype=bf, device=DEVICE)
+    kernels.grouped_linear(x[:1], gate_up, order1, meta1, top=top, by_token=True, max_tiles=tiles1, pair_weight=weights.view(-1)[:top],
+                           out_act=act1, wide=kind, clamp=(0.5, 1.702), fault=fault)
+    for j in range(top):
+        if int(chosen[j]) < experts:
+            assert torch.equal(act1[int(place1[j])], act[int(place[j])])
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("experts,top,gates,hidden", [(12, 1, 1, 64), (40, 3, 0, 50), (2, 2, 2, 33), (70, 8, 1, 128)])
 def test_router_scores_choices_and_gates(experts, top, gates, hidden, dtype):
