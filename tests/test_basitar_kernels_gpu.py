@@ -117,6 +117,27 @@ def test_a_product_per_head(tokens, heads, n_out, k, x_width, out_width, x_col0,
     assert bool((got[..., n_out:] == 5.0).all())
 
 
+@pytest.mark.parametrize("tokens", [1, 16, 17, 33, 64])
+@pytest.mark.parametrize("heads,n_out,k,x_width,out_width,x_col0", [
+    (3, 192, 128, 192, 256, 0), (16, 128, 192, 256, 128, 0), (2, 40, 8, 24, 48, 8), (1, 6, 64, 64, 6, 0), (4, 17, 72, 80, 19, 8), (2, 33, 200, 208, 40, 8),
+    (1, 256, 256, 256, 256, 0), (2, 24, 264, 264, 24, 0)])
+def test_a_product_per_head_of_a_few_rows(tokens, heads, n_out, k, x_width, out_width, x_col0):
+    """Steps of up to 64 rows: remainders of 16 rows and columns, of 64 steps of the reduction, the widest row the kernel
+    holds and the first behind it; what lies behind the columns stays."""
+    from rapid_llm_b200.ops import kernels
+
+    g = torch.Generator().manual_seed(tokens + k)
+    x = torch.randn(tokens, heads * x_width, generator=g).to(torch.bfloat16).to(DEVICE)
+    weight = (torch.randn(heads, n_out, k, generator=g) / math.sqrt(k)).to(torch.bfloat16).to(DEVICE)
+    out = torch.full((tokens, heads * out_width), 5.0, dtype=torch.bfloat16, device=DEVICE)
+    kernels.heads_linear(x, weight, out, x_col0=x_col0)
+    got = out.view(tokens, heads, out_width).float()
+    want = torch.einsum("thk,hnk->thn", x.view(tokens, heads, x_width)[..., x_col0 : x_col0 + k].double(), weight.double())
+    # one rounding to bfloat16 (2^-9 of the value) and the float32 sums' own error
+    torch.testing.assert_close(got[..., :n_out].double(), want, rtol=2.0 ** -8, atol=1e-4)
+    assert bool((got[..., n_out:] == 5.0).all())
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("heads,width", [(3, 24), (1, 64), (5, 6), (16, 40)])
 def test_a_sigmoid_gate_per_head(heads, width, dtype):
