@@ -573,6 +573,7 @@ int launch_attention(const AttentionArgs& args, int n_items, bool pdl, cudaStrea
 
 #include "attention_decode_tc.cuh"
 #include "attention_prefill_tc.cuh"
+#include "attention_plane_tc.cuh"
 
 namespace rl {
 namespace RL_ATTENTION_NS {
@@ -610,6 +611,37 @@ static int launch_prefill_tc(const AttentionArgs& a, int n_items, bool pdl, cuda
   }
   return launch_kernel(kernel, dim3(a.hkv, n_items), dim3(kPfThreads), kPfSmemBytes, stream, pdl,
                        map, t);
+}
+
+// Whether the one-plane tcgen05 chunk kernel takes this geometry.
+static bool plane_tc_supported(int page_size) { return kPlTakes && page_size % 8 == 0; }
+
+// Chunk tiles of 128 packed rows over a cache of one plane.
+static int launch_plane_tc(const AttentionArgs& a, int n_items, bool pdl, cudaStream_t stream) {
+  if constexpr (!kPlTakes) {
+    return static_cast<int>(cudaErrorInvalidValue);
+  } else {
+    static bool configured = false;
+    if (!configured) {
+      cudaError_t e = cudaFuncSetAttribute(attention_plane_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPlSmemBytes);
+      if (e != cudaSuccess) return static_cast<int>(e);
+      configured = true;
+    }
+    PlaneTcArgs t;
+    t.box_rows = a.page_size % 32 == 0 ? 32 : a.page_size % 16 == 0 ? 16 : 8;
+    CUtensorMap map;
+    const long long rows = static_cast<long long>(a.num_pages) * a.hkv * a.page_size;
+    if (rows > 0x7fffffff) return static_cast<int>(cudaErrorInvalidValue);
+    int status = make_map(&map, a.cache, rows, kD, t.box_rows);
+    if (status != 0) return status;
+    t.q = a.q; t.out = a.out; t.part_out = a.part_out; t.part_lse = a.part_lse; t.items = a.items;
+    t.cu_seqlens = a.cu_seqlens; t.entry_start = a.entry_start; t.entry_slot = a.entry_slot;
+    t.block_table = a.block_table; t.hq = a.hq; t.hkv = a.hkv; t.page_size = a.page_size;
+    t.num_pages = a.num_pages; t.max_pages = a.max_pages; t.slots = a.slots; t.window = a.window; t.chunk = a.chunk;
+    t.splits = a.splits; t.scale_log2 = a.scale_log2; t.fault = a.fault; t.sink = a.sink;
+    t.out_stride = a.out_stride; t.gate = a.gate; t.gate_stride = a.gate_stride;
+    return launch_kernel(attention_plane_tc_kernel, dim3(a.hkv, n_items), dim3(kPlThreads), kPlSmemBytes, stream, pdl, map, t);
+  }
 }
 
 static bool g_decode_tc_configured[5][2][2] = {};   // per row-count, ring-depth and dressed instantiation; file-local on purpose
@@ -721,10 +753,13 @@ int rl_attention_head_dim() { return attn::kD; }
 int rl_attention_chunk_rows() { return 64; }
 // ... of a chunk tile of the tcgen05 kernel, or 0 where this build (head size) has none.
 int rl_attention_chunk_rows_tc() { return attn::kD == attn::kPfD ? attn::kPfRows : 0; }
+// ... of the tcgen05 kernel over a cache of one plane, or 0.
+int rl_attention_chunk_rows_plane() { return attn::kPlTakes ? attn::kPlRows : 0; }
 int rl_attention_decode_rows() { return 16; }
 
 // chunk_rows: packed rows per chunk item: 64 (or 0) = the mma.sync tiles, 256 = the tcgen05
-// kernel (head size 128, pages it takes, splits == 1).
+// kernel (head size 128, pages it takes, splits == 1), 128 = the tcgen05 kernel over a cache of one plane (rows of 64 and
+// more numbers, pages of a multiple of 8 tokens, scores that are not squashed).
 // decode_splits: key ranges of the decode tiles where they differ from `splits` (a step of prompt portions, which
 // the tcgen05 kernel does not split, beside single tokens with long contexts); 0 = the same.
 // decode_kernel: 0 = the tcgen05 kernel for decode tiles where it applies, 1 = always the
@@ -773,7 +808,9 @@ int rl_attention_mma(const void* q, const void* cache, void* out, float* part_ou
     if (!(softcap > 0.0f) || (decode_splits > 0 && decode_splits != splits)) return static_cast<int>(cudaErrorInvalidValue);
     decode_kernel = 1;
   }
-  if (kv_planes == 1) {         // rows that are keys and values at once: the mma.sync tiles read them, the tcgen05 tiles do not
+  if (chunk_rows == attn::kPlRows && (kv_planes != 1 || softcap != 0.0f || !attn::plane_tc_supported(page_size)))
+    return static_cast<int>(cudaErrorInvalidValue);
+  if (kv_planes == 1) {         // rows that are keys and values at once: tiles of 128 or the mma.sync tiles read them
     if (slopes != nullptr || chunk_rows == attn::kPfRows || (decode_splits > 0 && decode_splits != splits)) return static_cast<int>(cudaErrorInvalidValue);
     decode_kernel = 1;
   } else if (kv_planes != 2) {
@@ -817,6 +854,8 @@ int rl_attention_mma(const void* q, const void* cache, void* out, float* part_ou
       if (attn::kD != attn::kPfD || !attn::decode_tc_supported(page_size) || splits != 1)
         return static_cast<int>(cudaErrorInvalidValue);
       status = attn::launch_prefill_tc(args, n_chunk_items, pdl != 0, stream);
+    } else if (chunk_rows == attn::kPlRows) {
+      status = attn::launch_plane_tc(args, n_chunk_items, pdl != 0, stream);
     } else if (chunk_rows == 64 || chunk_rows == 0) {
       status = attn::launch_attention<4, 1, 2>(args, n_chunk_items, pdl != 0, stream);
     } else {

@@ -598,10 +598,17 @@ _ATTENTION_LIBS: dict[int, ctypes.CDLL] = {}
 
 CHUNK_TILE_ROWS = 64       # packed rows (token, head of the group) of a chunk tile of the mma.sync kernel
 CHUNK_TILE_ROWS_TC = 256   # ... of the tcgen05 kernel (head size 128, unsplit key ranges)
+CHUNK_TILE_ROWS_PLANE = 128   # ... of the tcgen05 kernel over rows that are keys and values at once
 DECODE_TILE_ROWS = 16      # ... of a decode tile
 TC_HEAD_DIM = 128
+PLANE_TC_MIN_DIM = 64     # narrowest row of the tcgen05 chunk tiles over a cache of one plane
 DECODE_TC_KEYS = 128      # keys per block of the tcgen05 decode kernel
 MMA_KEYS = 64             # ... of the mma.sync tiles
+
+
+def attention_plane_tc_takes(head_dim: int, page_size: int) -> bool:
+    """Whether the tcgen05 chunk tiles over a cache of one plane take this row and page size."""
+    return PLANE_TC_MIN_DIM <= head_dim <= 256 and head_dim % 16 == 0 and page_size > 0 and page_size % 8 == 0
 
 
 def attention_tc_takes(head_dim: int, page_size: int) -> bool:
@@ -631,6 +638,8 @@ def attention_lib(head_dim: int) -> ctypes.CDLL:
             raise KernelError("the attention library's tile sizes differ from the host's")
         if lib.rl_attention_chunk_rows_tc() != (CHUNK_TILE_ROWS_TC if head_dim == TC_HEAD_DIM else 0):
             raise KernelError("the attention library's tensor-core tile size differs from the host's")
+        if lib.rl_attention_chunk_rows_plane() != (CHUNK_TILE_ROWS_PLANE if head_dim >= PLANE_TC_MIN_DIM else 0):
+            raise KernelError("the attention library's tile size for caches of one plane differs from the host's")
         _ATTENTION_LIBS[head_dim] = lib
     return lib
 
@@ -687,7 +696,8 @@ def attention_mma(
     a multiple of 128 tokens) unless ``decode_kernel`` is ``"mma"``; ``decode_rows`` is the most
     packed rows any decode tile has (0 = not known), which lets that kernel unroll over fewer rows.
     ``chunk_rows`` says how the chunk items were cut: :data:`CHUNK_TILE_ROWS` for the mma.sync
-    tiles, :data:`CHUNK_TILE_ROWS_TC` for the tcgen05 kernel (``splits`` must then be 1).
+    tiles, :data:`CHUNK_TILE_ROWS_TC` for the tcgen05 kernel (``splits`` must then be 1),
+    :data:`CHUNK_TILE_ROWS_PLANE` for the one over a cache of one plane.
 
     ``chunk_items`` / ``decode_items`` are int32 ``[n, 4]`` rows ``(entry, first packed row,
     split, 0)`` for tiles of :data:`CHUNK_TILE_ROWS` / :data:`DECODE_TILE_ROWS` packed rows

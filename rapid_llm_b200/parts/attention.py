@@ -104,7 +104,7 @@ class AttentionItems(StepPlanner):
     context length (where the tcgen05 decode kernel merges the parts inside a thread-block cluster: the
     largest cluster of which that many run at one time); bounded by the longest context otherwise.  Chunk tiles have 256 rows
     for the tcgen05 kernel, which takes head size 128, the usual page sizes and unsplit key
-    ranges, and 64 rows for the mma.sync kernel otherwise.  The tcgen05 kernel is several times
+    ranges, 128 rows for the one that reads caches of one plane, and 64 rows for the mma.sync kernel otherwise.  The tcgen05 kernel is several times
     faster per key, so it also runs, unsplit, where a split would have been wanted, unless its
     CTAs are few and the context long (a few dozen prompt tokens behind thousands of cached ones).
     The longest tiles come first in the list, and the kernels' grids start them in that order.
@@ -114,13 +114,16 @@ class AttentionItems(StepPlanner):
 
     def __init__(self, group: int, num_kv_heads: int, head_dim: int = 0, sms: int = DEFAULT_SMS,
                  decode_clusters: dict[int, int] | None = None, tensor_core: bool = True,
-                 decode_tensor_core: bool = True, chunk: int = 0, window: int = 0) -> None:
+                 decode_tensor_core: bool = True, chunk: int = 0, window: int = 0, one_plane: bool = False) -> None:
         self.group, self.num_kv_heads, self.head_dim = int(group), int(num_kv_heads), int(head_dim)
         # decode_tensor_core False: the mixer's scores are squashed, which the tcgen05 chunk tiles and the mma.sync tiles
         # compute, the tcgen05 decode tiles not; tensor_core False: mma.sync tiles only.  chunk: the most keys a
         # position sees (0 = all before it), which bounds the key ranges worth having.
         self.tensor_core = bool(tensor_core)
         self.decode_tensor_core = self.tensor_core and bool(decode_tensor_core)
+        # one_plane: the cached rows are keys and values at once; chunk tiles then have 128 rows where the tcgen05
+        # kernel for such caches takes the row and page size.
+        self.one_plane = bool(one_plane)
         # window: the same bound for the key ranges where a mixer asks for it (0 = not bounded).
         self.chunk, self.window = int(chunk), int(window)
         self.decode_clusters = dict(decode_clusters or DEFAULT_DECODE_CLUSTERS)
@@ -128,7 +131,8 @@ class AttentionItems(StepPlanner):
         # step, whose kernel keeps a whole multiprocessor's shared memory busy
         self.target_ctas, self.decode_target_ctas = 2 * int(sms), int(sms)
         self.key = ("attention_items", self.group, self.num_kv_heads, self.head_dim, int(sms),
-                    tuple(sorted(self.decode_clusters.items())), self.tensor_core, self.decode_tensor_core, self.chunk, self.window)
+                    tuple(sorted(self.decode_clusters.items())), self.tensor_core, self.decode_tensor_core, self.chunk, self.window,
+                    self.one_plane)
 
     def capacity(self, max_tokens: int, max_entries: int) -> int:
         chunk_tiles = -(-max_tokens * self.group // kernels.CHUNK_TILE_ROWS) + max_entries
@@ -145,11 +149,16 @@ class AttentionItems(StepPlanner):
             seen_last = np.minimum(starts % self.chunk + lengths, self.chunk + lengths - 1)
         is_decode = (lengths == 1) | (rows <= kernels.DECODE_TILE_ROWS)
         tensor_core = self.tensor_core and kernels.attention_tc_takes(self.head_dim, shape.page_size)
-        for chunk_rows in ((kernels.CHUNK_TILE_ROWS_TC, kernels.CHUNK_TILE_ROWS) if tensor_core else (kernels.CHUNK_TILE_ROWS,)):
+        plane = self.one_plane and kernels.attention_plane_tc_takes(self.head_dim, shape.page_size)
+        if plane:
+            is_decode = np.zeros_like(is_decode)
+        for chunk_rows in ((kernels.CHUNK_TILE_ROWS_PLANE,) if plane else
+                           (kernels.CHUNK_TILE_ROWS_TC, kernels.CHUNK_TILE_ROWS) if tensor_core else (kernels.CHUNK_TILE_ROWS,)):
             tile_rows = np.where(is_decode, kernels.DECODE_TILE_ROWS, chunk_rows)
             tiles = -(-rows // tile_rows)
             ctas = int(tiles.sum()) * self.num_kv_heads
-            target = self.decode_target_ctas if shape.decode_only else self.target_ctas
+            # (a tile of 128 rows has a multiprocessor to itself, as in a decode-only step)
+            target = self.decode_target_ctas if shape.decode_only or plane else self.target_ctas
             splits = max(1, min(MAX_SPLITS, target // max(ctas, 1)))
             if self.chunk:
                 splits = max(1, min(splits, -(-self.chunk // kernels.MMA_KEYS)))
@@ -171,7 +180,7 @@ class AttentionItems(StepPlanner):
                     real = len(lengths) - int(shape.padding)
                     counted = max(1, int(tiles[:real].sum()) * self.num_kv_heads)
                 splits = min(cluster_splits(counted, self.decode_clusters), 1 << (blocks.bit_length() - 1))
-            if splits == 1 or chunk_rows == kernels.CHUNK_TILE_ROWS or bool(is_decode.all()):
+            if splits == 1 or chunk_rows != kernels.CHUNK_TILE_ROWS_TC or bool(is_decode.all()):
                 break
             # The tcgen05 chunk kernel does not split key ranges, but it is several times faster per
             # key than the mma.sync tiles: it runs unsplit unless it would leave most of the GPU

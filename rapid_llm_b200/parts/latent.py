@@ -101,8 +101,8 @@ class LatentAttention(Mixer):
         self.o = self.new_storage((self.hidden, self.h * self.vdim), MATRIX)
         device = torch.device(device)
         sms = torch.cuda.get_device_properties(device).multi_processor_count if device.type == "cuda" else DEFAULT_SMS
-        # the mma.sync tiles read a cache of one plane; the tcgen05 tiles do not
-        self._items = AttentionItems(self.h, 1, self.d, sms, None, tensor_core=False, window=self.window)
+        # a cache of one plane: chunk tiles of its own tcgen05 kernel, decode tiles on mma.sync
+        self._items = AttentionItems(self.h, 1, self.d, sms, None, tensor_core=False, window=self.window, one_plane=True)
 
     # -- needs ----------------------------------------------------------------- #
     def cache_need(self) -> CacheNeed:
@@ -228,7 +228,7 @@ class LatentAttention(Mixer):
                 part_out=part_out, part_lse=part_lse, cu_seqlens=batch.cu_seqlens, entry_start=batch.entry_start,
                 entry_slot=batch.entry_slot, block_table=group.block_table, num_heads=self.h, num_kv_heads=1,
                 head_dim=self.d, window=self.window, scale=self.scale, fault=batch.fault, sink=self.sink, decode_kernel="mma",
-                decode_rows=plan.get("decode_rows", 0), chunk_rows=kernels.CHUNK_TILE_ROWS)
+                decode_rows=plan.get("decode_rows", 0), chunk_rows=plan["chunk_rows"])
             return
         kernels.attention_generic(
             q, pages, out, positions=batch.positions, token_slot=batch.token_slot, block_table=group.block_table,

@@ -133,3 +133,22 @@ def test_chunk_tiles_follow_the_kernel_that_will_run():
     assert AttentionItems(4, 8, 64).plan(whole)["chunk_rows"] == kernels.CHUNK_TILE_ROWS
     odd = StepShape(np.asarray([2048], dtype=np.int32), np.asarray([0], dtype=np.int32), False, page_size=4)
     assert planner.plan(odd)["chunk_rows"] == kernels.CHUNK_TILE_ROWS
+
+
+@pytest.mark.parametrize("group,head_dim,page_size", [(16, 256, 16), (5, 144, 8), (128, 64, 64), (16, 256, 12), (16, 48, 16)])
+@pytest.mark.parametrize("seed", range(4))
+def test_a_cache_of_one_plane_gets_tiles_of_its_own(group, head_dim, page_size, seed):
+    rng = np.random.default_rng(seed)
+    entries = int(rng.integers(1, 9))
+    lengths = rng.choice([1, 1, 2, 16, 17, 100, 700], size=entries).astype(np.int32)
+    starts = rng.integers(0, 3000, size=entries).astype(np.int32)
+    planner = AttentionItems(group, 1, head_dim, tensor_core=False, one_plane=True)
+    plan = planner.plan(StepShape(lengths, starts, decode_only=bool(lengths.max() == 1), page_size=page_size))
+    taken = page_size % 8 == 0 and head_dim >= 64
+    assert plan["chunk_rows"] == (kernels.CHUNK_TILE_ROWS_PLANE if taken else kernels.CHUNK_TILE_ROWS)
+    rows = lengths.astype(np.int64) * group
+    seen = covered(plan["chunk_items"], plan["chunk_rows"], rows, plan["splits"])
+    for key, count in covered(plan["decode_items"], kernels.DECODE_TILE_ROWS, rows, plan["splits"]).items():
+        seen[key] = seen.get(key, 0) + count
+    assert all(count == 1 for count in seen.values()) and len(seen) == int(rows.sum()) * plan["splits"]
+    assert 4 * (len(plan["chunk_items"]) + len(plan["decode_items"])) <= planner.capacity(int(lengths.sum()), entries)

@@ -321,6 +321,51 @@ def test_tiles_over_one_plane_with_a_window_and_a_sink(hq, d, page, window, spli
     torch.testing.assert_close(out.float().cpu(), _plain(case, hq, 1, lengths, new, d ** -0.5, window, sink), rtol=3e-2, atol=8e-3)
 
 
+@pytest.mark.parametrize("hq,hkv,d,page,window,splits", [
+    (16, 1, 256, 16, 0, None), (16, 1, 256, 8, 65, 3), (6, 2, 256, 48, 0, 1), (40, 1, 240, 64, 0, None), (16, 1, 208, 24, 130, 1), (5, 1, 144, 128, 0, 5),
+    (128, 1, 128, 16, 0, 2), (1, 1, 80, 16, 96, 1), (12, 3, 64, 32, 0, None)])
+def test_tensor_core_tiles_over_one_plane(hq, hkv, d, page, window, splits):
+    """Portions that end inside and on a tile of 128 rows, ranges that end inside and on a block of 96 keys and on a box,
+    more key ranges than blocks, rows that are no multiple of 64 numbers; places that nothing wrote hold NaN."""
+    from rapid_llm_b200.ops import kernels
+    from rapid_llm_b200.parts.attention import AttentionItems
+    from rapid_llm_b200.parts.base import StepShape
+
+    lengths, new = [17, 96, 97, 129, 200, 64, 700, 301, 288, 5], [17, 96, 1, 129, 33, 64, 300, 1, 3, 5]
+    case = _case(torch.bfloat16, hq, hkv, d, page, lengths, new, seed=d + page, planes=1)
+    case["cache"][case["cache"] == 50.0] = float("nan")
+    starts = np.asarray(lengths, np.int32) - np.asarray(new, np.int32)
+    plan = AttentionItems(hq // hkv, hkv, d, tensor_core=False, window=window, one_plane=True).plan(
+        StepShape(np.asarray(new, np.int32), starts, decode_only=False, page_size=page))
+    assert plan["chunk_rows"] == kernels.CHUNK_TILE_ROWS_PLANE and len(plan["chunk_items"])
+
+    def spread(items, count):
+        base = items[items[:, 2] == 0]
+        again = np.repeat(base, count, axis=0)
+        again[:, 2] = np.tile(np.arange(count, dtype=np.int32), len(base))
+        return torch.from_numpy(again).to(DEVICE)
+
+    count = splits or plan["splits"]
+    sink = torch.linspace(-4.0, 3.0, hq, device=DEVICE) if page != 16 else None
+    gate = torch.randn(case["q"].shape[0], hq, device=DEVICE).to(torch.bfloat16) if page == 64 else None
+    part_out = torch.full((case["q"].shape[0] * hq * count, d), float("nan"), device=DEVICE)
+    part_lse = torch.full((case["q"].shape[0] * hq * count,), float("nan"), device=DEVICE)
+    wide = torch.full((case["q"].shape[0], hq * d + 8), 7.0, dtype=torch.bfloat16, device=DEVICE)
+    fault = _word()
+    kernels.attention_mma(
+        case["q"], case["cache"], wide[:, : hq * d], chunk_items=spread(plan["chunk_items"], count), decode_items=spread(plan["decode_items"], count),
+        splits=count, part_out=part_out, part_lse=part_lse, cu_seqlens=torch.tensor([0] + list(np.cumsum(new)), dtype=torch.int32, device=DEVICE),
+        entry_start=torch.from_numpy(starts).to(DEVICE), entry_slot=case["slots"], block_table=case["table"], num_heads=hq, num_kv_heads=hkv,
+        head_dim=d, window=window, scale=d ** -0.5, fault=fault, decode_kernel="mma", decode_rows=plan["decode_rows"], chunk_rows=plan["chunk_rows"],
+        sink=sink, gate=gate)
+    assert int(fault.item()) == 0
+    want = _plain(case, hq, hkv, lengths, new, d ** -0.5, window, sink)
+    if gate is not None:
+        want = (want.view(-1, hq, d) * torch.sigmoid(gate.float().cpu())[:, :, None]).reshape(want.shape)
+    torch.testing.assert_close(wide[:, : hq * d].float().cpu(), want, rtol=3e-2, atol=8e-3)
+    assert bool((wide[:, hq * d :] == 7.0).all())
+
+
 def test_slopes_over_one_plane_are_refused_by_the_tiles():
     from rapid_llm_b200.ops import kernels
 
