@@ -8,19 +8,20 @@
 //     S[row, key]  = Q[row, :] . R[key, :]      tcgen05.mma  M = 128, N = 96 keys, K = D
 //     O[row, d]   += P[row, key] . R[key, d]    A = P from tensor memory, M = 128, N = D, K = 96 keys
 //
-// What bounds it is the tensor core's two products per block, so the scores of block j + 1 are issued before the
-// values of block j and the softmax of one block runs under the products of its neighbours: O takes D columns of
-// tensor memory, two blocks of scores 2 x 128 (P lies over the scores it came from).  Blocks of 96: three tiles
-// of 96 x 256 fit beside the queries, and a tile is held from its scores to its values, one block later; with two tiles
-// of 128 the next scores would wait for a whole fetch.  The softmax is that of the two-plane kernel: a thread owns a row,
-// the reference point of the exponentials moves only when the maximum has grown by more than 2^8, scores, maxima, sums
+// What bounds it is the chain from a block's scores through its softmax to its values (1.3 us; the two products alone
+// take 0.8), so the scores of block j + 1 are issued before the values of block j, two threads share a row and the softmax of
+// one block runs under the products of its neighbours: O takes D columns of tensor memory, two blocks of scores 2 x 128 (P
+// lies over the scores it came from).  Blocks of 96: three tiles of 96 x 256 fit beside the queries, and a tile is held from its scores to its values, one block later; with two tiles
+// of 128 the next scores would wait for a whole fetch, and blocks of 64 with the queries in tensor memory and six tiles
+// pay the chain more often (60 us against 52 for the prompt below).  The softmax is that of the two-plane kernel: the
+// reference point of the exponentials moves only when the maximum has grown by more than 2^8, scores, maxima, sums
 // and O are float32 and P is rounded to bfloat16.
 //
 // Rows behind the range come as zeros (whole boxes from outside the tensor, the rest of a box cleared here): what lies
 // in memory that nothing wrote yet must not reach the product, where zero times it could be NaN.
 //
-// 16 heads, rows of 256: 2,048 tokens of a prompt 55 us (the mma.sync tiles 236), 8 portions of 130 behind 500 tokens 27
-// (85), 64 single tokens behind 1,024 34 (50), behind 4,096 63 (101); 128 heads, the same single tokens 42 (125), 71 (374).
+// 16 heads, rows of 256: 2,048 tokens of a prompt 52 us (the mma.sync tiles 236), 8 portions of 130 behind 500 tokens 27
+// (85), 64 single tokens behind 1,024 34 (50), behind 4,096 60 (101); 128 heads, the same single tokens 42 (125), 71 (374).
 //
 // Takes rows of 64 to 256 numbers and pages of a multiple of 8 tokens; others run on the mma.sync tiles.
 #pragma once
@@ -36,7 +37,8 @@ constexpr int kPlKeys = 96;                     // rows per block
 constexpr int kPlRows = 128;                    // packed query rows per work item
 constexpr int kPlStages = 3;
 constexpr int kPlAtoms = (kPlD + 63) / 64;      // 64-wide columns of swizzled 128-byte rows
-constexpr int kPlThreads = 256;                 // warp 0: TMA, warp 1: MMA, warps 4..7: softmax, one row a thread
+constexpr int kPlThreads = 384;                 // warp 0: TMA, warp 1: MMA, warps 4..11: softmax, two threads a row
+constexpr int kPlHalfKeys = kPlKeys / 2;        // scores per softmax thread and block
 constexpr int kPlQAtomBytes = kPlRows * 128;
 constexpr int kPlAtomBytes = kPlKeys * 128;
 constexpr int kPlQBytes = kPlAtoms * kPlQAtomBytes;
@@ -78,6 +80,7 @@ attention_plane_tc_kernel(const __grid_constant__ CUtensorMap map_cache, const P
   __shared__ uint32_t tmem_slot;
   __shared__ int aborted_flag;
   __shared__ int staged_pages[kPlStagedPages];
+  __shared__ float exchange[2][2][kPlRows];       // [block parity][half][row]
   volatile int* aborted = &aborted_flag;
 
   pdl_trigger();
@@ -110,7 +113,7 @@ attention_plane_tc_kernel(const __grid_constant__ CUtensorMap map_cache, const P
   const int k_end = min(hi, k_begin + n_blocks * kPlKeys);
   const int* table = args.block_table + static_cast<size_t>(bad ? 0 : slot) * args.max_pages;
 
-  const int live = bad ? 1 : min(4, (n_rows + 31) / 32);    // softmax warps that have rows; what the others' lanes hold is never read
+  const int live = max(1, min(4, (n_rows + 31) / 32));    // softmax warps that have rows; what the others' lanes hold is never read
 
   // ---- set-up --------------------------------------------------------------------------
   if (tid == 0) {
@@ -120,10 +123,10 @@ attention_plane_tc_kernel(const __grid_constant__ CUtensorMap map_cache, const P
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_addr(&score_ready[i]), 1);
-      mbar_init(smem_addr(&p_ready[i]), live);
+      mbar_init(smem_addr(&p_ready[i]), 2 * live);
       mbar_init(smem_addr(&value_done[i]), 1);
     }
-    mbar_init(smem_addr(&q_ready), live);
+    mbar_init(smem_addr(&q_ready), 2 * live);
     mbar_init(smem_addr(&drained), 1);
     aborted_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -264,9 +267,12 @@ attention_plane_tc_kernel(const __grid_constant__ CUtensorMap map_cache, const P
       mbar_wait(smem_addr(&drained), 0, aborted, args.fault, 1 << 12);
     }
     __syncwarp();
-  } else if (warp >= 4 && warp < 4 + live) {
+  } else if (warp >= 4 && (warp & 3) < live) {
     // -------------------------------------------------------------------- softmax and output
+    // Warps 4 + i and 8 + i share the rows of lane quarter i, a half of the columns each.  What leads one of them past
+    // a meeting point leads the other: they vote there.
     const int quarter = warp & 3;                      // tensor-memory lanes this warp may touch
+    const int half = (warp - 4) >> 2;
     const int r = quarter * 32 + lane;                 // row of the tile = lane of S and O
     const uint32_t lane_bits = static_cast<uint32_t>(quarter * 32) << 16;
     const int p = row0 + r;                            // packed row of the request
@@ -276,72 +282,81 @@ attention_plane_tc_kernel(const __grid_constant__ CUtensorMap map_cache, const P
     const int lo_pos = first_visible(pos, args.window, args.chunk);
     pdl_wait();                                        // queries come from the kernel before
     if (n_blocks > 0) {
-      // the warp's 32 rows of Q into the K-major operand [row][64] per 64 columns, swizzled
-      constexpr int kChunks = kPlD / 8;                // 16-byte pieces of a row
+      // the 32 rows of Q into the K-major operand [row][64] per 64 columns, swizzled; each warp half of the pieces
+      constexpr int kPieces = kPlD / 16;               // 16-byte pieces a lane fetches
+      constexpr int kChunks = kPlD / 8;                // ... of a row
       const int shift = (group & (group - 1)) == 0 ? 31 - __clz(group) : -1;
+      uint4 fetched[kPieces];
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint4 fetched[kChunks / 2];
+      for (int i = 0; i < kPieces; ++i) {
+        const int at = (half * kPieces + i) * 32 + lane;
+        const int rr = quarter * 32 + at / kChunks, c = at % kChunks;
+        const int pp = row0 + rr;
+        const int tt = shift >= 0 ? pp >> shift : pp / group;
+        fetched[i] = make_uint4(0, 0, 0, 0);
+        if (rr < n_rows)
+          fetched[i] = __ldcg(reinterpret_cast<const uint4*>(
+              args.q + (static_cast<size_t>(tok_begin + tt) * args.hq + kv_head * group + (pp - tt * group)) * kPlD + c * 8));
+      }
 #pragma unroll
-        for (int i = 0; i < kChunks / 2; ++i) {
-          const int at = (half * (kChunks / 2) + i) * 32 + lane;
-          const int rr = quarter * 32 + at / kChunks, c = at % kChunks;
-          const int pp = row0 + rr;
-          const int tt = shift >= 0 ? pp >> shift : pp / group;
-          fetched[i] = make_uint4(0, 0, 0, 0);
-          if (rr < n_rows)
-            fetched[i] = __ldcg(reinterpret_cast<const uint4*>(
-                args.q + (static_cast<size_t>(tok_begin + tt) * args.hq + kv_head * group + (pp - tt * group)) * kPlD + c * 8));
-        }
-#pragma unroll
-        for (int i = 0; i < kChunks / 2; ++i) {
-          const int at = (half * (kChunks / 2) + i) * 32 + lane;
-          const int rr = quarter * 32 + at / kChunks, c = at % kChunks;
-          const uint32_t dst = q_tile + (c >> 3) * kPlQAtomBytes + rr * 128 + (((c & 7) ^ (rr & 7)) << 4);
-          asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(fetched[i].x), "r"(fetched[i].y), "r"(fetched[i].z), "r"(fetched[i].w) : "memory");
-        }
+      for (int i = 0; i < kPieces; ++i) {
+        const int at = (half * kPieces + i) * 32 + lane;
+        const int rr = quarter * 32 + at / kChunks, c = at % kChunks;
+        const uint32_t dst = q_tile + (c >> 3) * kPlQAtomBytes + rr * 128 + (((c & 7) ^ (rr & 7)) << 4);
+        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(fetched[i].x), "r"(fetched[i].y), "r"(fetched[i].z), "r"(fetched[i].w) : "memory");
       }
       fence_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_addr(&q_ready));
     }
 
-    float ref_max = -INFINITY;                         // exponentials are taken against ref_max
-    unsigned long long row_sum2 = pf_pack2(0.0f, 0.0f);
+    float ref_max = -INFINITY;                         // exponentials are taken against ref_max, the same in both threads
+    unsigned long long row_sum2 = pf_pack2(0.0f, 0.0f);   // of this thread's columns
     bool ok = true;
     for (int b = 0; b < n_blocks; ++b) {
-      const int kb = k_begin + b * kPlKeys;
-      ok = __all_sync(0xffffffffu, mbar_wait(smem_addr(&score_ready[b & 1]), (b >> 1) & 1, aborted, args.fault, 1 << 13));
+      const int kb = k_begin + b * kPlKeys + half * kPlHalfKeys;     // this thread's first key
+      if (ok) ok = __all_sync(0xffffffffu, mbar_wait(smem_addr(&score_ready[b & 1]), (b >> 1) & 1, aborted, args.fault, 1 << 13));
       // (the values product two blocks back has ended: it was issued before these scores; the wait keeps the barrier's
       // phases in step with the blocks)
       if (ok && b >= 2)
         ok = __all_sync(0xffffffffu, mbar_wait(smem_addr(&value_done[b & 1]), ((b - 2) >> 1) & 1, aborted, args.fault, 1 << 14));
+      float score[kPlHalfKeys];
+      float half_max = -INFINITY;
+      if (ok) {
+        tc_fence_after();
+        uint32_t low[32];
+        float high[16];
+        tmem_load32(tmem_score(b) + lane_bits + half * kPlHalfKeys, low);
+        tmem_load16(tmem_score(b) + lane_bits + half * kPlHalfKeys + 32, high);      // waits for both
+#pragma unroll
+        for (int i = 0; i < 32; ++i) score[i] = __uint_as_float(low[i]);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) score[32 + i] = high[i];
+        if (kb + kPlHalfKeys - 1 > pos || kb < lo_pos) {
+#pragma unroll
+          for (int i = 0; i < kPlHalfKeys; ++i) {
+            const int key = kb + i;
+            if (!(key <= pos && key >= lo_pos)) score[i] = -INFINITY;
+          }
+        }
+        float lane_max[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) lane_max[i] = fmaxf(score[i], score[i + 8]);
+#pragma unroll
+        for (int i = 16; i < kPlHalfKeys; i += 16) {
+#pragma unroll
+          for (int c = 0; c < 8; ++c) lane_max[c] = pf_max3(lane_max[c], score[i + c], score[i + c + 8]);
+        }
+        half_max = fmaxf(pf_max3(lane_max[0], lane_max[1], lane_max[2]),
+                         fmaxf(pf_max3(lane_max[3], lane_max[4], lane_max[5]), fmaxf(lane_max[6], lane_max[7])));
+        exchange[b & 1][half][r] = half_max;
+      }
+      // both have their scores in registers now, so that P may go over them
+      tc_fence_before();
+      ok = named_barrier_and(1 + quarter, 64, ok);
       if (!ok) break;
       tc_fence_after();
-      uint32_t score[3][32];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) tmem_load32(tmem_score(b) + lane_bits + c * 32, score[c]);
-      tmem_wait_ld();
-      if (kb + kPlKeys - 1 > pos || kb < lo_pos) {
-#pragma unroll
-        for (int i = 0; i < kPlKeys; ++i) {
-          const int key = kb + i;
-          if (!(key <= pos && key >= lo_pos)) score[i >> 5][i & 31] = 0xff800000u;
-        }
-      }
-      float lane_max[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) lane_max[i] = fmaxf(__uint_as_float(score[0][i]), __uint_as_float(score[0][i + 8]));
-#pragma unroll
-      for (int i = 16; i < kPlKeys; i += 16) {
-#pragma unroll
-        for (int c = 0; c < 8; ++c)
-          lane_max[c] = pf_max3(lane_max[c], __uint_as_float(score[(i + c) >> 5][(i + c) & 31]),
-                                __uint_as_float(score[(i + c + 8) >> 5][(i + c + 8) & 31]));
-      }
-      float block_max = fmaxf(fmaxf(fmaxf(lane_max[0], lane_max[1]), fmaxf(lane_max[2], lane_max[3])),
-                              fmaxf(fmaxf(lane_max[4], lane_max[5]), fmaxf(lane_max[6], lane_max[7])));
-      block_max *= args.scale_log2;                    // the scale is positive
+      const float block_max = fmaxf(half_max, exchange[b & 1][half ^ 1][r]) * args.scale_log2;     // the scale is positive
       const bool moves = block_max > ref_max + kPfRescaleStep || (ref_max == -INFINITY && block_max > -INFINITY);
       float alpha = 1.0f;
       if (moves) {
@@ -351,14 +366,14 @@ attention_plane_tc_kernel(const __grid_constant__ CUtensorMap map_cache, const P
         pf_unpack2(row_sum2, even, odd);
         row_sum2 = pf_pack2(even * alpha, odd * alpha);
       }
-      // a warp one of whose rows moves rewrites its rows of O (the others times one), after the product of the block
-      // before; the next one waits for this block's P
+      // warps one of whose rows moves rewrite their rows of O (the others times one), after the product of the block
+      // before; the next one waits for this block's P.  A wait that ran out is told at the next meeting point.
       if (b > 0 && __any_sync(0xffffffffu, moves)) {
         ok = __all_sync(0xffffffffu, mbar_wait(smem_addr(&value_done[(b - 1) & 1]), ((b - 1) >> 1) & 1, aborted, args.fault, 1 << 15));
-        if (!ok) break;
+        if (!ok) continue;
         tc_fence_after();
-#pragma unroll
-        for (int c = 0; c < kPlD / 16; ++c) {
+#pragma unroll 2
+        for (int c = half; c < kPlD / 16; c += 2) {
           float value[16];
           uint32_t raw[16];
           tmem_load16(tmem_out + lane_bits + c * 16, value);
@@ -369,19 +384,25 @@ attention_plane_tc_kernel(const __grid_constant__ CUtensorMap map_cache, const P
       }
       const float shift = ref_max == -INFINITY ? 0.0f : ref_max;
       const unsigned long long scale2 = pf_pack2(args.scale_log2, args.scale_log2), shift2 = pf_pack2(-shift, -shift);
+      uint32_t packed[kPlHalfKeys / 2];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        uint32_t packed[16];
+      for (int i = 0; i < kPlHalfKeys / 2; ++i) {
+        float x0, x1;
+        pf_unpack2(pf_fma2(pf_pack2(score[2 * i], score[2 * i + 1]), scale2, shift2), x0, x1);
+        const float e0 = fast_exp2(x0), e1 = fast_exp2(x1);
+        row_sum2 = pf_add2(row_sum2, pf_pack2(e0, e1));
+        const __nv_bfloat162 pair = __floats2bfloat162_rn(e0, e1);
+        packed[i] = *reinterpret_cast<const uint32_t*>(&pair);
+      }
+      {
+        const uint32_t to = tmem_score(b) + lane_bits + half * (kPlHalfKeys / 2);
+        uint32_t first[16], second[8];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          float x0, x1;
-          pf_unpack2(pf_fma2(pf_pack2(__uint_as_float(score[c][2 * i]), __uint_as_float(score[c][2 * i + 1])), scale2, shift2), x0, x1);
-          const float e0 = fast_exp2(x0), e1 = fast_exp2(x1);
-          row_sum2 = pf_add2(row_sum2, pf_pack2(e0, e1));
-          const __nv_bfloat162 pair = __floats2bfloat162_rn(e0, e1);
-          packed[i] = *reinterpret_cast<const uint32_t*>(&pair);
-        }
-        tmem_store16(tmem_score(b) + lane_bits + c * 16, packed);
+        for (int i = 0; i < 16; ++i) first[i] = packed[i];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) second[i] = packed[16 + i];
+        tmem_store16(to, first);
+        tmem_store8(to + 16, second);
       }
       tmem_wait_st();
       tc_fence_before();
@@ -390,15 +411,16 @@ attention_plane_tc_kernel(const __grid_constant__ CUtensorMap map_cache, const P
     }
     if (ok && n_blocks > 0)
       ok = mbar_wait(smem_addr(&value_done[(n_blocks - 1) & 1]), ((n_blocks - 1) >> 1) & 1, aborted, args.fault, 1 << 16);
-    if (__all_sync(0xffffffffu, ok)) {
+    float even, odd;
+    pf_unpack2(row_sum2, even, odd);
+    exchange[n_blocks & 1][half][r] = even + odd;
+    if (named_barrier_and(1 + quarter, 64, ok)) {
       tc_fence_after();
       const int head = kv_head * group + (p - token * group);
       const size_t row = static_cast<size_t>(tok_begin + token) * args.hq + head;
-      float even, odd;
-      pf_unpack2(row_sum2, even, odd);
-      float row_sum = even + odd;
+      float row_sum = exchange[n_blocks & 1][0][r] + exchange[n_blocks & 1][1][r];
       const bool whole = args.splits == 1;
-      if (!whole && exists)
+      if (!whole && exists && half == 0)
         args.part_lse[row * args.splits + split] = row_sum > 0.0f ? ref_max + log2f(row_sum) : -INFINITY;
       if (whole && args.sink != nullptr && exists) {
         // the sink's term against the same reference point as the keys' (an infinite one: it alone counts, the row is zero)
@@ -411,7 +433,7 @@ attention_plane_tc_kernel(const __grid_constant__ CUtensorMap map_cache, const P
       float* part = args.part_out + (row * args.splits + split) * kPlD;
       if (whole || n_blocks > 0) {                     // (the merge does not read a part without keys)
 #pragma unroll 4
-        for (int c = 0; c < kPlD / 16; ++c) {
+        for (int c = half; c < kPlD / 16; c += 2) {
           float value[16];
           if (n_blocks > 0) {
             tmem_load16(tmem_out + lane_bits + c * 16, value);

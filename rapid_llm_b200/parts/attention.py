@@ -124,6 +124,7 @@ class AttentionItems(StepPlanner):
         # one_plane: the cached rows are keys and values at once; chunk tiles then have 128 rows where the tcgen05
         # kernel for such caches takes the row and page size.
         self.one_plane = bool(one_plane)
+        self.plane_decode_tiles = int(sms)
         # window: the same bound for the key ranges where a mixer asks for it (0 = not bounded).
         self.chunk, self.window = int(chunk), int(window)
         self.decode_clusters = dict(decode_clusters or DEFAULT_DECODE_CLUSTERS)
@@ -150,14 +151,18 @@ class AttentionItems(StepPlanner):
         is_decode = (lengths == 1) | (rows <= kernels.DECODE_TILE_ROWS)
         tensor_core = self.tensor_core and kernels.attention_tc_takes(self.head_dim, shape.page_size)
         plane = self.one_plane and kernels.attention_plane_tc_takes(self.head_dim, shape.page_size)
-        if plane:
+        # Single tokens, too: their heads are the rows of a tile.  A tile of fewer than 16 rows costs the mma.sync kernel no
+        # more than it costs a multiprocessor to itself once there are more tiles than those and the context is short
+        # (4 heads, 200 tokens: 28 against 33 us behind 256 keys, 102 against 96 behind 2,048; 16 heads: 34 and 34, 110
+        # and 97; 64 tokens of 4 heads behind 1,024: 42 against 34).
+        if plane and (self.group >= kernels.DECODE_TILE_ROWS or int(is_decode.sum()) * self.num_kv_heads <= self.plane_decode_tiles):
             is_decode = np.zeros_like(is_decode)
         for chunk_rows in ((kernels.CHUNK_TILE_ROWS_PLANE,) if plane else
                            (kernels.CHUNK_TILE_ROWS_TC, kernels.CHUNK_TILE_ROWS) if tensor_core else (kernels.CHUNK_TILE_ROWS,)):
             tile_rows = np.where(is_decode, kernels.DECODE_TILE_ROWS, chunk_rows)
             tiles = -(-rows // tile_rows)
             ctas = int(tiles.sum()) * self.num_kv_heads
-            # (a tile of 128 rows has a multiprocessor to itself, as in a decode-only step)
+            # (a tile of 128 rows has a multiprocessor to itself, as a tile has in a decode-only step)
             target = self.decode_target_ctas if shape.decode_only or plane else self.target_ctas
             splits = max(1, min(MAX_SPLITS, target // max(ctas, 1)))
             if self.chunk:
