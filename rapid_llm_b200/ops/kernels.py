@@ -1592,16 +1592,22 @@ def moe_wide_takes(dtype: torch.dtype, *inner_sizes: int) -> bool:
     return dtype == torch.bfloat16 and all(size % 8 == 0 for size in inner_sizes)
 
 
-MOE_FEW_PAIRS, MOE_TENSOR_PAIRS = 8, 32      # pairs per expert up to and from which a kernel is the fastest
+# Where the product kernels' lines lie, in elements (a pair's inner product sizes, hidden x inter).  Measured with cold
+# weights, both products together, few / 64-pair tiles / tensor, us.  hidden 2,048, inter 512, 2 of 16 experts: 1 token
+# 23 / 39 / 38, 8 tokens 42 / 44 / 41, 32 tokens 53 / 53 / 47, 2,048 tokens - / 139 / 90; hidden 4,096, inter 1,024:
+# 1 token 33 / 63 / 58, 8 tokens 101 / 110 / 93, 2,048 tokens - / 449 / 195; hidden 1,024, inter 256, 1 of 8: 8 tokens
+# 21 / 29 / 30, 64 tokens 22 / 29 / 31, 128 tokens 27 / 29 / 30, 2,048 tokens - / 37 / 39.
+MOE_FEW_ELEMENTS = 1 << 24        # pairs x hidden x inter up to which the weights' stream is short
+MOE_TENSOR_ELEMENTS = 1 << 19     # hidden x inter from which a tile of the tensor cores is worth its start
 
 
-def moe_kind(dtype: torch.dtype, pairs: int, experts: int, hidden: int, inter: int):
+def moe_kind(dtype: torch.dtype, pairs: int, hidden: int, inter: int):
     """Which product kernels a step's pairs run on (see :func:`moe_tile_rows`)."""
     if not moe_wide_takes(dtype, hidden, inter):
         return False
-    if pairs <= MOE_FEW_PAIRS * experts and max(hidden, inter) <= 6144:
+    if pairs * hidden * inter <= MOE_FEW_ELEMENTS and max(hidden, inter) <= 6144:
         return "few"
-    return "tensor" if pairs >= MOE_TENSOR_PAIRS * experts else True
+    return "tensor" if hidden * inter >= MOE_TENSOR_ELEMENTS else True
 
 
 def moe_max_tiles(pairs: int, experts: int, wide=False) -> int:
