@@ -115,7 +115,7 @@ def kernel_figures(width: int, hbm_gbs: float) -> dict:
         timed("latent_rotate_queries", tokens, entries, tokens * heads * (ROT + d - KV_RANK) * 2,
               lambda: kernels.latent_rotate_queries(q, wide, heads=heads, dim=PLAIN, rot=ROT, kv_rank=KV_RANK, positions=positions,
                                                     freq=freq, magnitude=1.2, layout=kernels.ROTATE_NEIGHBOURS))
-        planner = AttentionItems(heads, 1, d, tensor_core=False)
+        planner = AttentionItems(heads, 1, d, tensor_core=False, one_plane=True)
         plan = planner.plan(StepShape(lengths=np.full(entries, per, dtype=np.int32), starts=np.full(entries, start, dtype=np.int32),
                                       decode_only=per == 1, page_size=page))
         chunk = torch.from_numpy(plan["chunk_items"]).to(device)
@@ -133,7 +133,7 @@ def kernel_figures(width: int, hbm_gbs: float) -> dict:
                   part_out=part_out, part_lse=part_lse, cu_seqlens=batch.cu_seqlens, entry_start=batch.entry_start,
                   entry_slot=batch.entry_slot, block_table=table, num_heads=heads, num_kv_heads=1, head_dim=d, window=0,
                   scale=(PLAIN + ROT) ** -0.5, fault=fault, decode_kernel="mma", decode_rows=plan.get("decode_rows", 0),
-                  chunk_rows=kernels.CHUNK_TILE_ROWS),
+                  chunk_rows=plan["chunk_rows"]),
               flops=4.0 * keys * heads * d)
         values = torch.empty(tokens, heads * VDIM, dtype=torch.bfloat16, device=device)
         timed("heads_linear, values out of the latent", tokens, entries,

@@ -164,7 +164,7 @@ def kernel_figures(width: int, hbm_gbs: float) -> dict:
         wide_out = torch.empty_like(wide_q)
         sink = f32(heads)
         for label, window, term in (("attention over cached rows, window of 512, sink", WINDOW, sink), ("attention over cached rows, all keys (like kernel)", 0, None)):
-            plan = AttentionItems(heads, 1, wide_d, tensor_core=False, window=window).plan(step)
+            plan = AttentionItems(heads, 1, wide_d, tensor_core=False, window=window, one_plane=True).plan(step)
             items = {name: torch.from_numpy(plan[name]).to(device) for name in ("chunk_items", "decode_items")}
             splits = plan["splits"]
             part_out = torch.empty(tokens * heads * splits, wide_d, device=device) if splits > 1 else None
@@ -176,7 +176,7 @@ def kernel_figures(width: int, hbm_gbs: float) -> dict:
                 wide_q, rows_cache.view(-1, 1, 1, page, wide_d), wide_out, splits=splits, part_out=part_out, part_lse=part_lse,
                 cu_seqlens=batch.cu_seqlens, entry_start=batch.entry_start, entry_slot=batch.entry_slot, block_table=table, num_heads=heads,
                 num_kv_heads=1, head_dim=wide_d, window=window, scale=(PLAIN + ROT) ** -0.5, fault=fault, sink=term, decode_kernel="mma",
-                decode_rows=plan["decode_rows"], chunk_rows=kernels.CHUNK_TILE_ROWS, **items), flops=4.0 * keys * heads * wide_d)
+                decode_rows=plan["decode_rows"], chunk_rows=plan["chunk_rows"], **items), flops=4.0 * keys * heads * wide_d)
         # -- the recurrent mixer: decays from the low-rank rows with q, k and v as float32, beside wkv's three kernels
         c, rec_heads = width, width // WKV_DIM
         proj = bf(tokens, 4 * c + RANK)
