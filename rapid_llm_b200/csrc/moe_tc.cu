@@ -109,12 +109,11 @@ grouped_linear_tc_kernel(const __grid_constant__ CUtensorMap map_w, const MoeTcA
           if (++stage == kMoeTcStages) { stage = 0; phase ^= 1u; }
         }
       }
-      if (!ok || *aborted) {
-        // copies still in flight must land before the CTA may exit
-        for (int s = 0; s < kMoeTcStages; ++s) {
-          const int fills = (filled - s + kMoeTcStages - 1) / kMoeTcStages;
-          if (fills > 0) mbar_wait(smem_addr(&weights_bar[s]), static_cast<uint32_t>((fills - 1) & 1), aborted, args.fault);
-        }
+      // the copies land before the shared memory goes, also when the others have given up
+      volatile int go_on = 0;
+      for (int s = 0; s < kMoeTcStages; ++s) {
+        const int fills = (filled - s + kMoeTcStages - 1) / kMoeTcStages;
+        if (fills > 0) mbar_wait(smem_addr(&weights_bar[s]), static_cast<uint32_t>((fills - 1) & 1), &go_on, args.fault);
       }
     }
   } else if (warp == 1) {

@@ -1,0 +1,20 @@
+"""Rules of the CUDA sources that a run on a GPU shows only when something else has already gone wrong."""
+
+import re
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parent.parent / "rapid_llm_b200" / "csrc"
+
+
+@pytest.mark.parametrize("name", ["moe_tc.cu", "attention_plane_tc.cuh"])
+def test_copies_in_flight_are_waited_for_after_the_others_gave_up(name):
+    """A wait under the block's abort flag gives up at once when the flag is set: the last wait for the copies has a flag of
+    its own, and nothing skips it."""
+    source = (CSRC / name).read_text()
+    drain = source.index("volatile int go_on = 0;")
+    loop = source[drain : source.index("\n    }\n", drain)]
+    waits = re.findall(r"mbar_wait\((.*)\);", loop)
+    assert waits and all("&go_on" in wait and "aborted" not in wait for wait in waits)
+    assert "*aborted" not in source[source.rindex("tma_load_2d(", 0, drain) : drain]
