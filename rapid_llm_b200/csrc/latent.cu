@@ -112,7 +112,7 @@ __global__ void latent_rotate_queries_kernel(const T* q, int heads, int dim, int
 // rows[t, h, 0:width] *= sigmoid(gate[t, gate_col0 + h]), in place.
 // kVec elements (16 bytes) a thread and round where a head's width is a multiple of kVec; else one.
 template <typename T, int kVec>
-__global__ void sigmoid_scale_heads_kernel(T* __restrict__ rows, int heads, int width, const T* __restrict__ gate,
+__global__ void sigmoid_scale_heads_kernel(T* __restrict__ rows, int heads, int width, const T* gate,
                                            int gate_stride, int gate_col0, long long total) {
   pdl_trigger();
   pdl_wait();
@@ -149,7 +149,7 @@ __global__ void sigmoid_scale_heads_kernel(T* __restrict__ rows, int heads, int 
 constexpr int kHeadTile = 64, kHeadStep = 16;
 
 template <typename T>
-__global__ void __launch_bounds__(256) heads_linear_kernel(const T* __restrict__ x, int x_width, int x_col0,
+__global__ void __launch_bounds__(256) heads_linear_kernel(const T* x, int x_width, int x_col0,
                                                            const T* __restrict__ w, T* __restrict__ out,
                                                            int out_width, int tokens, int heads, int N, int K) {
   __shared__ float xs[kHeadStep][kHeadTile + 4];
@@ -210,7 +210,7 @@ constexpr int kHeadRowRegs = 8, kHeadColumnsPerCta = 8, kHeadTokensPerCta = 8;
 
 template <typename T>
 __global__ void __launch_bounds__(32 * kHeadColumnsPerCta) heads_linear_few_kernel(
-    const T* __restrict__ x, int x_width, int x_col0, const T* __restrict__ w, T* __restrict__ out, int out_width,
+    const T* x, int x_width, int x_col0, const T* __restrict__ w, T* __restrict__ out, int out_width,
     int tokens, int heads, int N, int K) {
   pdl_trigger();
   const int h = blockIdx.x, lane = threadIdx.x & 31;

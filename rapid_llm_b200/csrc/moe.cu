@@ -273,7 +273,7 @@ router_topk_kernel(const T* x, int x_stride, const float* __restrict__ w, int hi
 // One block.  meta: [0] tiles, then per tile (expert, first place, rows).  `sorted` [pairs] receives pair
 // indices expert by expert.  `place_of` [pairs]: where pair i went (the inverse of sorted).  Bound by its few trips to
 // memory one after the other (4,096 pairs: 16 us while a thread walked an expert's pairs, 12 with all counting at once).
-__global__ void moe_plan_kernel(const int* __restrict__ ids, int pairs, int experts, int* __restrict__ sorted,
+__global__ void moe_plan_kernel(const int* ids, int pairs, int experts, int* __restrict__ sorted,
                                 int* __restrict__ place_of, int* __restrict__ meta, int max_tiles, int tile_m,
                                 int* __restrict__ fault) {
   extern __shared__ int moe_counts[];      // [experts] counts, [experts] cursors
@@ -346,8 +346,8 @@ __global__ void moe_plan_kernel(const int* __restrict__ ids, int pairs, int expe
 // : y[pair, N] (float32).
 template <typename T, bool kGated>
 __global__ void __launch_bounds__(kMoeThreads)
-grouped_linear_fma_kernel(const T* a, int a_stride, const T* __restrict__ w, const int* __restrict__ sorted,
-                          const int* __restrict__ meta, const float* __restrict__ pair_weight, int top, int by_token,
+grouped_linear_fma_kernel(const T* a, int a_stride, const T* __restrict__ w, const int* sorted,
+                          const int* meta, const float* pair_weight, int top, int by_token,
                           int n, int k, T* out_act, float* out_y, float glu_limit, float glu_alpha) {
   __shared__ float sa[kMoeTileM][kMoeTileK + 1];
   __shared__ float sw[kGated ? 2 : 1][kMoeTileN][kMoeTileK + 1];
@@ -438,8 +438,8 @@ __device__ __forceinline__ void moe_mma_bf16(float (&c)[4], const uint32_t (&a)[
 template <bool kGated>
 __global__ void __launch_bounds__(kMoeThreads)
 grouped_linear_mma_kernel(const __nv_bfloat16* a, int a_stride, const __nv_bfloat16* __restrict__ w,
-                          const int* __restrict__ sorted, const int* __restrict__ meta,
-                          const float* __restrict__ pair_weight, int top, int by_token, int n, int k,
+                          const int* sorted, const int* meta,
+                          const float* pair_weight, int top, int by_token, int n, int k,
                           __nv_bfloat16* out_act, float* out_y, float glu_limit, float glu_alpha) {
   constexpr int kStride = kMoeTileK + 8;      // elements; rows stay 16-byte aligned and spread over the banks
   __shared__ __align__(16) __nv_bfloat16 sa[kMoeTileM][kStride];
@@ -582,8 +582,8 @@ constexpr int moe_wide_smem_bytes() {
 template <bool kGated>
 __global__ void __launch_bounds__(kMoeThreads)
 grouped_linear_wide_kernel(const __nv_bfloat16* a, int a_stride, const __nv_bfloat16* __restrict__ w,
-                           const int* __restrict__ sorted, const int* __restrict__ meta,
-                           const float* __restrict__ pair_weight, int top, int by_token, int n, int k,
+                           const int* sorted, const int* meta,
+                           const float* pair_weight, int top, int by_token, int n, int k,
                            __nv_bfloat16* out_act, float* out_y, float glu_limit, float glu_alpha) {
   constexpr int kStride = kMoeWideK + 8;
   constexpr int kWRows = (kGated ? 2 : 1) * kMoeTileN;
@@ -896,9 +896,9 @@ __global__ void __launch_bounds__(256) moe_combine_wide_kernel(const float* y, i
 }
 
 template <typename T>
-__global__ void moe_combine_kernel(const float* __restrict__ y, int top, const T* shared, const float* __restrict__ gate,
+__global__ void moe_combine_kernel(const float* y, int top, const T* shared, const float* gate,
                                    int gate_stride, T* __restrict__ out, int tokens, int hidden, const float* weights,
-                                   const int* __restrict__ ids, int experts, const T* __restrict__ x, int x_stride) {
+                                   const int* ids, int experts, const T* x, int x_stride) {
   pdl_trigger();
   pdl_wait();
   const long long total = static_cast<long long>(tokens) * hidden;
@@ -930,8 +930,8 @@ __global__ void moe_combine_kernel(const float* __restrict__ y, int top, const T
 // as the mean of squared deviations; the stream takes n, out its rounding.  The row waits in shared memory between
 // the passes; the sums run down the block's fixed tree.
 template <typename T>
-__global__ void moe_combine_layernorm_kernel(const float* __restrict__ y, int top, const float* __restrict__ weights,
-                                             const int* __restrict__ ids, int experts, const T* __restrict__ x,
+__global__ void moe_combine_layernorm_kernel(const float* y, int top, const float* weights,
+                                             const int* ids, int experts, const T* x,
                                              int x_stride, float* __restrict__ stream, float res_scale,
                                              const float* __restrict__ ln_weight, const float* __restrict__ ln_bias,
                                              float eps, T* __restrict__ out, int hidden) {

@@ -18,3 +18,15 @@ def test_copies_in_flight_are_waited_for_after_the_others_gave_up(name):
     waits = re.findall(r"mbar_wait\((.*)\);", loop)
     assert waits and all("&go_on" in wait and "aborted" not in wait for wait in waits)
     assert "*aborted" not in source[source.rindex("tma_load_2d(", 0, drain) : drain]
+
+
+# what no kernel of a step writes: weights, tables made when the weights are loaded, the step's uploaded metadata
+STEADY = {"w", "wq", "wc", "bias", "correction", "weight", "ln_weight", "ln_bias", "taps", "rate", "mu", "pq", "freq", "inv_freq",
+          "cu_seqlens", "entry_slot", "entry_start", "positions", "kv_dest"}
+
+
+@pytest.mark.parametrize("name", ["moe.cu", "moe_tc.cu", "latent.cu", "recurrent.cu"])
+def test_what_a_step_writes_is_not_read_as_invariant(name):
+    """A load through a const restrict pointer may be moved above the wait for the kernel before."""
+    invariant = set(re.findall(r"const [\w:]+\* ?__restrict__ (\w+)", (CSRC / name).read_text()))
+    assert invariant <= STEADY, sorted(invariant - STEADY)
