@@ -1261,6 +1261,16 @@ def scan_takes_pieces(dim: int, vdim: int) -> bool:
     return 32 < dim <= 128 and dim % 4 == 0 and vdim % 4 == 0
 
 
+def scan_buffers(space, tokens: int, heads: int, dim: int, vdim: int, corrected: bool):
+    """States, products of decays (without a correction) and matrices (with one) of the pieces a step can have: sized once
+    for the largest step ``space`` is made for, so that prompts of growing length allocate nothing."""
+    most, piece = max(space.max_tokens, tokens), scan_piece(heads, vdim, corrected)
+    rows = most // piece + most // (piece + 1)      # whole pieces, and a remainder of each entry longer than one
+    get = lambda name, cols: space.get(name, rows, cols, torch.float32, min_rows=rows)      # noqa: E731
+    states = get("scan_states", heads * dim * vdim)
+    return (states, None, get("scan_mats", heads * dim * dim)) if corrected else (states, get("scan_decays", heads * dim), None)
+
+
 def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, out: torch.Tensor,
                 state: torch.Tensor, batch, *, heads: int, kv_heads: int, dim: int, vdim: int,
                 beta: torch.Tensor | None = None, v_scale: torch.Tensor | None = None,
@@ -1308,12 +1318,7 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.
     if pieces is not None and scan_takes_pieces(dim, vdim) and batch.max_query_len >= scan_pieces_from(heads, vdim, beta is not None):
         piece = scan_piece(heads, vdim, beta is not None)
         blocks = tokens // piece + batch.num_entries
-        kept = tokens // piece + min(batch.num_entries, tokens // (piece + 1))      # of entries longer than a piece
-        states = pieces.get("scan_states", kept, heads * dim * vdim, torch.float32, min_rows=kept)
-        if beta is None:
-            decays = pieces.get("scan_decays", kept, heads * dim, torch.float32, min_rows=kept)
-        else:
-            mats = pieces.get("scan_mats", kept, heads * dim * dim, torch.float32, min_rows=kept)
+        states, decays, mats = scan_buffers(pieces, tokens, heads, dim, vdim, beta is not None)
     _check(
         recurrent().rl_linear_scan(
             _ptr(q), _row_stride("q", q), _ptr(k), _row_stride("k", k), _ptr(v), _row_stride("v", v), _ptr(decay), mode,
