@@ -632,12 +632,12 @@ __global__ void rotate_heads_kernel(const T* in, int in_stride, int q_col0, int 
 // Then the instructions a token takes (about 90 a warp) with one warp a scheduler to issue them (0.3 a cycle): a walk from
 // end to end cannot use the rest of the GPU, so in 16-bit engines long prompts are walked in pieces (below).
 // A correction (beta) makes a token wait for the sum over the whole column of the token before it: there a column has
-// few lanes with many rows each, since an exchange between lanes waits as long as eight multiply-adds.
-// 2,048 tokens, us, before / from end to end / in pieces: 16 heads of 128, fixed decay 432 / 288 / 183; 32 heads of 64, row
-// decays 380 / 249 / 136; with a bonus 333 / 270 / 148; 32 heads of 128, fixed, 3 prompts 551 / 420 / 331; with a
-// correction, 16 heads of 128, 632 / 567 / 433.  64 single tokens: 64 heads of 64, row decays 54 / 31 (4.3 TB/s), 16 heads of
-// 128, fixed 53 / 31 (see the kernel).  Against 64 bits the error is what it was (1.1e-7; fixed decays 2.6e-7; with a correction
-// 1.4e-7 from end to end and 1.41e-7 in pieces of 256, 1.54e-7 in pieces of 128).
+// few lanes with many rows each, since an exchange between lanes waits as long as eight multiply-adds, and prompts are
+// walked from end to end (in pieces the state has to go through a matrix per piece, which costs digits).
+// 2,048 tokens, us, before / from end to end / in pieces: 16 heads of 128, fixed decay 432 / 288 / 187; 32 heads of 64, row
+// decays 383 / 255 / 138; with a bonus 334 / 278 / 151; 32 heads of 128, fixed, 3 prompts 552 / 410 / 339; with a
+// correction, 16 heads of 128, 632 / 572.  64 single tokens: 64 heads of 64, row decays 54 / 31 (4.3 TB/s), 16 heads of
+// 128, fixed 53 / 31 (see the kernel).
 struct ScanArgs {
   const float* q; int q_stride;
   const float* k; int k_stride;
@@ -658,7 +658,6 @@ struct ScanArgs {
   int segment;            // 0: a block walks its entry from end to end; else at most so many tokens, from a state of its own
   float* seg_states;      // [pieces, heads, vdim, dim]: what a piece alone leaves, then what it starts from
   float* seg_decays;      // [pieces, heads, dim]: the product of a piece's decays
-  float* seg_mats;        // [pieces, heads, dim, dim]: with beta, what a piece makes of each unit column
 };
 
 // The piece that block `index` owns: of which entry, which one of the entry's, its tokens, its place in the arrays of
@@ -851,17 +850,6 @@ struct ScanColumns {
       }
     }
   }
-  // Column c becomes the unit vector of row `row0 + c`; columns before row 0 stay as they are.
-  __device__ __forceinline__ void units(int row0, int part) {
-#pragma unroll
-    for (int c = 0; c < kCols; ++c) {
-#pragma unroll
-      for (int r = 0; r < kRows / 2; ++r) {
-        const int row = ((r / 2) * kPartners + part) * 4 + (r & 1) * 2;
-        if (row0 + c >= 0) S[c][r] = pair_of<P>(row == row0 + c ? 1.0f : 0.0f, row + 1 == row0 + c ? 1.0f : 0.0f);
-      }
-    }
-  }
   __device__ __forceinline__ void clear() {
 #pragma unroll
     for (int c = 0; c < kCols; ++c)
@@ -946,8 +934,7 @@ __global__ void __launch_bounds__(kScanThreads) linear_scan_kernel(const ScanArg
   constexpr int kPadded = kPartners * kRows;
   const int col_in_tile = (warp * kSpread + lane / kPartners) * kCols;
   const int col = blockIdx.z * kTile + col_in_tile;
-  // columns of this lane that exist; with a correction a piece also takes the unit columns, which lie behind the values'
-  const int left = a.vdim + (!kRead && kKind == kScanDelta ? a.dim : 0) - col;
+  const int left = a.vdim - col;      // columns of this lane that exist
   const int kv_head = head / (a.heads / a.kv_heads);
 
   const int first = seg.first, length = seg.length, start = a.entry_start[e];
@@ -1049,7 +1036,6 @@ __global__ void __launch_bounds__(kScanThreads) linear_scan_kernel(const ScanArg
   ScanColumns<kRows, kPartners, kCols, kKind, kRowDecay, kRead, P> mine;
   if constexpr (!kRead) {
     mine.clear();
-    if constexpr (kKind == kScanDelta) mine.units(col - a.vdim, part);
   } else if (seg.of == 1) {
     if (start > 0) mine.load(home, a.dim, part, left, wide); else mine.clear();
   } else if (start > 0 || seg.number > 0) {
@@ -1152,7 +1138,7 @@ __global__ void __launch_bounds__(kScanThreads) linear_scan_kernel(const ScanArg
         if constexpr (kRead) {
 #pragma unroll
           for (int c = 0; c < kCols; ++c) o[g * kCols + c] = one[c];
-        } else if constexpr (kKind != kScanDelta) {
+        } else {
           multiply(now, decay);
         }
       }
@@ -1165,19 +1151,15 @@ __global__ void __launch_bounds__(kScanThreads) linear_scan_kernel(const ScanArg
       const float decay = kRowDecay ? 1.0f : sdecay[tt];
       mine.take(now, decay, scaled, o);
       if constexpr (kRead) finish(std::integral_constant<int, 1>{}, o, tt);
-      else if constexpr (kKind != kScanDelta) multiply(now, decay);
+      else multiply(now, decay);
     }
     __syncthreads();     // the buffer is free for the run after the next
   }
   pdl_trigger();
   if (left <= 0) return;
   if constexpr (!kRead) {
-    const int values = a.vdim - col;      // columns of this lane in front of the unit columns
-    // (a lane's columns are all values' or all units': vdim is a multiple of kCols here)
-    if (values > 0) mine.store(a.seg_states + own * a.vdim + in_head, a.dim, part, min(left, values), true);
-    if constexpr (kKind == kScanDelta) {
-      if (values <= 0) mine.store(a.seg_mats + own * a.dim + static_cast<size_t>(-values) * a.dim, a.dim, part, left, true);
-    } else if (blockIdx.z == 0 && threadIdx.x < kPartners) {
+    mine.store(a.seg_states + own * a.vdim + in_head, a.dim, part, left, true);
+    if (blockIdx.z == 0 && threadIdx.x < kPartners) {
 #pragma unroll
       for (int r = 0; r < kRows / 2; ++r) {
         const int row = ((r / 2) * kPartners + part) * 4 + (r & 1) * 2;
@@ -1221,92 +1203,6 @@ __global__ void __launch_bounds__(256) scan_join_kernel(const ScanArgs a) {
     const float4 left = *state, d = *reinterpret_cast<const float4*>(a.seg_decays + own + row);
     *state = S;
     S.x = fmaf(S.x, d.x, left.x); S.y = fmaf(S.y, d.y, left.y); S.z = fmaf(S.z, d.z, left.z); S.w = fmaf(S.w, d.w, left.w);
-  }
-}
-
-// The same with a correction: start' = M start + left, M the piece's matrix (its unit columns).  A block owns eight columns
-// of S, which lie in shared memory; a thread forms two rows of them, the matrix read once per block from L2, sixteen of its
-// columns on their way while sixteen are multiplied (without that a piece took 14 us, with it 7).
-constexpr int kJoinCols = 8, kJoinThreads = 64;
-__global__ void __launch_bounds__(kJoinThreads) scan_join_delta_kernel(const ScanArgs a) {
-  __shared__ __align__(16) float start[2 * kJoinThreads][kJoinCols];
-  const int e = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * kJoinCols;
-  int place;
-  const int pieces = scan_pieces_of(a, e, place);
-  int slot = a.entry_slot[e];
-  if (slot < 0 || slot >= a.slots) slot = 0;      // the walk says so in the fault word
-  pdl_wait();
-  if (pieces <= 1) return;
-  const bool carried = a.entry_start[e] > 0;
-  const float* home = a.state + slot * a.state_stride + a.state_off + static_cast<size_t>(head) * a.dim * a.vdim;
-  const int count = min(kJoinCols, a.vdim - col0);
-  const int rows[2] = {min(static_cast<int>(threadIdx.x), a.dim - 1), min(static_cast<int>(threadIdx.x) + kJoinThreads, a.dim - 1)};
-  float S[2][kJoinCols];
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int row = threadIdx.x + h * kJoinThreads;
-#pragma unroll
-    for (int c = 0; c < kJoinCols; ++c)
-      S[h][c] = carried && row < a.dim && c < count ? home[static_cast<size_t>(col0 + c) * a.dim + row] : 0.0f;
-  }
-  for (int p = 0; p < pieces; ++p) {
-    const size_t own = (static_cast<size_t>(place + p) * a.heads + head) * a.dim;
-    float* states = a.seg_states + own * a.vdim + static_cast<size_t>(col0) * a.dim;
-    const float* mat = a.seg_mats + own * a.dim;
-    const bool last = p == pieces - 1;
-    constexpr int kAhead = 16;
-    float m[2][kAhead][2];
-    auto fetch = [&](int buffer, int j0) {
-#pragma unroll
-      for (int j = 0; j < kAhead; ++j)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) m[buffer][j][h] = mat[static_cast<size_t>(min(j0 + j, a.dim - 1)) * a.dim + rows[h]];
-    };
-    if (!last) fetch(0, 0);
-    float next[2][kJoinCols];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const bool mine = static_cast<int>(threadIdx.x) + h * kJoinThreads < a.dim;
-#pragma unroll
-      for (int c = 0; c < kJoinCols; ++c) next[h][c] = mine && c < count && !last ? states[static_cast<size_t>(c) * a.dim + rows[h]] : 0.0f;
-#pragma unroll
-      for (int c = 0; c < kJoinCols; ++c)
-        if (mine && c < count) states[static_cast<size_t>(c) * a.dim + rows[h]] = S[h][c];
-    }
-    if (last) break;
-    __syncthreads();      // the piece before has been read
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
-#pragma unroll
-      for (int c = 0; c < kJoinCols; ++c) start[threadIdx.x + h * kJoinThreads][c] = S[h][c];
-    __syncthreads();
-    auto multiply = [&](int buffer, int j0) {
-#pragma unroll
-      for (int j = 0; j < kAhead; ++j) {
-        if (j0 + j >= a.dim) break;
-        float s[kJoinCols];
-#pragma unroll
-        for (int c = 0; c < kJoinCols; c += 4) {
-          const float4 four = *reinterpret_cast<const float4*>(&start[j0 + j][c]);
-          s[c] = four.x; s[c + 1] = four.y; s[c + 2] = four.z; s[c + 3] = four.w;
-        }
-#pragma unroll
-        for (int c = 0; c < kJoinCols; ++c) {
-          next[0][c] = fmaf(m[buffer][j][0], s[c], next[0][c]);
-          next[1][c] = fmaf(m[buffer][j][1], s[c], next[1][c]);
-        }
-      }
-    };
-    for (int j0 = 0; j0 < a.dim; j0 += 2 * kAhead) {
-      fetch(1, j0 + kAhead);
-      multiply(0, j0);
-      fetch(0, j0 + 2 * kAhead);
-      multiply(1, j0 + kAhead);
-    }
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
-#pragma unroll
-      for (int c = 0; c < kJoinCols; ++c) S[h][c] = next[h][c];
   }
 }
 
@@ -1650,8 +1546,7 @@ static int launch_scan(ScanArgs a, int blocks, int pdl, cudaStream_t stream) {
   constexpr int kRun = 20 * 1024 / 4 / kPerToken;      // two buffers of a run each within 40 KB
   a.run = kRun > 16 ? 16 : (kRun < 1 ? 1 : kRun);
   const size_t smem = 2 * static_cast<size_t>((a.run * kPerToken + 3) & ~3) * sizeof(float);
-  const int columns = a.vdim + (!kRead && kKind == kScanDelta ? a.dim : 0);
-  const dim3 grid(blocks, a.heads, (columns + kTile - 1) / kTile);
+  const dim3 grid(blocks, a.heads, (a.vdim + kTile - 1) / kTile);
   return launch_kernel(linear_scan_kernel<kRows, kPartners, kCols, kKind, kRowDecay, kRead>, grid, dim3(kScanThreads), smem,
                        stream, pdl != 0, a);
 }
@@ -1687,14 +1582,8 @@ static int launch_delta_scan(const ScanArgs& a, int blocks, int pdl, cudaStream_
 // In pieces there are blocks enough: more rows a lane and four columns, fewer exchanges and fetches a column.
 template <int kKind, bool kRowDecay, bool kRead>
 static int launch_pieces(const ScanArgs& a, int blocks, int pdl, cudaStream_t stream) {
-  if constexpr (kKind == kScanDelta) {
-    // four columns a lane where a column has eight lanes and its read-outs are summed: 194 -> 163 us at 16 heads of 128
-    if (a.dim <= 64) return launch_scan<16, 4, 2, kKind, true, kRead>(a, blocks, pdl, stream);
-    return launch_scan<16, 8, kRead ? 4 : 2, kKind, true, kRead>(a, blocks, pdl, stream);
-  } else {
-    return a.dim <= 64 ? launch_scan<8, 8, 4, kKind, kRowDecay, kRead>(a, blocks, pdl, stream)
-                       : launch_scan<8, 16, 4, kKind, kRowDecay, kRead>(a, blocks, pdl, stream);
-  }
+  return a.dim <= 64 ? launch_scan<8, 8, 4, kKind, kRowDecay, kRead>(a, blocks, pdl, stream)
+                     : launch_scan<8, 16, 4, kKind, kRowDecay, kRead>(a, blocks, pdl, stream);
 }
 
 template <int kRows, int kPartners, int kCols, int kKind, bool kRowDecay>
@@ -1870,7 +1759,7 @@ int rl_linear_scan(const float* q, int q_stride, const float* k, int k_stride, c
                    const float* bonus, float* out, int out_stride, float* state, long long state_stride, int state_off,
                    const int* cu_seqlens, const int* entry_slot, const int* entry_start, int entries, int tokens, int heads,
                    int kv_heads, int dim, int vdim, int slots, int* fault, int segment, int segments, float* seg_states,
-                   float* seg_decays, float* seg_mats, int pdl, cudaStream_t stream) {
+                   float* seg_decays, int pdl, cudaStream_t stream) {
   if (entries == 0) return 0;
   if (heads < 1 || kv_heads < 1 || heads % kv_heads || dim < 1 || dim > 1024 || vdim < 1 || decay_mode < 0 ||
       decay_mode > 2 || decay == nullptr || (bonus != nullptr && beta != nullptr))
@@ -1887,7 +1776,7 @@ int rl_linear_scan(const float* q, int q_stride, const float* k, int k_stride, c
               aligned(q) && aligned(k) && aligned(v) && (decay_mode != 2 || aligned(decay));
   a.entries = entries;
   a.segment = segment;
-  a.seg_states = seg_states; a.seg_decays = seg_decays; a.seg_mats = seg_mats;
+  a.seg_states = seg_states; a.seg_decays = seg_decays;
   using namespace rl;
   // single tokens of the common head sizes: the same rows a lane and lanes a column as the walk, so the same sums
   if (segment == 0 && tokens == entries && a.wide_in && dim > 32 && dim <= 128) {
@@ -1910,20 +1799,12 @@ int rl_linear_scan(const float* q, int q_stride, const float* k, int k_stride, c
     return launch_plain_scan<kScanPlain, false>(a, entries, pdl, stream);
   }
   // in pieces side by side: sizes and pieces the kernels are made for
-  if (segment < 0 || dim <= 32 || dim > 128 || dim % 4 || vdim % 4 || segments < 1 || seg_states == nullptr ||
-      (beta ? seg_mats == nullptr : seg_decays == nullptr) || !aligned(seg_states) || !aligned(seg_decays) || !aligned(seg_mats))
+  if (segment < 0 || beta != nullptr || dim <= 32 || dim > 128 || dim % 4 || vdim % 4 || segments < 1 || seg_states == nullptr ||
+      seg_decays == nullptr || !aligned(seg_states) || !aligned(seg_decays))
     return static_cast<int>(cudaErrorInvalidValue);
-  int e;
-  if (beta) {
-    e = launch_pieces<kScanDelta, true, false>(a, segments, pdl, stream);
-    if (e == 0)
-      e = launch_kernel(scan_join_delta_kernel, dim3(entries, heads, (vdim + kJoinCols - 1) / kJoinCols), dim3(kJoinThreads), 0,
-                        stream, pdl != 0, a);
-    return e ? e : launch_pieces<kScanDelta, true, true>(a, segments, pdl, stream);
-  }
   // with a bonus the state moves as without one
-  e = bonus || decay_mode == 2 ? launch_pieces<kScanPlain, true, false>(a, segments, pdl, stream)
-                               : launch_pieces<kScanPlain, false, false>(a, segments, pdl, stream);
+  int e = bonus || decay_mode == 2 ? launch_pieces<kScanPlain, true, false>(a, segments, pdl, stream)
+                                   : launch_pieces<kScanPlain, false, false>(a, segments, pdl, stream);
   if (e == 0)
     e = launch_kernel(scan_join_kernel, dim3(entries, heads, (vdim * (dim / 4) + 255) / 256), dim3(256), 0, stream, pdl != 0, a);
   if (e) return e;

@@ -1111,7 +1111,7 @@ def recurrent() -> ctypes.CDLL:
         lib.rl_linear_scan.argtypes = [
             c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
             c_void_p, c_int, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-            c_int, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
+            c_int, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p,
         ]
         lib.rl_exp_decay.argtypes = [c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]
         lib.rl_low_rank_decay.argtypes = [c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_float, c_void_p,
@@ -1240,35 +1240,35 @@ def rotate_heads(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.T
     return out
 
 
-def scan_piece(heads: int, vdim: int, corrected: bool) -> int:
+def scan_piece(heads: int, vdim: int) -> int:
     """Tokens of a piece of a prompt that is walked in pieces side by side: as many pieces as it takes to fill the GPU, and no
-    more, since what joins them costs by the piece (a matrix product each with a correction, else one more pass over the
-    pieces' states).  2,048 tokens in pieces of 64, 128, 256, us: 16 heads of 128, fixed decays 206, 187, 202; 32 heads 556,
-    374, 332; with a correction, 16 heads, 663, 508, 469."""
-    return 256 if corrected or heads * vdim >= 4096 else 128
+    more, since what joins them is one more pass over the pieces' states.  2,048 tokens in pieces of 64, 128, 256, us: 16 heads
+    of 128, fixed decays 206, 187, 202; 32 heads 556, 374, 332."""
+    return 256 if heads * vdim >= 4096 else 128
 
 
-def scan_pieces_from(heads: int, vdim: int, corrected: bool) -> int:
+def scan_pieces_from(heads: int, vdim: int) -> int:
     """The shortest prompt that is walked in pieces: every piece but the last is walked twice, and what joins them comes on
     top.  From end to end and in pieces, us: 8 heads of 128, 300 tokens 43 and 56; 32 heads of 128, 1,015 tokens beside
-    shorter ones 420 and 331; with a correction, 32 heads of 64, the same prompts 252 and 275, 2,048 tokens of 16 heads 567
-    and 433."""
-    return scan_piece(heads, vdim, corrected) * (4 if corrected else 3)
+    shorter ones 420 and 331."""
+    return scan_piece(heads, vdim) * 3
 
 
-def scan_takes_pieces(dim: int, vdim: int) -> bool:
-    """Whether the recurrence's kernels walk prompts of this head size in pieces."""
-    return 32 < dim <= 128 and dim % 4 == 0 and vdim % 4 == 0
+def scan_takes_pieces(dim: int, vdim: int, corrected: bool = False) -> bool:
+    """Whether the recurrence's kernels walk prompts of this head size in pieces.  With a correction they do not: a piece's
+    matrix took the place of its decays, whose product with the state lost digits (1,300 tokens, 16 heads of 128, against 64
+    bits: states 2.1e-7 off in pieces, 1.5e-7 from end to end), and a GPU that is full walked the prompts twice for nothing
+    (four prompts of 1,024, 32 heads of 64: 386 us in pieces, 256 from end to end)."""
+    return not corrected and 32 < dim <= 128 and dim % 4 == 0 and vdim % 4 == 0
 
 
-def scan_buffers(space, tokens: int, heads: int, dim: int, vdim: int, corrected: bool):
-    """States, products of decays (without a correction) and matrices (with one) of the pieces a step can have: sized once
-    for the largest step ``space`` is made for, so that prompts of growing length allocate nothing."""
-    most, piece = max(space.max_tokens, tokens), scan_piece(heads, vdim, corrected)
+def scan_buffers(space, tokens: int, heads: int, dim: int, vdim: int):
+    """States and products of decays of the pieces a step can have: sized once for the largest step ``space`` is made for, so
+    that prompts of growing length allocate nothing."""
+    most, piece = max(space.max_tokens, tokens), scan_piece(heads, vdim)
     rows = most // piece + most // (piece + 1)      # whole pieces, and a remainder of each entry longer than one
-    get = lambda name, cols: space.get(name, rows, cols, torch.float32, min_rows=rows)      # noqa: E731
-    states = get("scan_states", heads * dim * vdim)
-    return (states, None, get("scan_mats", heads * dim * dim)) if corrected else (states, get("scan_decays", heads * dim), None)
+    return tuple(space.get(name, rows, cols, torch.float32, min_rows=rows)
+                 for name, cols in (("scan_states", heads * dim * vdim), ("scan_decays", heads * dim)))
 
 
 def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, out: torch.Tensor,
@@ -1285,7 +1285,8 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.
     are fine), ``decay`` ``[heads]`` (fixed), ``[T, heads]`` or ``[T, heads * dim]`` (one per row of ``S``),
     ``beta``/``v_scale`` ``[T, heads]``, ``skip`` ``[heads]``, ``out`` ``[T, heads * vdim]``.
 
-    With ``pieces`` (a workspace) a step with a long enough prompt (:func:`scan_pieces_from`) is walked in pieces side by side: the
+    With ``pieces`` (a workspace) a step with a long enough prompt (:func:`scan_pieces_from`) is walked in pieces side by side
+    where the kernels have that form (:func:`scan_takes_pieces`): the
     same sums in another order, which depends on where the step cuts the request.
     """
     _need_cuda(q, k, v, decay, out, state, beta, v_scale, skip, bonus)
@@ -1314,17 +1315,17 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.
     # of 0.6 ms for 2,048 tokens).  Steps of single tokens have many short blocks and keep the early start.
     early = PDL and tokens < 8 * batch.num_entries
     piece = blocks = 0
-    states = decays = mats = None
-    if pieces is not None and scan_takes_pieces(dim, vdim) and batch.max_query_len >= scan_pieces_from(heads, vdim, beta is not None):
-        piece = scan_piece(heads, vdim, beta is not None)
+    states = decays = None
+    if pieces is not None and scan_takes_pieces(dim, vdim, beta is not None) and batch.max_query_len >= scan_pieces_from(heads, vdim):
+        piece = scan_piece(heads, vdim)
         blocks = tokens // piece + batch.num_entries
-        states, decays, mats = scan_buffers(pieces, tokens, heads, dim, vdim, beta is not None)
+        states, decays = scan_buffers(pieces, tokens, heads, dim, vdim)
     _check(
         recurrent().rl_linear_scan(
             _ptr(q), _row_stride("q", q), _ptr(k), _row_stride("k", k), _ptr(v), _row_stride("v", v), _ptr(decay), mode,
             _ptr(beta), _ptr(v_scale), _ptr(skip), _ptr(bonus), _ptr(out), _row_stride("out", out), _ptr(state), stride, 0,
             _ptr(batch.cu_seqlens), _ptr(batch.entry_slot), _ptr(batch.entry_start), batch.num_entries, tokens, heads, kv_heads,
-            dim, vdim, slots, _ptr(batch.fault), piece, blocks, _ptr(states), _ptr(decays), _ptr(mats), int(early), _stream()),
+            dim, vdim, slots, _ptr(batch.fault), piece, blocks, _ptr(states), _ptr(decays), int(early), _stream()),
         f"linear_scan(dim={dim}, vdim={vdim})",
     )
     return out

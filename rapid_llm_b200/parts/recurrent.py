@@ -58,12 +58,11 @@ class _Recurrent(Mixer):
         after the other, so that its rows are the same bit for bit however they are cut into steps."""
         return batch.workspace if self.dtype == torch.bfloat16 else None
 
-    def _pieces_elements(self, heads: int, dim: int, vdim: int, corrected: bool = False) -> int:
+    def _pieces_elements(self, heads: int, dim: int, vdim: int) -> int:
         """Elements of the engine's dtype a token's share of the pieces' states takes at most."""
         if self.dtype != torch.bfloat16 or not kernels.scan_takes_pieces(dim, vdim):
             return 0
-        floats = heads * dim * (vdim + (dim if corrected else 1))
-        return 2 * 2 * -(-floats // kernels.scan_piece(heads, vdim, corrected))
+        return 2 * 2 * -(-heads * dim * (vdim + 1) // kernels.scan_piece(heads, vdim))
 
     def _state_views(self, cache) -> tuple[torch.Tensor, torch.Tensor]:
         state = cache.state
@@ -172,8 +171,7 @@ class ChannelDeltaRule(_Recurrent):
             raise KeyError(name)
 
     def workspace_elements_per_token(self) -> int:
-        return (3 * (self.w_in.shape[0] + self.w_high.shape[0]) + self.ra + self.rg + self.hidden
-                + self._pieces_elements(self.h, self.dim, self.vdim, corrected=True))
+        return 3 * (self.w_in.shape[0] + self.w_high.shape[0]) + self.ra + self.rg + self.hidden
 
     def forward(self, x, batch, cache):
         rows, space, f32 = x.shape[0], batch.workspace, torch.float32
@@ -190,7 +188,7 @@ class ChannelDeltaRule(_Recurrent):
         kernels.decay_gate(high[:, : self.h * self.dim], self.rate, self.dt_bias, self.dim, decay)
         read = space.get("delta_read", rows, self.cv, f32)
         kernels.linear_scan(conv[:, : self.cq], conv[:, self.cq : 2 * self.cq], conv[:, 2 * self.cq :], decay, read, S,
-                            batch, heads=self.h, kv_heads=self.hk, dim=self.dim, vdim=self.vdim, beta=beta, pieces=self._pieces(batch))
+                            batch, heads=self.h, kv_heads=self.hk, dim=self.dim, vdim=self.vdim, beta=beta)
         normed = space.get("delta_normed", rows, self.cv, x.dtype)
         kernels.gated_norm(read, normed, group=self.vdim, gate=high[:, self.h * self.dim :], act=kernels.GATE_SIGMOID,
                            weight=self.norm, eps=self.eps)
