@@ -1043,9 +1043,16 @@ __global__ void __launch_bounds__(kScanThreads) linear_scan_kernel(const ScanArg
   } else {
     mine.clear();
   }
-  P product[kRowDecay ? kRows / 2 : 1];      // of the piece's decays
+  // The product of the piece's decays, for the one warp that stores it: two floats a row, product - rest, so that it is
+  // rounded once and not at every token (slow decays would lose digits: the state is multiplied by what is left of 1).
+  constexpr int kFactors = kRowDecay ? kRows / 2 : 1;
+  const bool multiplies = !kRead && blockIdx.z == 0 && warp == 0;
+  P product[kFactors], rest[kFactors];
 #pragma unroll
-  for (int r = 0; r < (kRowDecay ? kRows / 2 : 1); ++r) product[r] = pair_of<P>(1.0f, 1.0f);
+  for (int r = 0; r < kFactors; ++r) {
+    product[r] = pair_of<P>(1.0f, 1.0f);
+    rest[r] = pair_of<P>(0.0f, 0.0f);
+  }
   if constexpr (kKind == kScanBonus) {
 #pragma unroll
     for (int r = 0; r < kRows / 2; ++r) {
@@ -1118,9 +1125,14 @@ __global__ void __launch_bounds__(kScanThreads) linear_scan_kernel(const ScanArg
       }
     };
     auto multiply = [&](const ScanToken<kRows, kCols, kRowDecay, P>& t, float decay) {
+      if (!multiplies) return;
+      const P minus_one = pair_of<P>(-1.0f, -1.0f);
 #pragma unroll
-      for (int r = 0; r < (kRowDecay ? kRows / 2 : 1); ++r)
-        product[r] = pair_mul(product[r], kRowDecay ? t.g[r] : pair_of<P>(decay, decay));
+      for (int r = 0; r < kFactors; ++r) {
+        const P d = kRowDecay ? t.g[r] : pair_of<P>(decay, decay), rounded = pair_mul(product[r], d);
+        rest[r] = pair_fma(rest[r], d, pair_fma(product[r], pair_mul(d, minus_one), rounded));
+        product[r] = rounded;
+      }
     };
     constexpr int kGroup = 4;
     const int whole = count / kGroup * kGroup;
@@ -1163,9 +1175,9 @@ __global__ void __launch_bounds__(kScanThreads) linear_scan_kernel(const ScanArg
 #pragma unroll
       for (int r = 0; r < kRows / 2; ++r) {
         const int row = ((r / 2) * kPartners + part) * 4 + (r & 1) * 2;
-        const float2 both = pair_halves(product[kRowDecay ? r : 0]);
-        if (row < a.dim) a.seg_decays[own + row] = both.x;
-        if (row + 1 < a.dim) a.seg_decays[own + row + 1] = both.y;
+        const float2 both = pair_halves(product[kRowDecay ? r : 0]), off = pair_halves(rest[kRowDecay ? r : 0]);
+        if (row < a.dim) a.seg_decays[own + row] = both.x - off.x;
+        if (row + 1 < a.dim) a.seg_decays[own + row + 1] = both.y - off.y;
       }
     }
   } else if (slot_ok && seg.number == seg.of - 1) {

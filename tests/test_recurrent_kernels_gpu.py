@@ -195,6 +195,47 @@ def test_prompts_walked_in_pieces(kind, dim, vdim):
         assert all(torch.equal(one, other) for one, other in zip(singles, mixed))
 
 
+@pytest.mark.parametrize("kind", ["fixed", "per_row", "bonus"])
+@pytest.mark.parametrize("heads,dim", [(16, 128), (16, 64)])
+def test_pieces_lose_no_digits(kind, heads, dim):
+    """Read-outs and final states in pieces are no further from 64-bit sums than those of the walk from end to end: decays
+    up to 1 - 2^-10, whose product over a piece is still near 1.  A run's figure is a mean over 10^5 roundings and more; 2 %
+    covers what another order of the same sums does to it."""
+    from rapid_llm_b200.engine.batch import Workspace
+    from rapid_llm_b200.ops import kernels
+
+    tokens = 5 * kernels.scan_piece(heads, dim) + 19
+    generator = torch.Generator(device=DEV).manual_seed(dim)
+    draw = lambda *shape: torch.randn(*shape, generator=generator, device=DEV)      # noqa: E731
+    q, k, v, given = draw(tokens, heads * dim), draw(tokens, heads * dim) * dim ** -0.5, draw(tokens, heads * dim), draw(1, heads * dim * dim) * 0.3
+    options = {"bonus": draw(heads, dim) * 0.5} if kind == "bonus" else {}
+    if kind == "fixed":
+        decay = 1 - 2.0 ** (-3 - 7 * torch.arange(heads, device=DEV) / (heads - 1))
+        rows = decay.double().view(1, heads, 1).expand(tokens, heads, dim)
+    else:
+        decay = torch.sigmoid(draw(tokens, heads * dim) + 2) ** (1 / 16)
+        rows = decay.double().view(tokens, heads, dim)
+    S, want = given.double().view(heads, dim, dim).transpose(1, 2).contiguous(), []
+    for t in range(tokens):
+        qt, kt, vt = (x[t].double().view(heads, dim) for x in (q, k, v))
+        pair = kt[:, :, None] * vt[:, None, :]
+        if options:
+            want.append(torch.einsum("hk,hkv->hv", qt, S + options["bonus"].double()[:, :, None] * pair))
+        S = S * rows[t][:, :, None] + pair
+        if not options:
+            want.append(torch.einsum("hk,hkv->hv", qt, S))
+    want, final = torch.stack(want).view(tokens, heads * dim), S.transpose(1, 2).reshape(1, -1)
+    off = []
+    for pieces in (None, Workspace(tokens, torch.device(DEV))):
+        batch = _batch([tokens], [0], [9])
+        batch.max_query_len = tokens
+        out, state = torch.empty_like(v), given.clone()
+        kernels.linear_scan(q, k, v, decay, out, state, batch, heads=heads, kv_heads=heads, dim=dim, vdim=dim, pieces=pieces, **options)
+        off.append([float((got.double() - exact).norm() / exact.norm()) for got, exact in ((out, want), (state, final))])
+    (walked, walked_state), (read, left) = off
+    assert read <= 1.02 * walked and left <= 1.02 * walked_state, off
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_norm_and_gate_in_their_three_orders(dtype):
     from rapid_llm_b200.ops import kernels
