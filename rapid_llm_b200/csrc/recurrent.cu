@@ -806,20 +806,24 @@ struct ScanColumns {
       for (int c = 0; c < kCols; ++c) {
         const float u = scaled ? t.strength * t.v[c] : t.v[c];
         const P u2 = pair_of<P>(u, u);
-        P sum[2] = {pair_of<P>(0.0f, 0.0f), pair_of<P>(0.0f, 0.0f)};
+        // one chain of up to four pairs: a chain's first product is rounded by itself, so two chains would lose digits
+        constexpr int kChains = kRows > 8 ? 2 : 1;
+        P sum[kChains];
+#pragma unroll
+        for (int i = 0; i < kChains; ++i) sum[i] = pair_of<P>(0.0f, 0.0f);
 #pragma unroll
         for (int r = 0; r < kRows / 2; ++r) {
           const P kv = pair_mul(t.k[r], u2);
           if constexpr (kKind == kScanBonus) {
             // read the state as the tokens before left it, the token's own pair weighed by the bonus; then decay and add
-            sum[r & 1] = pair_fma(pair_fma(bonus[r], kv, S[c][r]), t.q[r], sum[r & 1]);
+            sum[r % kChains] = pair_fma(pair_fma(bonus[r], kv, S[c][r]), t.q[r], sum[r % kChains]);
             S[c][r] = pair_fma(S[c][r], kRowDecay ? t.g[r] : d2, kv);
           } else {
             S[c][r] = pair_fma(S[c][r], kRowDecay ? t.g[r] : d2, kv);
-            if constexpr (kRead) sum[r & 1] = pair_fma(S[c][r], t.q[r], sum[r & 1]);
+            if constexpr (kRead) sum[r % kChains] = pair_fma(S[c][r], t.q[r], sum[r % kChains]);
           }
         }
-        if constexpr (kRead) o[c] = pair_sum(pair_add(sum[0], sum[1]));
+        if constexpr (kRead) o[c] = pair_sum(kChains == 2 ? pair_add(sum[0], sum[kChains - 1]) : sum[0]);
       }
     }
   }
