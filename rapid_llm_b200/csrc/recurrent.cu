@@ -656,39 +656,40 @@ struct ScanArgs {
   int* fault;
   int entries;
   int segment;            // 0: a block walks its entry from end to end; else at most so many tokens, from a state of its own
+  int from;               // entries of so many tokens and more are cut into pieces, the others walked (0: none is cut)
   float* seg_states;      // [pieces, heads, vdim, dim]: what a piece alone leaves, then what it starts from
   float* seg_decays;      // [pieces, heads, dim]: the product of a piece's decays
 };
 
 // The piece that block `index` owns: of which entry, which one of the entry's, its tokens, its place in the arrays of
-// pieces (entries of one piece have none: they start from the slot's state and leave it there); false behind the last.
+// pieces; false behind the last, and for a walk (segment 0) of an entry that is cut.
 struct ScanPiece { int entry, number, first, length, of, place; };
 __device__ __forceinline__ bool scan_piece(const ScanArgs& a, int index, ScanPiece& s) {
   if (a.segment == 0) {
     s = {index, 0, a.cu_seqlens[index], a.cu_seqlens[index + 1] - a.cu_seqlens[index], 1, 0};
-    return true;
+    return a.from == 0 || s.length < a.from;
   }
-  int at = 0, place = 0;
+  int at = 0;
   for (int e = 0; e < a.entries; ++e) {
     const int first = a.cu_seqlens[e], length = a.cu_seqlens[e + 1] - first;
-    const int count = (length + a.segment - 1) / a.segment;
+    const int count = length >= a.from ? (length + a.segment - 1) / a.segment : 0;
     if (index < at + count) {
       const int number = index - at, skipped = number * a.segment;
-      s = {e, number, first + skipped, min(a.segment, length - skipped), count, count > 1 ? place + number : 0};
+      s = {e, number, first + skipped, min(a.segment, length - skipped), count, index};
       return true;
     }
     at += count;
-    if (count > 1) place += count;
   }
   return false;
 }
-// The pieces of entry `e` and the place of its first.
+// The pieces of entry `e` (none where it is walked) and the place of its first.
 __device__ __forceinline__ int scan_pieces_of(const ScanArgs& a, int e, int& place) {
   place = 0;
   int count = 0;
   for (int i = 0; i <= e; ++i) {
-    if (count > 1) place += count;
-    count = (a.cu_seqlens[i + 1] - a.cu_seqlens[i] + a.segment - 1) / a.segment;
+    const int length = a.cu_seqlens[i + 1] - a.cu_seqlens[i];
+    place += count;
+    count = length >= a.from ? (length + a.segment - 1) / a.segment : 0;
   }
   return count;
 }
@@ -1200,7 +1201,7 @@ __global__ void __launch_bounds__(256) scan_join_kernel(const ScanArgs a) {
   int slot = a.entry_slot[e];
   if (slot < 0 || slot >= a.slots) slot = 0;      // the walk says so in the fault word
   pdl_wait();
-  if (col >= a.vdim || pieces <= 1) return;
+  if (col >= a.vdim || pieces == 0) return;
   float4 S = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   if (a.entry_start[e] > 0) {
     const float* home = a.state + slot * a.state_stride + a.state_off + static_cast<size_t>(head) * a.dim * a.vdim +
@@ -1774,8 +1775,8 @@ int rl_linear_scan(const float* q, int q_stride, const float* k, int k_stride, c
                    const float* decay, int decay_mode, const float* beta, const float* v_scale, const float* skip,
                    const float* bonus, float* out, int out_stride, float* state, long long state_stride, int state_off,
                    const int* cu_seqlens, const int* entry_slot, const int* entry_start, int entries, int tokens, int heads,
-                   int kv_heads, int dim, int vdim, int slots, int* fault, int segment, int segments, float* seg_states,
-                   float* seg_decays, int pdl, cudaStream_t stream) {
+                   int kv_heads, int dim, int vdim, int slots, int* fault, int segment, int from, int segments, int others,
+                   float* seg_states, float* seg_decays, int pdl, cudaStream_t stream) {
   if (entries == 0) return 0;
   if (heads < 1 || kv_heads < 1 || heads % kv_heads || dim < 1 || dim > 1024 || vdim < 1 || decay_mode < 0 ||
       decay_mode > 2 || decay == nullptr || (bonus != nullptr && beta != nullptr))
@@ -1792,6 +1793,7 @@ int rl_linear_scan(const float* q, int q_stride, const float* k, int k_stride, c
               aligned(q) && aligned(k) && aligned(v) && (decay_mode != 2 || aligned(decay));
   a.entries = entries;
   a.segment = segment;
+  a.from = segment ? from : 0;
   a.seg_states = seg_states; a.seg_decays = seg_decays;
   using namespace rl;
   // single tokens of the common head sizes: the same rows a lane and lanes a column as the walk, so the same sums
@@ -1814,12 +1816,23 @@ int rl_linear_scan(const float* q, int q_stride, const float* k, int k_stride, c
     if (decay_mode == 2) return launch_plain_scan<kScanPlain, true>(a, entries, pdl, stream);
     return launch_plain_scan<kScanPlain, false>(a, entries, pdl, stream);
   }
-  // in pieces side by side: sizes and pieces the kernels are made for
-  if (segment < 0 || beta != nullptr || dim <= 32 || dim > 128 || dim % 4 || vdim % 4 || segments < 1 || seg_states == nullptr ||
+  // in pieces side by side: sizes and pieces the kernels are made for (an entry that is cut has two pieces at least)
+  if (segment < 0 || from <= segment || beta != nullptr || dim <= 32 || dim > 128 || dim % 4 || vdim % 4 || segments < 1 || seg_states == nullptr ||
       seg_decays == nullptr || !aligned(seg_states) || !aligned(seg_decays))
     return static_cast<int>(cudaErrorInvalidValue);
+  // An entry's own length says whether it is cut, so that its sums are in the same order whatever else is in the step; the
+  // others are walked by themselves.
+  int e = 0;
+  if (others) {
+    ScanArgs walked = a;
+    walked.segment = 0;
+    e = bonus ? launch_plain_scan<kScanBonus, true>(walked, entries, pdl, stream)
+              : decay_mode == 2 ? launch_plain_scan<kScanPlain, true>(walked, entries, pdl, stream)
+                                : launch_plain_scan<kScanPlain, false>(walked, entries, pdl, stream);
+    if (e) return e;
+  }
   // with a bonus the state moves as without one
-  int e = bonus || decay_mode == 2 ? launch_pieces<kScanPlain, true, false>(a, segments, pdl, stream)
+  e = bonus || decay_mode == 2 ? launch_pieces<kScanPlain, true, false>(a, segments, pdl, stream)
                                    : launch_pieces<kScanPlain, false, false>(a, segments, pdl, stream);
   if (e == 0)
     e = launch_kernel(scan_join_kernel, dim3(entries, heads, (vdim * (dim / 4) + 255) / 256), dim3(256), 0, stream, pdl != 0, a);

@@ -1111,7 +1111,7 @@ def recurrent() -> ctypes.CDLL:
         lib.rl_linear_scan.argtypes = [
             c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
             c_void_p, c_int, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-            c_int, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p,
+            c_int, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p,
         ]
         lib.rl_exp_decay.argtypes = [c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]
         lib.rl_low_rank_decay.argtypes = [c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_float, c_void_p,
@@ -1242,16 +1242,22 @@ def rotate_heads(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.T
 
 def scan_piece(heads: int, vdim: int) -> int:
     """Tokens of a piece of a prompt that is walked in pieces side by side: as many pieces as it takes to fill the GPU, and no
-    more, since what joins them is one more pass over the pieces' states.  2,048 tokens in pieces of 64, 128, 256, us: 16 heads
-    of 128, fixed decays 206, 187, 202; 32 heads 556, 374, 332."""
+    more, since what joins them is one more pass over the pieces' states.  In pieces of 128 and 256, us: 2,048 tokens, 32 heads
+    of 64 120 and 128, 16 heads of 128 191 and 204, 32 heads of 128 384 and 335; two prompts of 2,048, 64 heads of 64 405 and
+    350."""
     return 256 if heads * vdim >= 4096 else 128
 
 
-def scan_pieces_from(heads: int, vdim: int) -> int:
-    """The shortest prompt that is walked in pieces: every piece but the last is walked twice, and what joins them comes on
-    top.  From end to end and in pieces, us: 8 heads of 128, 300 tokens 43 and 56; 32 heads of 128, 1,015 tokens beside
-    shorter ones 420 and 331."""
-    return scan_piece(heads, vdim) * 3
+def scan_pieces_from(heads: int, dim: int, vdim: int) -> int:
+    """The shortest entry that is cut into pieces: every piece but the last is walked twice, and what joins them comes on top.
+    One prompt from end to end and in pieces, us: 32 heads of 64, 520 tokens 63 and 75, 640 tokens 76 and 75, 1,024 tokens 117
+    and 77; 16 heads of 128, 640 tokens 94 and 95, 800 tokens 116 and 116, 1,024 tokens 145 and 119; 64 heads of 64, 1,024
+    tokens 135 and 161, 1,536 tokens 199 and 189; 32 heads of 128, 1,024 tokens 206 and 204, 1,536 tokens 301 and 279, 2,048
+    tokens 398 and 339.  The entry's length alone decides, not what else is in the step, which may fill the GPU by itself:
+    eight prompts of 1,024 take 628 and 761 at 16 heads of 128, 303 and 370 at 32 heads of 64."""
+    if heads * vdim >= 4096:
+        return 1536
+    return 1024 if heads * dim * vdim >= 1 << 18 else 640
 
 
 def scan_takes_pieces(dim: int, vdim: int, corrected: bool = False) -> bool:
@@ -1265,8 +1271,8 @@ def scan_takes_pieces(dim: int, vdim: int, corrected: bool = False) -> bool:
 def scan_buffers(space, tokens: int, heads: int, dim: int, vdim: int):
     """States and products of decays of the pieces a step can have: sized once for the largest step ``space`` is made for, so
     that prompts of growing length allocate nothing."""
-    most, piece = max(space.max_tokens, tokens), scan_piece(heads, vdim)
-    rows = most // piece + most // (piece + 1)      # whole pieces, and a remainder of each entry longer than one
+    most = max(space.max_tokens, tokens)
+    rows = most // scan_piece(heads, vdim) + most // scan_pieces_from(heads, dim, vdim)      # whole pieces and remainders
     return tuple(space.get(name, rows, cols, torch.float32, min_rows=rows)
                  for name, cols in (("scan_states", heads * dim * vdim), ("scan_decays", heads * dim)))
 
@@ -1285,9 +1291,9 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.
     are fine), ``decay`` ``[heads]`` (fixed), ``[T, heads]`` or ``[T, heads * dim]`` (one per row of ``S``),
     ``beta``/``v_scale`` ``[T, heads]``, ``skip`` ``[heads]``, ``out`` ``[T, heads * vdim]``.
 
-    With ``pieces`` (a workspace) a step with a long enough prompt (:func:`scan_pieces_from`) is walked in pieces side by side
-    where the kernels have that form (:func:`scan_takes_pieces`): the
-    same sums in another order, which depends on where the step cuts the request.
+    With ``pieces`` (a workspace) entries that are long enough (:func:`scan_pieces_from`) are walked in pieces side by side
+    where the kernels have that form (:func:`scan_takes_pieces`): the same sums in another order, which depends on the entry's
+    own length in this step, so on where a request is cut, and on nothing else in the step.
     """
     _need_cuda(q, k, v, decay, out, state, beta, v_scale, skip, bonus)
     for name, tensor in (("q", q), ("k", k), ("v", v), ("decay", decay), ("out", out), ("beta", beta),
@@ -1314,18 +1320,19 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.
     # before it still fills most multiprocessors, several of its few blocks on the same ones (measured: 1.1 ms instead
     # of 0.6 ms for 2,048 tokens).  Steps of single tokens have many short blocks and keep the early start.
     early = PDL and tokens < 8 * batch.num_entries
-    piece = blocks = 0
+    piece = first = blocks = others = 0
     states = decays = None
-    if pieces is not None and scan_takes_pieces(dim, vdim, beta is not None) and batch.max_query_len >= scan_pieces_from(heads, vdim):
-        piece = scan_piece(heads, vdim)
-        blocks = tokens // piece + batch.num_entries
+    if pieces is not None and scan_takes_pieces(dim, vdim, beta is not None) and batch.max_query_len >= scan_pieces_from(heads, dim, vdim):
+        piece, first = scan_piece(heads, vdim), scan_pieces_from(heads, dim, vdim)
+        blocks = tokens // piece + min(batch.num_entries, tokens // first)
+        others = int(batch.num_entries * batch.max_query_len != tokens)      # entries of other lengths, shorter ones perhaps
         states, decays = scan_buffers(pieces, tokens, heads, dim, vdim)
     _check(
         recurrent().rl_linear_scan(
             _ptr(q), _row_stride("q", q), _ptr(k), _row_stride("k", k), _ptr(v), _row_stride("v", v), _ptr(decay), mode,
             _ptr(beta), _ptr(v_scale), _ptr(skip), _ptr(bonus), _ptr(out), _row_stride("out", out), _ptr(state), stride, 0,
             _ptr(batch.cu_seqlens), _ptr(batch.entry_slot), _ptr(batch.entry_start), batch.num_entries, tokens, heads, kv_heads,
-            dim, vdim, slots, _ptr(batch.fault), piece, blocks, _ptr(states), _ptr(decays), int(early), _stream()),
+            dim, vdim, slots, _ptr(batch.fault), piece, first, blocks, others, _ptr(states), _ptr(decays), int(early), _stream()),
         f"linear_scan(dim={dim}, vdim={vdim})",
     )
     return out

@@ -135,15 +135,15 @@ def test_the_recurrence_over_steps_and_slots(kind, dim, vdim, heads, kv_heads):
 @pytest.mark.parametrize("kind", ["fixed", "per_token", "per_row", "bonus", "delta"])
 @pytest.mark.parametrize("dim,vdim", [(36, 44), (64, 64), (128, 128), (100, 132)])
 def test_prompts_walked_in_pieces(kind, dim, vdim):
-    """Entries of one piece, of exactly two, of five with a remainder and of a single token, from zeros and from a carried
-    state, in pieces against the walk from end to end (the same sums in another order) and its final states; and single tokens
+    """Entries of whole pieces, of pieces with a remainder, of fewer tokens than are cut and of a single one, from zeros and from
+    a carried state, in pieces against the walk from end to end (the same sums in another order) and its final states; and single tokens
     of the same heads, alone and behind another entry, bit for bit as the walk takes them.  With a correction nothing is cut."""
     from rapid_llm_b200.engine.batch import Workspace
     from rapid_llm_b200.ops import kernels
 
     heads, kv_heads = 4, 2
-    piece = kernels.scan_piece(heads, vdim)
-    lengths, starts, slots = [4 * piece + 37, 1, piece, 2 * piece], [0, 9, 5, 700], [3, 1, 0, 2]
+    piece, first = kernels.scan_piece(heads, vdim), kernels.scan_pieces_from(heads, dim, vdim)
+    lengths, starts, slots = [first + 37, 1, first - 1, -(-first // piece) * piece], [0, 9, 5, 700], [3, 1, 0, 2]
     tokens = sum(lengths)
     torch.manual_seed(dim)
     q, k = torch.randn(tokens, kv_heads * dim, device=DEV) / dim ** 0.5, torch.randn(tokens, kv_heads * dim, device=DEV)
@@ -179,7 +179,7 @@ def test_prompts_walked_in_pieces(kind, dim, vdim):
     if dim % 4 == 0 and vdim % 4 == 0:
         per_token = {name: t for name, t in options.items() if t.shape[0] == tokens}
         fixed = {name: t for name, t in options.items() if t.shape[0] != tokens}
-        rows = torch.tensor([3, 4 * piece + 37, 5], device=DEV)      # any three tokens, as single tokens and in an entry of two
+        rows = torch.tensor([3, first + 37, 5], device=DEV)      # any three tokens, as single tokens and in an entry of two
 
         def taken(index):
             return (q[index].contiguous(), k[index].contiguous(), v[index].contiguous(), decay if kind == "fixed" else decay[index].contiguous(),
@@ -195,6 +195,41 @@ def test_prompts_walked_in_pieces(kind, dim, vdim):
         assert all(torch.equal(one, other) for one, other in zip(singles, mixed))
 
 
+@pytest.mark.parametrize("kind", ["fixed", "per_token", "per_row", "bonus"])
+@pytest.mark.parametrize("dim,vdim", [(64, 64), (128, 128), (36, 44)])
+def test_an_entry_is_the_same_alone_and_beside_others(kind, dim, vdim):
+    """A long prompt, a single token and shorter entries, to the last bit: which of them is cut is a matter of its own length."""
+    from rapid_llm_b200.engine.batch import Workspace
+    from rapid_llm_b200.ops import kernels
+
+    heads, first = 3, kernels.scan_pieces_from(3, dim, vdim)
+    lengths, starts = [1, first + 150, 201, first - 1, first, 2], [8, 0, 40, 0, 7, 3]
+    tokens, count = sum(lengths), len(lengths)
+    generator = torch.Generator(device=DEV).manual_seed(dim)
+    draw = lambda *shape: torch.randn(*shape, generator=generator, device=DEV)      # noqa: E731
+    q, k, v, given = draw(tokens, heads * dim), draw(tokens, heads * dim) * dim ** -0.5, draw(tokens, heads * vdim), draw(count, heads * dim * vdim)
+    decay = 1 - 0.1 * torch.rand({"fixed": (heads,), "per_token": (tokens, heads)}.get(kind, (tokens, heads * dim)), generator=generator, device=DEV)
+    options = {"bonus": draw(heads, dim)} if kind == "bonus" else {}
+    space = Workspace(tokens, torch.device(DEV))
+
+    def walk(rows, entries):
+        batch = _batch([lengths[e] for e in entries], list(range(len(entries))), [starts[e] for e in entries])
+        batch.max_query_len = max(lengths[e] for e in entries)
+        part = lambda t: t[rows].contiguous()      # noqa: E731
+        out, state = torch.empty_like(part(v)), given[entries].clone()
+        kernels.linear_scan(part(q), part(k), part(v), decay if kind == "fixed" else part(decay), out, state, batch, heads=heads,
+                            kv_heads=heads, dim=dim, vdim=vdim, pieces=space, **options)
+        assert int(batch.fault.item()) == 0
+        return out, state
+
+    together, states = walk(slice(0, tokens), list(range(count)))
+    at = 0
+    for e, n in enumerate(lengths):
+        out, state = walk(slice(at, at + n), [e])
+        assert torch.equal(out, together[at : at + n]) and torch.equal(state[0], states[e]), n
+        at += n
+
+
 @pytest.mark.parametrize("kind", ["fixed", "per_row", "bonus"])
 @pytest.mark.parametrize("heads,dim", [(16, 128), (16, 64)])
 def test_pieces_lose_no_digits(kind, heads, dim):
@@ -204,7 +239,7 @@ def test_pieces_lose_no_digits(kind, heads, dim):
     from rapid_llm_b200.engine.batch import Workspace
     from rapid_llm_b200.ops import kernels
 
-    tokens = 5 * kernels.scan_piece(heads, dim) + 19
+    tokens = 1024 + 2 * kernels.scan_piece(heads, dim) + 19
     generator = torch.Generator(device=DEV).manual_seed(dim)
     draw = lambda *shape: torch.randn(*shape, generator=generator, device=DEV)      # noqa: E731
     q, k, v, given = draw(tokens, heads * dim), draw(tokens, heads * dim) * dim ** -0.5, draw(tokens, heads * dim), draw(1, heads * dim * dim) * 0.3
