@@ -30,6 +30,7 @@
 // behind a cp.async ring with ldmatrix fragments on tiles of 64 pairs, and tcgen05 on tiles of 128 (moe_tc.cu).
 // The plan is made for the tile the product kernels will use (`tile_m`).
 #include "common.cuh"
+#include "moe_unit.cuh"
 
 namespace rl {
 
@@ -49,17 +50,6 @@ int grouped_linear_tc(const void* a, int a_stride, const void* w, int experts, c
                       int most_tiles, float glu_limit, float glu_alpha, int* fault, int pdl, cudaStream_t stream);
 
 __device__ __forceinline__ float moe_sigmoid(float x) { return 1.0f / (1.0f + expf(-x)); }
-
-// The gated unit of an expert from its two float32 products: SiLU(g) * u, or with limit > 0 the clamped unit
-// min(g, limit) * sigmoid(alpha * min(g, limit)) * (clamp(u, -limit, limit) + 1).
-__device__ __forceinline__ float moe_unit(float g, float u, float limit, float alpha) {
-  if (limit > 0.0f) {
-    g = fminf(g, limit);
-    u = fminf(fmaxf(u, -limit), limit);
-    return g / (1.0f + expf(-alpha * g)) * (u + 1.0f);
-  }
-  return g / (1.0f + expf(-g)) * u;
-}
 
 // ------------------------------------------------------------------ router
 // One block per kRouterTokens tokens.  The block's warps share the inner range: warp w forms, for every router row

@@ -12,12 +12,13 @@
 // k, whatever else is in its tile.
 //
 // Bound by what a multiprocessor fetches per product: 48 KB for every 64 columns of a tile.  Before that the gated
-// results' divisions held it up, one behind the other (a tile's 128 outputs a thread: some 20 us), so they use the fast
-// division (2 ulp, ahead of the rounding to bfloat16).  Hidden 2,048, inter 512, 2 of 16 experts, 2,048 tokens: 47 + 43 us
-// (mma.sync tiles of 64 pairs: 80 + 59); hidden 4,096, inter 1,024: 113 + 82 (270 + 178).
+// results' divisions held it up, one behind the other (a tile's 128 outputs a thread: 20 to 35 us more), so sixteen are
+// formed together (moe_units).  Hidden 2,048, inter 512, 2 of 16 experts, 2,048 tokens: 51 + 41 us (mma.sync tiles of 64
+// pairs: 80 + 59; a plain division: 82 + 43); hidden 4,096, inter 1,024: 118 + 82 (270 + 178; 137 + 80).
 #include <cuda.h>
 
 #include "common.cuh"
+#include "moe_unit.cuh"
 #include "tc_common.cuh"
 
 namespace rl {
@@ -169,21 +170,17 @@ grouped_linear_tc_kernel(const __grid_constant__ CUtensorMap map_w, const MoeTcA
         if constexpr (kGated) {
           float u[16];
           tmem_load16(acc + kColumns + c, u);
-          __align__(16) __nv_bfloat16 packed[16];
-          if (args.glu_limit > 0.0f) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const float g = fminf(v[j] * scale, args.glu_limit), up = fminf(fmaxf(u[j] * scale, -args.glu_limit), args.glu_limit);
-              packed[j] = __float2bfloat16_rn(__fdividef(g, 1.0f + expf(-args.glu_alpha * g)) * (up + 1.0f));
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const float g = v[j] * scale;
-              packed[j] = __float2bfloat16_rn(__fdividef(g, 1.0f + expf(-g)) * (u[j] * scale));
-            }
-          }
           if (live) {
+            float unit[16];
+            __align__(16) __nv_bfloat16 packed[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              v[j] *= scale;
+              u[j] *= scale;
+            }
+            moe_units(v, u, args.glu_limit, args.glu_alpha, unit);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) packed[j] = __float2bfloat16_rn(unit[j]);
             __nv_bfloat16* o = args.out_act + static_cast<size_t>(place0 + row) * args.n + n0 + c;
 #pragma unroll
             for (int j = 0; j < 16; j += 8)             // n is a multiple of 8 here

@@ -225,3 +225,36 @@ def test_the_clamped_unit_rides_on_the_gate_up_product(tokens):
     assert int(fault.item()) == 0
     assert float((gate == limit).float().mean()) > 0.05 and float((up.abs() == limit).float().mean()) > 0.05      # the limits bite
     torch.testing.assert_close(act.float(), want, rtol=2e-2, atol=2e-2)
+
+
+@pytest.mark.parametrize("clamp", [None, (7.0, 1.702)])
+def test_the_gated_unit_is_the_same_to_the_last_bit_in_every_product_kernel(clamp):
+    """Rows with a single one pick a weight each, so that the kernels' sums are exact and what differs is the unit alone: over
+    ordinary gates, tiny ones, zeros and ones so far below zero that their sigmoid leaves the normal range."""
+    from rapid_llm_b200.ops import kernels
+
+    torch.manual_seed(5)
+    tokens, hidden, inter, bf = 320, 64, 256, torch.bfloat16
+    gate = torch.randn(inter, hidden, device=DEVICE)
+    gate[:64] *= 6.0
+    gate[64:128] = -70.0 - 25.0 * torch.rand(64, hidden, device=DEVICE)
+    gate[128:160] *= 2.0 ** torch.randint(-126, 0, (32, hidden), device=DEVICE).float()
+    gate[160:164] = 0.0
+    up = torch.randn(inter, hidden, device=DEVICE) * 2.0 ** torch.randint(0, 40, (inter, hidden), device=DEVICE).float()
+    gate_up = torch.cat([gate, up])[None].to(bf).contiguous()
+    x = torch.zeros(tokens, hidden, device=DEVICE)
+    x[torch.arange(tokens), torch.arange(tokens) % hidden] = 1.0
+    x, weights = x.to(bf), torch.rand(tokens, 1, device=DEVICE) + 0.5
+    ids, fault = torch.zeros(tokens, 1, dtype=torch.int32, device=DEVICE), torch.zeros(1, dtype=torch.int32, device=DEVICE)
+    results = []
+    for kind in (False, True, "few", "tensor"):
+        order, place = torch.zeros(tokens, dtype=torch.int32, device=DEVICE), torch.zeros(tokens, dtype=torch.int32, device=DEVICE)
+        meta = torch.zeros(1 + 3 * kernels.moe_max_tiles(tokens, 1, kind), dtype=torch.int32, device=DEVICE)
+        tiles = kernels.moe_plan(ids, 1, order, place, meta, fault, wide=kind)
+        act = torch.empty(tokens, inter, dtype=bf, device=DEVICE)
+        kernels.grouped_linear(x, gate_up, order, meta, top=1, by_token=True, max_tiles=tiles, pair_weight=weights.view(-1), out_act=act,
+                               wide=kind, clamp=clamp, fault=fault)
+        results.append(act[place.long()])
+    assert int(fault.item()) == 0
+    assert clamp is not None or bool((results[0][:, 64:128] != 0).any())
+    assert all(torch.equal(results[0], other) for other in results[1:])
