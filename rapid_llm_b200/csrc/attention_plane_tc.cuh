@@ -6,22 +6,28 @@
 // turned for the values (MN-major).
 //
 //     S[row, key]  = Q[row, :] . R[key, :]      tcgen05.mma  M = 128, N = 96 keys, K = D
-//     O[row, d]   += P[row, key] . R[key, d]    A = P from tensor memory, M = 128, N = D, K = 96 keys
+//     O[row, d]   += P[row, key] . R[key, d]    A = P from tensor memory, M = 128, N = D, K = 96 keys, twice
 //
-// What bounds it is the chain from a block's scores through its softmax to its values (1.3 us; the two products alone
-// take 0.8), so the scores of block j + 1 are issued before the values of block j, two threads share a row and the softmax of
+// P enters as two bfloat16 terms, its rounding and what that left.  Rounded once, every weight is up to 2^-9 off, also the
+// largest, which the mma.sync tiles take against itself and so without an error.  Root mean square error of the result
+// against 64 bits: 2,048 tokens 1.63e-3 (the mma.sync tiles 1.90e-3, one term 1.96e-3), 64 single tokens behind 1,024
+// 1.65e-3 (1.81e-3, 1.95e-3); rounding the result alone gives 1.6e-3.  One term against the running maximum itself: 1.91e-3
+// and 1.87e-3.
+//
+// What bounds it is the chain from a block's scores through its softmax to its values (1.4 us; the three products alone
+// take 1.2), so the scores of block j + 1 are issued before the values of block j, two threads share a row and the softmax of
 // one block runs under the products of its neighbours: O takes D columns of tensor memory, two blocks of scores 2 x 128 (P
 // lies over the scores it came from).  Blocks of 96: three tiles of 96 x 256 fit beside the queries, and a tile is held from its scores to its values, one block later; with two tiles
 // of 128 the next scores would wait for a whole fetch, and blocks of 64 with the queries in tensor memory and six tiles
-// pay the chain more often (60 us against 52 for the prompt below).  The softmax is that of the two-plane kernel: the
-// reference point of the exponentials moves only when the maximum has grown by more than 2^8, scores, maxima, sums
-// and O are float32 and P is rounded to bfloat16.
+// pay the chain more often (with one term of P 60 us against 52 for the prompt below).  The softmax is that of the two-plane kernel: the
+// reference point of the exponentials moves only when the maximum has grown by more than 2^8; scores, maxima, sums
+// and O are float32.
 //
 // Rows behind the range come as zeros (whole boxes from outside the tensor, the rest of a box cleared here): what lies
 // in memory that nothing wrote yet must not reach the product, where zero times it could be NaN.
 //
-// 16 heads, rows of 256: 2,048 tokens of a prompt 52 us (the mma.sync tiles 236), 8 portions of 130 behind 500 tokens 27
-// (85), 64 single tokens behind 1,024 34 (50), behind 4,096 60 (101); 128 heads, the same single tokens 42 (125), 71 (374).
+// 16 heads, rows of 256: 2,048 tokens of a prompt 58 us (the mma.sync tiles 236; one term of P 52), 64 single tokens behind
+// 1,024 34 (50; 32), behind 4,096 66 (101; 60); 32 heads, 2 prompts of 600 47 (105; 45).
 //
 // Takes rows of 64 to 256 numbers and pages of a multiple of 8 tokens; others run on the mma.sync tiles.
 #pragma once
@@ -255,8 +261,12 @@ attention_plane_tc_kernel(const __grid_constant__ CUtensorMap map_cache, const P
       if (lane == 0) {
         const uint64_t values_desc = operand_desc_mn(tile_at(b % kPlStages), kPlAtomBytes);
 #pragma unroll
-        for (int k = 0; k < kPlKeys / 16; ++k)
-          umma_bf16_ts(tmem_out, tmem_score(b) + k * 8, values_desc + k * (2048 >> 4), kPlIdescValue, (b > 0 || k > 0) ? 1u : 0u);
+        for (int part = 0; part < 2; ++part) {      // P as it rounds, then what the rounding left
+#pragma unroll
+          for (int k = 0; k < kPlKeys / 16; ++k)
+            umma_bf16_ts(tmem_out, tmem_score(b) + part * (kPlKeys / 2) + k * 8, values_desc + k * (2048 >> 4), kPlIdescValue,
+                         (b > 0 || part > 0 || k > 0) ? 1u : 0u);
+        }
         umma_commit(smem_addr(&value_done[b & 1]));
         umma_commit(smem_addr(&empty[b % kPlStages]));
       }
@@ -384,7 +394,7 @@ attention_plane_tc_kernel(const __grid_constant__ CUtensorMap map_cache, const P
       }
       const float shift = ref_max == -INFINITY ? 0.0f : ref_max;
       const unsigned long long scale2 = pf_pack2(args.scale_log2, args.scale_log2), shift2 = pf_pack2(-shift, -shift);
-      uint32_t packed[kPlHalfKeys / 2];
+      uint32_t packed[kPlHalfKeys / 2], rest[kPlHalfKeys / 2];
 #pragma unroll
       for (int i = 0; i < kPlHalfKeys / 2; ++i) {
         float x0, x1;
@@ -393,17 +403,21 @@ attention_plane_tc_kernel(const __grid_constant__ CUtensorMap map_cache, const P
         row_sum2 = pf_add2(row_sum2, pf_pack2(e0, e1));
         const __nv_bfloat162 pair = __floats2bfloat162_rn(e0, e1);
         packed[i] = *reinterpret_cast<const uint32_t*>(&pair);
+        const __nv_bfloat162 left = __floats2bfloat162_rn(e0 - __uint_as_float(packed[i] << 16), e1 - __uint_as_float(packed[i] & 0xffff0000u));
+        rest[i] = *reinterpret_cast<const uint32_t*>(&left);
       }
-      {
-        const uint32_t to = tmem_score(b) + lane_bits + half * (kPlHalfKeys / 2);
+      auto store = [&](uint32_t to, const uint32_t (&from)[kPlHalfKeys / 2]) {
         uint32_t first[16], second[8];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) first[i] = packed[i];
+        for (int i = 0; i < 16; ++i) first[i] = from[i];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) second[i] = packed[16 + i];
+        for (int i = 0; i < 8; ++i) second[i] = from[16 + i];
         tmem_store16(to, first);
         tmem_store8(to + 16, second);
-      }
+      };
+      const uint32_t to = tmem_score(b) + lane_bits + half * (kPlHalfKeys / 2);
+      store(to, packed);
+      store(to + kPlKeys / 2, rest);
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();

@@ -374,3 +374,41 @@ def test_slopes_over_one_plane_are_refused_by_the_tiles():
         _tiles(case, 2, 1, 32, 8, [20], [20], torch.empty_like(case["q"]), slopes=_slopes(2), decode_kernel="mma", tensor_core=False)
     with pytest.raises(kernels.KernelError, match="slopes"):
         _tiles(case, 2, 1, 32, 8, [20], [20], torch.empty_like(case["q"]), slopes=_slopes(3), decode_kernel="mma", tensor_core=False)
+
+
+@pytest.mark.parametrize("heads,requests,new,start,d", [(16, 1, 600, 0, 256), (16, 8, 1, 1000, 256), (32, 16, 1, 300, 256), (8, 2, 100, 250, 256),
+                                                        (16, 4, 1, 2000, 192), (12, 2, 333, 0, 128)])
+def test_tensor_core_tiles_over_one_plane_are_as_precise_as_the_others(heads, requests, new, start, d):
+    """Against 64 bits the tiles of 128 rows are no further off than the mma.sync tiles, which take a row's largest weight
+    without an error; half a percent is what the means over 10^5 roundings and more vary by."""
+    from rapid_llm_b200.ops import kernels
+    from rapid_llm_b200.parts.attention import AttentionItems
+    from rapid_llm_b200.parts.base import StepShape
+
+    page, scale = 16, 0.072 * (256 / d) ** 0.5
+    length = start + new
+    per = -(-length // page)
+    generator = torch.Generator(device=DEVICE).manual_seed(new + d)
+    cache = torch.randn(requests * per, 1, 1, page, d, generator=generator, device=DEVICE).to(torch.bfloat16)
+    q = torch.randn(requests * new, heads * d, generator=generator, device=DEVICE).to(torch.bfloat16)
+    table = torch.arange(requests * per, dtype=torch.int32, device=DEVICE).view(requests, per)
+    keys = cache.view(requests, per * page, d)[:, :length].double()
+    scores = torch.einsum("nthd,nkd->nhtk", q.view(requests, new, heads, d).double(), keys) * scale
+    hidden = torch.arange(length, device=DEVICE)[None, :] > (start + torch.arange(new, device=DEVICE))[:, None]
+    want = torch.einsum("nhtk,nkd->nthd", torch.softmax(scores.masked_fill(hidden, float("-inf")), -1), keys).reshape(requests * new, -1)
+    off = []
+    for plane in (False, True):
+        plan = AttentionItems(heads, 1, d, tensor_core=False, one_plane=plane).plan(
+            StepShape(np.full(requests, new, np.int32), np.full(requests, start, np.int32), decode_only=new == 1, page_size=page))
+        assert (plan["chunk_rows"] == kernels.CHUNK_TILE_ROWS_PLANE) == plane
+        rows, fault, out = requests * new * heads * plan["splits"], _word(), torch.empty_like(q)
+        kernels.attention_mma(
+            q, cache, out, chunk_items=torch.from_numpy(plan["chunk_items"]).to(DEVICE), decode_items=torch.from_numpy(plan["decode_items"]).to(DEVICE),
+            splits=plan["splits"], part_out=torch.empty(rows, d, device=DEVICE), part_lse=torch.empty(rows, device=DEVICE),
+            cu_seqlens=torch.arange(0, requests * new + 1, new, dtype=torch.int32, device=DEVICE),
+            entry_start=torch.full((requests,), start, dtype=torch.int32, device=DEVICE), entry_slot=torch.arange(requests, dtype=torch.int32, device=DEVICE),
+            block_table=table, num_heads=heads, num_kv_heads=1, head_dim=d, window=0, scale=scale, fault=fault, decode_kernel="mma",
+            decode_rows=plan["decode_rows"], chunk_rows=plan["chunk_rows"])
+        assert int(fault.item()) == 0
+        off.append(float((out.double() - want).norm() / want.norm()))
+    assert off[1] <= 1.005 * off[0], off
