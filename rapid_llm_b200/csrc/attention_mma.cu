@@ -759,7 +759,8 @@ int rl_attention_decode_rows() { return 16; }
 
 // chunk_rows: packed rows per chunk item: 64 (or 0) = the mma.sync tiles, 256 = the tcgen05
 // kernel (head size 128, pages it takes, splits == 1), 128 = the tcgen05 kernel over a cache of one plane (rows of 64 and
-// more numbers, pages of a multiple of 8 tokens, scores that are not squashed).
+// more numbers, pages of a multiple of 8 tokens, scores that are not squashed, a scale above zero: it masks and takes
+// maxima before it scales).
 // decode_splits: key ranges of the decode tiles where they differ from `splits` (a step of prompt portions, which
 // the tcgen05 kernel does not split, beside single tokens with long contexts); 0 = the same.
 // decode_kernel: 0 = the tcgen05 kernel for decode tiles where it applies, 1 = always the
@@ -808,7 +809,7 @@ int rl_attention_mma(const void* q, const void* cache, void* out, float* part_ou
     if (!(softcap > 0.0f) || (decode_splits > 0 && decode_splits != splits)) return static_cast<int>(cudaErrorInvalidValue);
     decode_kernel = 1;
   }
-  if (chunk_rows == attn::kPlRows && (kv_planes != 1 || softcap != 0.0f || !attn::plane_tc_supported(page_size)))
+  if (chunk_rows == attn::kPlRows && (kv_planes != 1 || softcap != 0.0f || !(scale > 0.0f) || !attn::plane_tc_supported(page_size)))
     return static_cast<int>(cudaErrorInvalidValue);
   if (kv_planes == 1) {         // rows that are keys and values at once: tiles of 128 or the mma.sync tiles read them
     if (slopes != nullptr || chunk_rows == attn::kPfRows || (decode_splits > 0 && decode_splits != splits)) return static_cast<int>(cudaErrorInvalidValue);

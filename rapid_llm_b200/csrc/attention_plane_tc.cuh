@@ -436,12 +436,13 @@ attention_plane_tc_kernel(const __grid_constant__ CUtensorMap map_cache, const P
       const bool whole = args.splits == 1;
       if (!whole && exists && half == 0)
         args.part_lse[row * args.splits + split] = row_sum > 0.0f ? ref_max + log2f(row_sum) : -INFINITY;
-      if (whole && args.sink != nullptr && exists) {
-        // the sink's term against the same reference point as the keys' (an infinite one: it alone counts, the row is zero)
-        const float sink2 = args.sink[head] * 1.4426950408889634f;
-        row_sum += fast_exp2(sink2 - (ref_max == -INFINITY ? 0.0f : ref_max));
-      }
       float inv = row_sum > 0.0f ? 1.0f / row_sum : 0.0f;
+      if (whole && args.sink != nullptr && exists && ref_max > -INFINITY) {
+        // the sink's term beside the keys', both against the larger of the two (an infinite one: it alone counts, the row is zero)
+        const float sink2 = args.sink[head] * 1.4426950408889634f;
+        const float top = fmaxf(ref_max, sink2), keys = exp2f(ref_max - top);
+        inv = sink2 == INFINITY ? 0.0f : keys / (row_sum * keys + exp2f(sink2 - top));
+      }
       if (whole && exists) inv *= head_gate(args.gate, args.gate_stride, tok_begin + token, head);
       bf16* dst = args.out + static_cast<size_t>(tok_begin + token) * args.out_stride + head * kPlD;
       float* part = args.part_out + (row * args.splits + split) * kPlD;

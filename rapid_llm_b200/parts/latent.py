@@ -101,8 +101,8 @@ class LatentAttention(Mixer):
         self.o = self.new_storage((self.hidden, self.h * self.vdim), MATRIX)
         device = torch.device(device)
         sms = torch.cuda.get_device_properties(device).multi_processor_count if device.type == "cuda" else DEFAULT_SMS
-        # a cache of one plane: chunk tiles of its own tcgen05 kernel, decode tiles on mma.sync
-        self._items = AttentionItems(self.h, 1, self.d, sms, None, tensor_core=False, window=self.window, one_plane=True)
+        # a cache of one plane: tiles of its own tcgen05 kernel, which wants a scale above zero; others on mma.sync
+        self._items = AttentionItems(self.h, 1, self.d, sms, None, tensor_core=False, window=self.window, one_plane=self.scale > 0.0)
 
     # -- needs ----------------------------------------------------------------- #
     def cache_need(self) -> CacheNeed:

@@ -152,3 +152,18 @@ def test_a_cache_of_one_plane_gets_tiles_of_its_own(group, head_dim, page_size, 
         seen[key] = seen.get(key, 0) + count
     assert all(count == 1 for count in seen.values()) and len(seen) == int(rows.sum()) * plan["splits"]
     assert 4 * (len(plan["chunk_items"]) + len(plan["decode_items"])) <= planner.capacity(int(lengths.sum()), entries)
+
+
+@pytest.mark.parametrize("scale,plane", [(0.07, True), (0.0, False), (-0.5, False)])
+def test_a_latent_mixer_keeps_the_general_tiles_where_its_scale_is_not_positive(scale, plane):
+    import torch
+
+    from rapid_llm_b200.config.model_spec import PartSpec
+    from rapid_llm_b200.parts.base import MIXERS
+
+    mixer = MIXERS.build(PartSpec("latent_attention", {
+        "hidden_size": 64, "num_heads": 4, "head_dim": 16, "rot_dim": 8, "value_dim": 16, "kv_rank": 56, "q_rank": 32, "scale": scale,
+        "norm_eps": 1e-6, "position": PartSpec("rotary_frequencies", {"rotary_dim": 8, "theta": 10000.0, "max_positions": 64})}),
+        dtype=torch.bfloat16, device="cpu")
+    shape = StepShape(lengths=np.asarray([40, 1], np.int32), starts=np.asarray([0, 9], np.int32), decode_only=False, page_size=16)
+    assert (mixer._items.plan(shape)["chunk_rows"] == kernels.CHUNK_TILE_ROWS_PLANE) == plane

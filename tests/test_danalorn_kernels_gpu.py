@@ -412,3 +412,40 @@ def test_tensor_core_tiles_over_one_plane_are_as_precise_as_the_others(heads, re
         assert int(fault.item()) == 0
         off.append(float((out.double() - want).norm() / want.norm()))
     assert off[1] <= 1.005 * off[0], off
+
+
+@pytest.mark.parametrize("lift", [-3.0, 60.0, 100.0, float("inf")])
+def test_a_sink_far_above_the_keys_leaves_their_sum_its_digits(lift):
+    """Large rows make what the sink leaves of them a number of the result's range: e^-100 of 10^30 is one.  One rounding of
+    the result and of the weights' sums, 2^-8, twice."""
+    from rapid_llm_b200.ops import kernels
+    from rapid_llm_b200.parts.attention import AttentionItems
+    from rapid_llm_b200.parts.base import StepShape
+
+    heads, d, page, tokens = 16, 256, 16, 40
+    generator = torch.Generator(device=DEVICE).manual_seed(3)
+    rows = (torch.randn(48, d, generator=generator, device=DEVICE) * 1e30).to(torch.bfloat16)
+    q = (torch.randn(tokens, heads * d, generator=generator, device=DEVICE) * 1e-30).to(torch.bfloat16)
+    scores = torch.einsum("thd,kd->thk", q.view(tokens, heads, d).double(), rows[:tokens].double()) / 16
+    scores.masked_fill_((torch.arange(tokens, device=DEVICE)[None] > torch.arange(tokens, device=DEVICE)[:, None])[:, None], float("-inf"))
+    sink = torch.full((heads,), lift, device=DEVICE)
+    with_sink = torch.cat([scores, sink.double().view(1, heads, 1).expand(tokens, heads, 1)], -1)
+    weights = torch.softmax(with_sink, -1)[..., :tokens] if math.isfinite(lift) else torch.zeros_like(scores)
+    want = torch.einsum("thk,kd->thd", weights, rows[:tokens].double()).reshape(tokens, -1)
+    plan = AttentionItems(heads, 1, d, tensor_core=False, one_plane=True).plan(
+        StepShape(np.asarray([tokens], np.int32), np.asarray([0], np.int32), decode_only=False, page_size=page))
+    assert plan["chunk_rows"] == kernels.CHUNK_TILE_ROWS_PLANE and plan["splits"] == 1
+    out, fault = torch.empty_like(q), _word()
+    call = lambda scale: kernels.attention_mma(      # noqa: E731
+        q, rows.view(3, 1, 1, page, d), out, chunk_items=torch.from_numpy(plan["chunk_items"]).to(DEVICE),
+        decode_items=torch.from_numpy(plan["decode_items"]).to(DEVICE), splits=1, part_out=None, part_lse=None,
+        cu_seqlens=torch.tensor([0, tokens], dtype=torch.int32, device=DEVICE), entry_start=torch.zeros(1, dtype=torch.int32, device=DEVICE),
+        entry_slot=torch.zeros(1, dtype=torch.int32, device=DEVICE), block_table=torch.arange(3, dtype=torch.int32, device=DEVICE).view(1, 3),
+        num_heads=heads, num_kv_heads=1, head_dim=d, window=0, scale=scale, fault=fault, decode_kernel="mma", decode_rows=plan["decode_rows"],
+        chunk_rows=plan["chunk_rows"], sink=sink)
+    call(1 / 16)
+    assert int(fault.item()) == 0
+    assert float((out.double() - want).norm()) <= 2.0 ** -7 * float(want.norm())
+    for scale in (0.0, -0.5):      # refused: the kernel masks and takes maxima before it scales
+        with pytest.raises(kernels.KernelError):
+            call(scale)
