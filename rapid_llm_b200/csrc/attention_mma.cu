@@ -551,13 +551,9 @@ int launch_attention_as(const AttentionArgs& args, int n_items, bool pdl, cudaSt
   auto kernel = attention_mma_kernel<kWarpsM, kWarpsN, kStages, kShared, kSloped>;
   constexpr size_t smem = attention_smem_bytes<kWarpsM, kWarpsN, kStages, kShared>();
   static_assert(smem <= 227 * 1024, "shared memory of one CTA");
-  static bool configured = false;   // one per instantiation and per library image
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
-    if (e != cudaSuccess) return static_cast<int>(e);
-    configured = true;
-  }
+  static std::atomic<unsigned long long> configured;   // one per instantiation and per library image
+  const cudaError_t e = allow_shared(kernel, static_cast<int>(smem), configured);
+  if (e != cudaSuccess) return static_cast<int>(e);
   return launch_kernel(kernel, dim3(args.hkv, n_items), dim3(kThreads), smem, stream, pdl, args);
 }
 
@@ -583,17 +579,14 @@ static bool decode_tc_supported(int page_size) {
   return kD == kTcD && page_size % 8 == 0 && (kTcKeys % page_size == 0 || page_size % kTcKeys == 0);
 }
 
-static bool g_prefill_tc_configured[2] = {};   // per instantiation; file-local on purpose
+static std::atomic<unsigned long long> g_prefill_tc_configured[2];   // per instantiation; file-local on purpose
 
 // Chunk tiles of 256 packed rows on the tcgen05 kernel (unsplit key ranges only).
 static int launch_prefill_tc(const AttentionArgs& a, int n_items, bool pdl, cudaStream_t stream) {
   const bool sloped = a.slopes != nullptr;
   auto kernel = sloped ? attention_prefill_tc_kernel<true> : attention_prefill_tc_kernel<false>;
-  if (!g_prefill_tc_configured[sloped]) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmemBytes);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    g_prefill_tc_configured[sloped] = true;
-  }
+  const cudaError_t e = allow_shared(kernel, kPfSmemBytes, g_prefill_tc_configured[sloped]);
+  if (e != cudaSuccess) return static_cast<int>(e);
   CUtensorMap map;
   const long long rows = static_cast<long long>(a.num_pages) * 2 * a.hkv * a.page_size;
   int status = make_map(&map, a.cache, rows, kD, a.page_size < kPfKeys ? a.page_size : kPfKeys);
@@ -621,12 +614,9 @@ static int launch_plane_tc(const AttentionArgs& a, int n_items, bool pdl, cudaSt
   if constexpr (!kPlTakes) {
     return static_cast<int>(cudaErrorInvalidValue);
   } else {
-    static bool configured = false;
-    if (!configured) {
-      cudaError_t e = cudaFuncSetAttribute(attention_plane_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPlSmemBytes);
-      if (e != cudaSuccess) return static_cast<int>(e);
-      configured = true;
-    }
+    static std::atomic<unsigned long long> configured;
+    const cudaError_t e = allow_shared(attention_plane_tc_kernel, kPlSmemBytes, configured);
+    if (e != cudaSuccess) return static_cast<int>(e);
     PlaneTcArgs t;
     t.box_rows = a.page_size % 32 == 0 ? 32 : a.page_size % 16 == 0 ? 16 : 8;
     CUtensorMap map;
@@ -644,7 +634,7 @@ static int launch_plane_tc(const AttentionArgs& a, int n_items, bool pdl, cudaSt
   }
 }
 
-static bool g_decode_tc_configured[5][2][2] = {};   // per row-count, ring-depth and dressed instantiation; file-local on purpose
+static std::atomic<unsigned long long> g_decode_tc_configured[5][2][2];   // per row-count, ring-depth and dressed instantiation; file-local on purpose
 
 static int decode_tc_sm_count() {
   int device = 0, sms = 0;
@@ -656,17 +646,11 @@ static int decode_tc_sm_count() {
 
 template <int kRows, int kStages, bool kDressed>
 static int launch_decode_tc_as(const CUtensorMap& map, const DecodeTcArgs& t, int n_items, bool pdl,
-                                   cudaStream_t stream, bool* configured) {
+                                   cudaStream_t stream, std::atomic<unsigned long long>* configured) {
   auto kernel = attention_decode_tc_kernel<kRows, kStages, kDressed>;
   constexpr int kTcSmemBytes = tc_smem_bytes(kStages);
-  if (!*configured) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmemBytes);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    // clusters of more than 8 CTAs (up to 16 key ranges of a tile) have to be asked for
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    *configured = true;
-  }
+  const cudaError_t allowed = allow_shared(kernel, kTcSmemBytes, *configured, true);      // up to 16 key ranges of a tile
+  if (allowed != cudaSuccess) return static_cast<int>(allowed);
   // x: the key ranges of one tile (a cluster when they merge among themselves), y: the kv head,
   // z: the tile.  CTAs start in x, y, z order: the tiles of the item list, longest first, over
   // all heads, so that the last wave holds the shortest.
@@ -697,7 +681,7 @@ static int launch_decode_tc_as(const CUtensorMap& map, const DecodeTcArgs& t, in
 
 template <int kRows, int kStages>
 static int launch_decode_tc_stages(const CUtensorMap& map, const DecodeTcArgs& t, int n_items, bool pdl,
-                                   cudaStream_t stream, bool* configured) {
+                                   cudaStream_t stream, std::atomic<unsigned long long>* configured) {
   const bool dressed = t.sink != nullptr || t.slopes != nullptr || t.gate != nullptr || t.out_stride != t.hq * kTcD;
   if (dressed) return launch_decode_tc_as<kRows, kStages, true>(map, t, n_items, pdl, stream, configured + 1);
   return launch_decode_tc_as<kRows, kStages, false>(map, t, n_items, pdl, stream, configured);
@@ -709,7 +693,7 @@ static int launch_decode_tc_stages(const CUtensorMap& map, const DecodeTcArgs& t
 // `rings`: 0 = decide here, 2 = deep, 3 = shallow (for measurements).
 template <int kRows>
 static int launch_decode_tc_rows(const CUtensorMap& map, const DecodeTcArgs& t, int n_items, bool pdl,
-                                 cudaStream_t stream, bool (*configured)[2], int rings) {
+                                 cudaStream_t stream, std::atomic<unsigned long long> (*configured)[2], int rings) {
   const bool shallow = rings == 3 || (rings != 2 && !t.cluster_merge &&
                                       static_cast<long long>(n_items) * t.hkv > decode_tc_sm_count());
   if (shallow) return launch_decode_tc_stages<kRows, 1>(map, t, n_items, pdl, stream, configured[1]);

@@ -7,6 +7,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 namespace rl {
 
 // Element type tags shared with the Python side.
@@ -120,6 +122,21 @@ __device__ __forceinline__ float query_temperature(int pos, float coef, float ev
 template <typename T>
 __device__ __forceinline__ float head_gate(const T* gate, int stride, int token, int head) {
   return gate == nullptr ? 1.0f : 1.0f / (1.0f + expf(-to_float(gate[static_cast<size_t>(token) * stride + head])));
+}
+
+// More than 48 KB of shared memory has to be allowed once per kernel and device; `done` has a bit for each device.
+template <typename Kernel>
+inline cudaError_t allow_shared(Kernel kernel, int bytes, std::atomic<unsigned long long>& done, bool wide_clusters = false) {
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  const unsigned long long bit = 1ull << (device & 63);
+  if (device < 64 && (done.load(std::memory_order_acquire) & bit)) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  // clusters of more than 8 CTAs have to be asked for
+  if (e == cudaSuccess && wide_clusters) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess && device < 64) done.fetch_or(bit, std::memory_order_release);
+  return e;
 }
 
 inline int launch_status() { return static_cast<int>(cudaGetLastError()); }

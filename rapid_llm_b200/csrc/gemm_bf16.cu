@@ -513,7 +513,7 @@ static int sm_count() {
   return sms;
 }
 
-static bool g_gemm_configured[3][9] = {};   // [plain, swiglu, squared columns][BN / 32]; file-local on purpose
+static std::atomic<unsigned long long> g_gemm_configured[3][9];   // [plain, swiglu, squared columns][BN / 32]; file-local on purpose
 
 template <bool kSwiglu, int BN, bool kRelu2>
 static int launch_gemm(const CUtensorMap& map_w, const CUtensorMap& map_x, GemmArgs args, int forced_split,
@@ -521,13 +521,8 @@ static int launch_gemm(const CUtensorMap& map_w, const CUtensorMap& map_x, GemmA
   using Shape = GemmShape<kSwiglu, BN>;
   static_assert(!(kSwiglu && kRelu2), "one activation");
   auto kernel = gemm_bf16_kernel<kSwiglu, BN, kRelu2>;
-  bool& configured = g_gemm_configured[kRelu2 ? 2 : (kSwiglu ? 1 : 0)][BN / 32];
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(Shape::kSmemBytes));
-    if (e != cudaSuccess) return static_cast<int>(e);
-    configured = true;
-  }
+  const cudaError_t allowed = allow_shared(kernel, static_cast<int>(Shape::kSmemBytes), g_gemm_configured[kRelu2 ? 2 : (kSwiglu ? 1 : 0)][BN / 32]);
+  if (allowed != cudaSuccess) return static_cast<int>(allowed);
   // how many CTAs the GPU holds at once, and how finely to split k so that they all stream
   // (three CTAs of the plain products' small tiles fit an SM and splitting for three pays there; measured)
   const int resident = sm_count() * (Shape::kShareSm ? (!kSwiglu ? 3 : 2) : 1);

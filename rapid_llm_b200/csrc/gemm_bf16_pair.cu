@@ -556,7 +556,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
   }
 }
 
-static bool g_pair_configured[2] = {false, false};   // [swiglu]; file-local on purpose
+static std::atomic<unsigned long long> g_pair_configured[2];   // [swiglu]; file-local on purpose
 
 template <bool kSwiglu>
 static int launch_pair(const void* x, const void* w, void* out, PairArgs args, int pairs, cudaStream_t stream) {
@@ -568,12 +568,8 @@ static int launch_pair(const void* x, const void* w, void* out, PairArgs args, i
   status = make_map(&map_out, out, args.T, args.N, kPairRows);      // boxes of 128 tokens by 64 columns, swizzled
   if (status != 0) return status;
   auto kernel = gemm_bf16_pair_kernel<kSwiglu>;
-  bool& configured = g_pair_configured[kSwiglu ? 1 : 0];
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kPairSmemBytes));
-    if (e != cudaSuccess) return static_cast<int>(e);
-    configured = true;
-  }
+  const cudaError_t allowed = allow_shared(kernel, static_cast<int>(kPairSmemBytes), g_pair_configured[kSwiglu ? 1 : 0]);
+  if (allowed != cudaSuccess) return static_cast<int>(allowed);
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(2 * pairs);
   config.blockDim = dim3(kPairThreads);

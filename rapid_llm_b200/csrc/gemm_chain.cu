@@ -637,19 +637,14 @@ static int chain_split(int n_tiles, int k_blocks, int grid) {
 
 static int chain_token_tile(int tokens) { return tokens <= 16 ? 16 : tokens <= 32 ? 32 : 64; }
 
-static bool g_chain_configured[3] = {};
+static std::atomic<unsigned long long> g_chain_configured[3];
 
 template <int BN>
 static int launch_chain(const ChainMaps& maps, const ChainArgs& args, int grid, cudaStream_t stream) {
   using Shape = ChainShape<BN>;
   auto kernel = gemm_chain_kernel<BN>;
-  bool& configured = g_chain_configured[BN / 32];
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(Shape::kSmemBytes));
-    if (e != cudaSuccess) return static_cast<int>(e);
-    configured = true;
-  }
+  const cudaError_t allowed = allow_shared(kernel, static_cast<int>(Shape::kSmemBytes), g_chain_configured[BN / 32]);
+  if (allowed != cudaSuccess) return static_cast<int>(allowed);
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(grid);
   config.blockDim = dim3(kChainThreads);

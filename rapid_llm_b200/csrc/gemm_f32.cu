@@ -5,8 +5,6 @@
 // value does not depend on M, on the kernel or the tile it falls in, or on what else is in the batch.
 // The reference has no 32-bit path (rapid_llm/models/config.py:134-146 downgrades float32
 // checkpoints); its products go through a library call (rapid_llm/kernels/ops/gemm/linear.py:17-40).
-#include <atomic>
-
 #include "common.cuh"
 
 namespace rl {
@@ -214,19 +212,6 @@ gemm_f32_few_kernel(const float* __restrict__ a, const float* __restrict__ w, co
   }
 }
 
-// More than 48 KB of shared memory has to be allowed once per kernel and device (a bit each in `done`).
-template <typename Kernel>
-static cudaError_t f32_allow_shared(Kernel kernel, int bytes, std::atomic<unsigned long long>& done) {
-  int device = 0;
-  const cudaError_t found = cudaGetDevice(&device);
-  if (found != cudaSuccess) return found;
-  const unsigned long long bit = 1ull << (device & 63);
-  if (device < 64 && (done.load(std::memory_order_acquire) & bit)) return cudaSuccess;
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e == cudaSuccess && device < 64) done.fetch_or(bit, std::memory_order_release);
-  return e;
-}
-
 template <int kTx, int kTy, int kTm, int kTn>
 static int launch_f32_tiles(bool aligned, const float* a, const float* w, const float* bias, float* c, int m, int n, int k,
                             int lda, int ldc, cudaStream_t stream) {
@@ -235,7 +220,7 @@ static int launch_f32_tiles(bool aligned, const float* a, const float* w, const 
   constexpr int smem = kF32Stages * f32_stage_floats<kTx, kTy, kTm, kTn>() * static_cast<int>(sizeof(float));
   auto kernel = aligned ? gemm_f32_kernel<kTx, kTy, kTm, kTn, true> : gemm_f32_kernel<kTx, kTy, kTm, kTn, false>;
   static std::atomic<unsigned long long> configured[2];
-  const cudaError_t e = f32_allow_shared(kernel, smem, configured[aligned]);
+  const cudaError_t e = allow_shared(kernel, smem, configured[aligned]);
   if (e != cudaSuccess) return static_cast<int>(e);
   kernel<<<grid, kTx * kTy, smem, stream>>>(a, w, bias, c, m, n, k, lda, ldc);
   return launch_status();
@@ -247,7 +232,7 @@ static int launch_f32_few(const float* a, const float* w, const float* bias, flo
   using F = Few<kPer, kG, kR, kBk, kStages>;
   auto kernel = gemm_f32_few_kernel<kPer, kG, kR, kBk, kStages>;
   static std::atomic<unsigned long long> configured;
-  const cudaError_t e = f32_allow_shared(kernel, F::kSmem, configured);
+  const cudaError_t e = allow_shared(kernel, F::kSmem, configured);
   if (e != cudaSuccess) return static_cast<int>(e);
   kernel<<<(n + F::kRows - 1) / F::kRows, kFewThreads, F::kSmem, stream>>>(a, w, bias, c, m, n, k, lda, ldc);
   return launch_status();

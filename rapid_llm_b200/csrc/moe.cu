@@ -714,6 +714,7 @@ grouped_linear_wide_kernel(const __nv_bfloat16* a, int a_stride, const __nv_bflo
 // 42 (44).
 constexpr int kMoeFewWarps = 8;
 constexpr int kMoeFewAhead = 4;      // steps of 32 columns on their way per warp
+constexpr int kMoeFewSmem = 200 * 1024;      // most the pairs' rows may take
 
 template <bool kGated, int kNt>
 __global__ void __launch_bounds__(kMoeFewWarps * 32)
@@ -1017,14 +1018,11 @@ static int launch_grouped_wide(dim3 grid, cudaStream_t stream, bool pdl, const _
                                const __nv_bfloat16* w, const int* sorted, const int* meta, const float* pair_weight,
                                int top, int by_token, int n, int k, __nv_bfloat16* out_act, float* out_y,
                                float glu_limit, float glu_alpha) {
-  static bool configured = false;
+  static std::atomic<unsigned long long> configured;
   auto kernel = rl::grouped_linear_wide_kernel<kGated>;
   constexpr int smem = rl::moe_wide_smem_bytes<kGated>();
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    configured = true;
-  }
+  const cudaError_t e = rl::allow_shared(kernel, smem, configured);
+  if (e != cudaSuccess) return static_cast<int>(e);
   return rl::launch_kernel(kernel, grid, dim3(rl::kMoeThreads), smem, stream, pdl, a, a_stride, w, sorted, meta,
                            pair_weight, top, by_token, n, k, out_act, out_y, glu_limit, glu_alpha);
 }
@@ -1058,14 +1056,13 @@ int rl_grouped_linear(int dtype, const void* a, int a_stride, const void* w, con
       return rl::grouped_linear_tc(a, a_stride, w, experts, sorted, meta, pair_weight, top, by_token, n, k, gated, out_act, out_y,
                                    max_tiles, glu_limit, glu_alpha, fault, pdl, stream);
     const size_t smem = static_cast<size_t>(rl::kMoeFewM) * ((k + 31) / 32 * 32 + 32) * sizeof(bf);
-    if (k % 8 != 0 || a_stride % 8 != 0 || n < 1 || k < 1 || top < 1 || max_tiles > 65535 || smem > 200 * 1024 ||
+    if (k % 8 != 0 || a_stride % 8 != 0 || n < 1 || k < 1 || top < 1 || max_tiles > 65535 || smem > rl::kMoeFewSmem ||
         ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) & 15) != 0)
       return static_cast<int>(cudaErrorInvalidValue);
     auto kernel = gated ? rl::grouped_linear_few_kernel<true, 2> : rl::grouped_linear_few_kernel<false, 2>;
-    if (smem > 30 * 1024) {      // with its own 17 KB beyond what a kernel has without asking
-      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-      if (e != cudaSuccess) return static_cast<int>(e);
-    }
+    static std::atomic<unsigned long long> configured[2];
+    const cudaError_t e = rl::allow_shared(kernel, rl::kMoeFewSmem, configured[gated != 0]);
+    if (e != cudaSuccess) return static_cast<int>(e);
     const int columns = gated ? 16 : 32;
     return rl::launch_kernel(kernel, dim3((n + columns - 1) / columns, max_tiles), dim3(rl::kMoeFewWarps * 32), smem, stream, pdl != 0,
                              static_cast<const bf*>(a), a_stride, static_cast<const bf*>(w), sorted, meta, pair_weight, top, by_token,

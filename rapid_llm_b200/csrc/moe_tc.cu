@@ -259,15 +259,9 @@ grouped_linear_tc_kernel(const __grid_constant__ CUtensorMap map_w, const MoeTcA
 template <bool kGated>
 static int launch_grouped_tc(const CUtensorMap& map_w, const MoeTcArgs& args, int blocks, int pdl, cudaStream_t stream) {
   auto kernel = grouped_linear_tc_kernel<kGated>;
-  static bool configured[64] = {};      // more than 48 KB of shared memory has to be allowed once per device
-  int device = 0;
-  cudaError_t e = cudaGetDevice(&device);
+  static std::atomic<unsigned long long> configured;
+  const cudaError_t e = allow_shared(kernel, kMoeTcSmem, configured);
   if (e != cudaSuccess) return static_cast<int>(e);
-  if (device >= 64 || !configured[device]) {
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMoeTcSmem);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    if (device < 64) configured[device] = true;
-  }
   return launch_kernel(kernel, dim3(blocks), dim3(kMoeTcThreads), kMoeTcSmem, stream, pdl != 0, map_w, args);
 }
 

@@ -30,3 +30,10 @@ def test_what_a_step_writes_is_not_read_as_invariant(name):
     """A load through a const restrict pointer may be moved above the wait for the kernel before."""
     invariant = set(re.findall(r"const [\w:]+\* ?__restrict__ (\w+)", (CSRC / name).read_text()))
     assert invariant <= STEADY, sorted(invariant - STEADY)
+
+
+def test_a_permission_is_remembered_per_device():
+    """A kernel's shared memory beyond 48 KB belongs to the current device: what remembers that it was asked for has a bit for
+    each (`allow_shared`), and nothing a flag for the process."""
+    for path in sorted(CSRC.glob("*.cu*")):
+        assert not re.search(r"\bbool\b[^;\n]*configured", path.read_text()), path.name
