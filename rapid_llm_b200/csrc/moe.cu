@@ -22,7 +22,8 @@
 //   rl_moe_combine_layernorm  the same sum, and at once the layer norm that closes it in an arrangement with the norm
 //                     behind the sum: stream[t] <- LN(res_scale * stream[t] + sum), out[t] its rounding.
 // A row's result does not depend on its tile's other rows or on the order in which the pairs of an
-// expert were laid out: the inner sums run over k in a fixed order per row.
+// expert were laid out: the inner sums run over k in a fixed order per row and kernel.  Which kernel a
+// step's pairs take is a matter of their number and the sizes (`moe_kind` on the host).
 //
 // Five product kernels: float32 FMA tiles (the 32-bit engine; any sizes), mma.sync m16n8k16 tiles for
 // bfloat16 (float32 accumulators; any sizes), and for bfloat16 operands whose rows are multiples of 16 bytes: the same
@@ -716,13 +717,13 @@ constexpr int kMoeFewWarps = 8;
 constexpr int kMoeFewAhead = 4;      // steps of 32 columns on their way per warp
 constexpr int kMoeFewSmem = 200 * 1024;      // most the pairs' rows may take
 
-template <bool kGated, int kNt>
+template <bool kGated>
 __global__ void __launch_bounds__(kMoeFewWarps * 32)
 grouped_linear_few_kernel(const __nv_bfloat16* a, int a_stride, const __nv_bfloat16* __restrict__ w, const int* sorted,
                           const int* meta, const float* pair_weight, int top, int by_token, int n, int k,
                           __nv_bfloat16* out_act, float* out_y, float glu_limit, float glu_alpha) {
   extern __shared__ __align__(16) unsigned char moe_few_smem[];
-  constexpr int kPairs = 8 * kNt;
+  constexpr int kPairs = kMoeFewM, kNt = kPairs / 8;      // pairs of a tile, and groups of eight of them
   __shared__ int s_pair[kPairs];
   __shared__ float partial[kMoeFewWarps][2][16][kPairs + 1];
   const int steps = (k + 31) / 32, stride = steps * 32 + 32;      // 64 bytes between rows' ends: neighbouring rows meet in no bank
@@ -1059,7 +1060,7 @@ int rl_grouped_linear(int dtype, const void* a, int a_stride, const void* w, con
     if (k % 8 != 0 || a_stride % 8 != 0 || n < 1 || k < 1 || top < 1 || max_tiles > 65535 || smem > rl::kMoeFewSmem ||
         ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) & 15) != 0)
       return static_cast<int>(cudaErrorInvalidValue);
-    auto kernel = gated ? rl::grouped_linear_few_kernel<true, 2> : rl::grouped_linear_few_kernel<false, 2>;
+    auto kernel = gated ? rl::grouped_linear_few_kernel<true> : rl::grouped_linear_few_kernel<false>;
     static std::atomic<unsigned long long> configured[2];
     const cudaError_t e = rl::allow_shared(kernel, rl::kMoeFewSmem, configured[gated != 0]);
     if (e != cudaSuccess) return static_cast<int>(e);
