@@ -17,7 +17,7 @@ __device__ __forceinline__ float moe_unit(float g, float u, float limit, float a
 // Sixteen of them, bit for bit, for a warp that has a multiprocessor's quarter to itself: a division's own test for odd
 // operands keeps the next one from starting before it has ended.  The quotients come from an approximate reciprocal,
 // refined once, and are corrected by their remainders, which leaves them rounded to nearest (Markstein, IBM Journal of
-// Research and Development 34, 1990) while the remainders stay in the normal range; where one might not (also zeros,
+// Research and Development 34, 1990) while a remainder has room below its quotient; where one might not (also zeros,
 // infinities, NaN) all sixteen are divided.
 __device__ __forceinline__ void moe_units(float (&g)[16], float (&u)[16], float limit, float alpha, float (&out)[16]) {
   float by[16];
@@ -29,11 +29,10 @@ __device__ __forceinline__ void moe_units(float (&g)[16], float (&u)[16], float 
       u[j] = fminf(fmaxf(u[j], -limit), limit) + 1.0f;
     }
     by[j] = 1.0f + expf(limit > 0.0f ? -alpha * g[j] : -g[j]);
-    const float size = fabsf(g[j]);
-    plain = plain && by[j] < 0x1p60f && size > 0x1p-64f && size < 0x1p60f;
     float inverse = __fdividef(1.0f, by[j]);
     inverse = fmaf(fmaf(-by[j], inverse, 1.0f), inverse, inverse);
     const float near = g[j] * inverse;
+    plain = plain && by[j] < 0x1p126f && fabsf(near) > 0x1p-100f && fabsf(g[j]) < 0x1p100f;
     out[j] = fmaf(fmaf(-by[j], near, g[j]), inverse, near) * u[j];
   }
   if (plain) return;
