@@ -1605,20 +1605,26 @@ def moe_wide_takes(dtype: torch.dtype, *inner_sizes: int) -> bool:
     return dtype == torch.bfloat16 and all(size % 8 == 0 for size in inner_sizes)
 
 
-# Where the product kernels' lines lie, in elements (a pair's inner product sizes, hidden x inter).  Measured with cold
-# weights, both products together, few / 64-pair tiles / tensor, us.  hidden 2,048, inter 512, 2 of 16 experts: 1 token
-# 23 / 39 / 38, 8 tokens 42 / 44 / 41, 32 tokens 53 / 53 / 47, 2,048 tokens - / 139 / 90; hidden 4,096, inter 1,024:
-# 1 token 33 / 63 / 58, 8 tokens 101 / 110 / 93, 2,048 tokens - / 449 / 195; hidden 1,024, inter 256, 1 of 8: 8 tokens
-# 21 / 29 / 30, 64 tokens 22 / 29 / 31, 128 tokens 27 / 29 / 30, 2,048 tokens - / 37 / 39.
-MOE_FEW_ELEMENTS = 1 << 24        # pairs x hidden x inter up to which the weights' stream is short
+# Where the product kernels' lines lie.  Measured with cold weights, both products together, 64-pair tiles / few / tensor, us,
+# two choices a token.  hidden 2,048, inter 512: 8 experts, 8 tokens 38 / 30 / 42, 32 tokens 40 / 32 / 42, 64 tokens
+# 40 / 44 / 42; 16 experts, 1 token 36 / 19 / 38, 8 tokens 42 / 42 / 44, 16 tokens 48 / 46 / 46, 64 tokens 50 / 54 / 48; 32
+# experts, 8 tokens 46 / 41 / 44, 16 tokens 58 / 60 / 54; 64 experts, 8 tokens 54 / 46 / 46, 16 tokens 62 / 69 / 56, 256 tokens
+# 120 / 152 / 101.  hidden 4,096, inter 1,024: 8 experts, 2 tokens 65 / 42 / 60, 8 tokens 81 / 73 / 69; 16 experts, 1 token
+# 61 / 28 / 58, 8 tokens 103 / 93 / 87, 256 tokens 120 / 339 / 99.  hidden 1,024, inter 256: 8 experts, 32 tokens 24 / 19 / 30,
+# 256 tokens 28 / 38 / 32; 32 experts, 8 tokens 26 / 23 / 30, 16 tokens 30 / 30 / 34, 32 tokens 30 / 34 / 34.
+MOE_FEW_TILES = 14.5              # tiles of few pairs up to which they are ahead
+MOE_FEW_ELEMENTS = 1 << 24        # tiles x hidden x inter up to which the weights' stream is short
 MOE_TENSOR_ELEMENTS = 1 << 19     # hidden x inter from which a tile of the tensor cores is worth its start
 
 
-def moe_kind(dtype: torch.dtype, pairs: int, hidden: int, inter: int):
-    """Which product kernels a step's pairs run on (see :func:`moe_tile_rows`)."""
+def moe_kind(dtype: torch.dtype, pairs: int, experts: int, hidden: int, inter: int):
+    """Which product kernels a step's pairs run on (see :func:`moe_tile_rows`): the one for few pairs by the tiles that as
+    many pairs over so many experts fall into: one for each expert that chance lets them touch, more beyond eight pairs an
+    expert."""
     if not moe_wide_takes(dtype, hidden, inter):
         return False
-    if pairs * hidden * inter <= MOE_FEW_ELEMENTS and max(hidden, inter) <= 6144:
+    tiles = max(experts * (1.0 - (1.0 - 1.0 / experts) ** pairs), pairs / 8)
+    if tiles <= MOE_FEW_TILES and tiles * hidden * inter <= MOE_FEW_ELEMENTS and max(hidden, inter) <= 6144:
         return "few"
     return "tensor" if hidden * inter >= MOE_TENSOR_ELEMENTS else True
 

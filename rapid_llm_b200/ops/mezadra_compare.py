@@ -91,19 +91,21 @@ def kernel_figures(width: int, hbm_gbs: float) -> dict:
               lambda: kernels.router_topk(x, router, experts=EXPERTS, top=TOP, ids=ids, weights=weights, gates=gates))
         pairs = tokens * TOP
         order, place = (torch.empty(pairs, dtype=torch.int32, device=device) for _ in range(2))
-        meta = torch.zeros(1 + 3 * kernels.moe_max_tiles(pairs, EXPERTS, True), dtype=torch.int32, device=device)
-        timed("moe_plan", tokens, entries, pairs * 16, lambda: kernels.moe_plan(ids, EXPERTS, order, place, meta, fault, wide=True))
-        max_tiles = kernels.moe_max_tiles(pairs, EXPERTS, True)
-        gate_up, down = bf(EXPERTS, 2 * inter, width), bf(EXPERTS, width, inter)
+        kind = kernels.moe_kind(torch.bfloat16, pairs, EXPERTS, width, inter)      # the product kernels the engine takes
+        meta = torch.zeros(1 + 3 * kernels.moe_max_tiles(pairs, EXPERTS, kind), dtype=torch.int32, device=device)
+        timed("moe_plan", tokens, entries, pairs * 16, lambda: kernels.moe_plan(ids, EXPERTS, order, place, meta, fault, wide=kind))
+        max_tiles = kernels.moe_max_tiles(pairs, EXPERTS, kind)
+        gate_up, down = bf(EXPERTS, 2 * inter, width) / width ** 0.5, bf(EXPERTS, width, inter)
         act, each = torch.empty(pairs, inter, dtype=torch.bfloat16, device=device), torch.empty(pairs, width, device=device)
         touched = min(EXPERTS, pairs)          # experts whose weights a step streams
         timed("grouped_linear, gate and up with the activation", tokens, entries,
               touched * 2 * inter * width * 2 + tokens * width * 2 + pairs * inter * 2,
               lambda: kernels.grouped_linear(x, gate_up, order, meta, top=TOP, by_token=True, max_tiles=max_tiles,
-                                             pair_weight=weights.view(-1), out_act=act, wide=True),
+                                             pair_weight=weights.view(-1), out_act=act, wide=kind, fault=fault),
               flops=2.0 * pairs * 2 * inter * width)
         timed("grouped_linear, down", tokens, entries, touched * inter * width * 2 + pairs * inter * 2 + pairs * width * 4,
-              lambda: kernels.grouped_linear(act, down, order, meta, top=TOP, by_token=False, max_tiles=max_tiles, out_y=each, wide=True),
+              lambda: kernels.grouped_linear(act, down, order, meta, top=TOP, by_token=False, max_tiles=max_tiles, out_y=each, wide=kind,
+                                             fault=fault),
               flops=2.0 * pairs * inter * width)
         shared, combined = bf(tokens, width), torch.empty(tokens, width, dtype=torch.bfloat16, device=device)
         timed("moe_combine", tokens, entries, pairs * width * 4 + tokens * width * 4,

@@ -122,8 +122,9 @@ def kernel_figures(width: int, hbm_gbs: float) -> dict:
         # -- clamped experts over the pairs that chose one, beside SiLU experts over the same plan; the weighted sum
         pairs = tokens * TOP
         order, place = (torch.empty(pairs, dtype=torch.int32, device=device) for _ in range(2))
-        meta = torch.zeros(1 + 3 * kernels.moe_max_tiles(pairs, EXPERTS, True), dtype=torch.int32, device=device)
-        max_tiles = kernels.moe_plan(ids, EXPERTS, order, place, meta, fault, wide=True)
+        kind = kernels.moe_kind(torch.bfloat16, pairs, EXPERTS, width, inter)      # the product kernels the engine takes
+        meta = torch.zeros(1 + 3 * kernels.moe_max_tiles(pairs, EXPERTS, kind), dtype=torch.int32, device=device)
+        max_tiles = kernels.moe_plan(ids, EXPERTS, order, place, meta, fault, wide=kind)
         gate_up, down = bf(EXPERTS, 2 * inter, width) / width ** 0.5, bf(EXPERTS, width, inter)
         act, each = torch.zeros(pairs, inter, dtype=torch.bfloat16, device=device), torch.zeros(pairs, width, device=device)
         real = int((ids < EXPERTS).sum())
@@ -131,11 +132,11 @@ def kernel_figures(width: int, hbm_gbs: float) -> dict:
         moved = touched * 2 * inter * width * 2 + tokens * width * 2 + real * inter * 2
         timed("grouped_linear, gate and up, clamped unit", tokens, entries, moved,
               lambda: kernels.grouped_linear(x, gate_up, order, meta, top=TOP, by_token=True, max_tiles=max_tiles, out_act=act,
-                                             wide=True, clamp=(7.0, 1.702)), flops=2.0 * real * 2 * inter * width)
+                                             wide=kind, fault=fault, clamp=(7.0, 1.702)), flops=2.0 * real * 2 * inter * width)
         timed("grouped_linear, gate and up, SiLU (like kernel)", tokens, entries, moved,
               lambda: kernels.grouped_linear(x, gate_up, order, meta, top=TOP, by_token=True, max_tiles=max_tiles, out_act=act,
-                                             wide=True), flops=2.0 * real * 2 * inter * width)
-        kernels.grouped_linear(act, down, order, meta, top=TOP, by_token=False, max_tiles=max_tiles, out_y=each, wide=True)
+                                             wide=kind, fault=fault), flops=2.0 * real * 2 * inter * width)
+        kernels.grouped_linear(act, down, order, meta, top=TOP, by_token=False, max_tiles=max_tiles, out_y=each, wide=kind, fault=fault)
         combined = torch.empty(tokens, width, dtype=torch.bfloat16, device=device)
         timed("moe_combine, weights and identity experts", tokens, entries, pairs * width * 4 + tokens * width * 4,
               lambda: kernels.moe_combine(each, TOP, combined, weights=weights.view(-1), ids=ids, experts=EXPERTS, x=x))

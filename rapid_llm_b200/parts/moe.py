@@ -169,7 +169,7 @@ class RoutedExperts(FeedForward):
                             correction=self.correction, groups=self.groups, keep=self.keep)
         order = space.get("moe_sorted", tokens, top, i32).view(-1)
         place = space.get("moe_place", tokens, top, i32).view(-1)
-        wide = kernels.moe_kind(x.dtype, pairs, self.hidden, self.inter)      # which product kernels
+        wide = kernels.moe_kind(x.dtype, pairs, experts, self.hidden, self.inter)      # which product kernels
         most = kernels.moe_max_tiles(max(space.max_tokens, tokens) * top, experts, "few")      # the smallest tiles
         meta = space.get("moe_meta", 1, 1 + 3 * most, i32, min_rows=1).view(-1)
         max_tiles = kernels.moe_plan(ids, experts, order, place, meta, batch.fault, wide=wide)
