@@ -261,8 +261,8 @@ extern "C" int rl_gemm_f32(const float* a, const float* w, const float* bias, fl
     return many ? rl::launch_f32_few<8, 4, 2, 64, 3>(a, w, bias, c, m, n, k, lda, ldc, stream)
                 : rl::launch_f32_few<8, 4, 1, 64, 6>(a, w, bias, c, m, n, k, lda, ldc, stream);
   }
-  // 64 x 64 tiles (4 x 8 outputs a thread) or 112 x 64 (7 x 8): a round of tiles on all multiprocessors takes about 115 and
-  // 180 us at K = 4,096 (measured over 40 to 2,048 rows), so the rule compares the rounds
+  // 64 x 64 tiles (4 x 8 outputs a thread) or 112 x 64 (7 x 8): a round of tiles on the B200's 148 multiprocessors takes about
+  // 115 and 180 us at K = 4,096 (measured over 40 to 2,048 rows), both in proportion to K, so the rule compares the rounds
   const long long wide = (n + 63) / 64, sms = 148;
   const long long low = (((m + 63) / 64) * wide + sms - 1) / sms, high = (((m + 111) / 112) * wide + sms - 1) / sms;
   if (180 * high < 115 * low) return rl::launch_f32_tiles<8, 16, 7, 8>(aligned, a, w, bias, c, m, n, k, lda, ldc, stream);

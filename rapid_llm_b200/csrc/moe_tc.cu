@@ -13,8 +13,8 @@
 //
 // Bound by what a multiprocessor fetches per product: 48 KB for every 64 columns of a tile.  Before that the gated
 // results' divisions held it up, one behind the other (a tile's 128 outputs a thread: 20 to 35 us more), so sixteen are
-// formed together (moe_units).  Hidden 2,048, inter 512, 2 of 16 experts, 2,048 tokens: 51 + 41 us (mma.sync tiles of 64
-// pairs: 80 + 59; a plain division: 82 + 43); hidden 4,096, inter 1,024: 118 + 82 (270 + 178; 137 + 80).
+// formed together (moe_units).  Hidden 2,048, inter 512, 2 of 16 experts, 2,048 tokens: 50 + 43 us (mma.sync tiles of 64
+// pairs: 80 + 59; a plain division: 82 + 43); hidden 4,096, inter 1,024: 119 + 82 (270 + 178; 137 + 80).
 #include <cuda.h>
 
 #include "common.cuh"

@@ -7,8 +7,9 @@
 // one float32 row per slot (`state + slot * state_stride + offset`); a request at position 0 starts
 // from zeros whatever the row holds, so a slot needs no clearing when it changes hands.  Everything a
 // recurrence consumes (decays, step sizes, gates, unit vectors, the state) is float32 in both engine
-// precisions; the recurrence runs token by token in a fixed order, so a row's result does not depend
-// on how the tokens were cut into steps or on what else is in the batch.
+// precisions.  The recurrence runs token by token in a fixed order, so a row's result does not depend
+// on how the tokens were cut into steps or on what else is in the batch; in 16-bit engines long entries
+// are walked in pieces, whose order of sums depends on the entry's length in the step and on nothing else in it.
 //
 // Pointers to what an earlier kernel of the same step wrote (activations, the state) carry no `__restrict__`:
 // a load through a const restrict pointer counts as invariant and may be moved above the wait for the
@@ -623,8 +624,8 @@ __global__ void rotate_heads_kernel(const T* in, int in_stride, int q_col0, int 
 //
 // A column of S is shared by kPartners lanes of one warp, a lane holds kRows of its rows in registers (pieces of four,
 // kPartners pieces apart) for kCols neighbouring columns; sums over rows run down a lane's rows and then over lanes in a
-// fixed tree of exchanges (offsets from kPartners / 2 down), so a token's result depends on nothing but the tokens before
-// it: not on the step it came in, the group of tokens it was walked in, or kCols.  In the slot's row a head's state lies
+// fixed tree of exchanges (offsets from kPartners / 2 down), so in a walk a token's result depends on nothing but the tokens
+// before it: not on the step it came in, the group of tokens it was walked in, or kCols.  In the slot's row a head's state lies
 // column by column (S^T, [vdim][dim]).
 //
 // What bounds the walk: a token's k, q and row decays are wanted by every column, and shared memory hands a multiprocessor
@@ -634,10 +635,12 @@ __global__ void rotate_heads_kernel(const T* in, int in_stride, int q_col0, int 
 // A correction (beta) makes a token wait for the sum over the whole column of the token before it: there a column has
 // few lanes with many rows each, since an exchange between lanes waits as long as eight multiply-adds, and prompts are
 // walked from end to end (in pieces the state has to go through a matrix per piece, which costs digits).
-// 2,048 tokens, us, before / from end to end / in pieces: 16 heads of 128, fixed decay 432 / 288 / 187; 32 heads of 64, row
-// decays 383 / 255 / 138; with a bonus 334 / 278 / 151; 32 heads of 128, fixed, 3 prompts 552 / 410 / 339; with a
-// correction, 16 heads of 128, 632 / 572.  64 single tokens: 64 heads of 64, row decays 54 / 31 (4.3 TB/s), 16 heads of
-// 128, fixed 53 / 31 (see the kernel).
+// 2,048 tokens, us, before / from end to end / in pieces: 16 heads of 128, fixed decay 432 / 284 / 199; 32 heads of 64, row
+// decays 383 / 252 / 140; with a bonus 334 / 258 / 154; 32 heads of 128, fixed, 570 / 398 / 341; with a
+// correction, 16 heads of 128, 632 / 571.  64 single tokens: 64 heads of 64, row decays 54 / 31 (4.3 TB/s), 16 heads of
+// 128, fixed 53 / 31 (see the kernel).  Root mean square error against 64 bits, 1,300 tokens of 16 heads of 128, before /
+// from end to end / in pieces: fixed decays 3.52e-7 / 3.52e-7 / 2.50e-7, row decays 1.836e-7 / 1.838e-7 / 1.806e-7, with a
+// correction 1.646e-7 / 1.646e-7; their states 4.06e-7 / 4.06e-7 / 2.18e-7, 1.71e-7 / 1.71e-7 / 1.64e-7, 1.46e-7 / 1.47e-7.
 struct ScanArgs {
   const float* q; int q_stride;
   const float* k; int k_stride;

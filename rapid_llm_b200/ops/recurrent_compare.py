@@ -3,7 +3,7 @@ and every kernel of the recurrent mixers alone against the memory roofline.
 
     python bench.py --workload kopatar [--sizes 2048,4096]
     python -m rapid_llm_b200.ops.recurrent_compare [--sizes 2048,4096]
-    python -m rapid_llm_b200.ops.recurrent_compare --scan fixed|delta      # three launches of the recurrence, for ncu
+    python -m rapid_llm_b200.ops.recurrent_compare --scan fixed|pieces|delta      # three launches of the recurrence, for ncu
 
 Random weights, bfloat16, one GPU.  A model of width ``W`` has heads of 128, a feed-forward of ``4 W`` (Qwen3's
 gated one gets ``8 W / 3`` rounded to 256, the same number of weights) and the layers
@@ -186,7 +186,8 @@ def kernel_figures(width: int, hbm_gbs: float) -> dict:
 
 def scan_alone(kind: str, width: int = 2048, launches: int = 3) -> None:
     """A few launches of the recurrence kernel over one 2,048-token prompt and nothing else: the case a profiler
-    captures (``--scan fixed`` or ``--scan delta``)."""
+    captures (``--scan fixed``, ``--scan delta``, or ``--scan pieces``: fixed decays as a 16-bit engine walks them)."""
+    from ..engine.batch import Workspace
     from . import kernels
 
     device, heads, dim, tokens = "cuda:0", width // 128, 128, PREFILL
@@ -195,7 +196,8 @@ def scan_alone(kind: str, width: int = 2048, launches: int = 3) -> None:
         cu_seqlens=torch.tensor([0, tokens], dtype=torch.int32, device=device),
         entry_slot=torch.zeros(1, dtype=torch.int32, device=device),
         entry_start=torch.full((1,), 512, dtype=torch.int32, device=device), num_entries=1,
-        fault=torch.zeros(1, dtype=torch.int32, device=device))
+        fault=torch.zeros(1, dtype=torch.int32, device=device), max_query_len=tokens)
+    pieces = Workspace(tokens, torch.device(device)) if kind == "pieces" else None
     q, k, v, read = (torch.randn(tokens, c, device=device) for _ in range(4))
     state = torch.zeros(1, heads * dim * dim, device=device)
     for _ in range(launches):
@@ -204,7 +206,7 @@ def scan_alone(kind: str, width: int = 2048, launches: int = 3) -> None:
                                 kv_heads=heads, dim=dim, vdim=dim, beta=torch.rand(tokens, heads, device=device))
         else:
             kernels.linear_scan(q, k, v, torch.rand(heads, device=device), read, state, batch, heads=heads,
-                                kv_heads=heads, dim=dim, vdim=dim)
+                                kv_heads=heads, dim=dim, vdim=dim, pieces=pieces)
     torch.cuda.synchronize()
 
 
@@ -226,7 +228,7 @@ def main() -> int:
     parser = argparse.ArgumentParser(description=__doc__.splitlines()[0])
     parser.add_argument("--sizes", default="2048,4096")
     parser.add_argument("--hbm-gbs", type=float, default=6650.0)
-    parser.add_argument("--scan", choices=["fixed", "delta"], default=None,
+    parser.add_argument("--scan", choices=["fixed", "pieces", "delta"], default=None,
                         help="only launch the recurrence kernel a few times (for a profiler)")
     args = parser.parse_args()
     if args.scan:

@@ -1,8 +1,8 @@
 """Mixers that carry a state of fixed size per request: linear recurrences over a matrix ``S``.
 
 All of them keep, per head, a float32 matrix ``S`` of ``key_dim x value_dim`` in the request's state row
-and advance it token by token in one kernel (``ops.kernels.linear_scan``), which serves portions of
-prompts and single decoded tokens alike:
+and advance it token by token (``ops.kernels.linear_scan``, portions of prompts and single decoded tokens alike);
+in bfloat16 engines long portions are walked in pieces side by side, except with the delta rule:
 
 * :class:`ChannelDeltaRule` (``gated_delta_rule``) — the delta rule with a decay per head and key channel:
   ``S <- diag(g) S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q``.
@@ -54,7 +54,7 @@ class _Recurrent(Mixer):
         return StateNeed((self.state_size + self.tail_size,), torch.float32)
 
     def _pieces(self, batch):
-        """Where a long prompt is walked in pieces side by side: in bfloat16.  The 32-bit path walks a request's tokens one
+        """Where a long entry is walked in pieces side by side: in bfloat16.  The 32-bit path walks a request's tokens one
         after the other, so that its rows are the same bit for bit however they are cut into steps."""
         return batch.workspace if self.dtype == torch.bfloat16 else None
 
