@@ -113,7 +113,7 @@ attention_decode_tc_kernel(const __grid_constant__ CUtensorMap map_cache, const 
   volatile int* aborted = &aborted_flag;
 
   pdl_trigger();
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   const uint32_t base = (smem_addr(tc_smem_raw) + 1023u) & ~1023u;
   auto k_tile = [&](int s) { return base + s * kTcStageBytes; };
   auto v_tile = [&](int s) { return base + s * kTcStageBytes + kTcTileBytes; };
@@ -193,7 +193,7 @@ attention_decode_tc_kernel(const __grid_constant__ CUtensorMap map_cache, const 
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = tmem_slot;
+  const uint32_t tmem_base = uniform(tmem_slot);
   // tensor-memory columns of team `team`, buffer `buf`: scores, then values
   auto tmem_score = [&](int team, int buf) { return tmem_base + (team * 4 + buf) * kTcRows; };
   auto tmem_value = [&](int team, int buf) { return tmem_base + (team * 4 + 2 + buf) * kTcRows; };
@@ -270,47 +270,54 @@ attention_decode_tc_kernel(const __grid_constant__ CUtensorMap map_cache, const 
     // value buffers.  Scores are issued as soon as their keys have arrived and their buffer is
     // free (the block four before has been through its softmax), values as soon as P^T and the
     // value tile are there: the thread looks at both in turn, so neither waits behind the other.
-    if (lane == 0) {
-      bool ok = n_blocks > 0;
-      if (ok) ok = mbar_wait(smem_addr(&q_ready), 0, aborted, args.fault);
+    {
+      const int blocks = uniform(n_blocks);
+      const bool issues = elect_one();
+      auto there = [&](uint64_t* bar, int phase) { return __all_sync(0xffffffffu, mbar_test(smem_addr(bar), phase & 1)); };
+      bool ok = blocks > 0;
+      if (ok) ok = __all_sync(0xffffffffu, mbar_wait(smem_addr(&q_ready), 0, aborted, args.fault));
       const uint64_t q_desc = operand_desc(q_tile);
       int next_s = 0, next_pv = 0;
       uint32_t idle = 0;
-      while (ok && next_pv < n_blocks) {
+      while (ok && next_pv < blocks) {
         bool progressed = false;
-        if (next_s < n_blocks && next_s < next_pv + 4 &&
-            mbar_test(smem_addr(&full_k[next_s % kTcStages]), (next_s / kTcStages) & 1)) {
+        if (next_s < blocks && next_s < next_pv + 4 && there(&full_k[next_s % kTcStages], next_s / kTcStages)) {
           const int stage = next_s % kTcStages, team = next_s & 1, buf = (next_s >> 1) & 1;
           tc_fence_after();
           const uint64_t keys_desc = operand_desc(k_tile(stage));
+          if (issues) {
 #pragma unroll
-          for (int k = 0; k < kTcD / 16; ++k) {
-            // descriptors count addresses in units of 16 bytes: 32 bytes further along a row = +2
-            const uint32_t half = (k >> 2), within = (k & 3) * 2;
-            umma_bf16(tmem_score(team, buf), keys_desc + half * (kTcHalfBytes >> 4) + within,
-                      q_desc + half * (kTcRows * 128 >> 4) + within, kTcIdescScore, k > 0 ? 1u : 0u);
+            for (int k = 0; k < kTcD / 16; ++k) {
+              // descriptors count addresses in units of 16 bytes: 32 bytes further along a row = +2
+              const uint32_t half = (k >> 2), within = (k & 3) * 2;
+              umma_bf16(tmem_score(team, buf), keys_desc + half * (kTcHalfBytes >> 4) + within,
+                        q_desc + half * (kTcRows * 128 >> 4) + within, kTcIdescScore, k > 0 ? 1u : 0u);
+            }
+            umma_commit(smem_addr(&score_ready[team][buf]));
+            umma_commit(smem_addr(&empty_k[stage]));
           }
-          umma_commit(smem_addr(&score_ready[team][buf]));
-          umma_commit(smem_addr(&empty_k[stage]));
+          __syncwarp();
           ++next_s;
           progressed = true;
         }
         if (next_pv < next_s) {
           const int stage = next_pv % kTcStages, team = next_pv & 1, buf = (next_pv >> 1) & 1;
-          if (mbar_test(smem_addr(&p_ready[team][buf]), (next_pv >> 2) & 1) &&
-              mbar_test(smem_addr(&full_v[stage]), (next_pv / kTcStages) & 1)) {
+          if (there(&p_ready[team][buf], next_pv >> 2) && there(&full_v[stage], next_pv / kTcStages)) {
             tc_fence_after();
             const uint64_t values_desc = operand_desc_mn(v_tile(stage), kTcHalfBytes);
             const uint64_t p_desc = operand_desc(p_tile(team, buf));
+            if (issues) {
 #pragma unroll
-            for (int k = 0; k < kTcKeys / 16; ++k) {
-              // 16 keys further: two groups of eight 128-byte rows in the value tile, 32 bytes in P^T
-              const uint32_t half = (k >> 2), within = (k & 3) * 2;
-              umma_bf16(tmem_value(team, buf), values_desc + k * (2048 >> 4),
-                        p_desc + half * (kTcRows * 128 >> 4) + within, kTcIdescValue, k > 0 ? 1u : 0u);
+              for (int k = 0; k < kTcKeys / 16; ++k) {
+                // 16 keys further: two groups of eight 128-byte rows in the value tile, 32 bytes in P^T
+                const uint32_t half = (k >> 2), within = (k & 3) * 2;
+                umma_bf16(tmem_value(team, buf), values_desc + k * (2048 >> 4),
+                          p_desc + half * (kTcRows * 128 >> 4) + within, kTcIdescValue, k > 0 ? 1u : 0u);
+              }
+              umma_commit(smem_addr(&value_ready[team][buf]));
+              umma_commit(smem_addr(&empty_v[stage]));
             }
-            umma_commit(smem_addr(&value_ready[team][buf]));
-            umma_commit(smem_addr(&empty_v[stage]));
+            __syncwarp();
             ++next_pv;
             progressed = true;
           }
@@ -319,7 +326,7 @@ attention_decode_tc_kernel(const __grid_constant__ CUtensorMap map_cache, const 
           idle = 0;
         } else {
           __nanosleep(32);                        // leave the issue slots to the softmax warps
-          if (++idle > (kSpinLimit >> 4) || ((idle & 255u) == 0 && *aborted)) {
+          if (++idle > (kSpinLimit >> 4) || ((idle & 255u) == 0 && __any_sync(0xffffffffu, *aborted))) {
             if (idle > (kSpinLimit >> 4)) {
               *aborted = 1;
               atomicOr(args.fault, kFaultWaitLimit);
@@ -328,7 +335,8 @@ attention_decode_tc_kernel(const __grid_constant__ CUtensorMap map_cache, const 
           }
         }
       }
-      umma_commit(smem_addr(&drained));
+      if (issues) umma_commit(smem_addr(&drained));
+      __syncwarp();
       mbar_wait(smem_addr(&drained), 0, aborted, args.fault);
     }
   }

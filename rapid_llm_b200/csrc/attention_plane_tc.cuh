@@ -90,7 +90,7 @@ attention_plane_tc_kernel(const __grid_constant__ CUtensorMap map_cache, const P
   volatile int* aborted = &aborted_flag;
 
   pdl_trigger();
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   const uint32_t q_tile = (smem_addr(pl_smem_raw) + 1023u) & ~1023u;
   auto tile_at = [&](int s) { return q_tile + kPlQBytes + s * kPlTileBytes; };
 
@@ -157,7 +157,7 @@ attention_plane_tc_kernel(const __grid_constant__ CUtensorMap map_cache, const P
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_out = tmem_slot;
+  const uint32_t tmem_out = uniform(tmem_slot);
   auto tmem_score = [&](int b) { return tmem_out + kPlScoreColumn + (b & 1) * 128; };
 
   if (warp == 0) {
@@ -213,7 +213,9 @@ attention_plane_tc_kernel(const __grid_constant__ CUtensorMap map_cache, const P
     // -------------------------------------------------------------------- tensor-core issuer
     // Products run in the order they are issued: the scores of block j + 2 overwrite the columns that held P of
     // block j only after the values product that read them.
-    bool ok = n_blocks > 0;
+    const int blocks = uniform(n_blocks);
+    const bool issues = elect_one();
+    bool ok = blocks > 0;
     auto wait = [&](uint64_t* bar, int phase, int where) {
       return __all_sync(0xffffffffu, mbar_wait(smem_addr(bar), phase & 1, aborted, args.fault, where));
     };
@@ -234,7 +236,7 @@ attention_plane_tc_kernel(const __grid_constant__ CUtensorMap map_cache, const P
       return true;
     };
     auto issue_scores = [&](int b) {
-      if (lane == 0) {
+      if (issues) {
         const uint64_t q_desc = operand_desc(q_tile), keys_desc = operand_desc(tile_at(b % kPlStages));
 #pragma unroll
         for (int k = 0; k < kPlD / 16; ++k) {
@@ -249,8 +251,8 @@ attention_plane_tc_kernel(const __grid_constant__ CUtensorMap map_cache, const P
     if (ok) ok = wait(&q_ready, 0, 1 << 10);
     if (ok) ok = rows_here(0);
     if (ok) issue_scores(0);
-    for (int b = 0; b < n_blocks && ok; ++b) {
-      if (b + 1 < n_blocks) {
+    for (int b = 0; b < blocks && ok; ++b) {
+      if (b + 1 < blocks) {
         ok = rows_here(b + 1);
         if (!ok) break;
         issue_scores(b + 1);
@@ -258,7 +260,7 @@ attention_plane_tc_kernel(const __grid_constant__ CUtensorMap map_cache, const P
       ok = wait(&p_ready[b & 1], b >> 1, 1 << 11);
       if (!ok) break;
       tc_fence_after();
-      if (lane == 0) {
+      if (issues) {
         const uint64_t values_desc = operand_desc_mn(tile_at(b % kPlStages), kPlAtomBytes);
 #pragma unroll
         for (int part = 0; part < 2; ++part) {      // P as it rounds, then what the rounding left
@@ -272,10 +274,9 @@ attention_plane_tc_kernel(const __grid_constant__ CUtensorMap map_cache, const P
       }
       __syncwarp();
     }
-    if (lane == 0) {
-      umma_commit(smem_addr(&drained));
-      mbar_wait(smem_addr(&drained), 0, aborted, args.fault, 1 << 12);
-    }
+    if (issues) umma_commit(smem_addr(&drained));
+    __syncwarp();
+    mbar_wait(smem_addr(&drained), 0, aborted, args.fault, 1 << 12);
     __syncwarp();
   } else if (warp >= 4 && (warp & 3) < live) {
     // -------------------------------------------------------------------- softmax and output

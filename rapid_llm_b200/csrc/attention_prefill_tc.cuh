@@ -122,7 +122,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_cache, const
   volatile int* aborted = &aborted_flag;
 
   pdl_trigger();
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   const uint32_t base = (smem_addr(pf_smem_raw) + 1023u) & ~1023u;
   auto q_tile = [&](int tile) { return base + tile * kPfTileBytes; };
   auto k_tile = [&](int s) { return base + (kPfTiles + s) * kPfTileBytes; };
@@ -198,7 +198,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_cache, const
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = tmem_slot;
+  const uint32_t tmem_base = uniform(tmem_slot);
   auto tmem_score = [&](int tile) { return tmem_base + tile * 256; };        // 128 columns; P over its first 64
   auto tmem_out = [&](int tile) { return tmem_base + tile * 256 + 128; };    // 128 columns
 
@@ -269,64 +269,80 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_cache, const
       // so that its softmax threads have work while the other tile's values are multiplied.
       // Products run in the order they are issued: the scores of block j + 1 overwrite the
       // columns that held P of block j only after the values product that read them.
-      if (lane == 0) {
-        bool ok = n_blocks > 0;
-        if (ok) ok = mbar_wait(smem_addr(&q_ready), 0, aborted, args.fault, 1 << 10);
-        auto issue_scores = [&](int tile, int b) {
-          const int stage = b % kPfStages;
-          const uint64_t q_desc = operand_desc(q_tile(tile)), keys_desc = operand_desc(k_tile(stage));
-  #pragma unroll
+      const int blocks = uniform(n_blocks);
+      int blocks_of[kPfTiles];
+      for (int tile = 0; tile < kPfTiles; ++tile) blocks_of[tile] = uniform(tile_blocks[tile]);
+      const bool issues = elect_one();
+      auto wait = [&](uint64_t* bar, int phase, int where) {
+        return __all_sync(0xffffffffu, mbar_wait(smem_addr(bar), phase & 1, aborted, args.fault, where));
+      };
+      bool ok = blocks > 0;
+      if (ok) ok = wait(&q_ready, 0, 1 << 10);
+      auto issue_scores = [&](int tile, int b) {
+        const int stage = b % kPfStages;
+        const uint64_t q_desc = operand_desc(q_tile(tile)), keys_desc = operand_desc(k_tile(stage));
+        if (issues) {
+#pragma unroll
           for (int k = 0; k < kPfD / 16; ++k) {
             const uint32_t half = (k >> 2), within = (k & 3) * 2;
             umma_bf16(tmem_score(tile), q_desc + half * (kPfHalfBytes >> 4) + within,
                       keys_desc + half * (kPfHalfBytes >> 4) + within, kPfIdescScore, k > 0 ? 1u : 0u);
           }
           umma_commit(smem_addr(&score_ready[tile]));
-        };
-        // the last tile that uses block b releases its key tile
-        auto release_keys = [&](int b) { umma_commit(smem_addr(&empty_k[b % kPfStages])); };
-        if (ok) {
-          ok = mbar_wait(smem_addr(&full_k[0]), 0, aborted, args.fault, 1 << 11);
-          if (ok) {
-            tc_fence_after();
-            for (int tile = 0; tile < kPfTiles; ++tile)
-              if (tile_blocks[tile] > 0) issue_scores(tile, 0);
-            release_keys(0);
-          }
         }
-        for (int b = 0; b < n_blocks && ok; ++b) {
-          const int stage = b % kPfStages;
-          bool keys_next = false;
-          for (int tile = 0; tile < kPfTiles && ok; ++tile) {
-            if (b >= tile_blocks[tile]) continue;
-            ok = mbar_wait(smem_addr(&p_ready[tile]), b & 1, aborted, args.fault, 1 << (12 + tile));
-            if (!ok) break;
-            ok = mbar_wait(smem_addr(&full_v[stage]), (b / kPfStages) & 1, aborted, args.fault, 1 << 14);
-            if (!ok) break;
-            tc_fence_after();
-            const uint64_t values_desc = operand_desc_mn(v_tile(stage), kPfHalfBytes);
-  #pragma unroll
+        __syncwarp();
+      };
+      // the last tile that uses block b releases its key tile
+      auto release_keys = [&](int b) {
+        if (issues) umma_commit(smem_addr(&empty_k[b % kPfStages]));
+        __syncwarp();
+      };
+      if (ok) {
+        ok = wait(&full_k[0], 0, 1 << 11);
+        if (ok) {
+          tc_fence_after();
+#pragma unroll
+          for (int tile = 0; tile < kPfTiles; ++tile)
+            if (blocks_of[tile] > 0) issue_scores(tile, 0);
+          release_keys(0);
+        }
+      }
+      for (int b = 0; b < blocks && ok; ++b) {
+        const int stage = b % kPfStages;
+        bool keys_next = false;
+#pragma unroll
+        for (int tile = 0; tile < kPfTiles; ++tile) {
+          if (!ok || b >= blocks_of[tile]) continue;
+          ok = wait(&p_ready[tile], b, 1 << (12 + tile)) && wait(&full_v[stage], b / kPfStages, 1 << 14);
+          if (!ok) continue;
+          tc_fence_after();
+          const uint64_t values_desc = operand_desc_mn(v_tile(stage), kPfHalfBytes);
+          if (issues) {
+#pragma unroll
             for (int k = 0; k < kPfKeys / 16; ++k)
               umma_bf16_ts(tmem_out(tile), tmem_score(tile) + k * 8, values_desc + k * (2048 >> 4), kPfIdescValue,
                            (b > 0 || k > 0) ? 1u : 0u);
             umma_commit(smem_addr(&value_done[tile]));
-            if (b + 1 < tile_blocks[tile]) {
-              if (!keys_next) {
-                ok = mbar_wait(smem_addr(&full_k[(b + 1) % kPfStages]), ((b + 1) / kPfStages) & 1, aborted, args.fault, 1 << 15);
-                if (!ok) break;
-                tc_fence_after();
-                keys_next = true;
-              }
-              issue_scores(tile, b + 1);
-            }
           }
-          if (!ok) break;
-          umma_commit(smem_addr(&empty_v[stage]));
-          if (keys_next) release_keys(b + 1);
+          __syncwarp();
+          if (b + 1 < blocks_of[tile]) {
+            if (!keys_next) {
+              ok = wait(&full_k[(b + 1) % kPfStages], (b + 1) / kPfStages, 1 << 15);
+              if (!ok) continue;
+              tc_fence_after();
+              keys_next = true;
+            }
+            issue_scores(tile, b + 1);
+          }
         }
-        umma_commit(smem_addr(&drained));
-        mbar_wait(smem_addr(&drained), 0, aborted, args.fault, 1 << 16);
+        if (!ok) break;
+        if (issues) umma_commit(smem_addr(&empty_v[stage]));
+        __syncwarp();
+        if (keys_next) release_keys(b + 1);
       }
+      if (issues) umma_commit(smem_addr(&drained));
+      __syncwarp();
+      mbar_wait(smem_addr(&drained), 0, aborted, args.fault, 1 << 16);
     }
   } else {
     // -------------------------------------------------------------------- softmax and output

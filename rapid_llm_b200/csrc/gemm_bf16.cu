@@ -150,7 +150,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   volatile int* aborted = &aborted_flag;
 
   if (args.pdl && threadIdx.x == 0) pdl_trigger();   // the successor may set itself up beside this kernel
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform(static_cast<int>(threadIdx.x) >> 5), lane = threadIdx.x & 31;
   const uint32_t smem_base = (smem_addr(gemm_smem_raw) + 1023u) & ~1023u;
   auto stage_a = [&](int s, int half) { return smem_base + s * Shape::kStageBytes + half * kTileN * kTileK * 2; };
   auto stage_b = [&](int s) { return smem_base + s * Shape::kStageBytes + kHalves * kTileN * kTileK * 2; };
@@ -215,7 +215,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = tmem_base_slot;
+  const uint32_t tmem_base = uniform(tmem_base_slot);
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -250,20 +250,21 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ tensor-core issuer
-    if (lane == 0) {
-      int stage = 0, buf = 0;
-      uint32_t phase = 0, acc_phase[2] = {0, 0};
-      bool ok = kb_count > 0;
-      for (int index = 0; index < my_tiles && ok; ++index) {
-        ok = mbar_wait(smem_addr(&acc_empty_bar[buf]), acc_phase[buf] ^ 1u, aborted, args.fault);
+    const bool issues = elect_one();
+    int stage = 0, buf = 0;
+    uint32_t phase = 0, acc_phase = 0;                 // acc_phase: a bit for each buffer
+    bool ok = kb_count > 0;
+    for (int index = 0; index < my_tiles && ok; ++index) {
+      ok = __all_sync(0xffffffffu, mbar_wait(smem_addr(&acc_empty_bar[buf]), ((acc_phase >> buf) & 1u) ^ 1u, aborted, args.fault));
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + buf * Shape::kAccColumns;
+      for (int kb = 0; kb < kb_count; ++kb) {
+        ok = __all_sync(0xffffffffu, mbar_wait(smem_addr(&full_bar[stage]), phase, aborted, args.fault));
         if (!ok) break;
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + buf * Shape::kAccColumns;
-        for (int kb = 0; kb < kb_count; ++kb) {
-          ok = mbar_wait(smem_addr(&full_bar[stage]), phase, aborted, args.fault);
-          if (!ok) break;
-          tc_fence_after();
-          const uint64_t b_desc = operand_desc(stage_b(stage));
+        const uint64_t b_desc = operand_desc(stage_b(stage));
+        if (issues) {
 #pragma unroll
           for (int half = 0; half < kHalves; ++half) {
             const uint64_t a_desc = operand_desc(stage_a(stage, half));
@@ -275,17 +276,20 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             }
           }
           umma_commit(smem_addr(&empty_bar[stage]));   // the stage is free once these products retire
-          if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
-        if (!ok) break;
-        umma_commit(smem_addr(&acc_full_bar[buf]));
-        acc_phase[buf] ^= 1u;
-        buf ^= 1;
+        __syncwarp();
+        if (++stage == kStages) { stage = 0; phase ^= 1u; }
       }
-      // nothing of this CTA may still be running on the tensor core when its memory is freed
-      umma_commit(smem_addr(&drain_bar));
-      mbar_wait(smem_addr(&drain_bar), 0, aborted, args.fault);
+      if (!ok) break;
+      if (issues) umma_commit(smem_addr(&acc_full_bar[buf]));
+      __syncwarp();
+      acc_phase ^= 1u << buf;
+      buf ^= 1;
     }
+    // nothing of this CTA may still be running on the tensor core when its memory is freed
+    if (issues) umma_commit(smem_addr(&drain_bar));
+    __syncwarp();
+    mbar_wait(smem_addr(&drain_bar), 0, aborted, args.fault);
   } else {
     // ------------------------------------------------------------------ epilogue (warps 2..5)
     const int quarter = warp & 3;                       // the 32 tensor-memory lanes this warp may read

@@ -58,7 +58,7 @@ grouped_linear_tc_kernel(const __grid_constant__ CUtensorMap map_w, const MoeTcA
   __shared__ int aborted_flag;
   volatile int* aborted = &aborted_flag;
   if (threadIdx.x == 0) pdl_trigger();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform(static_cast<int>(threadIdx.x) >> 5), lane = threadIdx.x & 31;
   const uint32_t smem_base = (smem_addr(moe_tc_raw) + 1023u) & ~1023u;
   auto stage_a = [&](int s) { return smem_base + s * (kMoeTcStageA + kMoeTcStageB); };
   auto stage_b = [&](int s) { return stage_a(s) + kMoeTcStageA; };
@@ -86,7 +86,7 @@ grouped_linear_tc_kernel(const __grid_constant__ CUtensorMap map_w, const MoeTcA
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = tmem_base_slot;
+  const uint32_t tmem_base = uniform(tmem_base_slot);
   pdl_wait();                                   // the plan, the rows and whoever still reads the results
   const int pair_tiles = args.meta[0];
   const int tiles = pair_tiles * n_tiles;       // neighbours share weights: the pairs' tiles run fastest
@@ -118,35 +118,40 @@ grouped_linear_tc_kernel(const __grid_constant__ CUtensorMap map_w, const MoeTcA
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      int stage = 0, buf = 0;
-      uint32_t phase = 0, acc_phase[2] = {0, 0};
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-        ok = mbar_wait(smem_addr(&acc_empty_bar[buf]), acc_phase[buf] ^ 1u, aborted, args.fault);
+    const bool issues = elect_one();
+    const int last_tile = uniform(tiles);
+    int stage = 0, buf = 0;
+    uint32_t phase = 0, acc_phase = 0;                  // acc_phase: a bit for each buffer
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < last_tile && ok; tile += gridDim.x) {
+      ok = __all_sync(0xffffffffu, mbar_wait(smem_addr(&acc_empty_bar[buf]), ((acc_phase >> buf) & 1u) ^ 1u, aborted, args.fault));
+      if (!ok) break;
+      tc_fence_after();
+      for (int step = 0; step < steps; ++step) {
+        ok = __all_sync(0xffffffffu, mbar_wait(smem_addr(&weights_bar[stage]), phase, aborted, args.fault) &&
+                                         mbar_wait(smem_addr(&rows_bar[stage]), phase, aborted, args.fault));
         if (!ok) break;
         tc_fence_after();
-        for (int step = 0; step < steps; ++step) {
-          ok = mbar_wait(smem_addr(&weights_bar[stage]), phase, aborted, args.fault) &&
-               mbar_wait(smem_addr(&rows_bar[stage]), phase, aborted, args.fault);
-          if (!ok) break;
-          tc_fence_after();
-          const uint64_t a_desc = operand_desc(stage_a(stage)), b_desc = operand_desc(stage_b(stage));
+        const uint64_t a_desc = operand_desc(stage_a(stage)), b_desc = operand_desc(stage_b(stage));
+        if (issues) {
 #pragma unroll
           for (int k = 0; k < kMoeTcK / 16; ++k)
             umma_bf16(tmem_base + buf * kMoeTcN, a_desc + 2 * k, b_desc + 2 * k, kIdesc, (step > 0 || k > 0) ? 1u : 0u);
           umma_commit(smem_addr(&empty_bar[stage]));
-          if (++stage == kMoeTcStages) { stage = 0; phase ^= 1u; }
         }
-        if (!ok) break;
-        umma_commit(smem_addr(&acc_full_bar[buf]));
-        acc_phase[buf] ^= 1u;
-        buf ^= 1;
+        __syncwarp();
+        if (++stage == kMoeTcStages) { stage = 0; phase ^= 1u; }
       }
-      // nothing of this CTA may still be running on the tensor core when its memory is freed
-      umma_commit(smem_addr(&drain_bar));
-      mbar_wait(smem_addr(&drain_bar), 0, aborted, args.fault);
+      if (!ok) break;
+      if (issues) umma_commit(smem_addr(&acc_full_bar[buf]));
+      __syncwarp();
+      acc_phase ^= 1u << buf;
+      buf ^= 1;
     }
+    // nothing of this CTA may still be running on the tensor core when its memory is freed
+    if (issues) umma_commit(smem_addr(&drain_bar));
+    __syncwarp();
+    mbar_wait(smem_addr(&drain_bar), 0, aborted, args.fault);
   } else if (warp < 6) {
     const int quarter = warp & 3;                       // the 32 tensor-memory lanes this warp may read
     const int row = quarter * 32 + lane;

@@ -112,6 +112,18 @@ __device__ __forceinline__ void tc_fence_before() {
 __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
+// What issues tensor-core instructions: a whole warp goes through the loop, with operands and conditions that the compiler
+// knows to be the same in every lane (loop counters, shared-memory addresses, `uniform` of what was loaded), and one lane of it
+// issues.  Then an instruction leaves every 20 to 40 cycles; issued from a branch that only one lane takes, its operands go
+// through moves of their own and it leaves every 75 (measured with clock64 around twelve of them), which is longer than a
+// product of 128 x 64 x 16 takes.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t chosen;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(chosen));
+  return chosen != 0;
+}
+template <typename T>
+__device__ __forceinline__ T uniform(T value) { return __shfl_sync(0xffffffffu, value, 0); }
 __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
                                           uint32_t idesc, uint32_t accumulate) {
   asm volatile(
