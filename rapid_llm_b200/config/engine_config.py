@@ -37,7 +37,7 @@ class EngineConfig:
 
     Attributes:
         dtype: ``torch.bfloat16`` (serving precision) or ``torch.float32`` (every
-            product and sum in true 32-bit).
+            product and sum as near as 32-bit arithmetic is, or nearer).
         max_seq_len: Longest sequence (prompt plus generated) a request may reach.
         page_size: Tokens per cache page.
         num_pages: Pages per cache group, the reserved null page not counted;

@@ -1,13 +1,19 @@
-// True 32-bit matrix product: C[M, N] = A[M, K] * W[N, K]^T (+ bias), float32 in, float32
-// fused multiply-adds, float32 out.  No tensor cores and no reduced-precision mode.
+// 32-bit matrix product: C[M, N] = A[M, K] * W[N, K]^T (+ bias), float32 in, float32 out, no reduced-precision mode.
 //
-// Every output element is accumulated over k = 0 .. K-1 in that order by one thread, so its
-// value does not depend on M, on the kernel or the tile it falls in, or on what else is in the batch.
+// Weights of a few million numbers and more run on the tensor cores, with every float32 cut into three exact parts
+// (gemm_f32_split.cu); the others here, in float32 fused multiply-adds.  The weight alone decides, and either way an output's
+// value does not depend on M, on the tile it falls in, or on what else is in the batch: here it is accumulated over
+// k = 0 .. K-1 in that order by one thread.
 // The reference has no 32-bit path (rapid_llm/models/config.py:134-146 downgrades float32
 // checkpoints); its products go through a library call (rapid_llm/kernels/ops/gemm/linear.py:17-40).
 #include "common.cuh"
 
 namespace rl {
+
+bool gemm_f32_split_takes(const float* w, int n, int k);
+long long gemm_f32_split_scratch(const float* a, int m, int k, int lda);
+int gemm_f32_split(const float* a, const float* w, const float* bias, float* c, int m, int n, int k, int lda, int ldc,
+                   __nv_bfloat16* parts, int* fault, cudaStream_t stream);
 
 __device__ __forceinline__ void f32_copy16(float* shared, const float* global, bool ok) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(shared))),
@@ -240,11 +246,18 @@ static int launch_f32_few(const float* a, const float* w, const float* bias, flo
 
 }  // namespace rl
 
-// a: [m, k] with row stride lda; w: [n, k] contiguous; c: [m, n] with row stride ldc.
+// The 16-bit numbers of scratch the product wants as `parts` (0: none), on a 16-byte boundary.
+extern "C" long long rl_gemm_f32_scratch(const float* a, const float* w, int m, int n, int k, int lda) {
+  return m > 0 && rl::gemm_f32_split_takes(w, n, k) ? rl::gemm_f32_split_scratch(a, m, k, lda) : 0;
+}
+
+// a: [m, k] with row stride lda; w: [n, k] contiguous; c: [m, n] with row stride ldc.  `fault` may be null.
 extern "C" int rl_gemm_f32(const float* a, const float* w, const float* bias, float* c, int m,
-                           int n, int k, int lda, int ldc, cudaStream_t stream) {
+                           int n, int k, int lda, int ldc, void* parts, int* fault, cudaStream_t stream) {
   if (m == 0 || n == 0) return 0;
   if (k <= 0 || lda < k || ldc < n) return static_cast<int>(cudaErrorInvalidValue);
+  if (rl::gemm_f32_split_takes(w, n, k))
+    return rl::gemm_f32_split(a, w, bias, c, m, n, k, lda, ldc, static_cast<__nv_bfloat16*>(parts), fault, stream);
   const bool aligned = (k % 4 == 0) && (lda % 4 == 0) &&
                        (reinterpret_cast<uintptr_t>(a) % 16 == 0) &&
                        (reinterpret_cast<uintptr_t>(w) % 16 == 0);

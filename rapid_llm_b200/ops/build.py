@@ -43,6 +43,7 @@ LIBRARIES: dict[str, list[str]] = {
         "rope_kv.cu",
         "attention_generic.cu",
         "gemm_f32.cu",
+        "gemm_f32_split.cu",
         "sampling.cu",
     ],
     "gemm": ["gemm_bf16.cu", "gemm_chain.cu", "gemm_bf16_pair.cu"],

@@ -1,6 +1,6 @@
 """Dense matrix products ``y = x @ W^T`` of the linear layers.
 
-float32 runs the hand-written true 32-bit kernel.  bfloat16 steps of up to
+float32 runs the hand-written 32-bit kernels.  bfloat16 steps of up to
 :data:`TENSOR_CORE_MAX_TOKENS` tokens (decoding, small portions) run the hand-written
 tcgen05/TMA kernel, which streams the weight once at close to memory speed; larger steps call
 the library product (cuBLAS through ``torch.mm``), which is where the reference's engine
@@ -163,7 +163,7 @@ def linear(x, weight: torch.Tensor, out: torch.Tensor, fault: torch.Tensor | Non
     if x.shape[0] == 0:
         return out
     if x.dtype == torch.float32:
-        kernels.gemm_f32(x, weight, out, bias)
+        kernels.gemm_f32(x, weight, out, bias, fault)
         return _square_columns(out, relu2_columns)
     if fault is not None and use_tensor_core_kernel(x, weight):
         rows, width = out.shape

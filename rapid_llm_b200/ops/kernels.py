@@ -148,7 +148,9 @@ def core() -> ctypes.CDLL:
             c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_int, c_float,
             c_void_p, c_void_p,
         ]
-        lib.rl_gemm_f32.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p]
+        lib.rl_gemm_f32.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p]
+        lib.rl_gemm_f32_scratch.argtypes = [c_void_p, c_void_p, c_int, c_int, c_int, c_int]
+        lib.rl_gemm_f32_scratch.restype = c_longlong
         lib.rl_sample.argtypes = [
             c_int, c_void_p, c_int, c_int, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p,
             c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
@@ -755,9 +757,11 @@ def attention_mma(
     return out
 
 
-def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
-    """``out[M, N] = a[M, K] @ w[N, K]^T`` in true float32."""
-    _need_cuda(a, w, out, bias)
+def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: torch.Tensor | None = None,
+             fault: torch.Tensor | None = None) -> torch.Tensor:
+    """``out[M, N] = a[M, K] @ w[N, K]^T`` in 32 bits: a row's values depend on the row and the weight alone.  Scratch for the
+    rows' parts (6 bytes a number, 1,024 rows at most) comes from torch's allocator where the kernel wants it."""
+    _need_cuda(a, w, out, bias, fault)
     for name, tensor in (("a", a), ("w", w), ("out", out), ("bias", bias)):
         _expect(name, tensor, torch.float32)
     _contig("w", w)
@@ -765,11 +769,16 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: torch.Te
         raise KernelError(f"gemm_f32: shapes {tuple(a.shape)} x {tuple(w.shape)}^T -> {tuple(out.shape)} do not agree")
     if a.stride(1) != 1 or out.stride(1) != 1:
         raise KernelError("gemm_f32: rows of a and out must be contiguous")
+    rows, columns, inner = a.shape[0], w.shape[0], a.shape[1]
+    wanted = core().rl_gemm_f32_scratch(_ptr(a), _ptr(w), rows, columns, inner, a.stride(0))
+    parts = torch.empty(wanted, dtype=torch.bfloat16, device=a.device) if wanted else None
     _check(
-        core().rl_gemm_f32(_ptr(a), _ptr(w), _ptr(bias), _ptr(out), a.shape[0], w.shape[0], a.shape[1],
-                           a.stride(0), out.stride(0), _stream()),
+        core().rl_gemm_f32(_ptr(a), _ptr(w), _ptr(bias), _ptr(out), rows, columns, inner, a.stride(0), out.stride(0), _ptr(parts),
+                           _ptr(fault), _stream()),
         "gemm_f32",
     )
+    if wanted:
+        LAUNCHES.count += 2 * -(-rows // 1024) - 1      # the rows' parts and the product, 1,024 rows at a time
     return out
 
 

@@ -1,0 +1,74 @@
+"""32-bit products on the tensor cores: three exact bfloat16 parts a number, at the edges of its tiles and rings."""
+
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda:0"
+
+
+def k():
+    from rapid_llm_b200.ops import kernels
+
+    return kernels
+
+
+def product(a, w, bias=None):
+    out = torch.full((a.shape[0], w.shape[0] + 4), 7.0, device=DEV)
+    fault = torch.zeros(1, dtype=torch.int32, device=DEV)
+    k().gemm_f32(a, w, out[:, : w.shape[0]], bias, fault)
+    assert int(fault) == 0 and bool((out[:, w.shape[0] :] == 7.0).all())
+    return out[:, : w.shape[0]]
+
+
+# weights on the line of the rule; rows that are no whole tile; columns of one to eight segments, of a last step with four columns
+# (a sum of one step behind whole ones, steps of odd number) and of no whole 16 bytes of parts
+@pytest.mark.parametrize("n,inner", [(8192, 1024), (2100, 4100), (1025, 8460), (24700, 1284)])
+def test_rows_are_near_and_the_same_at_every_count(n, inner):
+    torch.manual_seed(5)
+    rows = [1, 16, 17, 32, 33, 64, 65, 112, 128, 129, 208, 209, 300, 1025]
+    a, w, bias = torch.randn(max(rows), inner, device=DEV), torch.randn(n, inner, device=DEV), torch.randn(n, device=DEV)
+    want = a.double() @ w.double().t() + bias.double()
+    # Of the sum S of the products' magnitudes: a sum of 256 columns is cut off 16 times below 2^-23 of what it holds, the parts'
+    # products that are left out stay below 3 x 2^-24, the small ones (2^-7 of the whole) are cut off 5 k / 16 times below 2^-23
+    # of theirs, and the float32 sums of k / 256 such round to 2^-24
+    magnitude = a.abs().double() @ w.abs().double().t() + bias.abs().double()
+    bound = magnitude * (16 + 2 + 5 * inner / 16 / 128 + inner / 512 + 1) * 2.0 ** -23
+    # and as random sums go, a small part of it: no further off than one multiply-add after the other would be on average
+    typical = 0.5 * math.sqrt(inner) * 2.0 ** -24
+    first = None
+    for m in rows:
+        got = product(a[:m], w, bias)
+        assert bool(((got.double() - want[:m]).abs() <= bound[:m]).all()), m
+        assert float((got.double() - want[:m]).norm() / want[:m].norm()) < typical, m
+        first = got[:1].clone() if first is None else first
+        assert torch.equal(got[:1], first), m
+
+
+@pytest.mark.parametrize("offset", [1, 2, 3])
+def test_rows_off_a_16_byte_boundary(offset):
+    torch.manual_seed(6)
+    wide, w = torch.randn(70, 4101, device=DEV), torch.randn(2048, 4096, device=DEV)
+    for m in (1, 20, 70):
+        view = wide[:m, offset : offset + 4096]
+        assert torch.equal(product(view, w), product(view.contiguous(), w))
+
+
+@pytest.mark.parametrize("m", [3, 40, 130])
+def test_what_is_not_finite_stays_in_its_row_and_column(m):
+    torch.manual_seed(7)
+    a, w = torch.randn(m, 4096, device=DEV), torch.randn(2048, 4096, device=DEV)
+    clean = product(a, w)
+    a[1, 5], w[7, 9] = math.inf, math.nan
+    a[2, 11], w[9, 100] = 3.0e38, 3.0e38
+    got = product(a, w)
+    want = (a.double() @ w.double().t()).float()
+    assert bool(got[:, 7].isnan().all()) and torch.equal(got[1].isinf(), want[1].isinf())
+    assert torch.equal(got[1, want[1].isinf()], want[1, want[1].isinf()])
+    kept = torch.ones_like(got, dtype=torch.bool)
+    kept[1:3], kept[:, 7], kept[:, 9] = False, False, False
+    assert torch.equal(got[kept], clean[kept])
+    assert bool(torch.isfinite(got[2][torch.isfinite(want[2])]).all())
