@@ -9,7 +9,8 @@
 // recurrence consumes (decays, step sizes, gates, unit vectors, the state) is float32 in both engine
 // precisions.  The recurrence runs token by token in a fixed order, so a row's result does not depend
 // on how the tokens were cut into steps or on what else is in the batch; in 16-bit engines long entries
-// are walked in pieces, whose order of sums depends on the entry's length in the step and on nothing else in it.
+// are walked in pieces or taken in blocks of tokens (scan_blocks.cu), whose order of sums depends on the entry's length in the
+// step and on nothing else in it.
 //
 // Pointers to what an earlier kernel of the same step wrote (activations, the state) carry no `__restrict__`:
 // a load through a const restrict pointer counts as invariant and may be moved above the wait for the
@@ -18,6 +19,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "scan_blocks.cuh"
 
 namespace rl {
 
@@ -634,7 +636,8 @@ __global__ void rotate_heads_kernel(const T* in, int in_stride, int q_col0, int 
 // end to end cannot use the rest of the GPU, so in 16-bit engines long prompts are walked in pieces (below).
 // A correction (beta) makes a token wait for the sum over the whole column of the token before it: there a column has
 // few lanes with many rows each, since an exchange between lanes waits as long as eight multiply-adds, and prompts are
-// walked from end to end (in pieces the state has to go through a matrix per piece, which costs digits).
+// walked from end to end (in pieces the state has to go through a matrix per piece, which costs digits) or, where that is
+// ahead, taken in blocks of tokens.
 // 2,048 tokens, us, before / from end to end / in pieces: 16 heads of 128, fixed decay 432 / 284 / 199; 32 heads of 64, row
 // decays 383 / 252 / 140; with a bonus 334 / 258 / 154; 32 heads of 128, fixed, 570 / 398 / 341; with a
 // correction, 16 heads of 128, 632 / 571.  64 single tokens: 64 heads of 64, row decays 54 / 31 (4.3 TB/s), 16 heads of
@@ -662,6 +665,7 @@ struct ScanArgs {
   int from;               // entries of so many tokens and more are cut into pieces, the others walked (0: none is cut)
   float* seg_states;      // [pieces, heads, vdim, dim]: what a piece alone leaves, then what it starts from
   float* seg_decays;      // [pieces, heads, dim]: the product of a piece's decays
+  int in_blocks;          // entries of so many tokens and more are taken in blocks of tokens (scan_blocks.cu) and left out here (0: none)
 };
 
 // The piece that block `index` owns: of which entry, which one of the entry's, its tokens, its place in the arrays of
@@ -670,7 +674,7 @@ struct ScanPiece { int entry, number, first, length, of, place; };
 __device__ __forceinline__ bool scan_piece(const ScanArgs& a, int index, ScanPiece& s) {
   if (a.segment == 0) {
     s = {index, 0, a.cu_seqlens[index], a.cu_seqlens[index + 1] - a.cu_seqlens[index], 1, 0};
-    return a.from == 0 || s.length < a.from;
+    return (a.from == 0 || s.length < a.from) && (a.in_blocks == 0 || s.length < a.in_blocks);
   }
   int at = 0;
   for (int e = 0; e < a.entries; ++e) {
@@ -1779,7 +1783,8 @@ int rl_linear_scan(const float* q, int q_stride, const float* k, int k_stride, c
                    const float* bonus, float* out, int out_stride, float* state, long long state_stride, int state_off,
                    const int* cu_seqlens, const int* entry_slot, const int* entry_start, int entries, int tokens, int heads,
                    int kv_heads, int dim, int vdim, int slots, int* fault, int segment, int from, int segments, int others,
-                   float* seg_states, float* seg_decays, int pdl, cudaStream_t stream) {
+                   float* seg_states, float* seg_decays, int blocks_from, int blocks, float* records, int record_floats, int pdl,
+                   cudaStream_t stream) {
   if (entries == 0) return 0;
   if (heads < 1 || kv_heads < 1 || heads % kv_heads || dim < 1 || dim > 1024 || vdim < 1 || decay_mode < 0 ||
       decay_mode > 2 || decay == nullptr || (bonus != nullptr && beta != nullptr))
@@ -1798,9 +1803,19 @@ int rl_linear_scan(const float* q, int q_stride, const float* k, int k_stride, c
   a.segment = segment;
   a.from = segment ? from : 0;
   a.seg_states = seg_states; a.seg_decays = seg_decays;
+  a.in_blocks = blocks_from;
   using namespace rl;
+  if (blocks_from > 0) {
+    // An entry's own length says how it is taken, so that its sums are in the same order whatever else is in the step.
+    if (segment != 0 || record_floats != scan_record_floats(dim, beta != nullptr)) return static_cast<int>(cudaErrorInvalidValue);
+    const ScanBlockArgs in_blocks = {q, q_stride, k, k_stride, v, v_stride, decay, decay_mode, beta, v_scale, skip, bonus, out, out_stride,
+                                     state + state_off, state_stride, cu_seqlens, entry_slot, entry_start, heads, kv_heads, dim, vdim, slots,
+                                     entries, blocks_from, a.wide_in, records, fault};
+    const int e = scan_blocks(in_blocks, blocks, stream);
+    if (e || !others) return e;
+  }
   // single tokens of the common head sizes: the same rows a lane and lanes a column as the walk, so the same sums
-  if (segment == 0 && tokens == entries && a.wide_in && dim > 32 && dim <= 128) {
+  if (segment == 0 && blocks_from == 0 && tokens == entries && a.wide_in && dim > 32 && dim <= 128) {
     if (beta)
       return dim <= 64 ? launch_single_scan<16, 4, 2, kScanDelta, true>(a, pdl, stream)
                        : launch_single_scan<16, 8, 2, kScanDelta, true>(a, pdl, stream);

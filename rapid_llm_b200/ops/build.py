@@ -47,7 +47,7 @@ LIBRARIES: dict[str, list[str]] = {
         "sampling.cu",
     ],
     "gemm": ["gemm_bf16.cu", "gemm_chain.cu", "gemm_bf16_pair.cu"],
-    "recurrent": ["recurrent.cu"],
+    "recurrent": ["recurrent.cu", "scan_blocks.cu"],
     "moe": ["moe.cu", "moe_tc.cu"],
     "latent": ["latent.cu"],
 }

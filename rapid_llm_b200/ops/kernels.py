@@ -1120,7 +1120,7 @@ def recurrent() -> ctypes.CDLL:
         lib.rl_linear_scan.argtypes = [
             c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
             c_void_p, c_int, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-            c_int, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p,
+            c_int, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p,
         ]
         lib.rl_exp_decay.argtypes = [c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]
         lib.rl_low_rank_decay.argtypes = [c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_float, c_void_p,
@@ -1286,10 +1286,44 @@ def scan_buffers(space, tokens: int, heads: int, dim: int, vdim: int):
                  for name, cols in (("scan_states", heads * dim * vdim), ("scan_decays", heads * dim)))
 
 
+SCAN_BLOCK = 32     # tokens of a block of ``csrc/scan_blocks.cu``
+
+
+def scan_blocks_from(heads: int, dim: int, vdim: int, corrected: bool = False) -> int:
+    """The shortest entry that is taken in blocks of tokens (0: none is): with a correction, where the alternative is a walk from
+    end to end, and without one where heads are wide and many, ahead of the pieces.  One prompt, us, walked or in pieces / in
+    blocks: with a correction 16 heads of 128, 2,048 tokens 571 / 255, 1,024 293 / 138; 32 heads of 64 500 / 230 and 254 / 126;
+    32 heads of 128 573 / 486 and 293 / 257; without one, fixed decays, 32 heads of 128, 2,048 tokens 342 / 276, 700 + 333 + 1,015
+    412 / 290, 128 tokens 29 / 27 (16 heads: 199 / 249, so they stay in pieces; 64 heads of 64 208 / 216).  The entry's length
+    alone decides, not what else is in the step: several long prompts at once fill the GPU by themselves, and a walk is ahead
+    there with a correction (four of 1,024 tokens, 16 heads of 128, 408 / 493, 32 heads of 64 256 / 339), which is why entries
+    that can come in such numbers in a step of a few thousand tokens are walked."""
+    if not 32 < dim <= 128 or dim % 4 or vdim % 4:
+        return 0
+    if corrected:
+        return 640 if heads * vdim <= 2048 else 1536
+    return 256 if dim > 64 and heads * vdim >= 4096 else 0
+
+
+def scan_record(dim: int, corrected: bool = False) -> int:
+    """Floats that a block of a head keeps for its walk (``BlockRecord`` of the kernels)."""
+    padded, parts = 64 if dim <= 64 else 128, 2 if corrected else 1
+    return parts * 32 * (padded + 8) + padded * 40 + parts * 32 * 40 + padded
+
+
+def scan_records(space, tokens: int, heads: int, dim: int, first: int, corrected: bool = False) -> torch.Tensor:
+    """Records of the blocks a step can have: sized once for the largest step ``space`` is made for, so that prompts of growing
+    length allocate nothing."""
+    most = max(space.max_tokens, tokens)
+    rows = most // SCAN_BLOCK + most // first      # whole blocks and remainders
+    return space.get("scan_records", rows, heads * scan_record(dim, corrected), torch.float32, min_rows=rows)
+
+
 def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, out: torch.Tensor,
                 state: torch.Tensor, batch, *, heads: int, kv_heads: int, dim: int, vdim: int,
                 beta: torch.Tensor | None = None, v_scale: torch.Tensor | None = None,
-                skip: torch.Tensor | None = None, bonus: torch.Tensor | None = None, pieces=None) -> torch.Tensor:
+                skip: torch.Tensor | None = None, bonus: torch.Tensor | None = None, pieces=None,
+                blocks_from: int = 0) -> torch.Tensor:
     """The recurrence ``S <- decay * S; u = beta * (v - S^T k)`` (or ``v_scale * v`` without ``beta``);
     ``S <- S + k u^T; out = S^T q + skip * v`` per head over every entry's tokens, from and into
     ``state [slots, heads * dim * vdim]`` (float32; a request at position 0 starts from zeros).  With ``bonus``
@@ -1302,7 +1336,8 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.
 
     With ``pieces`` (a workspace) entries that are long enough (:func:`scan_pieces_from`) are walked in pieces side by side
     where the kernels have that form (:func:`scan_takes_pieces`): the same sums in another order, which depends on the entry's
-    own length in this step, so on where a request is cut, and on nothing else in the step.
+    own length in this step, so on where a request is cut, and on nothing else in the step.  With ``blocks_from`` (and
+    ``pieces``) entries of so many tokens and more are taken in blocks of 32 tokens instead, corrections included.
     """
     _need_cuda(q, k, v, decay, out, state, beta, v_scale, skip, bonus)
     for name, tensor in (("q", q), ("k", k), ("v", v), ("decay", decay), ("out", out), ("beta", beta),
@@ -1330,8 +1365,16 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.
     # of 0.6 ms for 2,048 tokens).  Steps of single tokens have many short blocks and keep the early start.
     early = PDL and tokens < 8 * batch.num_entries
     piece = first = blocks = others = 0
-    states = decays = None
-    if pieces is not None and scan_takes_pieces(dim, vdim, beta is not None) and batch.max_query_len >= scan_pieces_from(heads, dim, vdim):
+    states = decays = records = None
+    record = 0
+    if pieces is None or batch.max_query_len < blocks_from:
+        blocks_from = 0
+    if blocks_from:
+        record = scan_record(dim, beta is not None)
+        blocks = tokens // SCAN_BLOCK + min(batch.num_entries, tokens // blocks_from)
+        others = int(batch.num_entries * batch.max_query_len != tokens)      # entries of other lengths, shorter ones perhaps
+        records = scan_records(pieces, tokens, heads, dim, blocks_from, beta is not None)
+    elif pieces is not None and scan_takes_pieces(dim, vdim, beta is not None) and batch.max_query_len >= scan_pieces_from(heads, dim, vdim):
         piece, first = scan_piece(heads, vdim), scan_pieces_from(heads, dim, vdim)
         blocks = tokens // piece + min(batch.num_entries, tokens // first)
         others = int(batch.num_entries * batch.max_query_len != tokens)      # entries of other lengths, shorter ones perhaps
@@ -1341,9 +1384,11 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.
             _ptr(q), _row_stride("q", q), _ptr(k), _row_stride("k", k), _ptr(v), _row_stride("v", v), _ptr(decay), mode,
             _ptr(beta), _ptr(v_scale), _ptr(skip), _ptr(bonus), _ptr(out), _row_stride("out", out), _ptr(state), stride, 0,
             _ptr(batch.cu_seqlens), _ptr(batch.entry_slot), _ptr(batch.entry_start), batch.num_entries, tokens, heads, kv_heads,
-            dim, vdim, slots, _ptr(batch.fault), piece, first, blocks, others, _ptr(states), _ptr(decays), int(early), _stream()),
+            dim, vdim, slots, _ptr(batch.fault), piece, first, blocks, others, _ptr(states), _ptr(decays), blocks_from, blocks, _ptr(records), record,
+            int(early), _stream()),
         f"linear_scan(dim={dim}, vdim={vdim})",
     )
+    LAUNCHES.count += 1 + others if blocks_from else 0
     return out
 
 

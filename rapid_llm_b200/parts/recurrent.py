@@ -2,7 +2,7 @@
 
 All of them keep, per head, a float32 matrix ``S`` of ``key_dim x value_dim`` in the request's state row
 and advance it token by token (``ops.kernels.linear_scan``, portions of prompts and single decoded tokens alike);
-in bfloat16 engines long portions are walked in pieces side by side, except with the delta rule:
+in bfloat16 engines long portions are walked in pieces side by side or taken in blocks of tokens:
 
 * :class:`ChannelDeltaRule` (``gated_delta_rule``) — the delta rule with a decay per head and key channel:
   ``S <- diag(g) S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q``.
@@ -62,7 +62,18 @@ class _Recurrent(Mixer):
         """Elements of the engine's dtype a token's share of the pieces' states takes at most."""
         if self.dtype != torch.bfloat16 or not kernels.scan_takes_pieces(dim, vdim):
             return 0
+        first = kernels.scan_blocks_from(heads, dim, vdim)
+        if first:
+            return self._blocks_elements(heads, dim, vdim)
         return 2 * 2 * -(-heads * dim * (vdim + 1) // kernels.scan_piece(heads, vdim))
+
+    def _blocks_elements(self, heads: int, dim: int, vdim: int, corrected: bool = False) -> int:
+        """The same for the records of blocks of tokens."""
+        first = kernels.scan_blocks_from(heads, dim, vdim, corrected)
+        if self.dtype != torch.bfloat16 or not first:
+            return 0
+        floats = heads * kernels.scan_record(dim, corrected)
+        return 2 * (-(-floats // kernels.SCAN_BLOCK) + -(-floats // first))
 
     def _state_views(self, cache) -> tuple[torch.Tensor, torch.Tensor]:
         state = cache.state
@@ -171,7 +182,8 @@ class ChannelDeltaRule(_Recurrent):
             raise KeyError(name)
 
     def workspace_elements_per_token(self) -> int:
-        return 3 * (self.w_in.shape[0] + self.w_high.shape[0]) + self.ra + self.rg + self.hidden
+        return (3 * (self.w_in.shape[0] + self.w_high.shape[0]) + self.ra + self.rg + self.hidden
+                + self._blocks_elements(self.h, self.dim, self.vdim, corrected=True))
 
     def forward(self, x, batch, cache):
         rows, space, f32 = x.shape[0], batch.workspace, torch.float32
@@ -188,7 +200,8 @@ class ChannelDeltaRule(_Recurrent):
         kernels.decay_gate(high[:, : self.h * self.dim], self.rate, self.dt_bias, self.dim, decay)
         read = space.get("delta_read", rows, self.cv, f32)
         kernels.linear_scan(conv[:, : self.cq], conv[:, self.cq : 2 * self.cq], conv[:, 2 * self.cq :], decay, read, S,
-                            batch, heads=self.h, kv_heads=self.hk, dim=self.dim, vdim=self.vdim, beta=beta)
+                            batch, heads=self.h, kv_heads=self.hk, dim=self.dim, vdim=self.vdim, beta=beta,
+                            pieces=self._pieces(batch), blocks_from=kernels.scan_blocks_from(self.h, self.dim, self.vdim, True))
         normed = space.get("delta_normed", rows, self.cv, x.dtype)
         kernels.gated_norm(read, normed, group=self.vdim, gate=high[:, self.h * self.dim :], act=kernels.GATE_SIGMOID,
                            weight=self.norm, eps=self.eps)
@@ -261,8 +274,8 @@ class Retention(_Recurrent):
                              self.inv_freq, heads=self.h, dim=self.dim, vdim=self.vdim, k_scale=self.dim ** -0.5)
         read = space.get("ret_read", rows, cv, f32)
         kernels.linear_scan(qkv[:, :cq], qkv[:, cq : 2 * cq], qkv[:, 2 * cq :], self.decay, read, S, batch,
-                            heads=self.h, kv_heads=self.h, dim=self.dim, vdim=self.vdim,
-                            pieces=self._pieces(batch))
+                            heads=self.h, kv_heads=self.h, dim=self.dim, vdim=self.vdim, pieces=self._pieces(batch),
+                            blocks_from=kernels.scan_blocks_from(self.h, self.dim, self.vdim))
         normed = space.get("ret_normed", rows, cv, x.dtype)
         kernels.gated_norm(read, normed, group=self.vdim, gate=proj[:, 2 * cq + cv :], act=kernels.GATE_SILU, eps=self.eps)
         return gemm.linear(normed, self.o, space.get("ret_out", rows, self.hidden, x.dtype), batch.fault)
@@ -329,8 +342,8 @@ class Lightning(_Recurrent):
         qkv = kernels.activate_rows(proj[:, : 2 * cq + cv], space.get("lightning_qkv", rows, 2 * cq + cv, f32), act=True)
         read = space.get("lightning_read", rows, cv, f32)
         kernels.linear_scan(qkv[:, :cq], qkv[:, cq : 2 * cq], qkv[:, 2 * cq :], self.decay, read, S, batch,
-                            heads=self.h, kv_heads=self.h, dim=self.dim, vdim=self.vdim,
-                            pieces=self._pieces(batch))
+                            heads=self.h, kv_heads=self.h, dim=self.dim, vdim=self.vdim, pieces=self._pieces(batch),
+                            blocks_from=kernels.scan_blocks_from(self.h, self.dim, self.vdim))
         normed = space.get("lightning_normed", rows, cv, x.dtype)
         kernels.gated_norm(read, normed, group=cv, gate=proj[:, 2 * cq + cv :], act=kernels.GATE_SIGMOID,
                            weight=self.norm, eps=self.eps)
@@ -419,7 +432,7 @@ class StateSpaceDual(_Recurrent):
         read = space.get("ssd_read", rows, inner, f32)
         kernels.linear_scan(conv[:, inner + gn :], conv[:, inner : inner + gn], conv[:, :inner], decay, read, S, batch,
                             heads=self.h, kv_heads=self.groups, dim=self.n, vdim=self.vdim, v_scale=step, skip=self.skip,
-                            pieces=self._pieces(batch))
+                            pieces=self._pieces(batch), blocks_from=kernels.scan_blocks_from(self.h, self.n, self.vdim))
         normed = space.get("ssd_normed", rows, inner, x.dtype)
         kernels.gated_norm(read, normed, group=inner // self.norm_groups, gate=proj[:, :inner], act=kernels.GATE_SILU,
                            gate_first=True, weight=self.norm, eps=self.eps)
@@ -517,8 +530,8 @@ class ShiftedDecay(_Recurrent):
         rkv = kernels.activate_rows(proj[: 3 * rows], space.get("wkv_rkv", 3 * rows, c, f32), act=False)
         read = space.get("wkv_read", rows, c, f32)
         kernels.linear_scan(rkv[:rows], rkv[rows : 2 * rows], rkv[2 * rows :], decay, read, S, batch, heads=self.h,
-                            kv_heads=self.h, dim=self.dim, vdim=self.dim, bonus=self.bonus,
-                            pieces=self._pieces(batch))
+                            kv_heads=self.h, dim=self.dim, vdim=self.dim, bonus=self.bonus, pieces=self._pieces(batch),
+                            blocks_from=kernels.scan_blocks_from(self.h, self.dim, self.dim))
         normed = space.get("wkv_normed", rows, c, x.dtype)
         kernels.gated_norm(read, normed, group=self.dim, gate=proj[3 * rows :], act=kernels.GATE_SILU, weight=self.norm,
                            eps=self.eps)
@@ -606,8 +619,8 @@ class GatedLinear(_Recurrent):
                                self.tau, qkv, decay)
         read = space.get("gla_read", rows, cv, f32)
         kernels.linear_scan(qkv[:, :cq], qkv[:, cq : 2 * cq], qkv[:, 2 * cq :], decay, read, S, batch,
-                            heads=self.h, kv_heads=self.h, dim=self.dim, vdim=self.vdim,
-                            pieces=self._pieces(batch))
+                            heads=self.h, kv_heads=self.h, dim=self.dim, vdim=self.vdim, pieces=self._pieces(batch),
+                            blocks_from=kernels.scan_blocks_from(self.h, self.dim, self.vdim))
         normed = space.get("gla_normed", rows, cv, x.dtype)
         kernels.gated_norm(read, normed, group=self.vdim, gate=proj[:, self.g_col0 : self.g_col0 + cv], act=kernels.GATE_SILU,
                            weight=self.norm, eps=self.eps * self.dim)
