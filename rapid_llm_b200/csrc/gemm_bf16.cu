@@ -79,6 +79,9 @@ struct GemmArgs {
   // feed-forward's); a multiple of 4
   int relu2_columns;
   float residual_scale;    // what the result is multiplied by when it joins the residual
+  // several products of as many rows each in one launch: weight tiles per product (0: one product); product p reads the rows
+  // of x from p * T on and writes those of out
+  int plane_tiles;
 };
 
 __device__ __forceinline__ float relu_squared(float v) {
@@ -132,8 +135,8 @@ struct GemmShape {
 
 // grid = (k_split, tile CTAs); with k_split > 1 the x dimension is one cluster and every CTA
 // has exactly one tile; otherwise a CTA walks the tiles blockIdx.y, blockIdx.y + gridDim.y, ...
-// kRelu2: the first relu2_columns columns of a plain product take the square of relu.
-template <bool kSwiglu, int BN, bool kRelu2>
+// kRelu2: the first relu2_columns columns of a plain product take the square of relu.  kPlanes: see GemmArgs::plane_tiles.
+template <bool kSwiglu, int BN, bool kRelu2, bool kPlanes>
 __global__ void __launch_bounds__(kGemmThreads)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                  const GemmArgs args) {
@@ -183,7 +186,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   };
   auto load_b = [&](const Cursor& c, int stage) {
     const int t_tile = tile_of(c.index) % args.t_tiles;
-    tma_load_2d(stage_b(stage), &map_x, smem_addr(&full_bar[stage]), (kb_begin + c.kb) * kTileK, t_tile * BN);
+    const int plane = kPlanes ? tile_of(c.index) / args.plane_tiles : 0;      // (of one token tile each)
+    tma_load_2d(stage_b(stage), &map_x, smem_addr(&full_bar[stage]), (kb_begin + c.kb) * kTileK, plane * args.T + t_tile * BN);
   };
   const int prefetch = static_cast<int>(min(static_cast<long long>(kStages), total_iters));
   Cursor cursor = {0, 0};
@@ -326,7 +330,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
       const int n_tile = tile / args.t_tiles, t_tile = tile - n_tile * args.t_tiles;
       // (a tile of fewer rows than lanes: only unsplit SwiGLU products, whose lanes past the tile's rows look like
       // columns past the matrix's edge)
-      const int n = n_local < args.tile_rows ? n_tile * args.tile_rows + n_local : args.N;
+      const int plane = kPlanes ? n_tile / args.plane_tiles : 0;
+      const int n = n_local < args.tile_rows ? (n_tile - plane * args.plane_tiles) * args.tile_rows + n_local : args.N;
+      bf16* out = args.out + static_cast<size_t>(plane) * args.T * args.N;
       const int t0 = t_tile * BN;
       ok = mbar_wait(smem_addr(&acc_full_bar[buf]), acc_phase[buf], aborted, args.fault);
       if (!ok) break;
@@ -371,7 +377,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
 #pragma unroll
             for (int j = 0; j < 16; ++j)
               if (t0 + c + j < args.T)
-                args.out[static_cast<size_t>(t0 + c + j) * args.N + n] = __float2bfloat16_rn(v[j]);
+                out[static_cast<size_t>(t0 + c + j) * args.N + n] = __float2bfloat16_rn(v[j]);
           }
         }
       } else if (Shape::kCanSplit) {
@@ -406,7 +412,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
       const int tile = static_cast<int>(blockIdx.y);
       const int n_tile = tile / args.t_tiles, t_tile = tile - n_tile * args.t_tiles;
       const int rows0 = 4 * lane;                                // this lane's rows of the tile
-      const int n = n_tile * kTileN + rows0, t0 = t_tile * BN;
+      const int plane = kPlanes ? n_tile / args.plane_tiles : 0;
+      const int n = (n_tile - plane * args.plane_tiles) * kTileN + rows0, t0 = t_tile * BN;
+      bf16* out = args.out + static_cast<size_t>(plane) * args.T * args.N;
       // where the other ranks keep these rows of a column of the partial tile
       uint32_t peer[8];
 #pragma unroll
@@ -485,11 +493,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
           uint2 packed;
           packed.x = *reinterpret_cast<const uint32_t*>(&lo);
           packed.y = *reinterpret_cast<const uint32_t*>(&hi);
-          *reinterpret_cast<uint2*>(args.out + at) = packed;
+          *reinterpret_cast<uint2*>(out + at) = packed;
         } else {
 #pragma unroll
           for (int r = 0; r < 4; ++r)
-            if (n + r < args.N) args.out[at + r] = __float2bfloat16_rn(result[r]);
+            if (n + r < args.N) out[at + r] = __float2bfloat16_rn(result[r]);
         }
       }
     }
@@ -517,15 +525,15 @@ static int sm_count() {
   return sms;
 }
 
-static std::atomic<unsigned long long> g_gemm_configured[3][9];   // [plain, swiglu, squared columns][BN / 32]; file-local on purpose
+static std::atomic<unsigned long long> g_gemm_configured[4][9];   // [plain, swiglu, squared columns, planes][BN / 32]; file-local on purpose
 
-template <bool kSwiglu, int BN, bool kRelu2>
+template <bool kSwiglu, int BN, bool kRelu2, bool kPlanes = false>
 static int launch_gemm(const CUtensorMap& map_w, const CUtensorMap& map_x, GemmArgs args, int forced_split,
                        cudaStream_t stream) {
   using Shape = GemmShape<kSwiglu, BN>;
   static_assert(!(kSwiglu && kRelu2), "one activation");
-  auto kernel = gemm_bf16_kernel<kSwiglu, BN, kRelu2>;
-  const cudaError_t allowed = allow_shared(kernel, static_cast<int>(Shape::kSmemBytes), g_gemm_configured[kRelu2 ? 2 : (kSwiglu ? 1 : 0)][BN / 32]);
+  auto kernel = gemm_bf16_kernel<kSwiglu, BN, kRelu2, kPlanes>;
+  const cudaError_t allowed = allow_shared(kernel, static_cast<int>(Shape::kSmemBytes), g_gemm_configured[kPlanes ? 3 : kRelu2 ? 2 : (kSwiglu ? 1 : 0)][BN / 32]);
   if (allowed != cudaSuccess) return static_cast<int>(allowed);
   // how many CTAs the GPU holds at once, and how finely to split k so that they all stream
   // (three CTAs of the plain products' small tiles fit an SM and splitting for three pays there; measured)
@@ -661,6 +669,7 @@ int rl_gemm_bf16_norm(const void* x, const void* w, void* out, int tokens, int n
   args.bias = bias;
   args.glu_limit = glu_limit; args.glu_alpha = glu_alpha;
   args.relu2_columns = relu2_columns; args.residual_scale = residual_scale;
+  args.plane_tiles = 0;
 #define RL_GEMM_CASE(SW, BNV, R2) \
   if ((swiglu != 0) == SW && bn == BNV && (relu2_columns > 0) == R2) \
     return rl::launch_gemm<SW, BNV, R2>(map_w, map_x, args, k_split, stream);
@@ -677,6 +686,40 @@ int rl_gemm_bf16(const void* x, const void* w, void* out, int tokens, int n_out,
                  int k_split, int* fault, cudaStream_t stream) {
   return rl_gemm_bf16_norm(x, w, out, tokens, n_out, k, swiglu, pdl, k_split, nullptr, nullptr, nullptr, nullptr, 0,
                            0.0f, 0, nullptr, 0.0f, 0.0f, 0, 0, 1.0f, fault, stream);
+}
+
+// `planes` products of at most 64 tokens in one launch: out[p] [tokens, n_out] = x[p] [tokens, k] * w[p] [n_out, k]^T, each of the
+// three contiguous over p; n_out a multiple of 128, so that a tile belongs to one product.  One launch because a product of a
+// few megabytes costs more in its start and end than in its stream: four of 4,096 x 4,096 at 64 tokens take 54 us one after the
+// other and 32 together, of 2,048 x 2,048 31 and 13, of 1,024 x 1,024 at one token 17 and 6.
+int rl_gemm_bf16_planes(const void* x, const void* w, void* out, int planes, int tokens, int n_out, int k, int pdl, int* fault,
+                        cudaStream_t stream) {
+  if (planes == 0 || tokens == 0 || n_out == 0) return 0;
+  if (planes < 0 || tokens < 0 || tokens > 64 || n_out < 0 || n_out % rl::kTileN != 0 || k <= 0 || k % 8 != 0 ||
+      ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(out)) & 15))
+    return static_cast<int>(cudaErrorInvalidValue);
+  const int bn = rl::token_tile(tokens, false);
+  CUtensorMap map_w, map_x;
+  int status = rl::make_map(&map_w, w, static_cast<long long>(planes) * n_out, k, rl::kTileN);
+  if (status != 0) return status;
+  status = rl::make_map(&map_x, x, static_cast<long long>(planes) * tokens, k, bn);
+  if (status != 0) return status;
+  rl::GemmArgs args = {};
+  args.out = static_cast<rl::bf16*>(out);
+  args.fault = fault;
+  args.T = tokens; args.N = n_out; args.K = k;
+  args.up_offset = n_out;
+  args.tile_rows = rl::kTileN;
+  args.plane_tiles = n_out / rl::kTileN;
+  args.n_tiles = planes * args.plane_tiles;
+  args.t_tiles = 1;
+  args.k_blocks = (k + rl::kTileK - 1) / rl::kTileK;
+  args.k_split = 1;
+  args.pdl = pdl;
+  args.residual_scale = 1.0f;
+  if (bn == 16) return rl::launch_gemm<false, 16, false, true>(map_w, map_x, args, 0, stream);
+  if (bn == 32) return rl::launch_gemm<false, 32, false, true>(map_w, map_x, args, 0, stream);
+  return rl::launch_gemm<false, 64, false, true>(map_w, map_x, args, 0, stream);
 }
 
 // columns of the table of partial sums of squares that a product of `n_out` output columns writes per token

@@ -195,6 +195,20 @@ def _square_columns(out: torch.Tensor, columns: int) -> torch.Tensor:
     return out
 
 
+def planes_linear(x: torch.Tensor, weights: torch.Tensor, out: torch.Tensor, fault: torch.Tensor | None = None) -> torch.Tensor:
+    """Products of inputs of their own, ``out[p] = x[p] @ weights[p]^T`` with ``weights [P, N, K]``, ``x [P * T, K]`` and
+    ``out [P * T, N]``: one launch of the tensor-core kernel where a step is small enough for it, else one product after the other."""
+    planes, width, _ = weights.shape
+    rows = x.shape[0] // planes
+    if (fault is not None and 0 < rows <= kernels.GEMM_PLANES_MAX_TOKENS and width % 128 == 0 and x.is_contiguous() and out.is_contiguous()
+            and use_tensor_core_kernel(x[:rows], weights[0])):
+        flush()
+        return kernels.gemm_bf16_planes(x, weights, out, fault)
+    for plane in range(planes):
+        linear(x[plane * rows : (plane + 1) * rows], weights[plane], out[plane * rows : (plane + 1) * rows], fault)
+    return out
+
+
 def heads_linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, *, x_col0: int = 0) -> torch.Tensor:
     """A product per head, ``out[t, h, :N] = x[t, h, x_col0 : x_col0 + K] @ weight[h]^T`` with ``weight [heads, N, K]``,
     ``x [T, heads * x_width]`` and ``out [T, heads * out_width]``; columns of ``out`` behind ``N`` in a head stay.

@@ -796,6 +796,8 @@ def gemm_lib() -> ctypes.CDLL:
                                           c_void_p, c_void_p, c_void_p, c_void_p, c_int, ctypes.c_float, c_int,
                                           c_void_p, c_float, c_float, c_int, c_int, c_float, c_void_p, c_void_p]
         lib.rl_gemm_bf16_norm.restype = c_int
+        lib.rl_gemm_bf16_planes.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p]
+        lib.rl_gemm_bf16_planes.restype = c_int
         lib.rl_gemm_bf16_sumsq_count.argtypes = [c_int]
         lib.rl_gemm_bf16_sumsq_count.restype = c_int
         _GEMM_LIB = lib
@@ -805,6 +807,28 @@ def gemm_lib() -> ctypes.CDLL:
 def gemm_bf16_supports(x: torch.Tensor, w: torch.Tensor) -> bool:
     """Whether the tensor-core product takes these operands (TMA wants 16-byte rows)."""
     return x.shape[1] % 8 == 0 and (x.shape[0] <= 1 or x.stride(0) % 8 == 0) and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
+
+
+GEMM_PLANES_MAX_TOKENS = 64   # most rows of each of several products in one launch
+
+
+def gemm_bf16_planes(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, fault: torch.Tensor) -> torch.Tensor:
+    """Several products in one launch: ``out[p] = x[p] @ w[p]^T`` with ``w [P, N, K]``, ``x [P * T, K]`` and ``out [P * T, N]``,
+    bfloat16 and contiguous, ``N`` a multiple of 128, at most :data:`GEMM_PLANES_MAX_TOKENS` rows each."""
+    _need_cuda(x, w, out, fault)
+    for name, tensor in (("x", x), ("w", w), ("out", out)):
+        _expect(name, tensor, torch.bfloat16), _contig(name, tensor)
+    if w.dim() != 3 or x.dim() != 2 or out.dim() != 2:
+        raise KernelError("gemm_bf16_planes: w is [planes, N, K], x and out are matrices")
+    planes, n_out, k = w.shape
+    if (planes == 0 or x.shape[0] % planes or x.shape[1] != k or out.shape != (x.shape[0], n_out) or n_out % 128
+            or x.shape[0] // planes > GEMM_PLANES_MAX_TOKENS):
+        raise KernelError(f"gemm_bf16_planes: shapes {tuple(x.shape)} x {tuple(w.shape)}^T -> {tuple(out.shape)} do not agree")
+    if not gemm_bf16_supports(x, w):
+        raise KernelError("gemm_bf16_planes: the inner size must be a multiple of 8 and the operands 16-byte aligned")
+    _check(gemm_lib().rl_gemm_bf16_planes(_ptr(x), _ptr(w), _ptr(out), planes, x.shape[0] // planes, n_out, k, int(PDL), _ptr(fault),
+                                          _stream()), "gemm_bf16_planes")
+    return out
 
 
 GEMM_NORM_MAX_TOKENS = 64   # most rows of a product that carries a norm's add or a norm's open scale

@@ -518,9 +518,7 @@ class ShiftedDecay(_Recurrent):
         S, kept = self._state_views(cache)
         blends = kernels.shift_mix(x, self.mu, space.get("wkv_blends", 5 * rows, self.hidden, x.dtype), kept, batch)
         proj = space.get("wkv_proj", 4 * rows, c, x.dtype)               # planes r | k | v | g
-        for index in range(4):
-            gemm.linear(blends[index * rows : (index + 1) * rows], self.w_rkvg[index],
-                        proj[index * rows : (index + 1) * rows], batch.fault)
+        gemm.planes_linear(blends[: 4 * rows], self.w_rkvg, proj, batch.fault)
         low = gemm.linear(blends[4 * rows :], self.w1, space.get("wkv_low", rows, self.rank, x.dtype), batch.fault)
         gemm.flush()
         kernels.tanh_rows(low, low)
