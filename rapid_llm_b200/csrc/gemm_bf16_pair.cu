@@ -201,7 +201,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
   __shared__ int aborted_flag;
   volatile int* aborted = &aborted_flag;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform(static_cast<int>(threadIdx.x) >> 5), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_cta_rank();                 // 0: the CTA that issues the products
   const bool leader = rank == 0;
   const int pair = static_cast<int>(blockIdx.x) >> 1, pairs = static_cast<int>(gridDim.x) >> 1;
@@ -241,7 +241,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
   __syncthreads();
   cluster_sync();                                 // the partner's barriers exist before anything is signalled to them
   tc_fence_after();
-  const uint32_t tmem_base = tmem_base_slot;
+  const uint32_t tmem_base = uniform(tmem_base_slot);
   if (args.pdl && threadIdx.x == 0) pdl_trigger();
 
   if (warp == 0) {
@@ -294,35 +294,43 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ products (the first CTA only)
-    if (leader && lane == 0) {
+    // The whole warp waits, one elected thread issues (elect_one in tc_common.cuh says why): the layers of a 2,048-token
+    // prompt, four products each, go from 3,107 to 2,999 us with the head.
+    if (leader) {
+      const bool issues = elect_one();
       int stage = 0, buf = 0;
-      uint32_t phase = 0, acc_phase[2] = {0, 0};
+      uint32_t phase = 0, acc_phase = 0;          // acc_phase: a bit for each buffer
       bool ok = true;
       PairRun run(args, pair, pairs);
       int tile, kb0, len;
       while (ok && run.next(tile, kb0, len)) {
-        ok = mbar_wait(smem_addr(&acc_empty_bar[buf]), acc_phase[buf] ^ 1u, aborted, args.fault, 1 << 9);
+        ok = __all_sync(0xffffffffu, mbar_wait(smem_addr(&acc_empty_bar[buf]), ((acc_phase >> buf) & 1u) ^ 1u, aborted, args.fault, 1 << 9));
         if (!ok) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + buf * kPairCols;
         for (int kb = 0; kb < len; ++kb) {
-          ok = mbar_wait(smem_addr(&full_bar[stage]), phase, aborted, args.fault, 1 << 10);
+          ok = __all_sync(0xffffffffu, mbar_wait(smem_addr(&full_bar[stage]), phase, aborted, args.fault, 1 << 10));
           if (!ok) break;
           tc_fence_after();
           const uint64_t a_desc = operand_desc(stage_a(stage));
           const uint64_t b_desc = operand_desc(stage_b(stage));
+          if (issues) {
 #pragma unroll
-          for (int k = 0; k < kPairTileK / 16; ++k)
-            umma_bf16_pair(d_tmem, a_desc + 2 * k, b_desc + 2 * k, kPairIdesc, (kb > 0 || k > 0) ? 1u : 0u);
-          umma_commit_pair(smem_addr(&empty_bar[stage]), 3);     // the stage is free in both CTAs
+            for (int k = 0; k < kPairTileK / 16; ++k)
+              umma_bf16_pair(d_tmem, a_desc + 2 * k, b_desc + 2 * k, kPairIdesc, (kb > 0 || k > 0) ? 1u : 0u);
+            umma_commit_pair(smem_addr(&empty_bar[stage]), 3);     // the stage is free in both CTAs
+          }
+          __syncwarp();
           if (++stage == kPairStages) { stage = 0; phase ^= 1u; }
         }
         if (!ok) break;
-        umma_commit_pair(smem_addr(&acc_full_bar[buf]), 3);
-        acc_phase[buf] ^= 1u;
+        if (issues) umma_commit_pair(smem_addr(&acc_full_bar[buf]), 3);
+        __syncwarp();
+        acc_phase ^= 1u << buf;
         buf ^= 1;
       }
-      umma_commit_pair(smem_addr(&drain_bar), 1);
+      if (issues) umma_commit_pair(smem_addr(&drain_bar), 1);
+      __syncwarp();
       mbar_wait(smem_addr(&drain_bar), 0, aborted, args.fault);
     }
   } else {
