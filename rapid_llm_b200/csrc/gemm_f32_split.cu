@@ -3,12 +3,12 @@
 // A float32 number is exactly the sum of three bfloat16 ones: its leading 8 bits, the next 8 and the last 8 (truncation, so
 // every remainder is exact and nothing overflows).  Of the nine products of two such sums the six that reach 2^-24 of the
 // whole are formed, each exact in the tensor core's float32:
-//   w0 x0                                          summed over 64 columns, then added to a float32 sum in registers
+//   w0 x0                                          summed over 256 columns, then added to a float32 sum in registers
 //   w0 x1, w1 x0, w1 x1, w0 x2, w2 x0              summed over all columns in an accumulator of their own
-// The tensor core cuts off what lies below its accumulator's last bit; 64 columns at a time, and with the small products
+// The tensor core cuts off what lies below its accumulator's last bit; 256 columns at a time, and with the small products
 // apart, that costs less than the roundings of one fused multiply-add after the other.
 //
-// An output is a sum in an order that n and k alone decide (64 columns, then the columns of a segment, then the segments,
+// An output is a sum in an order that n and k alone decide (256 columns, then the columns of a segment, then the segments,
 // whose number `split_segments` takes from n and k): not M, the tile it falls in, or what else is in the batch.
 // A product of an infinity's or a NaN's parts is not finite; such outputs are formed again, one column after the other.
 //
