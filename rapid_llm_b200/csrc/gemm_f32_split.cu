@@ -302,11 +302,35 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                                        mbar_wait(smem_addr(&empty_bar[b]), phase, aborted, fault));
       if (!ok) break;
       tc_fence_after();
+      // few tokens, where the weights' stream is the bound: a place of the ring goes back as soon as its numbers are in registers, and
+      // only the rows there are are cut.  One row by 24,576 x 4,096 87 -> 78 us (5.2 TB/s), 4,096 x 12,288 56 -> 40
+      float early[kCopied ? 1 : 32];
+      if constexpr (!kCopied) {
+        float v[8];
+        const bool cuts = row < live;           // (rows behind the last: anything, for outputs that are not stored)
+        if (cuts) {
+          load_raw(raw_x(r), row, 2 * eight, v);
+          load_raw(raw_x(r), row, 2 * eight + 1, v + 4);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) load_raw(raw_w(r), w_row, j, early + 4 * j);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_addr(&raw_empty_bar[r]));
+        if (cuts) {
+          store_parts(buffer_x(b) + place, part_x, v);
+          fence_async_smem();
+        }
+      }
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         float v[16];
+        if constexpr (kCopied) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) load_raw(raw_w(r), w_row, half * 4 + j, v + 4 * j);
+          for (int j = 0; j < 4; ++j) load_raw(raw_w(r), w_row, half * 4 + j, v + 4 * j);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] = early[half * 16 + j];
+        }
 #pragma unroll
         for (int part = 0; part < 3; ++part) {
           uint32_t packed[8];
@@ -319,21 +343,12 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
           }
         }
       }
-      if constexpr (!kCopied) {
-        if (row < tokens) {
-          float v[8];
-          load_raw(raw_x(r), row, 2 * eight, v);
-          load_raw(raw_x(r), row, 2 * eight + 1, v + 4);
-          store_parts(buffer_x(b) + place, part_x, v);
-        }
-        fence_async_smem();
-      }
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) {
         mbar_arrive(smem_addr(&full_bar[b]));
-        mbar_arrive(smem_addr(&raw_empty_bar[r]));
+        if (kCopied) mbar_arrive(smem_addr(&raw_empty_bar[r]));
       }
       if ((b += 2) >= kBuffers) { b -= kBuffers; phase ^= 1u; }
       if ((r += 2) >= kRaw) { r -= kRaw; raw_phase ^= 1u; }
@@ -451,9 +466,9 @@ static int launch_split(SplitArgs args, __nv_bfloat16* parts, cudaStream_t strea
 
 // Whether the product runs here: a rule on the weight alone, so that a row's bits do not depend on what it comes with.  The line
 // lies where the weight's 32 MB are a few rounds of tiles; below it a product is its launches.  us at 1, 16, 64, 203 rows,
-// sums down the columns / here: 4,096 x 4,096 23, 58, 166, 252 / 23, 23, 30, 48; 24,576 x 4,096 70, 167, 351, 1,078 / 87, 89,
-// 112, 230; 4,096 x 12,288 63, 166, 488, 740 / 56, 57, 76, 128; 151,936 x 4,096 380, 753, 1,900, 5,830 / 415, 423, 581, 1,253
-// (a single row of wide weights is the one that loses: its stream runs at 0.85 to 0.9 of the sums' in registers).
+// sums down the columns / here: 4,096 x 4,096 23, 58, 166, 252 / 20, 21, 30, 48; 24,576 x 4,096 72, 167, 351, 1,078 / 78, 80,
+// 112, 230; 4,096 x 12,288 62, 166, 488, 740 / 40, 43, 76, 128; 151,936 x 4,096 384, 804, 1,900, 5,830 / 404, 453, 581, 1,253
+// (a single row of wide weights is the one that loses, by 5 to 9 %; a layer of one row and its head take as long either way).
 bool gemm_f32_split_takes(const float* w, int n, int k) {
   return k % 4 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0 && n >= 1024 && k >= 1024 &&
          static_cast<long long>(n) * k >= 1 << 23 && n <= 65535 * kSplitM;
