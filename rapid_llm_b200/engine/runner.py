@@ -165,6 +165,7 @@ class ModelRunner:
         return pages_that_fit(
             free, self.config.memory_fraction, per_page,
             reserve=self.config.max_num_batched_tokens * self.model.activation_bytes_per_token()
+            + self.model.product_scratch_bytes(self.config.max_num_batched_tokens)
             + self.config.max_num_seqs * self.model.spec.vocab_size * (element + 4),
             cap=self.config.max_num_seqs * self.config.max_pages_per_seq,
         )

@@ -11,8 +11,8 @@ import torch
 
 from ..config.model_spec import ModelSpec
 from ..engine.batch import LayerCache, StepBatch
-from ..ops import gemm
-from ..parts.base import BLOCKS, EMBEDDINGS, HEADS, NORMS, CacheNeed, StateNeed, StreamAddend, TensorSpec
+from ..ops import gemm, kernels
+from ..parts.base import BLOCKS, EMBEDDINGS, HEADS, MATRIX, NORMS, CacheNeed, StateNeed, StreamAddend, TensorSpec
 from ..parts.norm import ADD, PLAIN
 
 
@@ -94,6 +94,14 @@ class CausalLM:
         element = torch.empty((), dtype=self.dtype).element_size()
         widest = max(layer.workspace_elements_per_token() for layer in self.layers)
         return (widest + 2 * self.spec.hidden_size) * element + 4 * self.spec.hidden_size
+
+    def product_scratch_bytes(self, tokens: int) -> int:
+        """Bytes of the workspace's buffers for a step's 32-bit products (``ops.kernels.gemm_f32``): three 16-bit parts a number of
+        the rows that run at a time, for every width of rows a large weight takes."""
+        if self.dtype != torch.float32:
+            return 0
+        shapes = [spec.shape for spec in self.tensor_specs().values() if spec.kind == MATRIX and len(spec.shape) == 2]
+        return 6 * min(tokens, kernels.GEMM_F32_ROWS) * sum({-(-shape[1] // 8) * 8 for shape in shapes if shape[1] >= 1024})
 
     # -- what the cache manager has to provide -------------------------------------- #
     def cache_needs(self) -> list[CacheNeed | None]:

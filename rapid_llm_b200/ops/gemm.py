@@ -141,7 +141,7 @@ def _bias_as(bias: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
     return kept[2]
 
 
-def linear(x, weight: torch.Tensor, out: torch.Tensor, fault: torch.Tensor | None = None, *,
+def linear(x, weight: torch.Tensor, out: torch.Tensor, fault: torch.Tensor | None = None, space=None, *,
            then_norm: FollowingNorm | None = None, bias: torch.Tensor | None = None, defer: bool = False,
            relu2_columns: int = 0):
     """``out[T, N] = x[T, K] @ weight[N, K]^T (+ bias[N], float32)``; all on the GPU, same dtype.  ``x`` may be a view of
@@ -151,7 +151,8 @@ def linear(x, weight: torch.Tensor, out: torch.Tensor, fault: torch.Tensor | Non
     ``x`` may be :class:`ScaledRows`.  With ``then_norm`` the product may take the norm along:
     it then returns :class:`ScaledRows` (the residual is updated, ``out`` is not written);
     otherwise it returns ``out`` and the caller runs the norm.  With ``defer`` the product may be
-    queued (see the module's text): its result exists once :func:`flush` has run.
+    queued (see the module's text): its result exists once :func:`flush` has run.  ``space`` (a workspace) lends the
+    32-bit product its scratch.
     """
     x, scale = _open_scale(x)
     if not x.is_cuda:
@@ -163,7 +164,7 @@ def linear(x, weight: torch.Tensor, out: torch.Tensor, fault: torch.Tensor | Non
     if x.shape[0] == 0:
         return out
     if x.dtype == torch.float32:
-        kernels.gemm_f32(x, weight, out, bias, fault)
+        kernels.gemm_f32(x, weight, out, bias, fault, space)
         return _square_columns(out, relu2_columns)
     if fault is not None and use_tensor_core_kernel(x, weight):
         rows, width = out.shape
@@ -195,7 +196,8 @@ def _square_columns(out: torch.Tensor, columns: int) -> torch.Tensor:
     return out
 
 
-def planes_linear(x: torch.Tensor, weights: torch.Tensor, out: torch.Tensor, fault: torch.Tensor | None = None) -> torch.Tensor:
+def planes_linear(x: torch.Tensor, weights: torch.Tensor, out: torch.Tensor, fault: torch.Tensor | None = None,
+                  space=None) -> torch.Tensor:
     """Products of inputs of their own, ``out[p] = x[p] @ weights[p]^T`` with ``weights [P, N, K]``, ``x [P * T, K]`` and
     ``out [P * T, N]``: one launch of the tensor-core kernel where a step is small enough for it, else one product after the other."""
     planes, width, _ = weights.shape
@@ -205,7 +207,7 @@ def planes_linear(x: torch.Tensor, weights: torch.Tensor, out: torch.Tensor, fau
         flush()
         return kernels.gemm_bf16_planes(x, weights, out, fault)
     for plane in range(planes):
-        linear(x[plane * rows : (plane + 1) * rows], weights[plane], out[plane * rows : (plane + 1) * rows], fault)
+        linear(x[plane * rows : (plane + 1) * rows], weights[plane], out[plane * rows : (plane + 1) * rows], fault, space)
     return out
 
 
@@ -255,7 +257,7 @@ def gated_linear(x, gate_up: torch.Tensor, act: torch.Tensor, workspace, fault: 
         flush()
         return kernels.gemm_bf16_pair(x, gate_up, act, fault, swiglu=True, **unit)      # no [T, 2 I] intermediate
     wide = workspace.get("ffn_gate_up", x.shape[0], gate_up.shape[0], x.dtype)
-    linear(x, gate_up, wide, fault)
+    linear(x, gate_up, wide, fault, workspace)
     if clamp is not None:
         return kernels.clamped_glu(wide, act, clamp[0], clamp[1])
     return kernels.silu_mul(wide, act)

@@ -757,10 +757,14 @@ def attention_mma(
     return out
 
 
+GEMM_F32_ROWS = 1024        # rows of a 32-bit product by a large weight that run at a time
+
+
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: torch.Tensor | None = None,
-             fault: torch.Tensor | None = None) -> torch.Tensor:
+             fault: torch.Tensor | None = None, space=None) -> torch.Tensor:
     """``out[M, N] = a[M, K] @ w[N, K]^T`` in 32 bits: a row's values depend on the row and the weight alone.  Scratch for the
-    rows' parts (6 bytes a number, 1,024 rows at most) comes from torch's allocator where the kernel wants it."""
+    rows' parts (6 bytes a number, :data:`GEMM_F32_ROWS` rows at most) comes from the workspace ``space``, a buffer for each
+    width of rows, or without one from torch's allocator, where the kernel wants it."""
     _need_cuda(a, w, out, bias, fault)
     for name, tensor in (("a", a), ("w", w), ("out", out), ("bias", bias)):
         _expect(name, tensor, torch.float32)
@@ -771,15 +775,20 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: torch.Te
         raise KernelError("gemm_f32: rows of a and out must be contiguous")
     rows, columns, inner = a.shape[0], w.shape[0], a.shape[1]
     wanted = core().rl_gemm_f32_scratch(_ptr(a), _ptr(w), rows, columns, inner, a.stride(0))
-    parts = torch.empty(wanted, dtype=torch.bfloat16, device=a.device) if wanted else None
+    parts = None
+    if wanted and space is not None:
+        held = min(rows, GEMM_F32_ROWS)
+        parts = space.get("product_parts", held, wanted // held, torch.bfloat16, min_rows=max(held, min(space.max_tokens, GEMM_F32_ROWS)))
+    elif wanted:
+        parts = torch.empty(wanted, dtype=torch.bfloat16, device=a.device)
     _check(
         core().rl_gemm_f32(_ptr(a), _ptr(w), _ptr(bias), _ptr(out), rows, columns, inner, a.stride(0), out.stride(0), _ptr(parts),
                            _ptr(fault), _stream()),
         "gemm_f32",
     )
     if wanted:
-        # 1,024 rows at a time, a launch for their parts and one for the product; up to 32 left over are cut in the product itself
-        passes, left = -(-rows // 1024), (rows - 1) % 1024 + 1
+        # so many rows at a time, a launch for their parts and one for the product; up to 32 left over are cut in the product itself
+        passes, left = -(-rows // GEMM_F32_ROWS), (rows - 1) % GEMM_F32_ROWS + 1
         LAUNCHES.count += 2 * passes - 1 - int(left <= 32 and a.stride(0) % 4 == 0 and a.data_ptr() % 16 == 0)
     return out
 

@@ -500,16 +500,16 @@ class GQAAttention(Mixer):
     def forward(self, x, batch, cache, then_norm=None):
         rows = x.shape[0]
         qkv = batch.workspace.get("attn_qkv", rows, self.qkv.shape[0], x.dtype)
-        gemm.linear(x, self.qkv, qkv, batch.fault, bias=self.qkv_bias, defer=batch.defer_products)
+        gemm.linear(x, self.qkv, qkv, batch.fault, batch.workspace, bias=self.qkv_bias, defer=batch.defer_products)
         gate = None
         if self.gate_rides:
             gate = qkv[:, self.qkv_rows : self.qkv_rows + self.gate_width]          # the first product brought it along
         elif self.gate:
             gate = batch.workspace.get("attn_gate", rows, self.gate_width, x.dtype)
-            gemm.linear(x, self.g, gate, batch.fault)
+            gemm.linear(x, self.g, gate, batch.fault, batch.workspace)
         attended = self._attended(qkv, gate, batch.workspace.get("attn_heads", rows, self.hq * self.d, x.dtype), batch, cache)
         out = batch.workspace.get("attn_proj", rows, self.hidden, x.dtype)
-        return gemm.linear(attended, self.o, out, batch.fault, then_norm=then_norm, bias=self.o_bias, defer=batch.defer_products)
+        return gemm.linear(attended, self.o, out, batch.fault, batch.workspace, then_norm=then_norm, bias=self.o_bias, defer=batch.defer_products)
 
     def _attended(self, qkv, gate, out, batch, cache) -> torch.Tensor:
         """From the first product's result to the gated heads side by side in ``out``: norms, rotation, the cache's store,

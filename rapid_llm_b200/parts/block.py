@@ -374,9 +374,9 @@ class SharedNormBlock(PreNormBlock):
             gemm.flush()
             return kernels.scaled_sum(mixed, wide, 1.0, 1.0, space.get("shared_sum", rows, mixed.shape[1], mixed.dtype)), residual
         wide = space.get("shared_wide", rows, self.first.shape[0], normed.dtype)
-        gemm.linear(normed, self.first, wide, batch.fault, bias=self.first_bias, relu2_columns=self.ff_columns)
+        gemm.linear(normed, self.first, wide, batch.fault, batch.workspace, bias=self.first_bias, relu2_columns=self.ff_columns)
         self.mixer.middle(wide[:, self.ff_columns :], batch, cache)
         offer = then_norm.following(residual, batch) if then_norm is not None else None
         out = space.get("shared_out", rows, self.hidden, normed.dtype)
-        return gemm.linear(wide[:, : self.last.shape[1]], self.last, out, batch.fault, then_norm=offer,
+        return gemm.linear(wide[:, : self.last.shape[1]], self.last, out, batch.fault, batch.workspace, then_norm=offer,
                            bias=self.mixer.o_bias), residual

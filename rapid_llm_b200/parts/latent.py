@@ -189,7 +189,7 @@ class LatentAttention(Mixer):
             raise ValueError("latent attention: the cache the engine gave this layer does not match its role in the run order")
         group, space, rows = batch.groups[cache.group], batch.workspace, x.shape[0]
         pages = cache.pages                                       # [pages, page_size, D]
-        down = gemm.linear(x, self.down, space.get("latent_down", rows, self.down_rows, x.dtype), batch.fault)
+        down = gemm.linear(x, self.down, space.get("latent_down", rows, self.down_rows, x.dtype), batch.fault, batch.workspace)
         gemm.flush()
         c_q = space.get("latent_cq", rows, self.q_rank, x.dtype)      # no columns without a query latent
         kernels.latent_norm_write(
@@ -197,7 +197,7 @@ class LatentAttention(Mixer):
             q_weight=self.q_norm, c_weight=self.c_norm, eps=self.eps, q_out=c_q, cache=None if self.shares_cache else pages,
             kv_dest=None if self.shares_cache else group.kv_dest, positions=batch.positions, freq=self.freq,
             magnitude=self.magnitude, layout=self.layout, fault=batch.fault)
-        q = gemm.linear(x if self.direct_q else c_q, self.uq, space.get("latent_q", rows, self.uq.shape[0], x.dtype), batch.fault)
+        q = gemm.linear(x if self.direct_q else c_q, self.uq, space.get("latent_q", rows, self.uq.shape[0], x.dtype), batch.fault, batch.workspace)
         gemm.flush()
         wide = space.get("latent_wide", rows, self.h * self.d, x.dtype)
         gemm.heads_linear(q, self.uk_t, wide)                  # columns [0, kv_rank) of every head
@@ -212,7 +212,7 @@ class LatentAttention(Mixer):
             kernels.sigmoid_scale_heads(values, down[:, self.g_col0 :], heads=self.h)
         if self.wide_gate:
             values = kernels.sigmoid_gate(values, down[:, self.g_col0 :], space.get("latent_gated", rows, self.h * self.vdim, x.dtype))
-        return gemm.linear(values, self.o, space.get("latent_out", rows, self.hidden, x.dtype), batch.fault)
+        return gemm.linear(values, self.o, space.get("latent_out", rows, self.hidden, x.dtype), batch.fault, batch.workspace)
 
     def _attend(self, q, pages, out, batch, group) -> None:
         if q.dtype == torch.bfloat16 and not self.wide_row:

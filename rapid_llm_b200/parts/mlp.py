@@ -57,7 +57,7 @@ class SwiGLU(FeedForward):
         act = batch.workspace.get("ffn_act", rows, self.inter, x.dtype)
         gemm.gated_linear(x, self.gate_up, act, batch.workspace, batch.fault, defer=batch.defer_products)
         out = batch.workspace.get("ffn_out", rows, self.hidden, x.dtype)
-        return gemm.linear(act, self.down, out, batch.fault, then_norm=then_norm, defer=batch.defer_products)
+        return gemm.linear(act, self.down, out, batch.fault, batch.workspace, then_norm=then_norm, defer=batch.defer_products)
 
 
     def uses_libraries(self) -> set[str]:
@@ -83,7 +83,7 @@ class ClampedGLU(SwiGLU):
         rows = x.shape[0]
         act = batch.workspace.get("ffn_act", rows, self.inter, x.dtype)
         gemm.gated_linear(x, self.gate_up, act, batch.workspace, batch.fault, clamp=(self.limit, self.alpha))
-        return gemm.linear(act, self.down, batch.workspace.get("ffn_out", rows, self.hidden, x.dtype), batch.fault)
+        return gemm.linear(act, self.down, batch.workspace.get("ffn_out", rows, self.hidden, x.dtype), batch.fault, batch.workspace)
 
 
 # activation name -> (number of learned scalars, kernel over [T, I] rows, library it lives in)
@@ -143,13 +143,13 @@ class DenseFeedForward(FeedForward):
         rows = x.shape[0]
         wide = batch.workspace.get("ffn_up", rows, self.inter, x.dtype)
         if self.activation == "relu_squared":
-            act = gemm.linear(x, self.up, wide, batch.fault, relu2_columns=self.inter)
+            act = gemm.linear(x, self.up, wide, batch.fault, batch.workspace, relu2_columns=self.inter)
         else:
-            gemm.linear(x, self.up, wide, batch.fault)
+            gemm.linear(x, self.up, wide, batch.fault, batch.workspace)
             act = batch.workspace.get("ffn_act", rows, self.inter, x.dtype)
             ACTIVATIONS[self.activation][1](wide, act, self.scalars)
         out = batch.workspace.get("ffn_out", rows, self.hidden, x.dtype)
-        return gemm.linear(act, self.down, out, batch.fault)
+        return gemm.linear(act, self.down, out, batch.fault, batch.workspace)
 
     # -- in an arrangement that stacks its sublayers' products ------------------- #
     @property

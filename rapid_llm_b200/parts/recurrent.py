@@ -188,9 +188,9 @@ class ChannelDeltaRule(_Recurrent):
     def forward(self, x, batch, cache):
         rows, space, f32 = x.shape[0], batch.workspace, torch.float32
         S, tail = self._state_views(cache)
-        proj = gemm.linear(x, self.w_in, space.get("delta_in", rows, self.w_in.shape[0], x.dtype), batch.fault)
-        low = gemm.linear(x, self.w_low, space.get("delta_low", rows, self.w_low.shape[0], x.dtype), batch.fault)
-        high = gemm.linear(low, self.w_high, space.get("delta_high", rows, self.w_high.shape[0], x.dtype), batch.fault)
+        proj = gemm.linear(x, self.w_in, space.get("delta_in", rows, self.w_in.shape[0], x.dtype), batch.fault, batch.workspace)
+        low = gemm.linear(x, self.w_low, space.get("delta_low", rows, self.w_low.shape[0], x.dtype), batch.fault, batch.workspace)
+        high = gemm.linear(low, self.w_high, space.get("delta_high", rows, self.w_high.shape[0], x.dtype), batch.fault, batch.workspace)
         conv = space.get("delta_conv", rows, self.conv_channels, f32)
         kernels.causal_conv_silu(proj[:, : self.conv_channels], self.taps, None, tail, conv, batch)
         beta = space.get("delta_beta", rows, self.h, f32)
@@ -205,7 +205,7 @@ class ChannelDeltaRule(_Recurrent):
         normed = space.get("delta_normed", rows, self.cv, x.dtype)
         kernels.gated_norm(read, normed, group=self.vdim, gate=high[:, self.h * self.dim :], act=kernels.GATE_SIGMOID,
                            weight=self.norm, eps=self.eps)
-        return gemm.linear(normed, self.o, space.get("delta_out", rows, self.hidden, x.dtype), batch.fault)
+        return gemm.linear(normed, self.o, space.get("delta_out", rows, self.hidden, x.dtype), batch.fault, batch.workspace)
 
 
 @MIXERS.register("retention")
@@ -268,7 +268,7 @@ class Retention(_Recurrent):
         rows, space, f32 = x.shape[0], batch.workspace, torch.float32
         S, _ = self._state_views(cache)
         cq, cv = self.cq, self.cv
-        proj = gemm.linear(x, self.w_in, space.get("ret_in", rows, self.w_in.shape[0], x.dtype), batch.fault)
+        proj = gemm.linear(x, self.w_in, space.get("ret_in", rows, self.w_in.shape[0], x.dtype), batch.fault, batch.workspace)
         qkv = space.get("ret_qkv", rows, 2 * cq + cv, f32)
         kernels.rotate_heads(proj[:, :cq], proj[:, cq : 2 * cq], proj[:, 2 * cq : 2 * cq + cv], qkv, batch.positions,
                              self.inv_freq, heads=self.h, dim=self.dim, vdim=self.vdim, k_scale=self.dim ** -0.5)
@@ -278,7 +278,7 @@ class Retention(_Recurrent):
                             blocks_from=kernels.scan_blocks_from(self.h, self.dim, self.vdim))
         normed = space.get("ret_normed", rows, cv, x.dtype)
         kernels.gated_norm(read, normed, group=self.vdim, gate=proj[:, 2 * cq + cv :], act=kernels.GATE_SILU, eps=self.eps)
-        return gemm.linear(normed, self.o, space.get("ret_out", rows, self.hidden, x.dtype), batch.fault)
+        return gemm.linear(normed, self.o, space.get("ret_out", rows, self.hidden, x.dtype), batch.fault, batch.workspace)
 
 
 @MIXERS.register("lightning")
@@ -338,7 +338,7 @@ class Lightning(_Recurrent):
         rows, space, f32 = x.shape[0], batch.workspace, torch.float32
         S, _ = self._state_views(cache)
         cq, cv = self.cq, self.cv
-        proj = gemm.linear(x, self.w_in, space.get("lightning_in", rows, self.w_in.shape[0], x.dtype), batch.fault)
+        proj = gemm.linear(x, self.w_in, space.get("lightning_in", rows, self.w_in.shape[0], x.dtype), batch.fault, batch.workspace)
         qkv = kernels.activate_rows(proj[:, : 2 * cq + cv], space.get("lightning_qkv", rows, 2 * cq + cv, f32), act=True)
         read = space.get("lightning_read", rows, cv, f32)
         kernels.linear_scan(qkv[:, :cq], qkv[:, cq : 2 * cq], qkv[:, 2 * cq :], self.decay, read, S, batch,
@@ -347,7 +347,7 @@ class Lightning(_Recurrent):
         normed = space.get("lightning_normed", rows, cv, x.dtype)
         kernels.gated_norm(read, normed, group=cv, gate=proj[:, 2 * cq + cv :], act=kernels.GATE_SIGMOID,
                            weight=self.norm, eps=self.eps)
-        return gemm.linear(normed, self.o, space.get("lightning_out", rows, self.hidden, x.dtype), batch.fault)
+        return gemm.linear(normed, self.o, space.get("lightning_out", rows, self.hidden, x.dtype), batch.fault, batch.workspace)
 
 
 @MIXERS.register("state_space_dual")
@@ -424,7 +424,7 @@ class StateSpaceDual(_Recurrent):
         rows, space, f32 = x.shape[0], batch.workspace, torch.float32
         S, tail = self._state_views(cache)
         inner, gn, mixed = self.inner, self.groups * self.n, self.conv_channels
-        proj = gemm.linear(x, self.w_in, space.get("ssd_in", rows, self.w_in.shape[0], x.dtype), batch.fault)
+        proj = gemm.linear(x, self.w_in, space.get("ssd_in", rows, self.w_in.shape[0], x.dtype), batch.fault, batch.workspace)
         conv = space.get("ssd_conv", rows, mixed, f32)
         kernels.causal_conv_silu(proj[:, inner : inner + mixed], self.taps, self.conv_bias, tail, conv, batch)
         decay, step = space.get("ssd_decay", rows, self.h, f32), space.get("ssd_step", rows, self.h, f32)
@@ -436,7 +436,7 @@ class StateSpaceDual(_Recurrent):
         normed = space.get("ssd_normed", rows, inner, x.dtype)
         kernels.gated_norm(read, normed, group=inner // self.norm_groups, gate=proj[:, :inner], act=kernels.GATE_SILU,
                            gate_first=True, weight=self.norm, eps=self.eps)
-        return gemm.linear(normed, self.o, space.get("ssd_out", rows, self.hidden, x.dtype), batch.fault)
+        return gemm.linear(normed, self.o, space.get("ssd_out", rows, self.hidden, x.dtype), batch.fault, batch.workspace)
 
 
 @MIXERS.register("wkv")
@@ -518,11 +518,11 @@ class ShiftedDecay(_Recurrent):
         S, kept = self._state_views(cache)
         blends = kernels.shift_mix(x, self.mu, space.get("wkv_blends", 5 * rows, self.hidden, x.dtype), kept, batch)
         proj = space.get("wkv_proj", 4 * rows, c, x.dtype)               # planes r | k | v | g
-        gemm.planes_linear(blends[: 4 * rows], self.w_rkvg, proj, batch.fault)
-        low = gemm.linear(blends[4 * rows :], self.w1, space.get("wkv_low", rows, self.rank, x.dtype), batch.fault)
+        gemm.planes_linear(blends[: 4 * rows], self.w_rkvg, proj, batch.fault, batch.workspace)
+        low = gemm.linear(blends[4 * rows :], self.w1, space.get("wkv_low", rows, self.rank, x.dtype), batch.fault, batch.workspace)
         gemm.flush()
         kernels.tanh_rows(low, low)
-        high = gemm.linear(low, self.w2, space.get("wkv_high", rows, c, x.dtype), batch.fault)
+        high = gemm.linear(low, self.w2, space.get("wkv_high", rows, c, x.dtype), batch.fault, batch.workspace)
         gemm.flush()
         decay = kernels.exp_decay(high, self.w0, space.get("wkv_decay", rows, c, f32))
         rkv = kernels.activate_rows(proj[: 3 * rows], space.get("wkv_rkv", 3 * rows, c, f32), act=False)
@@ -533,7 +533,7 @@ class ShiftedDecay(_Recurrent):
         normed = space.get("wkv_normed", rows, c, x.dtype)
         kernels.gated_norm(read, normed, group=self.dim, gate=proj[3 * rows :], act=kernels.GATE_SILU, weight=self.norm,
                            eps=self.eps)
-        return gemm.linear(normed, self.o, space.get("wkv_out", rows, self.hidden, x.dtype), batch.fault)
+        return gemm.linear(normed, self.o, space.get("wkv_out", rows, self.hidden, x.dtype), batch.fault, batch.workspace)
 
 
 @MIXERS.register("gated_linear")
@@ -610,7 +610,7 @@ class GatedLinear(_Recurrent):
         rows, space, f32 = x.shape[0], batch.workspace, torch.float32
         S, _ = self._state_views(cache)
         cq, cv = self.cq, self.cv
-        proj = gemm.linear(x, self.w_in, space.get("gla_in", rows, self.w_in.shape[0], x.dtype), batch.fault)
+        proj = gemm.linear(x, self.w_in, space.get("gla_in", rows, self.w_in.shape[0], x.dtype), batch.fault, batch.workspace)
         gemm.flush()
         qkv, decay = space.get("gla_qkv", rows, 2 * cq + cv, f32), space.get("gla_decay", rows, cq, f32)
         kernels.low_rank_decay(proj[:, : 2 * cq + cv], proj[:, self.a_col0 : self.a_col0 + self.rank], self.a2, self.a2_bias,
@@ -622,4 +622,4 @@ class GatedLinear(_Recurrent):
         normed = space.get("gla_normed", rows, cv, x.dtype)
         kernels.gated_norm(read, normed, group=self.vdim, gate=proj[:, self.g_col0 : self.g_col0 + cv], act=kernels.GATE_SILU,
                            weight=self.norm, eps=self.eps * self.dim)
-        return gemm.linear(normed, self.o, space.get("gla_out", rows, self.hidden, x.dtype), batch.fault)
+        return gemm.linear(normed, self.o, space.get("gla_out", rows, self.hidden, x.dtype), batch.fault, batch.workspace)
