@@ -1783,7 +1783,7 @@ int rl_linear_scan(const float* q, int q_stride, const float* k, int k_stride, c
                    const float* bonus, float* out, int out_stride, float* state, long long state_stride, int state_off,
                    const int* cu_seqlens, const int* entry_slot, const int* entry_start, int entries, int tokens, int heads,
                    int kv_heads, int dim, int vdim, int slots, int* fault, int segment, int from, int segments, int others,
-                   float* seg_states, float* seg_decays, int blocks_from, int blocks, float* records, int record_floats, int pdl,
+                   float* seg_states, float* seg_decays, int blocks_from, int blocks, int taken, float* records, int record_floats, int pdl,
                    cudaStream_t stream) {
   if (entries == 0) return 0;
   if (heads < 1 || kv_heads < 1 || heads % kv_heads || dim < 1 || dim > 1024 || vdim < 1 || decay_mode < 0 ||
@@ -1811,7 +1811,7 @@ int rl_linear_scan(const float* q, int q_stride, const float* k, int k_stride, c
     const ScanBlockArgs in_blocks = {q, q_stride, k, k_stride, v, v_stride, decay, decay_mode, beta, v_scale, skip, bonus, out, out_stride,
                                      state + state_off, state_stride, cu_seqlens, entry_slot, entry_start, heads, kv_heads, dim, vdim, slots,
                                      entries, blocks_from, a.wide_in, records, fault};
-    const int e = scan_blocks(in_blocks, blocks, stream);
+    const int e = scan_blocks(in_blocks, blocks, taken, stream);
     if (e || !others) return e;
   }
   // single tokens of the common head sizes: the same rows a lane and lanes a column as the walk, so the same sums

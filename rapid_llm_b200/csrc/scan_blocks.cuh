@@ -28,7 +28,7 @@ struct ScanBlockArgs {
 
 // Floats a block of a head takes in `records`.
 int scan_record_floats(int dim, bool corrected);
-// `blocks`: a bound on the blocks of the step's entries.
-int scan_blocks(const ScanBlockArgs& args, int blocks, cudaStream_t stream);
+// `blocks`, `taken`: bounds on the blocks of the step's entries, and on the entries that have any.
+int scan_blocks(const ScanBlockArgs& args, int blocks, int taken, cudaStream_t stream);
 
 }  // namespace rl

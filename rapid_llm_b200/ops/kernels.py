@@ -1155,7 +1155,7 @@ def recurrent() -> ctypes.CDLL:
         lib.rl_linear_scan.argtypes = [
             c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
             c_void_p, c_int, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-            c_int, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p,
+            c_int, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_int, c_void_p,
         ]
         lib.rl_exp_decay.argtypes = [c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]
         lib.rl_low_rank_decay.argtypes = [c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_float, c_void_p,
@@ -1399,14 +1399,15 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.
     # before it still fills most multiprocessors, several of its few blocks on the same ones (measured: 1.1 ms instead
     # of 0.6 ms for 2,048 tokens).  Steps of single tokens have many short blocks and keep the early start.
     early = PDL and tokens < 8 * batch.num_entries
-    piece = first = blocks = others = 0
+    piece = first = blocks = taken = others = 0
     states = decays = records = None
     record = 0
     if pieces is None or batch.max_query_len < blocks_from:
         blocks_from = 0
     if blocks_from:
         record = scan_record(dim, beta is not None)
-        blocks = tokens // SCAN_BLOCK + min(batch.num_entries, tokens // blocks_from)
+        taken = min(batch.num_entries, tokens // blocks_from)      # entries that can be so long
+        blocks = tokens // SCAN_BLOCK + taken
         others = int(batch.num_entries * batch.max_query_len != tokens)      # entries of other lengths, shorter ones perhaps
         records = scan_records(pieces, tokens, heads, dim, blocks_from, beta is not None)
     elif pieces is not None and scan_takes_pieces(dim, vdim, beta is not None) and batch.max_query_len >= scan_pieces_from(heads, dim, vdim):
@@ -1419,8 +1420,8 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.
             _ptr(q), _row_stride("q", q), _ptr(k), _row_stride("k", k), _ptr(v), _row_stride("v", v), _ptr(decay), mode,
             _ptr(beta), _ptr(v_scale), _ptr(skip), _ptr(bonus), _ptr(out), _row_stride("out", out), _ptr(state), stride, 0,
             _ptr(batch.cu_seqlens), _ptr(batch.entry_slot), _ptr(batch.entry_start), batch.num_entries, tokens, heads, kv_heads,
-            dim, vdim, slots, _ptr(batch.fault), piece, first, blocks, others, _ptr(states), _ptr(decays), blocks_from, blocks, _ptr(records), record,
-            int(early), _stream()),
+            dim, vdim, slots, _ptr(batch.fault), piece, first, blocks, others, _ptr(states), _ptr(decays), blocks_from, blocks, taken,
+            _ptr(records), record, int(early), _stream()),
         f"linear_scan(dim={dim}, vdim={vdim})",
     )
     LAUNCHES.count += 1 + others if blocks_from else 0
