@@ -1354,6 +1354,14 @@ def scan_records(space, tokens: int, heads: int, dim: int, first: int, corrected
     return space.get("scan_records", rows, heads * scan_record(dim, corrected), torch.float32, min_rows=rows)
 
 
+def _walked_beside(batch, tokens: int, first: int) -> int:
+    """Whether a step has entries of fewer than ``first`` tokens, which are walked in a launch of their own."""
+    ends = getattr(batch, "h_cu_seqlens", None)
+    if ends is None:
+        return int(batch.num_entries * batch.max_query_len != tokens)      # entries of other lengths, shorter ones perhaps
+    return int((ends[1:] - ends[:-1]).min() < first)
+
+
 def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, out: torch.Tensor,
                 state: torch.Tensor, batch, *, heads: int, kv_heads: int, dim: int, vdim: int,
                 beta: torch.Tensor | None = None, v_scale: torch.Tensor | None = None,
@@ -1408,12 +1416,12 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.
         record = scan_record(dim, beta is not None)
         taken = min(batch.num_entries, tokens // blocks_from)      # entries that can be so long
         blocks = tokens // SCAN_BLOCK + taken
-        others = int(batch.num_entries * batch.max_query_len != tokens)      # entries of other lengths, shorter ones perhaps
+        others = _walked_beside(batch, tokens, blocks_from)
         records = scan_records(pieces, tokens, heads, dim, blocks_from, beta is not None)
     elif pieces is not None and scan_takes_pieces(dim, vdim, beta is not None) and batch.max_query_len >= scan_pieces_from(heads, dim, vdim):
         piece, first = scan_piece(heads, vdim), scan_pieces_from(heads, dim, vdim)
         blocks = tokens // piece + min(batch.num_entries, tokens // first)
-        others = int(batch.num_entries * batch.max_query_len != tokens)      # entries of other lengths, shorter ones perhaps
+        others = _walked_beside(batch, tokens, first)
         states, decays = scan_buffers(pieces, tokens, heads, dim, vdim)
     _check(
         recurrent().rl_linear_scan(

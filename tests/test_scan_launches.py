@@ -39,3 +39,12 @@ def test_entries_that_are_not_taken_in_blocks_get_no_ctas(monkeypatch, lengths):
     # enough for those that are, and no more than could be so long with as many tokens
     assert len(long) <= args[TAKEN] <= sum(lengths) // first
     assert sum(-(-n // kernels.SCAN_BLOCK) for n in long) <= args[BLOCKS] <= sum(lengths) // kernels.SCAN_BLOCK + args[TAKEN]
+
+
+@pytest.mark.parametrize("host", [True, False])
+@pytest.mark.parametrize("lengths", [[700, 333, 1015], [600] + [1] * 64, [256, 255], [300] * 4, [256]])
+def test_a_walk_is_launched_for_shorter_entries_alone(monkeypatch, lengths, host):
+    args, launched = asked_for(monkeypatch, lengths, 256, with_host_lengths=host)
+    shorter, uneven = min(lengths) < 256, len(set(lengths)) > 1
+    assert args[OTHERS] == int(shorter if host else uneven)      # (without the host's lengths, where there may be some)
+    assert launched == 2 + args[OTHERS]
