@@ -521,7 +521,9 @@ __global__ void __launch_bounds__(BlockShape<kDim, kKind>::kThreads) scan_blocks
   }
   float* home = a.state + slot * a.state_stride + static_cast<size_t>(head) * a.dim * a.vdim;
   const float* records = a.records + (static_cast<size_t>(before) * a.heads + head) * Record::kSize;
+  int fetched = 0;
   auto fetch = [&](int block) {      // one thread
+    ++fetched;
     const uint32_t bar = smem_addr(&full_bar[block % Shape::kBuffers]);
     mbar_expect_tx(bar, Record::kSize * 4);
     bulk_copy(smem_addr(block_floats + (block % Shape::kBuffers) * Shape::kRecord), records + static_cast<size_t>(block) * a.heads * Record::kSize,
@@ -611,7 +613,7 @@ __global__ void __launch_bounds__(BlockShape<kDim, kKind>::kThreads) scan_blocks
     return odd;
   };
   const float skip = a.skip ? a.skip[head] : 0.0f;
-  bool odd = false;
+  bool odd = false, gave_up = false;
   show_state(0);
   fetch_values(0);
   if constexpr (!kDelta) {
@@ -624,7 +626,7 @@ __global__ void __launch_bounds__(BlockShape<kDim, kKind>::kThreads) scan_blocks
     __syncwarp();
     bool strange = __syncthreads_or(odd);      // S and, without a correction, U are there; the record before is done with
     odd = false;
-    if (tid == 0 && block + Shape::kBuffers - 1 < blocks) {
+    if (tid == 0 && block + Shape::kBuffers - 1 < blocks && !*aborted) {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       fetch(block + Shape::kBuffers - 1);
     }
@@ -638,7 +640,9 @@ __global__ void __launch_bounds__(BlockShape<kDim, kKind>::kThreads) scan_blocks
     float mine[1][4];
     shared_half[(half ^ 1) * 32] = half ? make_float4(sums[0][0], sums[0][1], sums[0][2], sums[0][3])
                                         : make_float4(sums[1][0], sums[1][1], sums[1][2], sums[1][3]);
-    __syncthreads();
+    // a record that never came: nothing more is asked for (a barrier with bytes outstanding takes no others), nothing is kept
+    gave_up = __syncthreads_or(*aborted);
+    if (gave_up) break;
     {
       const float4 other = shared_half[half * 32];
       const float others[4] = {other.x, other.y, other.z, other.w};
@@ -703,7 +707,7 @@ __global__ void __launch_bounds__(BlockShape<kDim, kKind>::kThreads) scan_blocks
       }
     }
   }
-  if (slot_ok) {
+  if (slot_ok && !gave_up) {
 #pragma unroll
     for (int n = 0; n < Shape::kOwn; ++n) {
 #pragma unroll
@@ -713,10 +717,10 @@ __global__ void __launch_bounds__(BlockShape<kDim, kKind>::kThreads) scan_blocks
       }
     }
   }
-  if (*aborted && tid == 0) {      // copies land before the shared memory goes
+  if (gave_up && tid == 0) {      // copies land before the shared memory goes
     volatile int go_on = 0;
     for (int b = 0; b < Shape::kBuffers; ++b) {
-      const int fills = (blocks - b + Shape::kBuffers - 1) / Shape::kBuffers;
+      const int fills = (fetched - b + Shape::kBuffers - 1) / Shape::kBuffers;
       if (fills > 0) mbar_wait(smem_addr(&full_bar[b]), (fills - 1) & 1, &go_on, a.fault);
     }
   }
