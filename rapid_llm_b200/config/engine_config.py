@@ -37,7 +37,9 @@ class EngineConfig:
 
     Attributes:
         dtype: ``torch.bfloat16`` (serving precision) or ``torch.float32`` (every
-            product and sum as near as 32-bit arithmetic is, or nearer).
+            product and sum in 32 bits; rows by large weights are nearer to 64 bits
+            than one multiply-add after the other, except rows of two to four numbers
+            that are not zero, which are up to 1.2 times as far).
         max_seq_len: Longest sequence (prompt plus generated) a request may reach.
         page_size: Tokens per cache page.
         num_pages: Pages per cache group, the reserved null page not counted;

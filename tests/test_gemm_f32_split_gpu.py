@@ -33,7 +33,7 @@ def test_rows_are_near_and_the_same_at_every_count(n, inner):
     a, w, bias = torch.randn(max(rows), inner, device=DEV), torch.randn(n, inner, device=DEV), torch.randn(n, device=DEV)
     want = a.double() @ w.double().t() + bias.double()
     # Of the sum S of the products' magnitudes: a sum of 256 columns is cut off 16 times below 2^-23 of what it holds, the parts'
-    # products that are left out stay below 3 x 2^-24, the small ones (2^-7 of the whole) are cut off 5 k / 16 times below 2^-23
+    # products that are left out stay within 2^-24, the small ones (2^-7 of the whole) are cut off 5 k / 16 times below 2^-23
     # of theirs, and the float32 sums of k / 256 such round to 2^-24
     magnitude = a.abs().double() @ w.abs().double().t() + bias.abs().double()
     bound = magnitude * (16 + 2 + 5 * inner / 16 / 128 + inner / 512 + 1) * 2.0 ** -23
@@ -72,3 +72,34 @@ def test_what_is_not_finite_stays_in_its_row_and_column(m):
     kept[1:3], kept[:, 7], kept[:, 9] = False, False, False
     assert torch.equal(got[kept], clean[kept])
     assert bool(torch.isfinite(got[2][torch.isfinite(want[2])]).all())
+
+
+@pytest.mark.parametrize("n,inner", [(8192, 1024), (1025, 8460)])
+def test_a_row_is_the_same_in_every_tile_and_pass(n, inner):
+    torch.manual_seed(8)
+    a, w = torch.randn(1100, inner, device=DEV), torch.randn(n, inner, device=DEV)
+    for m in (33, 209, 416, 1024, 1060, 1100):
+        got = product(a[:m], w)
+        for at in {0, 15, 16, 31, 32, 104, 111, 112, 207, 208, 415, 831, 832, 1023, 1024, 1059, m - 1}:
+            if at < m:
+                assert torch.equal(got[at : at + 1], product(a[at : at + 1], w)), (m, at)
+
+
+@pytest.mark.parametrize("rows", [5, 70, 209])
+def test_a_product_by_itself_is_rounded_twice_at_most(rows):
+    """Rows with a single number that is not zero: what the parts' products leave out and the rounding of their sum, 2^-24 each
+    (a multiply-add has the second alone); either way as often as the other, and together hardly more than a rounding by itself."""
+    torch.manual_seed(9)
+    n, inner = 8192, 1028
+    w, a = torch.randn(n, inner, device=DEV), torch.zeros(rows, inner, device=DEV)
+    at = torch.randint(inner, (rows,), device=DEV)
+    a[torch.arange(rows, device=DEV), at] = torch.randn(rows, device=DEV)
+    a[0, at[0]] = 1 + 2.0 ** -7 - 2.0 ** -23           # cut off after 8 and 16 bits, both remainders are as large as they come
+    w[::2, at[0]] = 1 + 2.0 ** -7 - 2.0 ** -23
+    want = a.double() @ w.double().t()
+    off = (product(a, w).double() - want) / want.abs()
+    assert float(off.abs().max()) <= 2 * 2.0 ** -24 * (1 + 2.0 ** -5)
+    rounded = (want.float().double() - want) / want.abs()
+    assert float(off.norm()) <= 1.1 * float(rounded.norm())
+    # of 10^4 numbers of at most 2^-23 and of a size of 2.6e-8: their mean is within five of its own deviations
+    assert abs(float(off[1:].mean())) <= 5 * float(off[1:].std()) / (off[1:].numel() ** 0.5) + 2.0 ** -30
