@@ -1324,19 +1324,29 @@ def scan_buffers(space, tokens: int, heads: int, dim: int, vdim: int):
 SCAN_BLOCK = 32     # tokens of a block of ``csrc/scan_blocks.cu``
 
 
-def scan_blocks_from(heads: int, dim: int, vdim: int, corrected: bool = False) -> int:
-    """The shortest entry that is taken in blocks of tokens (0: none is): with a correction, where the alternative is a walk from
-    end to end, and without one where heads are wide and many, ahead of the pieces.  One prompt, us, walked or in pieces / in
-    blocks: with a correction 16 heads of 128, 2,048 tokens 571 / 255, 1,024 293 / 138; 32 heads of 64 500 / 230 and 254 / 126;
-    32 heads of 128 573 / 486 and 293 / 257; without one, fixed decays, 32 heads of 128, 2,048 tokens 342 / 276, 700 + 333 + 1,015
-    412 / 290, 128 tokens 29 / 27 (16 heads: 199 / 249, so they stay in pieces; 64 heads of 64 208 / 216).  The entry's length
-    alone decides, not what else is in the step: several long prompts at once fill the GPU by themselves, and a walk is ahead
-    there with a correction (four of 1,024 tokens, 16 heads of 128, 408 / 493, 32 heads of 64 256 / 339), which is why entries
-    that can come in such numbers in a step of a few thousand tokens are walked."""
+def scan_blocks_from(heads: int, dim: int, vdim: int, corrected: bool = False, max_tokens: int = 0) -> int:
+    """The shortest entry that is taken in blocks of tokens (0: none is) in an engine whose steps hold up to ``max_tokens`` tokens
+    (0: not said, a bound from below).  The entry's own length decides and what a step can hold, not what else is in this one.
+
+    With a correction the alternative is a walk from end to end, which takes as long for a few prompts as for one, where blocks
+    fill the GPU by themselves and the walk of shorter entries comes on top.  An entry is taken where the rest of a step cannot be
+    long enough to undo what it gains.  us, walked / in blocks, for 2,048 tokens alone, twice, four times, and eight times 1,024: 16
+    heads of 128 571 / 255, 572 / 486, 801 / 951, 768 / 871; 32 heads of 64 496 / 230, 496 / 335, 496 / 648, 369 / 624; 32 heads of 128
+    571 / 505, 801 / 951, 1,522 / 1,691, 1,260 / 1,717; 64 heads of 64 494 / 335, 496 / 648, 727 / 1,209, 694 / 1,193; 64 heads of 128
+    alone 801 / 947.  2,800 + 2,700 + 2,690 tokens with the longest in blocks and the others walked: 16 heads of 128 1,088 / 1,394, 32
+    of 64 674 / 962.  By itself a prompt takes 0.41 to 0.47 of its walk up to heads times value size 2,048, 0.6 to 0.88 up to 4,096, more
+    than all of it above: from two thirds and nine tenths of a step on, the worst mixture is no slower than its walk.
+
+    Without a correction heads that are wide and many are ahead of walk and pieces, one prompt or several.  Fixed decays, 32 heads of
+    128: 2,048 tokens 346 / 267, four such 1,282 / 1,019, 700 + 333 + 1,015 398 / 282, 256 57 / 50, 32 times 256 1,183 / 1,057, 600 beside
+    64 single tokens 262 / 204; 16 heads 199 / 249 and 64 heads of 64 208 / 216 for 2,048 tokens stay in pieces.  What it costs: 256
+    tokens beside 255, which are walked, 98 / 124, 300 beside three of 250 181 / 183."""
     if not 32 < dim <= 128 or dim % 4 or vdim % 4:
         return 0
     if corrected:
-        return 640 if heads * vdim <= 2048 else 1536
+        if heads * vdim > 4096:
+            return 0
+        return max(640, -(-2 * max_tokens // 3)) if heads * vdim <= 2048 else max(1536, -(-9 * max_tokens // 10))
     return 256 if dim > 64 and heads * vdim >= 4096 else 0
 
 

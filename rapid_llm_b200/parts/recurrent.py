@@ -201,7 +201,7 @@ class ChannelDeltaRule(_Recurrent):
         read = space.get("delta_read", rows, self.cv, f32)
         kernels.linear_scan(conv[:, : self.cq], conv[:, self.cq : 2 * self.cq], conv[:, 2 * self.cq :], decay, read, S,
                             batch, heads=self.h, kv_heads=self.hk, dim=self.dim, vdim=self.vdim, beta=beta,
-                            pieces=self._pieces(batch), blocks_from=kernels.scan_blocks_from(self.h, self.dim, self.vdim, True))
+                            pieces=self._pieces(batch), blocks_from=kernels.scan_blocks_from(self.h, self.dim, self.vdim, True, space.max_tokens))
         normed = space.get("delta_normed", rows, self.cv, x.dtype)
         kernels.gated_norm(read, normed, group=self.vdim, gate=high[:, self.h * self.dim :], act=kernels.GATE_SIGMOID,
                            weight=self.norm, eps=self.eps)

@@ -8,6 +8,7 @@ import torch
 
 from rapid_llm_b200.engine.batch import Workspace
 from rapid_llm_b200.ops import kernels
+from rapid_llm_b200.parts.recurrent import _Recurrent
 
 # what `rl_linear_scan` is given, by place from the end
 TAKEN, BLOCKS, BLOCKS_FROM, OTHERS = -5, -6, -7, -10
@@ -48,3 +49,38 @@ def test_a_walk_is_launched_for_shorter_entries_alone(monkeypatch, lengths, host
     shorter, uneven = min(lengths) < 256, len(set(lengths)) > 1
     assert args[OTHERS] == int(shorter if host else uneven)      # (without the host's lengths, where there may be some)
     assert launched == 2 + args[OTHERS]
+
+
+@pytest.mark.parametrize("heads,dim,vdim", [(8, 128, 128), (16, 128, 128), (32, 64, 64), (32, 128, 128), (64, 64, 64), (64, 128, 128)])
+@pytest.mark.parametrize("max_tokens", [64, 640, 2048, 8192, 65536])
+def test_with_a_correction_no_step_holds_two_entries_in_blocks(heads, dim, vdim, max_tokens):
+    """Several prompts are walked as fast as one, blocks of several take turns: what a step can hold beside an entry in blocks is
+    short enough for its walk to cost no more than the blocks gain."""
+    first = kernels.scan_blocks_from(heads, dim, vdim, True, max_tokens)
+    if heads * vdim > 4096:
+        assert first == 0
+        return
+    assert first >= kernels.scan_blocks_from(heads, dim, vdim, True) >= 640
+    # the share of its walk that a prompt takes in blocks, as measured: taken with the rest walked, or walked with it
+    share = 0.47 if heads * vdim <= 2048 else 0.88
+    if first <= max_tokens:
+        assert share * first + (max_tokens - first) <= first * 1.02
+
+
+@pytest.mark.parametrize("corrected", [False, True])
+@pytest.mark.parametrize("heads,dim,vdim", [(32, 128, 128), (16, 128, 128), (32, 64, 64), (4, 100, 132), (48, 128, 128)])
+def test_records_are_allocated_once_and_within_the_reserve(heads, dim, vdim, corrected):
+    most = 8192
+    first = kernels.scan_blocks_from(heads, dim, vdim, corrected, most)
+    reserve = _Recurrent._blocks_elements(SimpleNamespace(dtype=torch.bfloat16), heads, dim, vdim, corrected)
+    assert _Recurrent._blocks_elements(SimpleNamespace(dtype=torch.float32), heads, dim, vdim, corrected) == 0
+    if first == 0:
+        assert reserve == 0
+        return
+    space, sizes = Workspace(most, torch.device("meta")), set()
+    for tokens in range(first, most + 1, 64):
+        records = kernels.scan_records(space, tokens, heads, dim, first, corrected)
+        assert records.shape[0] >= tokens // kernels.SCAN_BLOCK + tokens // first      # whole blocks and a remainder an entry
+        sizes.add(space.nbytes())
+    assert not space._retired and len(sizes) == 1
+    assert sizes.pop() <= most * 2 * reserve      # what a mixer reserves a token, in bytes
