@@ -613,7 +613,7 @@ __global__ void __launch_bounds__(BlockShape<kDim, kKind>::kThreads) scan_blocks
     return odd;
   };
   const float skip = a.skip ? a.skip[head] : 0.0f;
-  bool odd = false, gave_up = false;
+  bool odd = false;
   show_state(0);
   fetch_values(0);
   if constexpr (!kDelta) {
@@ -626,6 +626,8 @@ __global__ void __launch_bounds__(BlockShape<kDim, kKind>::kThreads) scan_blocks
     __syncwarp();
     bool strange = __syncthreads_or(odd);      // S and, without a correction, U are there; the record before is done with
     odd = false;
+    // Once a record did not come nothing more is asked for (a barrier with bytes outstanding takes no others): what follows ends at
+    // once, and nothing of it is kept.  The threads do not agree on that block by block, which would take 5 % of a block's time.
     if (tid == 0 && block + Shape::kBuffers - 1 < blocks && !*aborted) {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       fetch(block + Shape::kBuffers - 1);
@@ -640,9 +642,7 @@ __global__ void __launch_bounds__(BlockShape<kDim, kKind>::kThreads) scan_blocks
     float mine[1][4];
     shared_half[(half ^ 1) * 32] = half ? make_float4(sums[0][0], sums[0][1], sums[0][2], sums[0][3])
                                         : make_float4(sums[1][0], sums[1][1], sums[1][2], sums[1][3]);
-    // a record that never came: nothing more is asked for (a barrier with bytes outstanding takes no others), nothing is kept
-    gave_up = __syncthreads_or(*aborted);
-    if (gave_up) break;
+    __syncthreads();
     {
       const float4 other = shared_half[half * 32];
       const float others[4] = {other.x, other.y, other.z, other.w};
@@ -707,6 +707,8 @@ __global__ void __launch_bounds__(BlockShape<kDim, kKind>::kThreads) scan_blocks
       }
     }
   }
+  __syncthreads();
+  const bool gave_up = *aborted;
   if (slot_ok && !gave_up) {
 #pragma unroll
     for (int n = 0; n < Shape::kOwn; ++n) {
