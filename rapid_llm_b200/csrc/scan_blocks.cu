@@ -12,6 +12,12 @@
 // scan_blocks_kernel walks an entry's blocks in order, a CTA per head and kCols columns of S; the records come by bulk copies
 // a block ahead.  Its products run on mma.sync with every float32 as three bfloat16 parts (tile_products).
 //
+// The parts of an infinity add up to NaN, those of a number that rounds to one, too, and a sum over a block's tokens lets it into
+// the read-outs before it.  So where q, k, V, beta, the bonus, the decays' products, R, U or the state an entry starts from are not
+// finite or beyond 2^60, the rest of the entry's tokens are walked one after the other, with the walk's infinities (2,048 tokens
+// that are not finite from the first on: 1.7 to 2.1 ms, a walk 0.4 to 0.6).  A record says whether its block is one of those, so that
+// the blocks themselves look at no more than V, R and U.
+//
 // An entry's sums depend on its own tokens in this step alone: not on the step's other entries.
 //
 // What bounds it: a block's chain of dependent steps (rows times S, with a correction R and U, the update, barriers between
@@ -45,7 +51,8 @@ struct BlockRecord {
   static constexpr int kP = kEnd + kDim * kTokenStride;                            // [32][40]
   static constexpr int kT = kP + kScanBlock * kTokenStride;
   static constexpr int kG = kT + (kDelta ? kScanBlock * kTokenStride : 0);         // G_32
-  static constexpr int kSize = kG + kDim;
+  static constexpr int kOdd = kG + kDim;                                           // not zero: the parts cannot say what is in the block
+  static constexpr int kSize = kOdd + 4;
   static_assert(kSize % 4 == 0, "records are copied 16 bytes at a time");
 };
 
@@ -58,6 +65,10 @@ __device__ __forceinline__ int blocks_of(const ScanBlockArgs& a, int e) {
   const int length = a.cu_seqlens[e + 1] - a.cu_seqlens[e];
   return length >= a.from ? (length + kScanBlock - 1) / kScanBlock : 0;
 }
+
+// What the products are made for: sums of such numbers stay finite.
+constexpr float kScanLargest = 0x1p60f;
+__device__ __forceinline__ bool is_plain(float x) { return fabsf(x) < kScanLargest; }
 
 // ------------------------------------------------------------------ float32 products on the tensor cores
 // Two neighbouring numbers as three pairs of bfloat16 each, every one what the ones before leave, rounded to nearest.
@@ -102,15 +113,6 @@ struct PartColumns {
       lower[i] = at[i * part + column * stride + (k >> 1)];
       upper[i] = at[i * part + column * stride + (k >> 1) + 4];
     }
-  }
-  __device__ __forceinline__ float value(int column, int k) const {
-    float sum = 0.0f;
-#pragma unroll
-    for (int i = 2; i >= 0; --i) {
-      const uint32_t word = at[i * part + column * stride + (k >> 1)];
-      sum += __uint_as_float(k & 1 ? word & 0xffff0000u : word << 16);
-    }
-    return sum;
   }
 };
 
@@ -227,6 +229,9 @@ __global__ void __launch_bounds__(256) scan_prepare_kernel(const ScanBlockArgs a
   const int first = a.cu_seqlens[e] + at * kScanBlock, length = min(kScanBlock, a.cu_seqlens[e + 1] - first);
   const int kv_head = head / (a.heads / a.kv_heads);
   float* record = a.records + (static_cast<size_t>(blockIdx.x) * a.heads + head) * Record::kSize;
+  __shared__ int odd_flag;
+  if (tid == 0) odd_flag = 0;
+  bool odd = false, grows = false;      // grows: decays above one, whose products may get anywhere
 
   for (int idx = tid; idx < kScanBlock * kDim / 4; idx += 256) {
     const int t = idx / (kDim / 4), c = (idx - t * (kDim / 4)) * 4;
@@ -250,13 +255,32 @@ __global__ void __launch_bounds__(256) scan_prepare_kernel(const ScanBlockArgs a
       }
       if (a.decay_mode != 2) g[0] = g[1] = g[2] = g[3] = pg[0];
     }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      odd = odd || !is_plain(q[i]) || !is_plain(k[i]);
+      grows = grows || !(fabsf(g[i]) <= 1.0f);
+    }
     *reinterpret_cast<float4*>(sq + t * kStride + c) = *reinterpret_cast<const float4*>(q);
     *reinterpret_cast<float4*>(sk + t * kStride + c) = *reinterpret_cast<const float4*>(k);
     *reinterpret_cast<float4*>(sg + t * kStride + c) = *reinterpret_cast<const float4*>(g);
   }
   for (int idx = tid; idx < 2 * kScanBlock * kTokenStride; idx += 256) sp[idx] = 0.0f;
-  if (kDelta && tid < kScanBlock) sbeta[tid] = tid < length ? a.beta[(static_cast<size_t>(first) + tid) * a.heads + head] : 0.0f;
-  __syncthreads();
+  if (kDelta && tid < kScanBlock) {
+    sbeta[tid] = tid < length ? a.beta[(static_cast<size_t>(first) + tid) * a.heads + head] : 0.0f;
+    odd = odd || !is_plain(sbeta[tid]);
+  }
+  if (__syncthreads_or(grows) && tid < kDim) {
+    double product = 1.0;
+    for (int t = 0; t < kScanBlock; ++t) {
+      product *= static_cast<double>(sg[t * kStride + tid]);
+      odd = odd || !is_plain(static_cast<float>(product));
+    }
+    product = 1.0;
+    for (int t = kScanBlock - 1; t > 0; --t) {
+      product *= static_cast<double>(sg[t * kStride + tid]);
+      odd = odd || !is_plain(static_cast<float>(product));
+    }
+  }
 
   // ---- products of decays from the start and to the end, a thread per channel each
   float to_end[kScanBlock];
@@ -289,12 +313,16 @@ __global__ void __launch_bounds__(256) scan_prepare_kernel(const ScanBlockArgs a
           make_float4(sk[t0 * kStride + c] * to_end[t0], sk[(t0 + 1) * kStride + c] * to_end[t0 + 1], sk[(t0 + 2) * kStride + c] * to_end[t0 + 2],
                       sk[(t0 + 3) * kStride + c] * to_end[t0 + 3]);
   }
+  if (odd) odd_flag = 1;
   if (__syncthreads_or(wide_range)) {
   {
     float w[4][kC], bonus[kC];
 #pragma unroll
     for (int c = 0; c < kC; ++c)
+    {
       bonus[c] = kKind == kBlockBonus && lane * kC + c < a.dim ? a.bonus[static_cast<size_t>(head) * a.dim + lane * kC + c] : 0.0f;
+      if (!is_plain(bonus[c])) odd_flag = 1;
+    }
     auto four_tokens = [&](int j0, int t0, auto own) {   // own: the keys' own four tokens
       constexpr bool kOwn = decltype(own)::value;
       constexpr int kValues = kDelta ? 32 : 16, kEach = kDelta ? 2 : 1;
@@ -384,7 +412,10 @@ __global__ void __launch_bounds__(256) scan_prepare_kernel(const ScanBlockArgs a
     if (kKind == kBlockBonus) {
       float bonus[kC];
 #pragma unroll
-      for (int c = 0; c < kC; ++c) bonus[c] = lane * kC + c < a.dim ? a.bonus[static_cast<size_t>(head) * a.dim + lane * kC + c] : 0.0f;
+      for (int c = 0; c < kC; ++c) {
+        bonus[c] = lane * kC + c < a.dim ? a.bonus[static_cast<size_t>(head) * a.dim + lane * kC + c] : 0.0f;
+        if (!is_plain(bonus[c])) odd_flag = 1;
+      }
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int t = warp * 4 + i;
@@ -430,6 +461,7 @@ __global__ void __launch_bounds__(256) scan_prepare_kernel(const ScanBlockArgs a
     }
   }
   __syncthreads();
+  if (tid == 255) record[Record::kOdd] = odd_flag ? 1.0f : 0.0f;
   if (kDelta && warp == 0) {
     // column `lane` of T: forward substitution, the sums over the tokens before in four chains
     float x[kScanBlock];
@@ -453,7 +485,66 @@ __global__ void __launch_bounds__(256) scan_prepare_kernel(const ScanBlockArgs a
   }
 }
 
-__device__ __forceinline__ bool is_finite(float x) { return fabsf(x) <= 3.402823466e38f; }
+// Tokens one after the other, as the walk takes them, for what the products cannot say.
+// `S`: a CTA's columns at the start, [kCols][kDim] in shared memory, afterwards those at the end; a lane holds kRows rows of one.
+template <int kDim, int kKind, int kCols, int kThreads>
+__device__ __noinline__ void walk_tokens(const ScanBlockArgs& args, float* S, int head, int col0, int first, int length) {
+  constexpr int kLanes = kThreads / kCols, kRows = kDim / kLanes;
+  static_assert(kLanes <= 32 && 32 % kLanes == 0 && kDim % kLanes == 0, "a column's lanes are neighbours in a warp");
+  const ScanBlockArgs a = args;      // (what is written below could lie anywhere)
+  const int col = static_cast<int>(threadIdx.x) / kLanes, part = static_cast<int>(threadIdx.x) % kLanes;
+  const bool inside = col0 + col < a.vdim;
+  const size_t kv_col = static_cast<size_t>(head / (a.heads / a.kv_heads)) * a.dim;
+  float* column = S + col * kDim;
+  auto column_sum = [](float x) {
+#pragma unroll
+    for (int off = kLanes / 2; off >= 1; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
+    return x;
+  };
+  float s[kRows], bonus[kRows];
+#pragma unroll
+  for (int i = 0; i < kRows; ++i) {
+    const int r = part + i * kLanes;
+    s[i] = column[r];
+    bonus[i] = kKind == kBlockBonus && r < a.dim ? a.bonus[static_cast<size_t>(head) * a.dim + r] : 0.0f;
+  }
+#pragma unroll 1
+  for (int t = 0; t < length; ++t) {
+    const size_t row = static_cast<size_t>(first) + t, own = row * a.heads + head;
+    const float* decay = a.decay + (a.decay_mode == 0 ? head : a.decay_mode == 1 ? own : own * a.dim);
+    const float v = inside ? a.v[row * a.v_stride + static_cast<size_t>(head) * a.vdim + col0 + col] : 0.0f;
+    const float strength = kKind == kBlockDelta ? a.beta[own] : a.v_scale ? a.v_scale[own] : 1.0f;
+    float q[kRows], k[kRows], g[kRows], seen = 0.0f, read = 0.0f;
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+      const int r = part + i * kLanes;
+      const bool good = r < a.dim;
+      q[i] = good ? a.q[row * a.q_stride + kv_col + r] : 0.0f;
+      k[i] = good ? a.k[row * a.k_stride + kv_col + r] : 0.0f;
+      g[i] = good ? decay[a.decay_mode == 2 ? r : 0] : 1.0f;
+    }
+    if (kKind == kBlockDelta) {
+#pragma unroll
+      for (int i = 0; i < kRows; ++i) {
+        s[i] *= g[i];
+        if (part + i * kLanes < a.dim) seen = fmaf(s[i], k[i], seen);
+      }
+      seen = column_sum(seen);
+    }
+    const float u = kKind == kBlockDelta ? strength * (v - seen) : a.v_scale ? strength * v : v;
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+      if (part + i * kLanes >= a.dim) continue;      // (rows that are not there take no part, whatever u is)
+      const float pair = k[i] * u, kept = s[i];
+      s[i] = kKind == kBlockDelta ? fmaf(k[i], u, kept) : fmaf(kept, g[i], pair);
+      read = fmaf(kKind == kBlockBonus ? fmaf(bonus[i], pair, kept) : s[i], q[i], read);
+    }
+    read = column_sum(read);
+    if (inside && part == 0) a.out[row * a.out_stride + static_cast<size_t>(head) * a.vdim + col0 + col] = a.skip ? read + a.skip[head] * v : read;
+  }
+#pragma unroll
+  for (int i = 0; i < kRows; ++i) column[part + i * kLanes] = s[i];
+}
 
 // Warps of a CTA: for every 16 rows times 16 columns of S two, half of the channels each; then the tiles of S are dealt to them.
 template <int kDim, int kKind>
@@ -475,8 +566,10 @@ __device__ __forceinline__ void bulk_copy(uint32_t to, const float* from, uint32
                "r"(bar) : "memory");
 }
 
+// Registers for one CTA a multiprocessor where shared memory holds no more (with a correction, keys of 128: 267 us with 128 registers a
+// thread, 256 with 164, 2,048 tokens of 16 heads); without a correction more of them are slower (290 us, 313 with 186).
 template <int kDim, int kKind>
-__global__ void __launch_bounds__(BlockShape<kDim, kKind>::kThreads) scan_blocks_kernel(const ScanBlockArgs a) {
+__global__ void __launch_bounds__(BlockShape<kDim, kKind>::kThreads, kDim == 128 && kKind == kBlockDelta ? 1 : 2) scan_blocks_kernel(const __grid_constant__ ScanBlockArgs a) {
   using Shape = BlockShape<kDim, kKind>;
   constexpr bool kDelta = Shape::kDelta;
   using Record = BlockRecord<kDim, kDelta>;
@@ -535,18 +628,6 @@ __global__ void __launch_bounds__(BlockShape<kDim, kKind>::kThreads) scan_blocks
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     for (int b = 0; b < Shape::kBuffers - 1 && b < blocks; ++b) fetch(b);
   }
-  // a lower triangle by U or R where one of their rows is not finite: rows behind a token stay out of its sum
-  auto causal = [&](float (&sums)[4], const float* lower, const PartColumns columns, int token, int col) {
-#pragma unroll 1
-    for (int i = 0; i < 4; ++i) {
-      const int at = token + g + (i >> 1) * 8;
-      float sum = 0.0f;
-      for (int j = 0; j <= at; ++j) sum = fmaf(lower[at * kTokenStride + j], columns.value(col + 2 * t + (i & 1), j), sum);
-      if (i == 0) sums[0] += sum; else if (i == 1) sums[1] += sum; else if (i == 2) sums[2] += sum; else sums[3] += sum;
-    }
-    __syncwarp();      // (the lanes' sums are of different lengths)
-  };
-
   // this warp's tile of rows (with a correction the first two of four make R, the others the read-outs) and its tiles of S
   const int task = warp >> 1, half = warp & 1, row_tile = task % Shape::kRowTiles, task_col = task / Shape::kRowTiles * 16;
   const bool reads = !kDelta || row_tile >= 2;
@@ -594,14 +675,14 @@ __global__ void __launch_bounds__(BlockShape<kDim, kKind>::kThreads) scan_blocks
       }
     }
   };
-  auto show_values = [&](int block) {      // without a correction: columns of U; true if one of them is not finite
+  auto show_values = [&](int block) {      // without a correction: columns of U; true if one of them is not plain
     bool odd = false;
     float x[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const bool inside = block * kScanBlock + v_token + (i >> 1) < length && col0 + v_col < a.vdim;      // vdim is a multiple of four
       x[i] = inside ? (a.v_scale ? v[i] * v_scale[i >> 1] : v[i]) : 0.0f;
-      odd = odd || !is_finite(x[i]);
+      odd = odd || !is_plain(x[i]);
     }
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
@@ -613,19 +694,34 @@ __global__ void __launch_bounds__(BlockShape<kDim, kKind>::kThreads) scan_blocks
     return odd;
   };
   const float skip = a.skip ? a.skip[head] : 0.0f;
+  // Blocks whose record says so are not taken here, nor those behind them.
+  __shared__ int first_odd;
+  if (tid == 0) first_odd = blocks;
+  __syncthreads();
+  for (int i = tid; i < blocks; i += Shape::kThreads)
+    if (records[static_cast<size_t>(i) * a.heads * Record::kSize + Record::kOdd] != 0.0f) atomicMin(&first_odd, i);
+  __syncthreads();
+  const int plain_blocks = first_odd;
   bool odd = false;
+  int walk_from = -1;      // the block from whose start on the tokens are walked, with its state in registers
+#pragma unroll
+  for (int n = 0; n < Shape::kOwn; ++n)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) odd = odd || !is_plain(S[n][i]);
   show_state(0);
   fetch_values(0);
   if constexpr (!kDelta) {
-    odd = show_values(0);
+    odd = show_values(0) || odd;
     if (blocks > 1) fetch_values(1);
   }
-  for (int block = 0; block < blocks; ++block) {
+  for (int block = 0; block < plain_blocks; ++block) {
     const float* record = block_floats + (block % Shape::kBuffers) * Shape::kRecord;
     const uint32_t* state = states + (block & 1) * Shape::kState;
     __syncwarp();
-    bool strange = __syncthreads_or(odd);      // S and, without a correction, U are there; the record before is done with
-    odd = false;
+    if (__syncthreads_or(odd)) {      // S and, without a correction, U are there; the record before is done with
+      walk_from = block;
+      break;
+    }
     // Once a record did not come nothing more is asked for (a barrier with bytes outstanding takes no others): what follows ends at
     // once, and nothing of it is kept.  The threads do not agree on that block by block, which would take 5 % of a block's time.
     if (tid == 0 && block + Shape::kBuffers - 1 < blocks && !*aborted) {
@@ -657,26 +753,29 @@ __global__ void __launch_bounds__(BlockShape<kDim, kKind>::kThreads) scan_blocks
         for (int i = 0; i < 4; ++i) {
           const int token = block * kScanBlock + token_tile + g + (i >> 1) * 8, col = col0 + my_col + 2 * t + (i & 1);
           left[i] = (token < length && col < a.vdim ? v[i] : 0.0f) - mine[0][i];
-          odd = odd || !is_finite(left[i]);
+          odd = odd || !is_plain(left[i]);
         }
         __syncwarp();
         show_tile(left, values + Shape::kValues, Shape::kValueStride, Shape::kValuePart, my_col, token_tile);
         if (block + 1 < blocks) fetch_values(block + 1);
       }
       __syncwarp();
-      const bool strange_r = __syncthreads_or(odd);      // R is there
-      odd = false;
+      if (__syncthreads_or(odd)) {      // R is there
+        walk_from = block;
+        break;
+      }
       if (!reads) {
         float rows[1][4] = {};
-        if (strange_r) causal(rows[0], record + Record::kT, value_columns(1, my_col), token_tile, 0);
-        else tile_products<kScanBlock / 16, 1>(rows, record + Record::kT + (token_tile + g) * kTokenStride, kTokenStride, value_columns(1, my_col));
+        tile_products<kScanBlock / 16, 1>(rows, record + Record::kT + (token_tile + g) * kTokenStride, kTokenStride, value_columns(1, my_col));
         show_tile(rows[0], values, Shape::kValueStride, Shape::kValuePart, my_col, token_tile);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) odd = odd || !is_finite(rows[0][i]);
+        for (int i = 0; i < 4; ++i) odd = odd || !is_plain(rows[0][i]);
       }
       __syncwarp();
-      strange = __syncthreads_or(odd);      // U is there
-      odd = false;
+      if (__syncthreads_or(odd)) {      // U is there
+        walk_from = block;
+        break;
+      }
     }
     float added[Shape::kOwn][4] = {};
     tile_products<kScanBlock / 16, Shape::kOwn>(added, record + Record::kEnd + s_row * kTokenStride, kTokenStride, value_columns(u, s_col));
@@ -691,8 +790,8 @@ __global__ void __launch_bounds__(BlockShape<kDim, kKind>::kThreads) scan_blocks
       if (block + 2 < blocks) fetch_values(block + 2);
     }
     if (reads) {
-      if (strange) causal(mine[0], record + Record::kP, value_columns(u, my_col), token_tile, 0);
-      else tile_products<kScanBlock / 16, 1>(mine, record + Record::kP + (token_tile + g) * kTokenStride, kTokenStride, value_columns(u, my_col));
+      __syncwarp();      // (keeps these loads behind the state's products: 2 % of the kernel without a correction)
+      tile_products<kScanBlock / 16, 1>(mine, record + Record::kP + (token_tile + g) * kTokenStride, kTokenStride, value_columns(u, my_col));
       const int col = col0 + my_col + 2 * t;
 #pragma unroll
       for (int i = 0; i < 4; i += 2) {
@@ -709,6 +808,22 @@ __global__ void __launch_bounds__(BlockShape<kDim, kKind>::kThreads) scan_blocks
   }
   __syncthreads();
   const bool gave_up = *aborted;
+  if (walk_from < 0 && plain_blocks < blocks) walk_from = plain_blocks;
+  if (walk_from >= 0 && !gave_up) {
+    float* plain = reinterpret_cast<float*>(states);      // the parts that lie there are done with
+    static_assert(kCols * kDim <= 2 * Shape::kState, "room for the state");
+    auto each = [&](auto act) {
+#pragma unroll
+      for (int n = 0; n < Shape::kOwn; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) act(S[n][i], plain + (s_col + n * 8 + 2 * t + (i & 1)) * kDim + s_row + (i >> 1) * 8);
+    };
+    each([](float& x, float* at) { *at = x; });
+    __syncthreads();
+    walk_tokens<kDim, kKind, kCols, Shape::kThreads>(a, plain, head, col0, first + walk_from * kScanBlock, length - walk_from * kScanBlock);
+    __syncthreads();
+    each([](float& x, float* at) { x = *at; });
+  }
   if (slot_ok && !gave_up) {
 #pragma unroll
     for (int n = 0; n < Shape::kOwn; ++n) {
@@ -719,7 +834,7 @@ __global__ void __launch_bounds__(BlockShape<kDim, kKind>::kThreads) scan_blocks
       }
     }
   }
-  if (gave_up && tid == 0) {      // copies land before the shared memory goes
+  if ((gave_up || walk_from >= 0) && tid == 0) {      // copies land before the shared memory goes
     volatile int go_on = 0;
     for (int b = 0; b < Shape::kBuffers; ++b) {
       const int fills = (fetched - b + Shape::kBuffers - 1) / Shape::kBuffers;

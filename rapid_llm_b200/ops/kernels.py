@@ -1353,7 +1353,7 @@ def scan_blocks_from(heads: int, dim: int, vdim: int, corrected: bool = False, m
 def scan_record(dim: int, corrected: bool = False) -> int:
     """Floats that a block of a head keeps for its walk (``BlockRecord`` of the kernels)."""
     padded, parts = 64 if dim <= 64 else 128, 2 if corrected else 1
-    return parts * 32 * (padded + 8) + padded * 40 + parts * 32 * 40 + padded
+    return parts * 32 * (padded + 8) + padded * 40 + parts * 32 * 40 + padded + 4
 
 
 def scan_records(space, tokens: int, heads: int, dim: int, first: int, corrected: bool = False) -> torch.Tensor:
