@@ -462,9 +462,10 @@ static int launch_split(SplitArgs args, __nv_bfloat16* parts, cudaStream_t strea
 
 // Whether the product runs here: a rule on the weight alone, so that a row's bits do not depend on what it comes with.  The line
 // lies where the weight's 32 MB are a few rounds of tiles; below it a product is its launches.  us at 1, 16, 64, 203 rows,
-// sums down the columns / here: 4,096 x 4,096 24, 58, 167, 253 / 21, 21, 28, 75; 24,576 x 4,096 70, 168, 353, 1,078 / 78, 80,
-// 100, 243; 4,096 x 12,288 62, 167, 490, 740 / 40, 41, 51, 172; 151,936 x 4,096 377, 726, 1,896, 5,830 / 398, 408, 549, 1,470
-// (a single row of wide weights is the one that loses, by 5 to 12 %; a layer of one row and its head take as long either way).
+// sums down the columns / here: 4,096 x 4,096 23, 58, 167, 253 / 20, 21, 28, 74; 24,576 x 4,096 69, 167, 352, 1,076 / 77, 79,
+// 99, 263; 4,096 x 12,288 62, 167, 490, 741 / 42, 42, 52, 176; 151,936 x 4,096 377, 790, 1,893, 5,828 / 395, 430, 617, 1,512
+// (a single row of wide weights is the one that loses, by 5 to 11 %; a decode step of one row, four layers of the 8B sizes and the
+// head, goes from 1,807 to 1,736).
 bool gemm_f32_split_takes(const float* w, int n, int k) {
   return k % 4 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0 && n >= 1024 && k >= 1024 &&
          static_cast<long long>(n) * k >= 1 << 23 && n <= 65535 * kSplitM;

@@ -6,7 +6,8 @@
 //   out = (G q) S + P U               P[t][j] = q_t (G_t / G_j) k_j, j <= t
 //   S <- G_32 S + ((G_32 / G) k)^T U
 // (a bonus reads before the token's own decay and weighs the diagonal of P).  The products from the block's start and to its
-// end run in float64 and are rounded once.
+// end run in float64 and are rounded once.  U and T are the WY form of a product of factors I - beta k k^T (Bischof and Van Loan
+// 1987), which the published chunked forms of the delta rule rest on.
 //
 // scan_prepare_kernel makes what does not depend on S, all blocks side by side: a record of G k, G q, (G_32 / G) k, P, T, G_32.
 // scan_blocks_kernel walks an entry's blocks in order, a CTA per head and kCols columns of S; the records come by bulk copies
@@ -23,10 +24,12 @@
 // What bounds it: a block's chain of dependent steps (rows times S, with a correction R and U, the update, barriers between
 // them), some 5,500 cycles with a correction and a CTA a multiprocessor, at 0.4 instructions a cycle and scheduler; the records'
 // kernel by its instructions.  us (records + blocks; walked or in pieces): 2,048 tokens, 16 heads of 128 with a correction
-// 48 + 198 (552); 32 heads of 64 61 + 160 (465); 700 + 333 + 1,015 tokens of 32 heads of 128, fixed decays, 59 + 220 (404).
+// 48 + 198 (552); 32 heads of 64 61 + 160 (465); 700 + 333 + 1,015 tokens of 32 heads of 128, fixed decays, 59 + 225 (404).
 // Float32 multiply-adds would be bound by shared memory (an 8 x 8 patch a thread takes as long to fetch as to multiply),
 // tcgen05 by its latencies at these sizes.  Root mean square error against 64 bits, 1,300 tokens of 16 heads of 128, here (read-
 // outs and states; walked): with a correction 1.24e-7, 9.3e-8 (1.65e-7, 1.47e-7); row decays 1.02e-7, 7.1e-8 (1.84e-7, 1.71e-7).
+// Those are decays near one, as the timed calls have them; where they are small a walk is nearer: drawn from 0.05 to 0.95, 900 tokens of
+// 8 heads, with a correction 1.14e-7, 7.0e-8 (8.8e-8, 4.9e-8), without one 9.0e-8, 4.4e-8 (8.3e-8, 4.0e-8).
 #include <cuda.h>
 
 #include <cuda_bf16.h>

@@ -1287,8 +1287,7 @@ def rotate_heads(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.T
 def scan_piece(heads: int, vdim: int) -> int:
     """Tokens of a piece of a prompt that is walked in pieces side by side: as many pieces as it takes to fill the GPU, and no
     more, since what joins them is one more pass over the pieces' states.  In pieces of 128 and 256, us: 2,048 tokens, 32 heads
-    of 64 120 and 128, 16 heads of 128 191 and 204, 32 heads of 128 384 and 335; two prompts of 2,048, 64 heads of 64 405 and
-    350."""
+    of 64 120 and 128, 16 heads of 128 191 and 204; two prompts of 2,048, 64 heads of 64 405 and 350."""
     return 256 if heads * vdim >= 4096 else 128
 
 
@@ -1296,8 +1295,7 @@ def scan_pieces_from(heads: int, dim: int, vdim: int) -> int:
     """The shortest entry that is cut into pieces: every piece but the last is walked twice, and what joins them comes on top.
     One prompt from end to end and in pieces, us: 32 heads of 64, 520 tokens 63 and 75, 640 tokens 76 and 75, 1,024 tokens 117
     and 77; 16 heads of 128, 640 tokens 94 and 95, 800 tokens 116 and 116, 1,024 tokens 145 and 119; 64 heads of 64, 1,024
-    tokens 135 and 161, 1,536 tokens 199 and 189; 32 heads of 128, 1,024 tokens 206 and 204, 1,536 tokens 301 and 279, 2,048
-    tokens 398 and 339.  The entry's length alone decides, not what else is in the step, which may fill the GPU by itself:
+    tokens 135 and 161, 1,536 tokens 199 and 189 (wider heads in such numbers go in blocks, :func:`scan_blocks_from`).  The entry's length alone decides, not what else is in the step, which may fill the GPU by itself:
     eight prompts of 1,024 take 628 and 761 at 16 heads of 128, 303 and 370 at 32 heads of 64."""
     if heads * vdim >= 4096:
         return 1536
