@@ -203,7 +203,7 @@ def planes_linear(x: torch.Tensor, weights: torch.Tensor, out: torch.Tensor, fau
     planes, width, _ = weights.shape
     rows = x.shape[0] // planes
     if (fault is not None and 0 < rows <= kernels.GEMM_PLANES_MAX_TOKENS and width % 128 == 0 and x.is_contiguous() and out.is_contiguous()
-            and use_tensor_core_kernel(x[:rows], weights[0])):
+            and weights.is_contiguous() and use_tensor_core_kernel(x[:rows], weights[0])):
         flush()
         return kernels.gemm_bf16_planes(x, weights, out, fault)
     for plane in range(planes):

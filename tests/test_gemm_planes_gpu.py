@@ -25,3 +25,17 @@ def test_planes_are_the_products_one_by_one(tokens, planes, width, inner):
     want = torch.einsum("ptk,pnk->ptn", x.view(planes, tokens, inner).double(), w.double()).view(planes * tokens, width)
     # one rounding to 8 bits of what float32 sums have left untouched at this size
     assert bool(((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all())
+
+
+def test_planes_of_a_wider_tensor_are_taken_one_by_one():
+    from rapid_llm_b200.ops import gemm
+
+    torch.manual_seed(3)
+    x = torch.randn(2 * 5, 256, device=DEV).bfloat16()
+    wide = (torch.randn(2, 384, 256, device=DEV) / 16).bfloat16()
+    fault = torch.zeros(1, dtype=torch.int32, device=DEV)
+    got, want = (torch.empty(10, 256, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    gemm.planes_linear(x, wide[:, :256], got, fault)
+    for plane in range(2):
+        gemm.linear(x[5 * plane : 5 * plane + 5], wide[plane, :256], want[5 * plane : 5 * plane + 5], fault)
+    assert int(fault) == 0 and torch.equal(got, want)
