@@ -15,7 +15,7 @@
 //
 // An output is a sum in an order that n and k alone decide (256 columns, then the columns of a segment, then the segments,
 // whose number `split_segments` takes from n and k): not M, the tile it falls in, or what else is in the batch.
-// A product of an infinity's or a NaN's parts is not finite; such outputs are formed again, one column after the other.
+// A product of an infinity's or a NaN's parts is not finite; such outputs are formed again from the numbers themselves.
 //
 // A CTA owns 128 weight rows (the lanes of the accumulators), up to 208 tokens and a segment of the columns.  TMA brings the
 // weights 32 columns at a time; eight warps cut them into their parts, which go to tensor memory: there they are an operand
@@ -100,16 +100,41 @@ __device__ __forceinline__ void load_four_or_zeros(float (&v)[4], const float* f
       : "=&f"(v[0]), "=&f"(v[1]), "=&f"(v[2]), "=&f"(v[3]) : "l"(from), "r"(static_cast<int>(good)));
 }
 
-// One output as a sum down the columns, for what the parts cannot say.
-__device__ __noinline__ float split_plain_sum(const float* a, const float* w, int k) {
-  float sum = 0.0f;
-  for (int i = 0; i < k; ++i) sum = fmaf(a[i], w[i], sum);
-  return sum;
-}
-__device__ __forceinline__ float split_result(const SplitArgs& args, float sum, int token, int row) {
-  if (!(fabsf(sum) <= 3.402823466e38f))
-    sum = split_plain_sum(args.a + static_cast<size_t>(token) * args.lda, args.w + static_cast<size_t>(row) * args.k, args.k);
-  return sum + (args.bias ? args.bias[row] : 0.0f);
+__device__ __forceinline__ bool split_finite(float sum) { return fabsf(sum) <= 3.402823466e38f; }
+
+// A warp's outputs of one token that are not finite, formed from the numbers themselves, for what the parts cannot say: NaN where
+// the token's row has one, else a sum over the columns that the lanes share out.  24,576 x 4,096, us: one of 64 rows with a NaN 231 (with
+// none 103; every output down the columns by a lane of its own 4,139), 203 rows of them 1,562 (249; 86,158), one of 64 with an infinity
+// 4,400.
+__device__ __noinline__ void split_again(const SplitArgs& args, float (&sums)[4], int token, int row0) {
+  const int lane = threadIdx.x & 31, k = args.k;
+  const float* a = args.a + static_cast<size_t>(token) * args.lda;
+  bool nan = false;
+#pragma unroll 8
+  for (int i = lane; i < k; i += 32) nan = nan || a[i] != a[i];
+  if (__any_sync(0xffffffffu, nan)) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sums[j] = __int_as_float(0x7fffffff);
+    return;
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    unsigned left = __ballot_sync(0xffffffffu, row0 + j < args.n && !split_finite(sums[j]));
+    while (left) {
+      const int whose = __ffs(left) - 1;
+      left &= left - 1;
+      const float* w = args.w + static_cast<size_t>(__shfl_sync(0xffffffffu, row0, whose) + j) * k;
+      float sum = 0.0f;
+#pragma unroll 8
+      for (int i = lane * 4; i < k; i += 128) {      // k is a multiple of four, w on a 16-byte boundary
+        const float4 four = *reinterpret_cast<const float4*>(w + i);
+        sum = fmaf(a[i + 3], four.w, fmaf(a[i + 2], four.z, fmaf(a[i + 1], four.y, fmaf(a[i], four.x, sum))));
+      }
+#pragma unroll
+      for (int off = 16; off >= 1; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+      if (lane == whose) sums[j] = sum;
+    }
+  }
 }
 
 // The parts of A's rows, one part after the other: [3][m][kp], kp columns of which those behind k are zeros.
@@ -132,7 +157,8 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float* a, int lda
 // kCopied: the tokens' parts lie in memory (map_x: [3 m, kp] of them), else their rows do (map_x: [m, k] of float32).
 template <int kTokens, bool kCopied>
 __global__ void __launch_bounds__(SplitShape<kTokens, kCopied>::kThreads, SplitShape<kTokens, kCopied>::kPerMultiprocessor)
-gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const SplitArgs args) {
+gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
+                      const __grid_constant__ SplitArgs args) {
   using Shape = SplitShape<kTokens, kCopied>;
   constexpr int kBuffers = Shape::kBuffers, kRaw = Shape::kRaw;
   constexpr int kAcc = (kTokens + 31) / 32 * 16;                    // outputs a thread
@@ -358,7 +384,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
       add_sum(tmem_base + kTokens);
       tc_fence_before();
     }
-    // a wait that ran out leaves no sum: such outputs are formed one column after the other, and the fault word says so
+    // a wait that ran out leaves no sum: such outputs are formed from the numbers themselves, and the fault word says so
     const float lost = *aborted ? __int_as_float(0x7fffffff) : 0.0f;
     const int at = (warp & 3) * 32 + lane;
 #pragma unroll
@@ -382,12 +408,15 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
       for (int s = 1; s < 8; ++s)
         if (s < segments) { sum.x += part[s].x; sum.y += part[s].y; sum.z += part[s].z; sum.w += part[s].w; }
       float* to = args.c + static_cast<size_t>(t0 + token) * args.ldc;
-      const float sums[4] = {sum.x, sum.y, sum.z, sum.w};
+      float sums[4] = {sum.x, sum.y, sum.z, sum.w};
+      const int row0 = n0 + lane * 4;
+      bool finite = true;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int row = n0 + lane * 4 + j;
-        if (row < args.n) to[row] = split_result(args, sums[j], t0 + token, row);
-      }
+      for (int j = 0; j < 4; ++j) finite = finite && (row0 + j >= args.n || split_finite(sums[j]));
+      if (!__all_sync(0xffffffffu, finite)) split_again(args, sums, t0 + token, row0);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (row0 + j < args.n) to[row0 + j] = sums[j] + (args.bias ? args.bias[row0 + j] : 0.0f);
     }
   }
   cluster_sync();      // the others may still be reading

@@ -103,3 +103,27 @@ def test_a_product_by_itself_is_rounded_twice_at_most(rows):
     assert float(off.norm()) <= 1.1 * float(rounded.norm())
     # of 10^4 numbers of at most 2^-23 and of a size of 2.6e-8: their mean is within five of its own deviations
     assert abs(float(off[1:].mean())) <= 5 * float(off[1:].std()) / (off[1:].numel() ** 0.5) + 2.0 ** -30
+
+
+@pytest.mark.parametrize("rows", [1, 64, 203])
+def test_what_is_not_finite_costs_no_more_than_a_few_products(rows):
+    """A request that went astray holds up the others of its step: NaN in every row, infinities in one, NaN in a weight."""
+    torch.manual_seed(10)
+    n, inner = 24576, 4096
+    w, spoilt = torch.randn(n, inner, device=DEV), torch.randn(n, inner, device=DEV)
+    spoilt[::64, 3] = math.nan
+    plain = torch.randn(rows, inner, device=DEV)
+    nan, inf = plain.clone(), plain.clone()
+    nan[:, 7], inf[rows // 2, 9] = math.nan, math.inf
+    product(plain, w)
+    for a, by in ((nan, w), (inf, w), (plain, spoilt)):
+        product(a, by)
+        begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        begin.record()
+        got = product(a, by)
+        end.record()
+        torch.cuda.synchronize()
+        want = a.double() @ by.double().t()
+        assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+        # an infinity's row is 4.4 ms of sums; 203 rows of NaN would be 86 ms of them (with a buffer's filling and checking, 0.3 ms)
+        assert begin.elapsed_time(end) < 15.0
